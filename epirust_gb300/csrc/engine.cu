@@ -1,7 +1,7 @@
 // engine.cu -- the engine handle and the C ABI of the GB300 tick.
 //
 // An engine holds R worlds ("replicates") on one device: their agents are concatenated in
-// 256-slot chunks, their bordered byte planes and claim planes laid end to end, and every
+// 256-slot chunks, their bordered bit and byte planes and claim planes laid end to end, and every
 // kernel of kernels.cuh serves all of them in one launch per hour.  The single-engine API
 // (epi_engine_*) is the R = 1 case; the ensemble API (epi_ensemble_*) runs many replicates
 // of uneven population and grid size in lockstep.  Hour segments between intervention
@@ -29,6 +29,9 @@
 using namespace epi;
 using namespace epi::kern;
 
+// k_commit takes no slots per thread any more; the launch shape keeps the field.
+constexpr int kCommitSlots = 4, kMaxCommitSlots = 8;
+
 enum KernelKind { kKDecide = 0, kKCommit, kKSleep, kKLock, kKVaccinate, kKBuildPlane, kKCheck, kKindCount };
 static const char* kKernelNames[kKindCount] = {"k_decide", "k_commit", "k_sleep", "k_lock", "k_vaccinate", "k_build_plane", "k_check"};
 
@@ -48,11 +51,13 @@ struct Replica {
     InterventionState iv;
     std::vector<epi_counts> rows;
     bool active = true;
+    uint32_t par = 0;  // the position and occupancy buffer that holds the current state
     // checkpoint of the host-side state (epi_engine_save_state)
     InterventionState s_iv;
     epi_geography s_geo{};
     uint32_t s_hosp_code = kHosp0;
     bool s_active = true;
+    uint32_t s_par = 0;
     std::vector<epi_counts> s_rows;
 };
 
@@ -60,25 +65,27 @@ struct epi_engine {
     std::vector<Replica> reps;
     uint32_t slots = 0;        // agent slots (chunk-padded replicates)
     size_t plane_bytes = 0;    // all bordered byte planes
+    size_t occ_words = 0;      // all bit planes (one buffer)
     size_t claim_cells = 0;    // all claim planes
     int grid_blocks = 0;       // grid of the counting kernels (k_decide, k_sleep)
-    int commit_slots = kCommitSlots;  // slots per k_commit thread and round (1 .. 8)
-    int commit_blocks = 0;
+    int commit_slots = kCommitSlots;  // of the launch shape (k_commit takes its work from lists)
     int resident_blocks = 0;   // SMs x resident k_decide blocks per SM
     // device
     DevParams* d_params = nullptr;
     uint32_t* d_chunk_rep = nullptr;  // null for a single replicate
-    uint32_t *d_pos = nullptr, *d_home = nullptr, *d_work = nullptr, *d_wsa = nullptr, *d_tgt = nullptr;
-    uint32_t* d_lost = nullptr;  // per slot: the hour in which the agent's claim was beaten
+    uint32_t *d_home = nullptr, *d_work = nullptr, *d_wsa = nullptr;
+    // Positions and occupancy bit planes have two buffers each (slots and occ_words long): the
+    // hours of day 7..22 write the next state to the other one, and Replica::par names the one
+    // holding the replicate's current state; the other bit plane is all zero between hours.
+    uint32_t *d_pos = nullptr, *d_occ = nullptr;
     uint2* d_st = nullptr;
-    // Byte planes of all replicates (plane_bytes).  A lone world keeps two (two_planes): the
-    // hours of day 7..22 rebuild the plane in the other one, and plane_par names the one
-    // holding the current state.
-    uint8_t* d_plane = nullptr;
-    bool two_planes = false;
-    uint32_t plane_par = 0;
-    uint8_t* d_danger = nullptr;  // infectious-neighbour counts, same layout as d_plane
+    uint8_t* d_cls = nullptr;     // class bytes (plane_bytes)
+    uint8_t* d_danger = nullptr;  // infectious-neighbour counts, same layout
     uint32_t* d_claim = nullptr;
+    uint32_t* d_displaced = nullptr;  // the hour's lists (HourLists)
+    uint2 *d_acts = nullptr, *d_list_n = nullptr;
+    uint32_t* d_piece_rep = nullptr;  // replicate of every kPieceWords of the bit planes (ensembles)
+    uint32_t* d_par = nullptr;        // Replica::par, uploaded for the checks
     uint32_t* d_counts = nullptr;  // [hour of segment][replicate][8]
     SegDev* d_seg = nullptr;       // hour base of the running piece and first hour of the chain
     uint32_t* d_ivn = nullptr;     // per replicate: the guard's new-infections figure
@@ -124,9 +131,8 @@ struct epi_engine {
     // device-side checkpoint
     uint32_t *s_pos = nullptr, *s_wsa = nullptr;
     uint2* s_st = nullptr;
-    uint8_t* s_plane = nullptr;
-    uint32_t s_plane_par = 0;
-    uint8_t* s_danger = nullptr;
+    uint32_t* s_occ = nullptr;
+    uint8_t *s_cls = nullptr, *s_danger = nullptr;
     bool saved = false;
 
     uint32_t R() const { return (uint32_t)reps.size(); }
@@ -180,6 +186,7 @@ static DevParams make_dev_params(const epi_params& p, const epi_geography& geo0,
     d.G = (int32_t)p.grid_size;
     d.W = d.G + 1;
     d.WP = d.G + 3;
+    d.PW = ((uint32_t)d.G + 3u + 31u) / 32u;
     d.hosp_code = kHosp0;
     d.area[kTransport] = to_rect(geo0.transport);
     d.area[kHousing] = to_rect(geo0.housing);
@@ -308,9 +315,8 @@ static int ensure_counts(epi_engine* h, uint32_t hours_needed) {
 }
 
 // ------------------------------------------------------------------ the hour loop
-using DecideKernel = void (*)(const DevParams*, const uint32_t*, uint32_t, const uint32_t*, uint2*, const uint32_t*,
-                              const uint32_t*, uint32_t*, const uint8_t*, const uint8_t*, uint32_t*, uint32_t*, uint32_t*,
-                              HourArgs, int*);
+using DecideKernel = void (*)(const DevParams*, const uint32_t*, uint32_t, const HourBuffers, HourArgs);
+using CommitKernel = void (*)(const DevParams*, const uint32_t*, uint32_t, const uint32_t*, const HourBuffers, HourArgs, uint64_t);
 
 // Hours 2..6 of a day change nothing once hour 1 has sent everyone but hospital staff home
 // (routine, citizen/mod.rs:244-248, sets current_area = home_location and nothing else), so
@@ -321,11 +327,9 @@ static bool sleep_hour_skipped(uint32_t first_hour, uint32_t k) {
     return k > 0 && hod >= 2u && hod <= 6u;
 }
 
-// The k_decide instance of an hour of the day.
 // The k_decide (single world) or k_decide_ens (ensemble) instance of an hour of the day.
-static DecideKernel decide_kernel(uint32_t hod, bool ensemble = false, bool full = false) {
-#define EPI_PICK(HC)                                                                                                 \
-    (ensemble ? (DecideKernel)k_decide_ens<HC> : full ? (DecideKernel)k_decide<HC, true> : (DecideKernel)k_decide<HC>)
+static DecideKernel decide_kernel(uint32_t hod, bool ensemble = false) {
+#define EPI_PICK(HC) (ensemble ? (DecideKernel)k_decide_ens<HC> : (DecideKernel)k_decide<HC>)
     switch (hour_class(hod)) {
         case kHcStart: return EPI_PICK(kHcStart);
         case kHcEnd: return EPI_PICK(kHcEnd);
@@ -337,47 +341,45 @@ static DecideKernel decide_kernel(uint32_t hod, bool ensemble = false, bool full
     }
 #undef EPI_PICK
 }
+static CommitKernel commit_kernel(bool patch, bool ensemble) {
+    return ensemble ? (patch ? (CommitKernel)k_commit<true, true> : (CommitKernel)k_commit<true, false>)
+                    : (patch ? (CommitKernel)k_commit<false, true> : (CommitKernel)k_commit<false, false>);
+}
 
-// The hours of day 7..22 of a lone world rebuild its plane in the other buffer (k_commit
-// REBUILD), 16 a day, so the buffer that holds the state after hour x is the parity of the
-// number of such hours among 1..x: a function of x mod 24.  The other hours update the
-// current buffer in place.
+// The hours of day 7..22 write positions and occupancy to the other buffers, 16 a day, so the
+// buffer that holds the state after hour x is the parity of the number of such hours among
+// 1..x: a function of x mod 24.  The other hours patch the current buffers in place.
 static bool rebuild_hour(uint32_t hod) { return hod >= 7u && hod <= 22u; }
-static uint32_t plane_parity(uint32_t hod) { return (hod >= 7u ? std::min(hod, 22u) - 6u : 0u) & 1u; }
-static uint8_t* plane_buf(const epi_engine* h, uint32_t par) {
-    return h->d_plane + (h->two_planes ? (size_t)par * h->plane_bytes : 0u);
+static uint32_t hour_parity(uint32_t hod) { return (hod >= 7u ? std::min(hod, 22u) - 6u : 0u) & 1u; }
+static uint32_t* pos_buf(const epi_engine* h, uint32_t par) { return h->d_pos + (size_t)par * h->slots; }
+static uint32_t* occ_buf(const epi_engine* h, uint32_t par) { return h->d_occ + (size_t)par * h->occ_words; }
+
+// The arrays of a launch that starts from buffer par.
+static HourBuffers hour_buffers(const epi_engine* h, uint32_t par) {
+    HourBuffers b;
+    b.pos = pos_buf(h, par);
+    b.pos_next = pos_buf(h, 1u - par);
+    b.st = h->d_st;
+    b.home = h->d_home;
+    b.work = h->d_work;
+    b.wsa = h->d_wsa;
+    b.occ = occ_buf(h, par);
+    b.occ_next = occ_buf(h, 1u - par);
+    b.cls = h->d_cls;
+    b.danger = h->d_danger;
+    b.claim = h->d_claim;
+    b.lists = HourLists{h->d_displaced, h->d_acts, h->d_list_n};
+    b.err = h->d_err;
+    return b;
 }
 
-static int commit_blocks_for(uint32_t slots, int per_thread = kCommitSlots) {
-    const uint32_t per_block = kThreads * (uint32_t)per_thread;
-    return (int)std::max<uint32_t>(1u, (slots + per_block - 1) / per_block);
-}
-
-// k_commit with S slots per thread and round; the sparse instance for the hours of day 0 and
-// 23, where hardly any agent acts.
-using CommitKernel = void (*)(const DevParams*, const uint32_t*, uint32_t, uint32_t*, const uint32_t*, uint8_t*,
-                              uint8_t*, uint32_t*, const uint32_t*, HourArgs, uint64_t, uint4*, uint32_t);
-static CommitKernel commit_kernel(int slots_per_thread, bool sparse = false, bool rebuild = false) {
-#define EPI_PICK(S)                                                                                                  \
-    (sparse ? (CommitKernel)k_commit<S, true> : rebuild ? (CommitKernel)k_commit<S, false, true> : (CommitKernel)k_commit<S, false>)
-    switch (slots_per_thread) {
-        case 1: return EPI_PICK(1);
-        case 2: return EPI_PICK(2);
-        case 3: return EPI_PICK(3);
-        case 4: return EPI_PICK(4);
-        case 5: return EPI_PICK(5);
-        case 6: return EPI_PICK(6);
-        case 7: return EPI_PICK(7);
-        default: return EPI_PICK(8);
-    }
-#undef EPI_PICK
-}
-
-// k_commit grid for S slots per thread: every slot once.  (Capping it at one wave of
-// resident blocks that loop over the rest was measured slower: the block scheduler's later
-// waves keep more loads in flight than a second round of the same threads.)
-static int commit_grid(epi_engine* h, int S, int* out) {
-    *out = commit_blocks_for(h->slots, S);
+// The citizen states at the end of hour k of a piece (arguments ha), into the stream buffers.
+static int record_state(epi_engine* h, uint32_t first_hour, uint32_t k, const HourArgs& ha) {
+    const uint32_t n = h->reps[0].n;
+    k_state_delta<<<(n + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(
+        h->d_params, ha, n, pos_buf(h, hour_parity((first_hour + k) % 24u)), h->d_st, h->d_prev,
+        h->d_codes + (size_t)k * h->slots, h->d_exc + (size_t)k * h->slots, h->d_exc_n + k);
+    CK(cudaGetLastError());
     return EPI_OK;
 }
 
@@ -389,6 +391,7 @@ static int enqueue_piece(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     const uint32_t row_words = h->R() * 8u;
     const uint32_t n_chunks = h->slots / kChunk;
     int last_row = -1;  // the latest hour of the piece whose counts the kernels computed
+    HourArgs recorded{};  // of the hour before (the citizen-state stream)
     for (uint32_t k = 0; k < nh; ++k) {
         const uint32_t hod = (first_hour + k) % 24u;
         // rows back to the previous computed hour: within the piece, or the hour before it
@@ -396,37 +399,25 @@ static int enqueue_piece(epi_engine* h, uint32_t first_hour, uint32_t nh) {
         const uint32_t prev_back = !h->stop_rule ? 0u : (last_row >= 0 ? k - (uint32_t)last_row : 1u);
         const HourArgs ha{h->d_seg, h->d_counts, row_words, k, prev_back};
         if (h->stream_file && k > 0) {  // record the previous hour's end state before this hour changes it
-            const uint32_t n = h->reps[0].n;
-            k_state_delta<<<(n + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(
-                n, h->d_pos, h->d_st, h->d_prev, h->d_codes + (size_t)(k - 1) * h->slots,
-                h->d_exc + (size_t)(k - 1) * h->slots, h->d_exc_n + (k - 1));
-            CK(cudaGetLastError());
+            const int rc = record_state(h, first_hour, k - 1, recorded);
+            if (rc) return rc;
         }
+        recorded = ha;
         if (sleep_hour_skipped(first_hour, k)) continue;
         last_row = (int)k;
         if (hod >= 1u && hod <= 6u) {
             LAUNCH(kKSleep, CK(launch_hour_kernel(k_sleep, h->grid_blocks, h->stream, (const DevParams*)h->d_params,
                                                   (const uint32_t*)h->d_chunk_rep, n_chunks, h->d_st, ha)));
         } else {
-            // the plane of the previous hour, and (a lone world's rebuilding hours) the other
-            // buffer, all zero, which k_commit fills before it zeroes the one the hour read
-            const bool rebuild = h->two_planes && rebuild_hour(hod);
-            uint8_t* read_plane = plane_buf(h, plane_parity((hod + 23u) % 24u));
-            uint8_t* next_plane = plane_buf(h, plane_parity(hod));
-            const DecideKernel decide = decide_kernel(hod, h->R() > 1, rebuild);
-            LAUNCH(kKDecide, CK(launch_hour_kernel(
-                                  decide, h->grid_blocks, h->stream, (const DevParams*)h->d_params,
-                                  (const uint32_t*)h->d_chunk_rep, n_chunks, (const uint32_t*)h->d_pos, h->d_st,
-                                  (const uint32_t*)h->d_home, (const uint32_t*)h->d_work, h->d_wsa,
-                                  (const uint8_t*)read_plane, (const uint8_t*)h->d_danger, h->d_claim, h->d_tgt, h->d_lost,
-                                  ha, h->d_err)));
-            const CommitKernel commit = commit_kernel(h->commit_slots, hod == 0u || hod == 23u, rebuild);
-            LAUNCH(kKCommit, CK(launch_hour_kernel(commit, h->commit_blocks, h->stream, (const DevParams*)h->d_params,
-                                                   (const uint32_t*)h->d_chunk_rep, h->slots, h->d_pos,
-                                                   (const uint32_t*)h->d_tgt, next_plane, h->d_danger, h->d_claim,
-                                                   (const uint32_t*)h->d_lost, ha, (uint64_t)h->claim_cells,
-                                                   rebuild ? reinterpret_cast<uint4*>(read_plane) : (uint4*)nullptr,
-                                                   (uint32_t)(rebuild ? h->plane_bytes / 16u : 0u))));
+            const HourBuffers b = hour_buffers(h, hour_parity((hod + 23u) % 24u));
+            const bool ens = h->R() > 1;
+            LAUNCH(kKDecide, CK(launch_hour_kernel(decide_kernel(hod, ens), h->grid_blocks, h->stream,
+                                                   (const DevParams*)h->d_params, (const uint32_t*)h->d_chunk_rep, n_chunks,
+                                                   b, ha)));
+            LAUNCH(kKCommit, CK(launch_hour_kernel(commit_kernel(!rebuild_hour(hod), ens), h->grid_blocks, h->stream,
+                                                   (const DevParams*)h->d_params, (const uint32_t*)h->d_chunk_rep,
+                                                   (uint32_t)(h->occ_words / kPieceWords), (const uint32_t*)h->d_piece_rep,
+                                                   b, ha, (uint64_t)h->claim_cells)));
         }
         // the run loop's guard after every day boundary but the piece's last hour (the piece
         // end below takes that one)
@@ -436,11 +427,8 @@ static int enqueue_piece(epi_engine* h, uint32_t first_hour, uint32_t nh) {
         }
     }
     if (h->stream_file) {
-        const uint32_t n = h->reps[0].n;
-        k_state_delta<<<(n + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(
-            n, h->d_pos, h->d_st, h->d_prev, h->d_codes + (size_t)(nh - 1) * h->slots, h->d_exc + (size_t)(nh - 1) * h->slots,
-            h->d_exc_n + (nh - 1));
-        CK(cudaGetLastError());
+        const int rc = record_state(h, first_hour, nh - 1, recorded);
+        if (rc) return rc;
     }
     const bool guard_last = h->stop_rule && (first_hour + nh - 1) % 24u == 0u;
     k_piece_end<<<1, kThreads, 0, h->stream>>>(h->d_params, h->R(), h->d_seg, h->d_counts, row_words,
@@ -495,6 +483,22 @@ static int piece_graph(epi_engine* h, uint32_t first_hour, uint32_t nh, cudaGrap
 
 static int check_error_flag(epi_engine* h);
 
+// Replicate r's state in the buffers of parity par, and its other bit plane zero, as the hours
+// want it (a chain that starts out of step: a restore, hours run out of order).
+static int move_to_buffer(epi_engine* h, uint32_t r, uint32_t par) {
+    Replica& rep = h->reps[r];
+    if (rep.par == par) return EPI_OK;
+    const size_t off = rep.hp.agent_off, w0 = rep.hp.occ_off,
+                 w1 = r + 1 < h->R() ? (size_t)h->reps[r + 1].hp.occ_off : h->occ_words;
+    CK(cudaMemcpyAsync(pos_buf(h, par) + off, pos_buf(h, rep.par) + off, (size_t)rep.n * sizeof(uint32_t),
+                       cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(occ_buf(h, par) + w0, occ_buf(h, rep.par) + w0, (w1 - w0) * sizeof(uint32_t),
+                       cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemsetAsync(occ_buf(h, rep.par) + w0, 0, (w1 - w0) * sizeof(uint32_t), h->stream));
+    rep.par = par;
+    return EPI_OK;
+}
+
 // Longest piece (one captured graph): two days.  Back-to-back pieces cost nothing measurable
 // on the device, while every new engine captures its pieces once: two-day pieces made a
 // fresh engine's 1M-agent 4,800-hour run 1.5 % faster than eight-day ones, at equal speed once warm.
@@ -515,19 +519,16 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     if (h->last_claim_hour >= 0 &&
         ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
         CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
-    if (h->last_claim_hour >= (int64_t)first_hour)  // loss marks of hours about to run again
-        CK(cudaMemsetAsync(h->d_lost, 0xFF, (size_t)h->slots * sizeof(uint32_t), h->stream));
     h->last_claim_hour = (int64_t)first_hour + nh - 1;
-    if (h->two_planes) {  // the chain reads the state after first_hour - 1 from its parity's buffer
-        const uint32_t need = plane_parity((first_hour + 23u) % 24u);
-        if (need != h->plane_par) {  // and the other buffer zero, as a rebuilding hour wants it
-            CK(cudaMemcpyAsync(plane_buf(h, need), plane_buf(h, h->plane_par), h->plane_bytes, cudaMemcpyDeviceToDevice,
-                               h->stream));
-            CK(cudaMemsetAsync(plane_buf(h, h->plane_par), 0, h->plane_bytes, h->stream));
-            h->plane_par = need;
-        }
+    // the chain reads the state after first_hour - 1 from its parity's buffers
+    const uint32_t need = hour_parity((first_hour + 23u) % 24u);
+    std::vector<uint8_t> ran(h->R(), 0);  // a world whose run has ended runs no hour kernel
+    for (uint32_t r = 0; r < h->R(); ++r) {
+        if (!h->reps[r].active) continue;
+        ran[r] = 1;
+        rc = move_to_buffer(h, r, need);
+        if (rc) return rc;
     }
-    const bool ran = h->reps[0].active;  // a lone world whose run has ended runs no hour kernel
     const size_t row_words = (size_t)h->R() * 8;
     CK(cudaMemsetAsync(h->d_counts, 0, (size_t)nh * row_words * sizeof(uint32_t), h->stream));
     if (h->stream_file) CK(cudaMemsetAsync(h->d_exc_n, 0, (size_t)nh * sizeof(uint32_t), h->stream));
@@ -567,14 +568,14 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     rc = check_error_flag(h);
     if (rc) return rc;
     std::vector<uint8_t> ended(h->R(), 0);  // stop rule met at an earlier hour of this chain
-    int end_row = -1;                       // the first such row (later hours ran no kernel)
+    std::vector<uint32_t> last(h->R(), nh - 1);  // the last row whose hour ran
     for (uint32_t k = 0; k < nh && h->halt_row < 0; ++k) {
         for (uint32_t r = 0; r < h->R(); ++r) {
             if (!h->reps[r].active || ended[r]) continue;
             const uint32_t* c = h->h_counts + ((size_t)k * h->R() + r) * 8;
             if (h->stop_rule && c[1] == 0 && c[2] == 0 && c[3] == 0) {
                 ended[r] = 1;
-                if (end_row < 0) end_row = (int)k;
+                last[r] = k;
             }
             const uint64_t total = (uint64_t)c[0] + c[1] + c[2] + c[3] + c[4] + c[5];
             if (total != h->reps[r].n) {  // assert_eq!(csv_record.total(), current_population), allocation_map.rs:128
@@ -585,11 +586,10 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
         }
         if (h->stop_rule && h->h_counts[(size_t)k * row_words + 6] != 0u) h->halt_row = (int)k;  // later rows did not run
     }
-    if (h->two_planes && ran) {  // the buffer of the last hour whose kernels ran
-        uint32_t last = nh - 1;
-        if (h->halt_row >= 0) last = std::min(last, (uint32_t)h->halt_row);
-        if (end_row >= 0) last = std::min(last, (uint32_t)end_row);
-        h->plane_par = plane_parity((first_hour + last) % 24u);
+    for (uint32_t r = 0; r < h->R(); ++r) {  // the buffers of the last hour whose kernels ran
+        if (!ran[r]) continue;
+        if (h->halt_row >= 0) last[r] = std::min(last[r], (uint32_t)h->halt_row);
+        h->reps[r].par = hour_parity((first_hour + last[r]) % 24u);
     }
     return EPI_OK;
 }
@@ -862,9 +862,10 @@ static void free_device(epi_engine* h) {
     destroy_graphs(h);
     stream_free(h);
     cudaFree(h->d_params); cudaFree(h->d_chunk_rep); cudaFree(h->d_pos); cudaFree(h->d_home); cudaFree(h->d_work);
-    cudaFree(h->d_wsa); cudaFree(h->d_tgt); cudaFree(h->d_lost); cudaFree(h->d_st); cudaFree(h->d_plane); cudaFree(h->d_danger); cudaFree(h->d_claim);
+    cudaFree(h->d_wsa); cudaFree(h->d_st); cudaFree(h->d_occ); cudaFree(h->d_cls); cudaFree(h->d_danger); cudaFree(h->d_claim);
+    cudaFree(h->d_displaced); cudaFree(h->d_acts); cudaFree(h->d_list_n); cudaFree(h->d_piece_rep); cudaFree(h->d_par);
     cudaFree(h->d_counts); cudaFree(h->d_seg); cudaFree(h->d_ivn); cudaFree(h->d_err); cudaFree(h->d_scratch);
-    cudaFree(h->s_pos); cudaFree(h->s_wsa); cudaFree(h->s_st); cudaFree(h->s_plane); cudaFree(h->s_danger);
+    cudaFree(h->s_pos); cudaFree(h->s_wsa); cudaFree(h->s_st); cudaFree(h->s_occ); cudaFree(h->s_cls); cudaFree(h->s_danger);
     if (h->h_counts) cudaFreeHost(h->h_counts);
     if (h->h_seg) cudaFreeHost(h->h_seg);
     if (h->h_ivn) cudaFreeHost(h->h_ivn);
@@ -939,12 +940,13 @@ static int build_on_device(epi_engine* h) {
     if (e == cudaSuccess && d_inf)
         e = cudaMemcpyAsync(d_inf, infections.data(), infections.size() * sizeof(uint4), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
-        // scratch: d_lost holds the eligibility flags, d_tgt the per-chunk counts (both reset after)
+        // scratch: the hour lists hold the eligibility flags and the per-chunk counts
+        uint32_t *d_elig = h->d_displaced, *d_chunk_elig = reinterpret_cast<uint32_t*>(h->d_acts);
         const int blocks = (int)std::min<uint64_t>(n_chunks, (uint64_t)h->resident_blocks * 2);
         k_world_citizens<<<blocks, kThreads, 0, h->stream>>>(d_w, h->d_chunk_rep, n_chunks, h->d_pos, h->d_st, h->d_home,
-                                                             h->d_work, h->d_wsa, h->d_lost, h->d_tgt, d_flags);
-        k_world_scan<<<1, 1024, 0, h->stream>>>(h->d_tgt, n_chunks);
-        k_world_pt<<<blocks, kThreads, 0, h->stream>>>(d_w, h->d_chunk_rep, n_chunks, h->d_lost, h->d_tgt, h->d_st);
+                                                             h->d_work, h->d_wsa, d_elig, d_chunk_elig, d_flags);
+        k_world_scan<<<1, 1024, 0, h->stream>>>(d_chunk_elig, n_chunks);
+        k_world_pt<<<blocks, kThreads, 0, h->stream>>>(d_w, h->d_chunk_rep, n_chunks, d_elig, d_chunk_elig, h->d_st);
         if (d_inf)
             k_world_infect<<<(int)std::min<size_t>((infections.size() + kThreads - 1) / kThreads, 1024), kThreads, 0,
                              h->stream>>>(d_inf, (uint32_t)infections.size(), h->d_st);
@@ -967,7 +969,7 @@ static int build_on_device(epi_engine* h) {
 static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_record* const* recs, uint32_t R) {
     if (R == 0) { h->err = "no replicates"; return EPI_ERR_ARG; }
     h->reps.resize(R);
-    uint64_t slots = 0, plane = 0, claim = 0;
+    uint64_t slots = 0, plane = 0, claim = 0, occ = 0;
     for (uint32_t r = 0; r < R; ++r) {
         Replica& rep = h->reps[r];
         rep.p = params[r];
@@ -981,15 +983,18 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
         rep.hp.agent_off = (uint32_t)slots;
         rep.hp.plane_off = plane;
         rep.hp.claim_off = claim;
+        rep.hp.occ_off = occ;
         const uint64_t side = (uint64_t)rep.p.grid_size + 1;
         slots += align_up(rep.n, kChunk);
         plane += align_up((side + 2) * (side + 2) + 16, 256);
         claim += side * side;
+        occ += align_up((side + 2) * rep.hp.PW, kPieceWords);
         if (slots >= 0xFFFFFFFFull - kChunk) { h->err = "too many agents for one engine"; return EPI_ERR_CAPACITY; }
     }
     h->slots = (uint32_t)slots;
     h->plane_bytes = plane;
     h->claim_cells = claim;
+    h->occ_words = occ;
     int dev = 0, sms = 0, per_sm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -998,10 +1003,6 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     const uint64_t n_chunks = slots / kChunk;
     h->resident_blocks = sms * per_sm;
     h->grid_blocks = (int)std::min<uint64_t>(n_chunks, (uint64_t)h->resident_blocks);
-    {
-        const int rc = commit_grid(h, h->commit_slots, &h->commit_blocks);
-        if (rc) return rc;
-    }
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     CK(cudaMalloc(&h->d_params, R * sizeof(DevParams)));
@@ -1013,24 +1014,34 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
         }
         CK(cudaMalloc(&h->d_chunk_rep, n_chunks * sizeof(uint32_t)));
         CK(cudaMemcpyAsync(h->d_chunk_rep, chunk_rep.data(), n_chunks * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
+        std::vector<uint32_t> piece_rep(occ / kPieceWords);
+        for (uint32_t r = 0; r < R; ++r) {
+            const uint64_t q1 = (r + 1 < R ? h->reps[r + 1].hp.occ_off : occ) / kPieceWords;
+            for (uint64_t q = h->reps[r].hp.occ_off / kPieceWords; q < q1; ++q) piece_rep[q] = r;
+        }
+        CK(cudaMalloc(&h->d_piece_rep, piece_rep.size() * sizeof(uint32_t)));
+        CK(cudaMemcpyAsync(h->d_piece_rep, piece_rep.data(), piece_rep.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                           h->stream));
         CK(cudaStreamSynchronize(h->stream));
     }
-    CK(cudaMalloc(&h->d_pos, slots * sizeof(uint32_t)));
+    CK(cudaMalloc(&h->d_pos, 2u * slots * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_home, slots * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_work, slots * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_wsa, slots * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_tgt, slots * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_lost, slots * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_st, slots * sizeof(uint2)));
-    h->two_planes = R == 1;
-    CK(cudaMalloc(&h->d_plane, h->plane_bytes * (h->two_planes ? 2u : 1u)));
+    CK(cudaMalloc(&h->d_occ, 2u * h->occ_words * sizeof(uint32_t)));
+    CK(cudaMalloc(&h->d_cls, h->plane_bytes));
     CK(cudaMalloc(&h->d_danger, h->plane_bytes));
+    CK(cudaMalloc(&h->d_displaced, slots * sizeof(uint32_t)));
+    CK(cudaMalloc(&h->d_acts, slots * sizeof(uint2)));
+    CK(cudaMalloc(&h->d_list_n, n_chunks * (kThreads / 32) * sizeof(uint2)));  // grids have at most n_chunks blocks
+    CK(cudaMalloc(&h->d_par, R * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_claim, h->claim_cells * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_seg, sizeof(SegDev)));
     CK(cudaMalloc(&h->d_ivn, R * sizeof(uint32_t)));
     CK(cudaMemset(h->d_ivn, 0, R * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_err, sizeof(int)));
-    CK(cudaMalloc(&h->d_scratch, 4 * sizeof(unsigned long long)));
+    CK(cudaMalloc(&h->d_scratch, 6 * sizeof(unsigned long long)));
     CK(cudaMallocHost(&h->h_seg, sizeof(SegDev)));
     CK(cudaMallocHost(&h->h_ivn, R * sizeof(uint32_t)));
     int rc = ensure_counts(h, 48);
@@ -1074,18 +1085,16 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
 
 // Everything after the agent arrays are on the device: scratch words, planes, parameters.
 static int finish_upload(epi_engine* h) {
-    const size_t slots = h->slots;
-    CK(cudaMemsetAsync(h->d_tgt, 0xFF, slots * sizeof(uint32_t), h->stream));
-    CK(cudaMemsetAsync(h->d_lost, 0xFF, slots * sizeof(uint32_t), h->stream));
-    CK(cudaMemsetAsync(h->d_plane, 0, h->plane_bytes * (h->two_planes ? 2u : 1u), h->stream));
+    CK(cudaMemsetAsync(h->d_occ, 0, 2u * h->occ_words * sizeof(uint32_t), h->stream));
+    CK(cudaMemsetAsync(h->d_cls, 0, h->plane_bytes, h->stream));
     CK(cudaMemsetAsync(h->d_danger, 0, h->plane_bytes, h->stream));
-    h->plane_par = 0;
     CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
+    for (auto& rep : h->reps) rep.par = 0;
     CK(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
     int rc = push_params(h);
     if (rc) return rc;
     LAUNCH(kKBuildPlane, (k_build_plane<<<blocks_for(h->slots), kThreads, 0, h->stream>>>(
-                              h->d_params, h->d_chunk_rep, h->slots, h->d_pos, h->d_st, h->d_plane, h->d_danger,
+                              h->d_params, h->d_chunk_rep, h->slots, h->d_pos, h->d_st, h->d_occ, h->d_cls, h->d_danger,
                               h->d_err)));
     CK(cudaStreamSynchronize(h->stream));
     rc = harvest_events(h);
@@ -1099,7 +1108,7 @@ static int snapshot_replica(epi_engine* h, uint32_t r, epi_agent_record* out, si
     const size_t off = rep.hp.agent_off;
     std::vector<uint32_t> pos(n), home(n), work(n), wsa(n);
     std::vector<uint2> st(n);
-    CK(cudaMemcpyAsync(pos.data(), h->d_pos + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(pos.data(), pos_buf(h, rep.par) + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(home.data(), h->d_home + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(work.data(), h->d_work + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaMemcpyAsync(wsa.data(), h->d_wsa + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
@@ -1134,25 +1143,30 @@ static int snapshot_replica(epi_engine* h, uint32_t r, epi_agent_record* out, si
 }
 
 static int check_all(epi_engine* h) {
-    CK(cudaMemsetAsync(h->d_scratch, 0, 4 * sizeof(unsigned long long), h->stream));
+    std::vector<uint32_t> par(h->R());
+    for (uint32_t r = 0; r < h->R(); ++r) par[r] = h->reps[r].par;
+    CK(cudaMemcpyAsync(h->d_par, par.data(), par.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemsetAsync(h->d_scratch, 0, 6 * sizeof(unsigned long long), h->stream));
     LAUNCH(kKCheck, (k_check_agents<<<blocks_for(h->slots), kThreads, 0, h->stream>>>(
-                         h->d_params, h->d_chunk_rep, h->slots, h->d_pos, h->d_st, plane_buf(h, h->plane_par),
-                         h->d_scratch)));
-    LAUNCH(kKCheck, (k_check_plane<<<h->grid_blocks, kThreads, 0, h->stream>>>(h->plane_bytes, plane_buf(h, h->plane_par),
-                                                                                h->d_scratch + 1)));
+                         h->d_params, h->d_chunk_rep, h->slots, h->d_pos, h->d_occ, h->occ_words, h->d_par, h->d_st,
+                         h->d_cls, h->d_scratch)));
+    LAUNCH(kKCheck, (k_check_planes<<<h->grid_blocks, kThreads, 0, h->stream>>>(
+                         h->R(), h->d_params, h->d_occ, h->occ_words, h->d_par, h->plane_bytes, h->d_cls,
+                         h->d_scratch + 2, h->d_scratch + 3, h->d_scratch + 4)));
     LAUNCH(kKCheck, (k_check_danger<<<dim3(64, std::min<uint32_t>(h->R(), 4096u)), kThreads, 0, h->stream>>>(
-                         h->d_params, h->R(), plane_buf(h, h->plane_par), h->d_danger, h->d_scratch + 2)));
-    unsigned long long v[4] = {0, 0, 0, 0};
+                         h->d_params, h->R(), h->d_cls, h->d_danger, h->d_scratch + 5)));
+    unsigned long long v[6] = {0, 0, 0, 0, 0, 0};
     CK(cudaMemcpyAsync(v, h->d_scratch, sizeof v, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     int rc = harvest_events(h);
     if (rc) return rc;
     uint64_t population = 0;
     for (const auto& rep : h->reps) population += rep.n;
-    if (v[0] || v[1] != population || v[2]) {
-        h->err = "invariants: " + std::to_string(v[0]) + " agents off their cell class, " + std::to_string(v[1]) +
-                 " occupied cells for " + std::to_string(population) + " agents, " + std::to_string(v[2]) +
-                 " cells with a wrong infectious-neighbour count";
+    if (v[0] || v[2] != population || v[3] || v[4] != v[1] || v[5]) {
+        h->err = "invariants: " + std::to_string(v[0]) + " agents off their cell class, " + std::to_string(v[2]) +
+                 " occupied cells for " + std::to_string(population) + " agents, " + std::to_string(v[3]) +
+                 " claims left in the spent plane, " + std::to_string(v[4]) + " class bytes for " + std::to_string(v[1]) +
+                 " infectious agents, " + std::to_string(v[5]) + " cells with a wrong infectious-neighbour count";
         return EPI_ERR_INVARIANT;
     }
     return EPI_OK;
@@ -1171,19 +1185,15 @@ static int set_launch_shape(epi_engine* h, uint32_t decide_blocks, uint32_t comm
     CK(cudaStreamSynchronize(h->stream));
     h->grid_blocks = (int)decide_blocks;
     h->commit_slots = (int)commit_slots;
-    {
-        const int rc = commit_grid(h, h->commit_slots, &h->commit_blocks);
-        if (rc) return rc;
-    }
     destroy_graphs(h);  // they bake the launch shapes in
     return EPI_OK;
 }
 
 // Launch-shape autotuner: times hours 1..hours of the engine's current world under each
-// candidate (k_decide grid: the resident grid, twice it, one chunk per block; k_commit: 1, 2
-// or 4 slots per thread), restarting every candidate from the same state, and keeps the
-// fastest.  Results do not depend on the shape; the state, the run's rows and the launch
-// counter are restored afterwards (the saved checkpoint is replaced).
+// candidate k_decide grid (three quarters of the resident grid, the resident grid, twice it,
+// one chunk per block), restarting every candidate from the same state, and keeps the fastest.
+// Results do not depend on the shape; the state, the run's rows and the launch counter are
+// restored afterwards (the saved checkpoint is replaced).
 static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
     if (hours == 0 || hours > 24u * 7u) { h->err = "autotune hours must be in [1, 168]"; return EPI_ERR_ARG; }
     const uint32_t n_chunks = h->slots / kChunk;
@@ -1196,59 +1206,69 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
         const uint32_t v = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(g, n_chunks));
         if (std::find(grids.begin(), grids.end(), v) == grids.end()) grids.push_back(v);
     }
-    const uint32_t slot_cands[3] = {1u, 2u, 4u};
     const bool prof = h->profiling;
     const uint64_t launched = h->kernels_launched;
     h->profiling = false;
     int rc = save_state(h);
     if (rc) return rc;
     double best = 1e300;
-    uint32_t best_g = (uint32_t)h->grid_blocks, best_c = (uint32_t)h->commit_slots;
+    uint32_t best_g = (uint32_t)h->grid_blocks;
     for (uint32_t g : grids) {
-        for (uint32_t c : slot_cands) {
-            rc = set_launch_shape(h, g, c);
-            double t_min = 1e300;
-            for (int rep = 0; rep < 5 && !rc; ++rep) {  // the first pass captures the graphs
-                rc = restore_state(h);
-                if (rc) break;
-                const auto t0 = std::chrono::steady_clock::now();
-                rc = run_hours(h, 1, hours);
-                const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-                if (rep > 0) t_min = std::min(t_min, t);
-            }
+        rc = set_launch_shape(h, g, (uint32_t)h->commit_slots);
+        double t_min = 1e300;
+        for (int rep = 0; rep < 5 && !rc; ++rep) {  // the first pass captures the graphs
+            rc = restore_state(h);
             if (rc) break;
-            if (t_min < best) { best = t_min; best_g = g; best_c = c; }
+            const auto t0 = std::chrono::steady_clock::now();
+            rc = run_hours(h, 1, hours);
+            const double t = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+            if (rep > 0) t_min = std::min(t_min, t);
         }
         if (rc) break;
+        if (t_min < best) { best = t_min; best_g = g; }
     }
     h->profiling = prof;
-    int rc2 = set_launch_shape(h, best_g, best_c);
+    int rc2 = set_launch_shape(h, best_g, (uint32_t)h->commit_slots);
     if (!rc2) rc2 = restore_state(h);
     h->kernels_launched = launched;
     if (rc) return rc;
     if (rc2) return rc2;
     if (out) {
         out->decide_blocks = best_g;
-        out->commit_slots = best_c;
+        out->commit_slots = (uint32_t)h->commit_slots;
         out->hour_us = best * 1e6 / hours;
+    }
+    return EPI_OK;
+}
+
+// Every replicate in the buffers of one parity (replicates that ended early may differ).
+static int same_buffer(epi_engine* h) {
+    for (uint32_t r = 1; r < h->R(); ++r) {
+        int rc = move_to_buffer(h, r, h->reps[0].par);
+        if (rc) return rc;
     }
     return EPI_OK;
 }
 
 static int save_state(epi_engine* h) {
     const size_t n = h->slots;
+    int rc = EPI_OK;
     if (!h->s_pos) {
         CK(cudaMalloc(&h->s_pos, n * sizeof(uint32_t)));
         CK(cudaMalloc(&h->s_wsa, n * sizeof(uint32_t)));
         CK(cudaMalloc(&h->s_st, n * sizeof(uint2)));
-        CK(cudaMalloc(&h->s_plane, h->plane_bytes));
+        CK(cudaMalloc(&h->s_occ, h->occ_words * sizeof(uint32_t)));
+        CK(cudaMalloc(&h->s_cls, h->plane_bytes));
         CK(cudaMalloc(&h->s_danger, h->plane_bytes));
     }
-    CK(cudaMemcpyAsync(h->s_pos, h->d_pos, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+    rc = same_buffer(h);
+    if (rc) return rc;
+    const uint32_t par = h->reps[0].par;
+    CK(cudaMemcpyAsync(h->s_pos, pos_buf(h, par), n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->s_wsa, h->d_wsa, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->s_st, h->d_st, n * sizeof(uint2), cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemcpyAsync(h->s_plane, plane_buf(h, h->plane_par), h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
-    h->s_plane_par = h->plane_par;
+    CK(cudaMemcpyAsync(h->s_occ, occ_buf(h, par), h->occ_words * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->s_cls, h->d_cls, h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->s_danger, h->d_danger, h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     for (auto& rep : h->reps) {
@@ -1256,6 +1276,7 @@ static int save_state(epi_engine* h) {
         rep.s_geo = rep.geo;
         rep.s_hosp_code = rep.hp.hosp_code;
         rep.s_active = rep.active;
+        rep.s_par = par;
         rep.s_rows = rep.rows;
     }
     h->s_loop_hour = h->loop_hour;
@@ -1266,15 +1287,14 @@ static int save_state(epi_engine* h) {
 static int restore_state(epi_engine* h) {
     if (!h->saved) { h->err = "no saved state"; return EPI_ERR_ARG; }
     const size_t n = h->slots;
-    CK(cudaMemcpyAsync(h->d_pos, h->s_pos, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+    const uint32_t par = h->reps[0].s_par;
+    CK(cudaMemcpyAsync(pos_buf(h, par), h->s_pos, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_wsa, h->s_wsa, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_st, h->s_st, n * sizeof(uint2), cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemcpyAsync(plane_buf(h, h->s_plane_par), h->s_plane, h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
-    if (h->two_planes) CK(cudaMemsetAsync(plane_buf(h, 1u - h->s_plane_par), 0, h->plane_bytes, h->stream));
-    h->plane_par = h->s_plane_par;
+    CK(cudaMemcpyAsync(occ_buf(h, par), h->s_occ, h->occ_words * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemsetAsync(occ_buf(h, 1u - par), 0, h->occ_words * sizeof(uint32_t), h->stream));
+    CK(cudaMemcpyAsync(h->d_cls, h->s_cls, h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->d_danger, h->s_danger, h->plane_bytes, cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaMemsetAsync(h->d_tgt, 0xFF, n * sizeof(uint32_t), h->stream));
-    CK(cudaMemsetAsync(h->d_lost, 0xFF, n * sizeof(uint32_t), h->stream));
     CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
     h->last_claim_hour = -1;
     for (auto& rep : h->reps) {
@@ -1283,6 +1303,7 @@ static int restore_state(epi_engine* h) {
         rep.hp.hosp_code = rep.s_hosp_code;
         rep.active = rep.s_active;
         rep.hp.active = rep.s_active ? 1u : 0u;
+        rep.par = rep.s_par;
         rep.rows = rep.s_rows;
     }
     h->loop_hour = h->s_loop_hour;
@@ -1807,7 +1828,7 @@ int epi_engine_state_stream_open(epi_engine* h, const char* path) {
     CK(cudaMallocHost(&h->h_codes, cap));
     CK(cudaMallocHost(&h->h_exc, (size_t)h->slots * sizeof(uint2)));
     CK(cudaMallocHost(&h->h_exc_n, kStreamChunk * sizeof(uint32_t)));
-    CK(cudaMemcpyAsync(h->d_prev, h->d_pos, (size_t)h->slots * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->d_prev, pos_buf(h, h->reps[0].par), (size_t)h->slots * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     destroy_graphs(h);  // hour graphs now carry the encoding kernel
     return EPI_OK;
@@ -1993,6 +2014,20 @@ std::mutex g_noalloc_mutex;
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
+using DecideBytesKernel = void (*)(const DevParams*, uint32_t, const uint32_t*, uint2*, const uint32_t*, const uint32_t*,
+                                   uint32_t*, const uint8_t*, uint32_t*, uint32_t*, HourArgs, int*);
+DecideBytesKernel decide_bytes_kernel(uint32_t hod) {
+    switch (hour_class(hod)) {
+        case kHcStart: return k_decide_bytes<kHcStart>;
+        case kHcEnd: return k_decide_bytes<kHcEnd>;
+        case kHcTransport: return k_decide_bytes<kHcTransport>;
+        case kHcWork: return k_decide_bytes<kHcWork>;
+        case kHcNoon: return k_decide_bytes<kHcNoon>;
+        case kHcHome: return k_decide_bytes<kHcHome>;
+        default: return k_decide_bytes<kHcMove>;
+    }
+}
+
 DevParams noalloc_params(const epi_params& p, uint32_t hospital_grown) {
     epi_geography g = define_geography(p.grid_size);
     resize_hospital(g, (int32_t)p.number_of_agents, 0.002, p.hospital_beds_percentage);
@@ -2022,7 +2057,7 @@ int noalloc_setup(int dev, NoAllocDevice** out) {
         NOALLOC_CK(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
         int sms = 0, per_sm = 0;
         NOALLOC_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        NOALLOC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)decide_kernel(9u), kThreads, 0));
+        NOALLOC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)decide_bytes_kernel(9u), kThreads, 0));
         d.grid_blocks = sms * std::max(per_sm, 1);
         d.base = static_cast<unsigned char*>(ptr);
     }
@@ -2087,11 +2122,9 @@ extern "C" int epi_tick_hour_noalloc(const epi_params* params, uint32_t hour, ui
         k_sleep<<<blocks, kThreads, 0, s>>>(d_params, nullptr, n_chunks, st, ha);
     } else {
         NOALLOC_CK(cudaMemsetAsync(d_claim, 0xFF, claim_bytes, s));
-        const DecideKernel decide = decide_kernel(hod);
-        decide<<<blocks, kThreads, 0, s>>>(d_params, nullptr, n_chunks, pos, st, home, work, work_start_at, plane, nullptr,
-                                           d_claim, d_tgt, nullptr, ha, d_err);
-        k_commit<kCommitSlots><<<commit_blocks_for(n), kThreads, 0, s>>>(d_params, nullptr, n, pos, d_tgt, plane, nullptr,
-                                                                         d_claim, nullptr, ha, 0ull, nullptr, 0u);
+        decide_bytes_kernel(hod)<<<blocks, kThreads, 0, s>>>(d_params, n_chunks, pos, st, home, work, work_start_at, plane,
+                                                             d_claim, d_tgt, ha, d_err);
+        k_commit_bytes<<<blocks, kThreads, 0, s>>>(d_params, n, pos, d_tgt, plane, d_claim);
     }
     NOALLOC_CK(cudaGetLastError());
     int err = 0;

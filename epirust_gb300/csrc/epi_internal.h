@@ -7,12 +7,15 @@
 //   home[i]  start corner of the 2x2 house  (packed like pos)
 //   work[i]  start corner of the 10x10 office (packed like pos; the house for non-workers)
 //   wsa[i]   work_start_at of hospital staff (read only for staff)
-// The occupancy plane is one byte per cell of the (G+1) x (G+1) plane (the reference's
-// areas reach row and column G, engine/src/geography/mod.rs:42-48), stored with a one-cell
-// border of zeros (pitch and height G+3, cell (x, y) at (y+1) * (G+3) + x+1):
-//   0 = vacant, 1 = occupied and not infectious, 2 = infectious at the regular rate,
-//   3 = infectious at the high rate.
-// A u32 claim plane of (G+1) x (G+1) resolves cell conflicts (lowest agent index wins).
+// pos has two buffers (kernels.cuh).  Planes cover the (G+1) x (G+1) cells (the reference's
+// areas reach row and column G, engine/src/geography/mod.rs:42-48) with a one-cell border of
+// zeros:
+//   occupancy  one bit per cell, two buffers: cell (x, y) is bit (x + 1) & 31 of word
+//              (y + 1) * PW + ((x + 1) >> 5), PW = ceil((G + 3) / 32) words a row
+//   class      one byte per cell (pitch G+3, cell (x, y) at (y+1) * (G+3) + x+1), non-zero only
+//              under an infectious agent: 0x01 regular rate, 0x10 high rate
+//   danger     one byte per cell, same layout: infectious agents on the 8 neighbours
+//   claim      a u32 per cell of (G+1) x (G+1), without border: the smallest claim key
 #pragma once
 
 #include <stdint.h>
@@ -45,7 +48,7 @@ constexpr uint32_t kDayMask = 0xFFFFu << kDayShift;
 // current_area codes; HOME/WORK decode through the agent's home/work corner
 enum AreaCode : uint32_t { kHome = 0, kWork = 1, kTransport = 2, kHousing = 3, kHosp0 = 4, kHosp1 = 5, kNumAreas = 6 };
 
-constexpr uint32_t kNoAction = 0xFFFFFFFFu;  // tgt[i]: nothing to commit
+constexpr uint32_t kNoAction = 0xFFFFFFFFu;  // a target word: nothing to commit
 constexpr uint32_t kNoClaim = 0xFFFFFFFFu;   // claim plane: free (larger than any key)
 // Claim keys: (127 - hour mod 128) << 25 | agent.  Within a window of 128 hours that starts
 // at a multiple of 128 a later hour has a smaller key, so atomicMin lets this hour's claims
@@ -87,6 +90,7 @@ struct DevParams {
     int32_t G;                  // grid size
     int32_t W;                  // claim-plane width G + 1
     int32_t WP;                 // byte-plane pitch G + 3 (one-cell border on each side)
+    uint32_t PW;                // words per row of the occupancy bit plane
     uint32_t hosp_code;         // kHosp0 or kHosp1: the current hospital_area
     Rect area[kNumAreas];       // global areas by code (HOME/WORK slots unused)
     uint32_t key0, key1;        // Philox key = seed
@@ -99,7 +103,8 @@ struct DevParams {
     // placement of this world among the replicates sharing the device arrays
     uint32_t agent_off;         // first agent slot (a multiple of the 256-slot chunk)
     uint32_t active;            // 0 once the run of this replicate has ended
-    uint64_t plane_off;         // byte offset of its bordered plane
+    uint64_t plane_off;         // byte offset of its class and danger planes
+    uint64_t occ_off;           // word offset of its bit plane
     uint64_t claim_off;         // word offset of its claim plane
     // day-boundary guard of the run loop: the data-dependent intervention triggers still armed
     uint32_t guard_flags;       // kGuard* bits

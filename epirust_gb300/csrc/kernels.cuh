@@ -10,10 +10,9 @@
 //
 // Per simulated hour (CitizenLocationMap::simulate, engine/src/allocation_map.rs:67-129):
 //   hours 1..6 of a day   k_sleep   current_area = home (non-staff), counts
-//   other hours           k_decide  per-agent rules on the previous-hour plane, proposals,
-//                                   atomicMin claims on the target cells, counts
-//                         k_commit  lowest claimant moves, losers stay, plane bytes updated;
-//                                   claims stay (a later hour's keys are smaller, see claim_key)
+//   other hours           k_decide  per-agent rules on the previous-hour planes, proposals,
+//                                   an occupancy bit claimed per agent, counts
+//                         k_commit  displaced claimants back to their cells, class planes, spent buffers zeroed
 #pragma once
 
 #include "tick.cuh"
@@ -31,19 +30,28 @@ constexpr int kThreads = (int)kChunk;
 // measured 1.7 % slower per hour than letting them start at its completion.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Warp-aggregated 6-bin histogram into shared memory: three ballots carry the bits of each
-// lane's bin (invalid lanes vote bin 7), and lane b (< 6) counts the lanes whose bits spell b.
-__device__ __forceinline__ void count_into(uint32_t* sh, bool valid, uint32_t bin) {
-    const uint32_t v = valid ? bin : 7u;
-    const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, v & 1u), b1 = __ballot_sync(0xFFFFFFFFu, v & 2u),
-                   b2 = __ballot_sync(0xFFFFFFFFu, v & 4u);
-    const uint32_t lane = threadIdx.x & 31u;
-    if (lane < 6u) {
-        const uint32_t m = ((lane & 1u) ? b0 : ~b0) & ((lane & 2u) ? b1 : ~b1) & ((lane & 4u) ? b2 : ~b2);
-        const uint32_t c = (uint32_t)__popc(m);
-        if (c) atomicAdd(&sh[lane], c);
+// Warp-aggregated 6-bin histogram: three ballots carry the bits of each lane's bin (invalid
+// lanes vote bin 7), lane b (< 6) counts the lanes whose bits spell b in a register, and the
+// warp adds its counts to the block's when they are due.
+struct Tally {
+    uint32_t n0, n1, n2, n = 0;  // all ones where the lane number's bit is clear
+    __device__ __forceinline__ Tally() {
+        const uint32_t lane = threadIdx.x & 31u;
+        n0 = (lane & 1u) - 1u;
+        n1 = ((lane >> 1) & 1u) - 1u;
+        n2 = ((lane >> 2) & 1u) - 1u;
     }
-}
+    __device__ __forceinline__ void add(bool valid, uint32_t bin) {
+        const uint32_t v = valid ? bin : 7u;
+        const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, v & 1u), b1 = __ballot_sync(0xFFFFFFFFu, v & 2u),
+                       b2 = __ballot_sync(0xFFFFFFFFu, v & 4u);
+        n += (uint32_t)__popc((b0 ^ n0) & (b1 ^ n1) & (b2 ^ n2));
+    }
+    __device__ __forceinline__ void flush(uint32_t* sh) {
+        if ((threadIdx.x & 31u) < 6u && n) atomicAdd(&sh[threadIdx.x & 31u], n);
+        n = 0;
+    }
+};
 
 // Consecutive chunks a block takes per grid-stride step.  An ensemble block that strides one
 // chunk at a time switches replicate at nearly every step (a parameter reload and a
@@ -104,7 +112,8 @@ __device__ __forceinline__ bool run_ended(const uint32_t* prev, uint32_t r) {
 // Switch the block to replicate r: flush the histogram of the previous one into its counts
 // row (counts[r * 8 + bin]), stage r's parameters, clear the histogram.  Block-uniform.
 __device__ __forceinline__ void switch_rep(BlockRep& br, uint32_t r, const DevParams* __restrict__ Pall, DevParams& sP,
-                                           uint32_t* sh, uint32_t* counts) {
+                                           Tally& tally, uint32_t* sh, uint32_t* counts) {
+    if (br.r != 0xFFFFFFFFu) tally.flush(sh);
     __syncthreads();
     if (br.r != 0xFFFFFFFFu && threadIdx.x < 6 && sh[threadIdx.x]) atomicAdd(&counts[br.r * 8 + threadIdx.x], sh[threadIdx.x]);
     __syncthreads();
@@ -115,14 +124,16 @@ __device__ __forceinline__ void switch_rep(BlockRep& br, uint32_t r, const DevPa
     br.r = r;
 }
 
-__device__ __forceinline__ void flush_rep(const BlockRep& br, uint32_t* sh, uint32_t* counts) {
+__device__ __forceinline__ void flush_rep(const BlockRep& br, Tally& tally, uint32_t* sh, uint32_t* counts) {
+    if (br.r != 0xFFFFFFFFu) tally.flush(sh);
     __syncthreads();
     if (br.r != 0xFFFFFFFFu && threadIdx.x < 6 && sh[threadIdx.x]) atomicAdd(&counts[br.r * 8 + threadIdx.x], sh[threadIdx.x]);
 }
 
 // First vacant hospital cell of the snapshot in AreaIterator order (area.rs:131-148), found
 // by the whole block; kNoAction when the hospital is full.
-__device__ uint32_t block_first_vacant(const DevParams& P, const PlaneView& pl) {
+template <class V>
+__device__ uint32_t block_first_vacant(const DevParams& P, const V& pl) {
     __shared__ uint32_t best;
     const Rect h = P.area[P.hosp_code];
     const uint32_t w = (uint32_t)(h.x1 - h.x0 + 1), total = w * (uint32_t)(h.y1 - h.y0 + 1);
@@ -146,9 +157,9 @@ __device__ uint32_t block_first_vacant(const DevParams& P, const PlaneView& pl) 
 // kernel is one load and a compare per agent, so one load round per chunk set its time).
 constexpr uint32_t kSleepBatch = 4;
 
-__device__ __forceinline__ void sleep_agent(uint2* __restrict__ st, uint32_t slot, bool valid, uint32_t s, uint32_t* sh) {
+__device__ __forceinline__ void sleep_agent(uint2* __restrict__ st, uint32_t slot, bool valid, uint32_t s, Tally& tally) {
     if (valid && st_ws(s) != EPI_WS_HOSPITAL_STAFF && st_area(s) != kHome) st[slot].x = with_area(s, kHome);
-    count_into(sh, valid, count_bin(s));
+    tally.add(valid, count_bin(s));
 }
 
 __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
@@ -158,10 +169,11 @@ __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict_
     dep_wait();
     const HourRow hr = hour_row(ha);
     BlockRep br;
+    Tally tally;
     bool ended = false;  // run_ended of the block's replicate (its prev row is fixed during the launch)
     if (!chunk_rep) {
         if (blockIdx.x < n_chunks) {
-            switch_rep(br, 0u, Pall, sP, sh, row_ptr(ha, hr.row));
+            switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
             ended = run_ended(prev_ptr(ha, hr.row), 0u);
         }
         if (blockIdx.x < n_chunks && sP.active && !ended) {
@@ -176,11 +188,11 @@ __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict_
                 for (uint32_t q = 0; q < kSleepBatch; ++q) {
                     const uint32_t c = c0 + q * gridDim.x, slot = c * kChunk + threadIdx.x;
                     if (c >= n_chunks) break;  // block-uniform
-                    sleep_agent(st, slot, slot < sP.n, sv[q], sh);
+                    sleep_agent(st, slot, slot < sP.n, sv[q], tally);
                 }
             }
         }
-        flush_rep(br, sh, row_ptr(ha, hr.row));
+        flush_rep(br, tally, sh, row_ptr(ha, hr.row));
         return;
     }
     const uint32_t grp = kEnsembleChunkGroup;  // chunks per stride step
@@ -188,27 +200,81 @@ __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict_
          c = (++k < grp) ? c + 1u : c + (gridDim.x - 1u) * grp + 1u, k = (k < grp) ? k : 0u) {
         const uint32_t r = chunk_rep ? chunk_rep[c] : 0u;
         if (r != br.r) {
-            switch_rep(br, r, Pall, sP, sh, row_ptr(ha, hr.row));
+            switch_rep(br, r, Pall, sP, tally, sh, row_ptr(ha, hr.row));
             ended = run_ended(prev_ptr(ha, hr.row), r);
         }
         if (!sP.active || ended) continue;
         const uint32_t slot = c * kChunk + threadIdx.x;
         const bool valid = slot - sP.agent_off < sP.n;
-        sleep_agent(st, slot, valid, valid ? st[slot].x : 0u, sh);
+        sleep_agent(st, slot, valid, valid ? st[slot].x : 0u, tally);
     }
-    flush_rep(br, sh, row_ptr(ha, hr.row));
+    flush_rep(br, tally, sh, row_ptr(ha, hr.row));
 }
 
-// The rules of one agent for the hour (slot valid): proposal, claim, infection update, state
-// and target words.  Returns the agent's counts bin.  FULL (a lone world with two plane
-// buffers, the hours whose commit rebuilds the plane): every agent's target word names its
-// cell and class.
-template <int HC, bool FULL = false>
-__device__ __forceinline__ uint32_t decide_agent(const DevParams& P, const PlaneView& pl, uint32_t* __restrict__ rclaim,
-                                                 uint32_t* __restrict__ wsa, uint2* __restrict__ st,
-                                                 uint32_t* __restrict__ tgt, uint32_t* __restrict__ lost, uint32_t slot,
-                                                 uint32_t i, uint32_t s, uint32_t at, uint32_t p, uint32_t hm, uint32_t wk,
-                                                 uint32_t hour, uint32_t hod, uint32_t hosp_first, int* err) {
+// ---------------------------------------------------------------- the hour's two kernels
+// Claims.  A mover claims its target with an atomicMin of claim_key (lowest index of the hour
+// wins) on the cell's claim word, and the value it finds names the claimant it competes with:
+// of the two the higher index has lost.  Every claimant but the cell's lowest is named so
+// exactly once -- by itself, which then simply stays, or by the one that displaces it, which
+// puts it on its warp's list.  The hour's blocks sweep the agents in index order, so most
+// losers find a lower index before them and few are ever displaced: k_commit, which sends the
+// listed ones back, has a short list (1.3 % of the agents in office hours, 0.04 % at home)
+// where a pass over all agents would settle every move.  One GB300, 1M agents on a 2,500 grid:
+// k_commit 5 us per waking hour in a launch list, against 9 us for a pass over target words,
+// loss marks and byte-plane stores; 4M agents 5.2 us against 26 us.
+//
+// The occupancy of the next hour is a bit plane that starts the hour all zero: the first
+// claimant of a cell sets the target's bit, an agent that stays or lost sets its own cell's.
+//
+// Positions have two buffers as well.  In the hours of day 7..22 every agent writes its
+// proposal to the other one, so the old cell of a claimant that lost is at hand; at hours 0
+// and 23 (PATCH), where few agents act, the current buffer and bit plane are patched in place
+// and the agents that act leave their old position in the other buffer.
+//
+// A warp's lists lie over the slots of its own chunks, in the order the warp takes them: entry
+// e of a warp is at the slot of lane e % 32 in the warp's (e / 32)-th chunk.
+struct HourLists {
+    uint32_t* displaced;  // slots of claimants that a lower index has displaced
+    uint2* acts;          // {slot, target word}: infectious agents that move or change class (PATCH: every mover too)
+    uint2* n;             // per warp: entries of the two lists
+};
+
+// The k-th chunk of block b (a grid of blocks): plain stride for a single world, groups of
+// kEnsembleChunkGroup for an ensemble.
+template <bool ENS>
+__device__ __forceinline__ uint32_t chunk_at(uint32_t b, uint32_t grid, uint32_t k) {
+    if (!ENS) return b + k * grid;
+    return ((k / kEnsembleChunkGroup) * grid + b) * kEnsembleChunkGroup + k % kEnsembleChunkGroup;
+}
+template <bool ENS>
+__device__ __forceinline__ uint32_t list_slot(uint32_t e) {
+    return chunk_at<ENS>(blockIdx.x, gridDim.x, e >> 5) * kChunk + (threadIdx.x & ~31u) + (e & 31u);
+}
+// Append the entries of the lanes with f set to the warp's list (whole warps; n is uniform).
+template <bool ENS, class T>
+__device__ __forceinline__ void list_append(T* list, uint32_t& n, bool f, const T& v) {
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, f);
+    if (f) list[list_slot<ENS>(n + (uint32_t)__popc(m & ((1u << (threadIdx.x & 31u)) - 1u)))] = v;
+    n += (uint32_t)__popc(m);
+}
+
+// What one agent's hour leaves to its warp: the counts bin and the list entries.
+struct AgentHour {
+    uint32_t bin = 0;
+    uint32_t target = 0;
+    uint32_t loser = 0;  // slot this agent displaced
+    bool displaces = false, act = false;
+};
+
+// The rules of one agent for the hour: proposal, claim, infection update, state and position
+// words.  next is the replicate's zeroed bit plane, pos_next the other position buffer.
+template <int HC, bool PATCH>
+__device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitView& pl, const StepTable& steps,
+                                                  uint32_t* __restrict__ next,
+                                                  uint32_t* __restrict__ rclaim, uint32_t* __restrict__ wsa,
+                                                  uint2* __restrict__ st, uint32_t* pos, uint32_t* pos_next, uint32_t slot,
+                                                  uint32_t i, uint32_t s, uint32_t at, uint32_t p, uint32_t hm, uint32_t wk,
+                                                  uint32_t hour, uint32_t hosp_first) {
     const uint32_t s0 = s, at0 = at;
     const Cell cell{unpack_x(p), unpack_y(p)};
     Draws dr{i, hour, P.key0, P.key1, P.move_key};
@@ -219,90 +285,114 @@ __device__ __forceinline__ uint32_t decide_agent(const DevParams& P, const Plane
     } else if (HC == kHcEnd) {
         nc = routine_end(P, pl, s, hm, cell, dr);
     } else {
-        const bool staff = st_ws(s) == EPI_WS_HOSPITAL_STAFF;
-        uint32_t w0 = staff ? wsa[slot] : 0u, w = w0;
-        nc = perform_movements<HC>(P, pl, s, w, hm, wk, cell, hod, hour, dr, infect);
-        if (staff && w != w0) wsa[slot] = w;
+        nc = perform_movements<HC>(P, pl, steps, s, wsa + slot, hm, wk, cell, hour, dr, infect);
     }
+    // (a proposal is the agent's cell, a vacant cell or a valid neighbour: inside the plane)
     bool moving = nc.x != cell.x || nc.y != cell.y;
-    if (moving && ((uint32_t)nc.x > (uint32_t)P.G || (uint32_t)nc.y > (uint32_t)P.G)) {
-        atomicOr(err, 4);  // unreachable for validated worlds; never write outside the plane
-        moving = false;
-        nc = cell;
-    }
     // The claim goes out before the infection update so that its round trip overlaps it.
+    AgentHour out;
     const uint32_t key = claim_key(hour, i);
-    const uint32_t old = moving ? atomicMin(&rclaim[(size_t)nc.y * P.W + nc.x], key) : kNoClaim;
+    const uint32_t found = moving ? atomicMin(&rclaim[(size_t)nc.y * P.W + nc.x], key) : kNoClaim;
     if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
-    if (moving) {
-        // The claim that atomicMin finds names an agent this one competes with: of the two
-        // the higher index loses.  Every claimant but the cell's lowest is named so, by
-        // itself or by the claimant that displaced it, so the loss marks settle the cell
-        // without a second read of the claim plane.
-        if (lost && old != kNoClaim && (old >> kClaimAgentBits) == (key >> kClaimAgentBits)) {
-            const uint32_t j = old & kMaxAgentsPerWorld;
-            if (j < i) {
-                moving = false;
-                nc = cell;
-            } else {
-                lost[P.agent_off + j] = hour;
-            }
+    // (an untouched word looks like a key of the window's first hour, but for its index)
+    if (found != kNoClaim && (found >> kClaimAgentBits) == (key >> kClaimAgentBits)) {
+        const uint32_t j = found & kMaxAgentsPerWorld;
+        if (j < i) {
+            moving = false;
+            nc = cell;
+        } else {
+            out.displaces = true;
+            out.loser = P.agent_off + j;
         }
     }
-    // the plane byte changes when the agent moves or its class changes (s == s0 keeps it)
-    uint32_t t = kNoAction;
-    if (moving || s != s0 || FULL) {
-        const uint32_t cls0 = cell_class(P, s0), cls = s == s0 ? cls0 : cell_class(P, s);
-        if (moving || cls != cls0 || FULL) t = encode_target(nc, cls, cls0);
+    const uint32_t q = pack_xy(nc.x, nc.y);
+    if (!PATCH) {
+        if (!out.displaces) {
+            const uint32_t X = (uint32_t)nc.x + 1u;
+            atomicOr(&next[((uint32_t)nc.y + 1u) * P.PW + (X >> 5)], 1u << (X & 31u));
+        }
+        pos_next[slot] = q;
     }
-    tgt[slot] = t;
+    if (infected(s0) || infected(s)) {  // the planes follow its class (a healthy agent's is 1 throughout)
+        const uint32_t cls0 = cell_class(P, s0), cls = cell_class(P, s);
+        out.act = (cls0 >= 2u || cls >= 2u) && (moving || cls != cls0);
+        out.target = encode_target(nc, cls, cls0);
+    }
+    if (PATCH && moving && !out.act) {
+        out.act = true;
+        out.target = encode_target(nc, 1u, 1u);
+    }
+    if (PATCH && out.act) {
+        pos_next[slot] = p;
+        if (moving) pos[slot] = q;
+    }
     if (s != s0 || at != at0) st[slot] = make_uint2(s, at);
-    return count_bin(s);
+    out.bin = count_bin(s);
+    return out;
 }
 
 // One hour of per-agent rules (hour of day 0, 7..22 or 23), specialised per hour class HC,
 // over one world (ENS false: slot = agent, the parameters staged once) or the chunks of many
 // replicates (ENS true: chunk_rep names each chunk's replicate).  The body is shared by two
-// kernels that differ in their launch bounds: k_decide for a single world (registers left to
-// the compiler) and k_decide_ens for ensembles (at least kEnsembleMinBlocks resident blocks:
-// 48 registers), whose per-chunk replicate switches favour occupancy; each was measured
-// faster on its own workload.
-constexpr int kEnsembleMinBlocks = 5;
+// kernels that differ in their launch bounds: k_decide for a single world (5 resident blocks,
+// 48 registers) and k_decide_ens for ensembles (6 blocks, 40 registers), whose per-chunk
+// replicate switches favour occupancy.  Every hour class has the same bound because one grid,
+// the resident one, serves them all: left to the compiler the mixed hours took 54 registers,
+// ran the 760-block grid in two waves and cost a run a quarter more.  (One GB300, two weeks of
+// hours: 1M agents 5.39 ms at 5 blocks, 5.43 at 6, 6.08 at 7; 4M agents 5.83, 5.69, 6.15; the
+// 256-replicate ensemble 49.9 at 4 blocks, 48.0 at 5, 47.1 at 6, 60.1 at 8.)
+//
+// What bounds it: issue and dependent latency together.  A walking agent costs about 390 warp
+// instructions per 32 agents and three dependent L2 round trips (its words, the rows around
+// its cell, the claim); 60 % of the issue slots are busy while warps are resident.
+constexpr int kWorldMinBlocks = 5;
+constexpr int kEnsembleMinBlocks = 6;
 
-template <int HC, bool ENS, bool FULL = false>
+// The arrays of an hour's launch (see the claims above).
+struct HourBuffers {
+    uint32_t* pos;        // positions before the hour
+    uint32_t* pos_next;   // the other buffer
+    uint2* st;
+    const uint32_t *home, *work;
+    uint32_t* wsa;
+    uint32_t* occ;        // occupancy before the hour
+    uint32_t* occ_next;   // the other buffer, all zero
+    uint8_t *cls, *danger;
+    uint32_t* claim;
+    HourLists lists;
+    int* err;
+};
+
+template <int HC, bool ENS>
 __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
-                                            uint32_t n_chunks, const uint32_t* __restrict__ pos, uint2* __restrict__ st,
-                                            const uint32_t* __restrict__ home, const uint32_t* __restrict__ work,
-                                            uint32_t* __restrict__ wsa, const uint8_t* __restrict__ plane,
-                                            const uint8_t* __restrict__ danger, uint32_t* __restrict__ claim,
-                                            uint32_t* __restrict__ tgt, uint32_t* __restrict__ lost, const HourArgs& ha,
-                                            int* err) {
+                                            uint32_t n_chunks, const HourBuffers& B, const HourArgs& ha) {
+    constexpr bool PATCH = HC == kHcStart || HC == kHcEnd;
     __shared__ uint32_t sh[8];
     __shared__ DevParams sP;
+    __shared__ StepTable steps;
     const DevParams& P = sP;
+    if (!PATCH) stage_steps(steps);  // read after switch_rep's barriers
     dep_wait();
     const HourRow hr = hour_row(ha);
     const uint32_t hour = hr.hour;
-    const uint32_t hod = hour % 24u;
     BlockRep br;
-    uint32_t hosp_first = kNoAction;
+    Tally tally;
+    uint32_t hosp_first = kNoAction, n_displaced = 0u, n_acts = 0u;
     bool hosp_known = false;
     if (!ENS) {
-        if (blockIdx.x >= n_chunks) return;  // block-uniform: nothing to do or count
-        switch_rep(br, 0u, Pall, sP, sh, row_ptr(ha, hr.row));
-        if (P.active && !run_ended(prev_ptr(ha, hr.row), 0u)) {
-            const PlaneView pl{plane + P.plane_off, P.G, P.WP, err, danger ? danger + P.plane_off : nullptr};
-            uint32_t* rclaim = claim + P.claim_off;
+        if (blockIdx.x < n_chunks) switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+        if (blockIdx.x < n_chunks && P.active && !run_ended(prev_ptr(ha, hr.row), 0u)) {
+            const BitView pl{B.occ, B.cls, B.danger, P.G, P.WP, P.PW, B.err};
             const uint32_t n = P.n;
             for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
                 const uint32_t slot = c * kChunk + threadIdx.x;  // = agent index (a lone world starts at slot 0)
                 const bool valid = slot < n;
                 uint32_t s = 0, at = 0, p = 0;
                 if (valid) {
-                    const uint2 sv = st[slot];
+                    const uint2 sv = B.st[slot];
                     s = sv.x;
                     at = sv.y;
-                    p = pos[slot];
+                    p = B.pos[slot];
                 }
                 if (HC == kHcStart) {
                     const bool need = valid && wants_hospital(P, infected(s) ? with_day(s, st_day(s) + 1u) : s);
@@ -311,40 +401,188 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                         hosp_known = true;
                     }
                 }
-                const uint32_t bin = valid ? decide_agent<HC, FULL>(P, pl, rclaim, wsa, st, tgt, lost, slot, slot, s, at, p,
-                                                                    home[slot], work[slot], hour, hod, hosp_first, err)
-                                           : 0u;
-                count_into(sh, valid, bin);
+                AgentHour a;
+                if (valid)
+                    a = decide_agent<HC, PATCH>(P, pl, steps, B.occ_next, B.claim, B.wsa, B.st, B.pos, B.pos_next, slot, slot, s, at, p,
+                                                B.home[slot], B.work[slot], hour, hosp_first);
+                tally.add(valid, a.bin);
+                if (__any_sync(0xFFFFFFFFu, a.displaces || a.act)) {
+                    list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
+                    list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
+                }
             }
         }
-        flush_rep(br, sh, row_ptr(ha, hr.row));
-        return;
-    }
-    bool ended = false;
-    const uint32_t grp = kEnsembleChunkGroup;  // chunks per stride step
-    // The replicate of the next chunk is read one chunk ahead, and a chunk's agent words are
-    // read before its replicate is known (every chunk of an ensemble is whole in the slot
-    // arrays), so neither waits on the other.
-    auto next_chunk = [&](uint32_t c, uint32_t k) { return k + 1u < grp ? c + 1u : c + (gridDim.x - 1u) * grp + 1u; };
-    uint32_t r_next = blockIdx.x * grp < n_chunks ? chunk_rep[blockIdx.x * grp] : 0u;
-    for (uint32_t c = blockIdx.x * grp, k = 0; c < n_chunks; c = next_chunk(c, k), k = (k + 1u < grp) ? k + 1u : 0u) {
-        const uint32_t r = r_next;
-        const uint32_t cn = next_chunk(c, k);
-        r_next = cn < n_chunks ? chunk_rep[cn] : 0u;
-        const uint32_t slot = c * kChunk + threadIdx.x;
-        const uint2 sv = st[slot];
-        const uint32_t pw = pos[slot], hw = home[slot], ww = work[slot];
-        if (r != br.r) {
-            switch_rep(br, r, Pall, sP, sh, row_ptr(ha, hr.row));
-            hosp_known = false;
-            ended = run_ended(prev_ptr(ha, hr.row), r);  // an earlier row: fixed during the launch
+    } else {
+        bool ended = false;
+        // The replicate of the next chunk is read one chunk ahead, and a chunk's agent words are
+        // read before its replicate is known (every chunk of an ensemble is whole in the slot
+        // arrays), so neither waits on the other.
+        uint32_t c = chunk_at<true>(blockIdx.x, gridDim.x, 0u);
+        uint32_t r_next = c < n_chunks ? chunk_rep[c] : 0u;
+        for (uint32_t k = 0; c < n_chunks; ++k) {
+            const uint32_t r = r_next;
+            const uint32_t slot = c * kChunk + threadIdx.x;
+            c = chunk_at<true>(blockIdx.x, gridDim.x, k + 1u);
+            r_next = c < n_chunks ? chunk_rep[c] : 0u;
+            const uint2 sv = B.st[slot];
+            const uint32_t pw = B.pos[slot], hw = B.home[slot], ww = B.work[slot];
+            if (r != br.r) {
+                switch_rep(br, r, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+                hosp_known = false;
+                ended = run_ended(prev_ptr(ha, hr.row), r);  // an earlier row: fixed during the launch
+            }
+            if (!P.active || ended) continue;
+            const BitView pl{B.occ + P.occ_off, B.cls + P.plane_off, B.danger + P.plane_off, P.G, P.WP, P.PW, B.err};
+            const uint32_t i = slot - P.agent_off;  // index within the replicate
+            const bool valid = i < P.n;
+            const uint32_t s = valid ? sv.x : 0u, at = valid ? sv.y : 0u, p = valid ? pw : 0u;
+            if (HC == kHcStart) {
+                const bool need = valid && wants_hospital(P, infected(s) ? with_day(s, st_day(s) + 1u) : s);
+                if (__syncthreads_or(need) && !hosp_known) {
+                    hosp_first = block_first_vacant(P, pl);
+                    hosp_known = true;
+                }
+            }
+            AgentHour a;
+            if (valid)
+                a = decide_agent<HC, PATCH>(P, pl, steps, B.occ_next + P.occ_off, B.claim + P.claim_off, B.wsa, B.st, B.pos,
+                                            B.pos_next, slot, i, s, at, p, hw, ww, hour, hosp_first);
+            tally.add(valid, a.bin);
+            if (__any_sync(0xFFFFFFFFu, a.displaces || a.act)) {
+                list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
+                list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
+            }
         }
-        if (!P.active || ended) continue;
-        const PlaneView pl{plane + P.plane_off, P.G, P.WP, err, danger ? danger + P.plane_off : nullptr};
-        uint32_t* rclaim = claim + P.claim_off;
-        const uint32_t i = slot - P.agent_off;  // index within the replicate
+    }
+    flush_rep(br, tally, sh, row_ptr(ha, hr.row));
+    if ((threadIdx.x & 31u) == 0u) B.lists.n[(blockIdx.x * kThreads + threadIdx.x) >> 5] = make_uint2(n_displaced, n_acts);
+}
+
+template <int HC>
+__global__ void __launch_bounds__(kThreads, kWorldMinBlocks) k_decide(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
+                                                     uint32_t n_chunks, const __grid_constant__ HourBuffers B, HourArgs ha) {
+    decide_body<HC, false>(Pall, chunk_rep, n_chunks, B, ha);
+}
+template <int HC>
+__global__ void __launch_bounds__(kThreads, kEnsembleMinBlocks)
+    k_decide_ens(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep, uint32_t n_chunks,
+                 const __grid_constant__ HourBuffers B, HourArgs ha) {
+    decide_body<HC, true>(Pall, chunk_rep, n_chunks, B, ha);
+}
+
+// A claimant that lost (slot of replicate P): back to its old cell.  dest holds its proposal,
+// old its position before the hour; occ is the plane of the hour's end.
+template <bool PATCH>
+__device__ __forceinline__ void send_back(const DevParams& P, uint32_t slot, const uint2* __restrict__ st,
+                                          uint32_t* dest, const uint32_t* old, uint32_t* occ, uint8_t* cls_plane,
+                                          uint8_t* danger) {
+    const uint32_t o = old[slot], s = st[slot].x, proposal = dest[slot];
+    // The position is changed by an atomic too: a plain store beside the atomic below made the
+    // launch wait 3.3 us (10,000 agents) to 5.6 us (1M agents, office hours) for its stores to
+    // drain at the end, whatever its cache operator.
+    atomicXor(&dest[slot], o ^ proposal);
+    const uint32_t X = (uint32_t)unpack_x(o) + 1u, w = ((uint32_t)unpack_y(o) + 1u) * P.PW + (X >> 5);
+    // PATCH: its entry in acts flips the bit too, so that two flips leave it set in either order
+    if (PATCH) atomicXor(&occ[w], 1u << (X & 31u));
+    else atomicOr(&occ[w], 1u << (X & 31u));
+    const uint32_t cls = cell_class(P, s);
+    if (cls >= 2u) {
+        class_add(cls_plane, danger, (uint32_t)P.WP, proposal, cls, true);
+        class_add(cls_plane, danger, (uint32_t)P.WP, o, cls, false);
+    }
+}
+
+// Completes the hour (the serial resolve of allocation_map.rs:93-102 in index order) from the
+// lists of k_decide, launched with the same grid: a warp takes its own lists.  Everything it
+// does to one word adds up or is idempotent, so the order of entries does not matter.  Not
+// PATCH: the planes and positions read this hour become the next hour's other buffers, so the
+// spent bit plane is zeroed (pieces of kPieceWords words; piece_rep names a piece's replicate
+// in an ensemble, where a replicate whose run has ended keeps its plane).
+constexpr uint32_t kPieceWords = 512;
+
+template <bool ENS, bool PATCH>
+__global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
+                                                     uint32_t n_pieces, const uint32_t* __restrict__ piece_rep,
+                                                     const __grid_constant__ HourBuffers B, HourArgs ha, uint64_t claim_cells) {
+    dep_wait();
+    const HourRow hr = hour_row(ha);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint2 n = B.lists.n[(blockIdx.x * kThreads + threadIdx.x) >> 5];
+    uint32_t* dest = PATCH ? B.pos : B.pos_next;
+    const uint32_t* old = PATCH ? B.pos_next : B.pos;
+    uint32_t* occ = PATCH ? B.occ : B.occ_next;
+    for (uint32_t e = lane; e < n.x; e += 32u) {
+        const uint32_t slot = B.lists.displaced[list_slot<ENS>(e)];
+        const DevParams& P = Pall[ENS ? chunk_rep[slot / kChunk] : 0u];
+        send_back<PATCH>(P, slot, B.st, dest, old, occ + P.occ_off, B.cls + P.plane_off, B.danger + P.plane_off);
+    }
+    for (uint32_t e = lane; e < n.y; e += 32u) {
+        const uint2 a = B.lists.acts[list_slot<ENS>(e)];
+        const DevParams& P = Pall[ENS ? chunk_rep[a.x / kChunk] : 0u];
+        const uint32_t o = old[a.x], t = target_xy(a.y), cls = target_class(a.y), cls0 = target_old_class(a.y);
+        uint8_t *cp = B.cls + P.plane_off, *dg = B.danger + P.plane_off;
+        if (cls0 >= 2u) class_add(cp, dg, (uint32_t)P.WP, o, cls0, true);
+        if (cls >= 2u) class_add(cp, dg, (uint32_t)P.WP, t, cls, false);
+        if (PATCH && t != o) {
+            const uint32_t Xo = (uint32_t)unpack_x(o) + 1u, X = (uint32_t)unpack_x(t) + 1u;
+            const uint32_t w = ((uint32_t)unpack_y(t) + 1u) * P.PW + (X >> 5);
+            uint32_t* ro = occ + P.occ_off;
+            atomicXor(&ro[((uint32_t)unpack_y(o) + 1u) * P.PW + (Xo >> 5)], 1u << (Xo & 31u));
+            atomicOr(&ro[w], 1u << (X & 31u));
+        }
+    }
+    if (!PATCH) {
+        const uint32_t* prev = prev_ptr(ha, hr.row);
+        const uint32_t per = kPieceWords / 4u;  // 16-byte words
+        const uint32_t stride = gridDim.x * (kThreads / per);
+        if (ENS || (Pall[0].active && !run_ended(prev, 0u)))
+            for (uint32_t q = blockIdx.x * (kThreads / per) + threadIdx.x / per; q < n_pieces; q += stride) {
+                if (ENS) {
+                    const uint32_t r = piece_rep[q];
+                    if (!Pall[r].active || run_ended(prev, r)) continue;
+                }
+                reinterpret_cast<uint4*>(B.occ)[(size_t)q * per + threadIdx.x % per] = make_uint4(0u, 0u, 0u, 0u);
+            }
+    }
+    // A new claim window (kClaimWindow hours) opens before the next hour that claims (hour of
+    // day 0 claims next at 7): every claim word is reset for it.
+    const uint32_t next = hr.hour % 24u == 0u ? hr.hour + 7u : hr.hour + 1u;
+    if (next / kClaimWindow != hr.hour / kClaimWindow)
+        for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < claim_cells; i += (size_t)gridDim.x * kThreads)
+            B.claim[i] = kNoClaim;
+}
+
+// ---------------------------------------------------------------- the caller-owned planes
+// The hour of epi_tick_hour_noalloc, whose caller owns one byte plane and no second buffers:
+// claims are an atomicMin per mover on a claim plane that every call resets, and
+// the commit reads the winner back and patches the plane in place.
+template <int HC>
+__global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __restrict__ Pall, uint32_t n_chunks,
+                                                           const uint32_t* __restrict__ pos, uint2* __restrict__ st,
+                                                           const uint32_t* __restrict__ home, const uint32_t* __restrict__ work,
+                                                           uint32_t* __restrict__ wsa, const uint8_t* __restrict__ plane,
+                                                           uint32_t* __restrict__ claim, uint32_t* __restrict__ tgt,
+                                                           HourArgs ha, int* err) {
+    __shared__ uint32_t sh[8];
+    __shared__ DevParams sP;
+    __shared__ StepTable steps;
+    const DevParams& P = sP;
+    stage_steps(steps);  // read after switch_rep's barriers
+    const HourRow hr = hour_row(ha);
+    const uint32_t hour = hr.hour;
+    BlockRep br;
+    Tally tally;
+    uint32_t hosp_first = kNoAction;
+    bool hosp_known = false;
+    if (blockIdx.x >= n_chunks) return;  // block-uniform
+    switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+    const ByteView pl{plane, P.G, P.WP, err};
+    for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+        const uint32_t i = c * kChunk + threadIdx.x;
         const bool valid = i < P.n;
-        const uint32_t s = valid ? sv.x : 0u, at = valid ? sv.y : 0u, p = valid ? pw : 0u;
+        uint2 sv = valid ? st[i] : make_uint2(0u, 0u);
+        uint32_t s = sv.x, at = sv.y;
+        const uint32_t p = valid ? pos[i] : 0u;
         if (HC == kHcStart) {
             const bool need = valid && wants_hospital(P, infected(s) ? with_day(s, st_day(s) + 1u) : s);
             if (__syncthreads_or(need) && !hosp_known) {
@@ -352,140 +590,48 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                 hosp_known = true;
             }
         }
-        const uint32_t bin = valid ? decide_agent<HC>(P, pl, rclaim, wsa, st, tgt, lost, slot, i, s, at, p, hw, ww, hour,
-                                                      hod, hosp_first, err)
-                                   : 0u;
-        count_into(sh, valid, bin);
-    }
-    flush_rep(br, sh, row_ptr(ha, hr.row));
-}
-
-#define EPI_DECIDE_PARAMS                                                                                              \
-    const DevParams *__restrict__ Pall, const uint32_t *__restrict__ chunk_rep, uint32_t n_chunks,                    \
-        const uint32_t *__restrict__ pos, uint2 *__restrict__ st, const uint32_t *__restrict__ home,                  \
-        const uint32_t *__restrict__ work, uint32_t *__restrict__ wsa, const uint8_t *__restrict__ plane,             \
-        const uint8_t *__restrict__ danger, uint32_t *__restrict__ claim, uint32_t *__restrict__ tgt,                 \
-        uint32_t *__restrict__ lost, HourArgs ha, int *err
-template <int HC, bool FULL = false>
-__global__ void __launch_bounds__(kThreads) k_decide(EPI_DECIDE_PARAMS) {
-    decide_body<HC, false, FULL>(Pall, chunk_rep, n_chunks, pos, st, home, work, wsa, plane, danger, claim, tgt, lost, ha,
-                                 err);
-}
-template <int HC>
-__global__ void __launch_bounds__(kThreads, kEnsembleMinBlocks) k_decide_ens(EPI_DECIDE_PARAMS) {
-    decide_body<HC, true>(Pall, chunk_rep, n_chunks, pos, st, home, work, wsa, plane, danger, claim, tgt, lost, ha, err);
-}
-#undef EPI_DECIDE_PARAMS
-
-// Resolve the claims of the hour: the lowest index that claimed a cell moves there
-// (the serial resolve of allocation_map.rs:93-102 in index order), others keep their cell.
-// With loss marks (lost != nullptr) a mover wins unless k_decide marked it beaten this
-// hour; without them the winner is read from the claim plane.  Each thread takes S slots a
-// block-width apart (S chosen by the launch-shape autotuner), issuing all their independent
-// loads first; the grid covers every slot once (a grid-stride loop here measured 1 % slower).
-// SPARSE (hours of day 0 and 23, where a few agents in a million move or change class) reads
-// the target words first and the position and loss mark only of the slots that act: about
-// 5 us per launch at 1M agents instead of 9-10 us.
-// REBUILD (a lone world with two plane buffers, the hours of day 7..22): `plane` is the other
-// buffer, all zero, and every agent writes its final cell's byte there (one scattered store
-// per agent instead of a cleared and a set byte per mover; k_decide then names every agent's
-// cell and class in its target word).  The launch then zeroes `spent`, the buffer the hour
-// read (clear_words 16-byte words), which the next rebuilding hour fills: nothing reads it
-// any more.
-constexpr int kCommitSlots = 4;   // default S
-constexpr int kMaxCommitSlots = 8;
-
-template <int S, bool SPARSE = false, bool REBUILD = false>
-__global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
-                                                     uint32_t n_slots, uint32_t* __restrict__ pos,
-                                                     const uint32_t* __restrict__ tgt, uint8_t* __restrict__ plane,
-                                                     uint8_t* __restrict__ danger, uint32_t* __restrict__ claim,
-                                                     const uint32_t* __restrict__ lost, HourArgs ha, uint64_t clear_cells,
-                                                     uint4* __restrict__ spent, uint32_t clear_words) {
-    dep_wait();
-    const HourRow hr = hour_row(ha);
-    const uint32_t* prev = prev_ptr(ha, hr.row);
-    const uint32_t hour = hr.hour;
-    // a single world's parameters once per thread; an ensemble looks each slot's replicate up
-    const bool one = chunk_rep == nullptr;
-    const uint32_t off0 = one ? Pall[0].agent_off : 0u, wp0 = one ? (uint32_t)Pall[0].WP : 0u;
-    const bool halted0 = one && (!Pall[0].active || run_ended(prev, 0u));  // the world does nothing this hour
-    {
-        const uint32_t base = blockIdx.x * (blockDim.x * S) + threadIdx.x;
-        uint32_t t[S], p[S], l[S];
-#pragma unroll
-        for (int k = 0; k < S; ++k) {
-            const uint32_t slot = base + k * blockDim.x;
-            t[k] = slot < n_slots ? tgt[slot] : kNoAction;
-            p[k] = !SPARSE && slot < n_slots ? pos[slot] : 0u;
-            l[k] = !SPARSE && lost && slot < n_slots ? lost[slot] : 0u;
+        if (valid) {
+            const uint32_t hm = home[i], wk = work[i];
+            const Cell cell{unpack_x(p), unpack_y(p)};
+            Draws dr{i, hour, P.key0, P.key1, P.move_key};
+            Cell nc;
+            bool infect = false;
+            if (HC == kHcStart) {
+                nc = routine_start(P, pl, s, hm, cell, hosp_first, dr);
+            } else if (HC == kHcEnd) {
+                nc = routine_end(P, pl, s, hm, cell, dr);
+            } else {
+                nc = perform_movements<HC>(P, pl, steps, s, wsa + i, hm, wk, cell, hour, dr, infect);
+            }
+            const bool moving = nc.x != cell.x || nc.y != cell.y;
+            if (moving) atomicMin(&claim[(size_t)nc.y * P.W + nc.x], i);
+            if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
+            const uint32_t cls0 = cell_class(P, sv.x), cls = cell_class(P, s);
+            tgt[i] = moving || cls != cls0 ? encode_target(nc, cls, cls0) : kNoAction;
+            if (s != sv.x || at != sv.y) st[i] = make_uint2(s, at);
         }
-#pragma unroll(SPARSE ? 1 : S)
-        for (int k = 0; k < S; ++k) {
-            if (t[k] == kNoAction) continue;
-            const uint32_t slot = base + k * blockDim.x;
-            const uint32_t pk = SPARSE ? pos[slot] : p[k];
-            const uint32_t lk = SPARSE ? (lost ? lost[slot] : 0u) : l[k];
-            uint32_t r = 0u, off = off0, WP = wp0;
-            uint64_t plane_off = 0u;
-            bool halted = halted0;
-            if (!one) {
-                r = chunk_rep[slot / kChunk];
-                const DevParams& P = Pall[r];
-                off = P.agent_off;
-                WP = (uint32_t)P.WP;
-                plane_off = P.plane_off;
-                halted = !P.active || run_ended(prev, r);
-            }
-            if (halted) continue;
-            const uint32_t xy = target_xy(t[k]), cls = target_class(t[k]), cls0 = target_old_class(t[k]);
-            bool win = false;
-            if (xy != pk) {
-                if (lost) {
-                    win = lk != hour;
-                } else {
-                    const DevParams& P = Pall[r];
-                    win = claim[P.claim_off + (size_t)unpack_y(xy) * (uint32_t)P.W + unpack_x(xy)] ==
-                          claim_key(hour, slot - off);
-                }
-            }
-            uint8_t* rplane = plane + plane_off;
-            const size_t old_cell = (size_t)(unpack_y(pk) + 1) * WP + (unpack_x(pk) + 1);
-            size_t new_cell = old_cell;
-            if (win) {
-                new_cell = (size_t)(unpack_y(xy) + 1) * WP + (unpack_x(xy) + 1);
-                pos[slot] = xy;
-            }
-            if (REBUILD) {
-                rplane[new_cell] = (uint8_t)cls;
-            } else if (win) {
-                rplane[old_cell] = 0;
-                rplane[new_cell] = (uint8_t)cls;
-            } else if (cls != cls0) {  // a beaten mover whose class held keeps its byte as it is
-                rplane[old_cell] = (uint8_t)cls;
-            }
-            // infectious-neighbour counts follow infectious agents that move or stop or start
-            // being infectious (rare: a few agents per hour)
-            const bool inf0 = cls0 >= 2u, inf1 = cls >= 2u;
-            if (danger && (inf0 || inf1) && (inf0 != inf1 || new_cell != old_cell)) {
-                uint8_t* rd = danger + plane_off;
-                if (inf0) danger_add(rd, old_cell, WP, -1);
-                if (inf1) danger_add(rd, new_cell, WP, +1);
-            }
-        }
+        tally.add(valid, valid ? count_bin(s) : 0u);
     }
-    // the spent buffer of a rebuilding hour (not when the world did nothing: it still holds the plane)
-    if (REBUILD && !halted0)
-        for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < clear_words; w += gridDim.x * blockDim.x)
-            spent[w] = make_uint4(0u, 0u, 0u, 0u);
-    // A new claim window (kClaimWindow hours) opens before the next hour that claims (hour of
-    // day 0 claims next at 7): every claim plane is reset for it.  Only with loss marks, where
-    // this kernel reads no claim.
-    if (clear_cells && lost) {
-        const uint32_t next = hour % 24u == 0u ? hour + 7u : hour + 1u;
-        if (next / kClaimWindow != hour / kClaimWindow)
-            for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < clear_cells; i += (size_t)gridDim.x * blockDim.x)
-                claim[i] = kNoClaim;
+    flush_rep(br, tally, sh, row_ptr(ha, hr.row));
+}
+
+// Winners move, losers stay, plane bytes updated (lowest index wins a cell).
+__global__ void __launch_bounds__(kThreads) k_commit_bytes(const DevParams* __restrict__ Pall, uint32_t n_agents,
+                                                           uint32_t* __restrict__ pos, const uint32_t* __restrict__ tgt,
+                                                           uint8_t* __restrict__ plane, const uint32_t* __restrict__ claim) {
+    const uint32_t WP = (uint32_t)Pall[0].WP, W = (uint32_t)Pall[0].W;
+    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n_agents; i += gridDim.x * kThreads) {
+        const uint32_t t = tgt[i];
+        if (t == kNoAction) continue;
+        const uint32_t p = pos[i], xy = target_xy(t), cls = target_class(t);
+        const size_t old_cell = (size_t)(unpack_y(p) + 1) * WP + (unpack_x(p) + 1);
+        if (xy != p && claim[(size_t)unpack_y(xy) * W + unpack_x(xy)] == i) {
+            pos[i] = xy;
+            plane[old_cell] = 0;
+            plane[(size_t)(unpack_y(xy) + 1) * WP + (unpack_x(xy) + 1)] = (uint8_t)cls;
+        } else if (cls != target_old_class(t)) {
+            plane[old_cell] = (uint8_t)cls;
+        }
     }
 }
 
@@ -526,20 +672,21 @@ __global__ void k_piece_end(const DevParams* __restrict__ Pall, uint32_t R, SegD
     if (advance && threadIdx.x == 0) seg->hour_base += advance;
 }
 
-// Plane bytes of every agent of every replicate (world upload).
+// Occupancy bits and class planes of every agent of every replicate (world upload; the planes
+// start all zero).
 __global__ void k_build_plane(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep, uint32_t n_slots,
-                              const uint32_t* __restrict__ pos, const uint2* __restrict__ st, uint8_t* __restrict__ plane,
-                              uint8_t* __restrict__ danger, int* err) {
+                              const uint32_t* __restrict__ pos, const uint2* __restrict__ st, uint32_t* __restrict__ occ,
+                              uint8_t* __restrict__ cls_plane, uint8_t* __restrict__ danger, int* err) {
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n_slots; slot += gridDim.x * blockDim.x) {
         const DevParams& P = Pall[chunk_rep ? chunk_rep[slot / kChunk] : 0u];
         if (slot - P.agent_off >= P.n) continue;
         const uint32_t p = pos[slot];
         const int32_t x = unpack_x(p), y = unpack_y(p);
         if (x > P.G || y > P.G) { atomicOr(err, 2); continue; }
-        const size_t c = (size_t)(y + 1) * P.WP + (x + 1);
+        const uint32_t X = (uint32_t)x + 1u;
+        atomicOr(&occ[P.occ_off + ((uint32_t)y + 1u) * P.PW + (X >> 5)], 1u << (X & 31u));
         const uint32_t cls = cell_class(P, st[slot].x);
-        plane[P.plane_off + c] = (uint8_t)cls;
-        if (danger && cls >= 2u) danger_add(danger + P.plane_off, c, (uint32_t)P.WP, +1);
+        if (cls >= 2u) class_add(cls_plane + P.plane_off, danger + P.plane_off, (uint32_t)P.WP, p, cls, false);
     }
 }
 
@@ -564,16 +711,24 @@ __global__ void k_vaccinate(uint2* __restrict__ st, uint32_t off, uint32_t n, ui
     }
 }
 
-// Invariants: each agent's cell holds its class.
+// Invariants: each agent's cell is occupied and holds its class byte (bad[0] counts those that
+// do not); bad[1] counts the agents that leave a class byte.  pos and occ are the two buffers
+// of each, par[r] the one that holds replicate r's state.
 __global__ void k_check_agents(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
-                               uint32_t n_slots, const uint32_t* __restrict__ pos, const uint2* __restrict__ st,
-                               const uint8_t* __restrict__ plane, unsigned long long* bad) {
+                               uint32_t n_slots, const uint32_t* __restrict__ pos, const uint32_t* __restrict__ occ,
+                               size_t occ_words, const uint32_t* __restrict__ par, const uint2* __restrict__ st,
+                               const uint8_t* __restrict__ cls_plane, unsigned long long* bad) {
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n_slots; slot += gridDim.x * blockDim.x) {
-        const DevParams& P = Pall[chunk_rep ? chunk_rep[slot / kChunk] : 0u];
+        const uint32_t r = chunk_rep ? chunk_rep[slot / kChunk] : 0u;
+        const DevParams& P = Pall[r];
         if (slot - P.agent_off >= P.n) continue;
-        const uint32_t p = pos[slot];
+        const uint32_t p = pos[(size_t)par[r] * n_slots + slot];
         const int32_t x = unpack_x(p), y = unpack_y(p);
-        if (x > P.G || y > P.G || plane[P.plane_off + (size_t)(y + 1) * P.WP + (x + 1)] != cell_class(P, st[slot].x))
+        const uint32_t cls = cell_class(P, st[slot].x), X = (uint32_t)x + 1u;
+        if (cls >= 2u) atomicAdd(bad + 1, 1ull);
+        if (x > P.G || y > P.G ||
+            !((occ[par[r] * occ_words + P.occ_off + ((uint32_t)y + 1u) * P.PW + (X >> 5)] >> (X & 31u)) & 1u) ||
+            cls_plane[P.plane_off + (size_t)(y + 1) * P.WP + (x + 1)] != (cls >= 2u ? class_amount(cls) : 0u))
             atomicAdd(bad, 1ull);
     }
 }
@@ -588,9 +743,12 @@ __device__ __forceinline__ uint32_t state_letter(uint32_t s) {
     return v == EPI_S ? 0u : v == EPI_E ? 1u : v == EPI_R ? 3u : v == EPI_D ? 4u : 2u;
 }
 
-__global__ void k_state_delta(uint32_t n, const uint32_t* __restrict__ pos, const uint2* __restrict__ st,
-                              uint32_t* __restrict__ prev, uint8_t* __restrict__ codes, uint2* __restrict__ exc,
-                              uint32_t* __restrict__ exc_count) {
+// An hour that did not run (ha are its hour's arguments) leaves prev as it is: the buffer its
+// parity names does not hold the state.
+__global__ void k_state_delta(const DevParams* __restrict__ Pall, HourArgs ha, uint32_t n, const uint32_t* __restrict__ pos,
+                              const uint2* __restrict__ st, uint32_t* __restrict__ prev, uint8_t* __restrict__ codes,
+                              uint2* __restrict__ exc, uint32_t* __restrict__ exc_count) {
+    if (!Pall[0].active || run_ended(prev_ptr(ha, hour_row(ha).row), 0u)) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < n;
     uint32_t code = 0u, p = 0u;
@@ -623,34 +781,52 @@ __global__ void k_state_delta(uint32_t n, const uint32_t* __restrict__ pos, cons
     }
 }
 
-// Cells of [0, G]^2 whose infectious-neighbour count differs from the 3x3 of the plane
+// Cells of [0, G]^2 whose infectious-neighbour count differs from the 3x3 of the class bytes
 // (replicates r = blockIdx.y, blockIdx.y + gridDim.y, ...).
-__global__ void k_check_danger(const DevParams* __restrict__ Pall, uint32_t R, const uint8_t* __restrict__ plane,
+__global__ void k_check_danger(const DevParams* __restrict__ Pall, uint32_t R, const uint8_t* __restrict__ cls_plane,
                                const uint8_t* __restrict__ danger, unsigned long long* bad) {
     unsigned long long b = 0;
     for (uint32_t r = blockIdx.y; r < R; r += gridDim.y) {
         const DevParams& P = Pall[r];
         const uint32_t side = (uint32_t)P.G + 1u, cells = side * side, WP = (uint32_t)P.WP;
-        const uint8_t* pl = plane + P.plane_off;
+        const uint8_t* pl = cls_plane + P.plane_off;
         const uint8_t* dg = danger + P.plane_off;
         for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < cells; q += gridDim.x * blockDim.x) {
             const size_t c = (size_t)(q / side + 1) * WP + (q % side + 1);
-            const uint32_t n = (pl[c - WP - 1] >= 2u) + (pl[c - WP] >= 2u) + (pl[c - WP + 1] >= 2u) +
-                               (pl[c - 1] >= 2u) + (pl[c + 1] >= 2u) + (pl[c + WP - 1] >= 2u) + (pl[c + WP] >= 2u) +
-                               (pl[c + WP + 1] >= 2u);
+            const uint32_t n = (pl[c - WP - 1] != 0u) + (pl[c - WP] != 0u) + (pl[c - WP + 1] != 0u) + (pl[c - 1] != 0u) +
+                               (pl[c + 1] != 0u) + (pl[c + WP - 1] != 0u) + (pl[c + WP] != 0u) + (pl[c + WP + 1] != 0u);
             b += n != dg[c];
         }
     }
     if (b) atomicAdd(bad, b);
 }
 
-// Occupied plane bytes over the whole buffer (borders and slack included: they must be 0).
-__global__ void k_check_plane(size_t plane_bytes, const uint8_t* __restrict__ plane, unsigned long long* occupied) {
-    unsigned long long o = 0;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < plane_bytes; k += stride) o += plane[k] != 0;
-    for (int off = 16; off; off >>= 1) o += __shfl_down_sync(0xFFFFFFFFu, o, off);
-    if ((threadIdx.x & 31) == 0 && o) atomicAdd(occupied, o);
+// Over the whole buffers, borders and slack included: occupied cells of the replicates' current
+// bit planes, set bits of their other buffers (which must be none), and class bytes in use.
+__global__ void k_check_planes(uint32_t R, const DevParams* __restrict__ Pall, const uint32_t* __restrict__ occ,
+                               size_t occ_words, const uint32_t* __restrict__ par, size_t plane_bytes,
+                               const uint8_t* __restrict__ cls_plane, unsigned long long* occupied, unsigned long long* stray,
+                               unsigned long long* classed) {
+    unsigned long long o = 0, x = 0, c = 0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (uint32_t r = 0; r < R; ++r) {
+        const size_t w0 = Pall[r].occ_off, w1 = r + 1 < R ? Pall[r + 1].occ_off : occ_words;
+        for (size_t k = w0 + first; k < w1; k += stride) {
+            o += __popc(occ[par[r] * occ_words + k]);
+            x += __popc(occ[(1u - par[r]) * occ_words + k]);
+        }
+    }
+    for (size_t k = first; k < plane_bytes; k += stride) c += cls_plane[k] != 0;
+    for (int off = 16; off; off >>= 1) {
+        o += __shfl_down_sync(0xFFFFFFFFu, o, off);
+        x += __shfl_down_sync(0xFFFFFFFFu, x, off);
+        c += __shfl_down_sync(0xFFFFFFFFu, c, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (o) atomicAdd(occupied, o);
+        if (x) atomicAdd(stray, x);
+        if (c) atomicAdd(classed, c);
+    }
 }
 
 }  // namespace kern

@@ -1,69 +1,29 @@
 // tick.cuh -- the per-agent hourly rules as sm_103a device code.
 //
 // One thread owns one agent for one hour.  It reads the agent's packed words and the
-// previous-hour occupancy plane (never another agent's record), proposes a target cell,
-// updates its own disease state, and claims the target with atomicMin on the claim plane.
+// previous-hour occupancy (never another agent's record), proposes a target cell, updates its
+// own disease state and claims the target (kernels.cuh).
 // The rules follow engine/src/citizen/mod.rs:215-454,
 // engine/src/state_machine/default_disease_handler.rs:31-103 and
 // engine/src/allocation_map.rs:136-163; random draws are fixed words of per-agent-hour
 // Philox blocks (movement: Philox2x32, counter = agent | which, hour; disease: Philox4x32,
 // counter = agent, hour, block, 0).
 //
-// Moore neighbourhoods are evaluated as bit masks: the byte plane carries a one-cell border,
-// so the 3x3 block around any cell of [0, G]^2 is in bounds; each of its three rows comes in
-// as two aligned 32-bit loads and a funnel shift, and SWAR tests turn the nine bytes into
-// 8-bit masks (bit k = k-th neighbour in NeighborIterator order) of occupied, infectious and
-// high-rate neighbours.  The area and grid filters of get_neighbors_of / is_point_in_grid
-// become a second mask built from six comparisons.  A per-cell count of infectious
-// neighbours (maintained by k_commit) lets a susceptible agent skip the exposure block when
-// it is zero.
+// Moore neighbourhoods are evaluated as bit masks of the 3x3 block (bit 3 (dy + 1) + dx + 1;
+// without the centre that is NeighborIterator order), which a view of the previous hour's
+// world delivers:
+//   BitView   the engine's: one occupancy bit per cell, a class byte per cell that is non-zero
+//             only under an infectious agent, and a per-cell count of infectious neighbours
+//             that lets a susceptible agent skip the exposure block when it is zero;
+//   ByteView  the caller's byte plane of epi_tick_hour_noalloc (0 vacant, 1 occupied, 2 / 3
+//             infectious at the regular / high rate).
+// Both carry a one-cell border, so the 3x3 block around any cell of [0, G]^2 is in bounds.
+// The area and grid filters of get_neighbors_of / is_point_in_grid become a second mask.
 #pragma once
 
 #include "epi_internal.h"
 
 namespace epi {
-
-// Moore offsets in NeighborIterator order (engine/src/geography/point.rs:59), packed as
-// 2-bit (d + 1) fields: k-th neighbour = (x + dx(k), y + dy(k)) with dx(k) + 1 the k-th field
-// of kMooreDx and dy(k) + 1 that of kMooreDy.
-constexpr uint32_t kMooreDx = 0x9224u, kMooreDy = 0xA940u;
-
-struct PlaneView {
-    const uint8_t* __restrict__ cells;  // padded plane: cell (x, y) at (y + 1) * WP + (x + 1)
-    int32_t G, WP;
-    int* err;
-    // Per cell, the number of infectious agents (class >= 2) on its 8 neighbours, same
-    // layout as cells; nullptr when the caller keeps none (the 3x3 is then read instead).
-    const uint8_t* __restrict__ danger;
-    // Cells outside [0, G]^2 are never addressed by construction; if one were, it is
-    // reported through err and treated as occupied instead of being dereferenced.
-    __device__ __forceinline__ bool inside(int32_t x, int32_t y) const {
-        return (uint32_t)x <= (uint32_t)G && (uint32_t)y <= (uint32_t)G;
-    }
-    __device__ __forceinline__ uint32_t at(int32_t x, int32_t y) const {
-        if (!inside(x, y)) {
-            atomicOr(err, 1);
-            return 1u;
-        }
-        return __ldg(cells + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1));
-    }
-    __device__ __forceinline__ bool vacant(int32_t x, int32_t y) const { return at(x, y) == 0u; }
-    __device__ __forceinline__ uint32_t danger_at(int32_t x, int32_t y) const {
-        if (!inside(x, y)) {
-            atomicOr(err, 1);
-            return 0u;
-        }
-        return __ldg(danger + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1));
-    }
-    // Bytes of (x-1, y), (x, y), (x+1, y) in bits 0-7, 8-15, 16-23 (bits 24-31: the next
-    // byte of the row, which no caller reads).
-    __device__ __forceinline__ uint32_t row3(int32_t x, int32_t y) const {
-        const uintptr_t a = (uintptr_t)(cells + (size_t)(y + 1) * (size_t)WP + (size_t)x);
-        const uint32_t* w = (const uint32_t*)(a & ~(uintptr_t)3);
-        const uint32_t lo = __ldg(w), hi = __ldg(w + 1);
-        return __funnelshift_r(lo, hi, (uint32_t)(a & 3u) * 8u);
-    }
-};
 
 // The eight neighbour bytes of a 3x3 block in NeighborIterator order, as two words: bytes of
 // lo = neighbours 0-3 (row 0 bytes 0-2, row 1 byte 0), bytes of hi = neighbours 4-7 (row 1
@@ -80,71 +40,148 @@ __device__ __forceinline__ Nb8 neighbour_bytes(uint32_t r0, uint32_t r1, uint32_
 __device__ __forceinline__ uint32_t pack4(uint32_t f) { return (f * 0x01020408u) >> 24; }
 __device__ __forceinline__ uint32_t pack8(uint32_t flo, uint32_t fhi) { return pack4(flo) | (pack4(fhi) << 4); }
 
-// The three rows of the 3x3 block around (x, y); a cell outside [0, G]^2 reads as a
-// block of occupied, non-infectious cells (and is reported).
+// 8 neighbours (NeighborIterator order) <-> the 9 cells of the block (centre bit 4 clear).
+constexpr uint32_t kNeighbours9 = 0x1EFu;
+__host__ __device__ constexpr uint32_t block9(uint32_t m8) { return (m8 & 0xFu) | ((m8 & 0xF0u) << 1); }
+__host__ __device__ constexpr uint32_t neighbours8(uint32_t m9) { return (m9 & 0xFu) | ((m9 >> 1) & 0xF0u); }
+
+// Bytes of (x-1, y), (x, y), (x+1, y) of a bordered byte plane (cell (x, y) at
+// (y + 1) * WP + x + 1) in bits 0-7, 8-15, 16-23 (bits 24-31: the next byte of the row, which
+// no caller reads): two aligned 32-bit loads and a funnel shift.
+__device__ __forceinline__ uint32_t byte_row3(const uint8_t* plane, int32_t WP, int32_t x, int32_t y) {
+    const uintptr_t a = (uintptr_t)(plane + (size_t)(y + 1) * (size_t)WP + (size_t)x);
+    const uint32_t* w = (const uint32_t*)(a & ~(uintptr_t)3);
+    const uint32_t lo = __ldg(w), hi = __ldg(w + 1);
+    return __funnelshift_r(lo, hi, (uint32_t)(a & 3u) * 8u);
+}
+
+// Three rows of the 3x3 block around a cell, in a view's own form.
 struct Rows3 {
     uint32_t r0, r1, r2;
 };
-__device__ __forceinline__ Rows3 rows_around(const PlaneView& pl, int32_t x, int32_t y) {
-    if (!pl.inside(x, y)) {
-        atomicOr(pl.err, 1);
-        return Rows3{0x010101u, 0x010101u, 0x010101u};
+// Infectious and high-rate neighbours of a cell, 8-bit masks in NeighborIterator order.
+struct InfMasks {
+    uint32_t inf, high;
+};
+
+// Cells outside [0, G]^2 are never addressed by construction; if one were, it is reported
+// through err and treated as occupied (and not infectious) instead of being dereferenced.
+__device__ __forceinline__ bool in_plane(int32_t G, int* err, int32_t x, int32_t y) {
+    if ((uint32_t)x <= (uint32_t)G && (uint32_t)y <= (uint32_t)G) return true;
+    atomicOr(err, 1);
+    return false;
+}
+
+// A caller's byte plane: bytes 0..3, occupied <=> bit0|bit1, infectious <=> bit1, high rate
+// <=> bit0&bit1.
+struct ByteView {
+    const uint8_t* __restrict__ cells;
+    int32_t G, WP;
+    int* err;
+    __device__ __forceinline__ bool inside(int32_t x, int32_t y) const { return in_plane(G, err, x, y); }
+    __device__ __forceinline__ bool vacant(int32_t x, int32_t y) const {
+        return inside(x, y) && __ldg(cells + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1)) == 0u;
     }
-    return Rows3{pl.row3(x, y - 1), pl.row3(x, y), pl.row3(x, y + 1)};
-}
+    __device__ __forceinline__ uint32_t row(int32_t x, int32_t y) const { return byte_row3(cells, WP, x, y); }
+    __device__ __forceinline__ Rows3 rows(int32_t x, int32_t y) const {
+        if (!inside(x, y)) return Rows3{0x010101u, 0x010101u, 0x010101u};
+        return Rows3{row(x, y - 1), row(x, y), row(x, y + 1)};
+    }
+    static __device__ __forceinline__ bool centre_vacant(uint32_t r1) { return ((r1 >> 8) & 0xFFu) == 0u; }
+    static __device__ __forceinline__ uint32_t occupied(const Rows3& r) {
+        const Nb8 b = neighbour_bytes(r.r0, r.r1, r.r2);
+        const uint32_t m = 0x01010101u;
+        return block9(pack8((b.lo | (b.lo >> 1)) & m, (b.hi | (b.hi >> 1)) & m));
+    }
+    // no infectious neighbour for sure (never known without reading the block)
+    __device__ __forceinline__ bool safe(int32_t, int32_t) const { return false; }
+    __device__ __forceinline__ InfMasks infectious(int32_t x, int32_t y) const {
+        const Rows3 r = rows(x, y);
+        const Nb8 b = neighbour_bytes(r.r0, r.r1, r.r2);
+        const uint32_t m = 0x01010101u;
+        return InfMasks{pack8((b.lo >> 1) & m, (b.hi >> 1) & m), pack8(b.lo & (b.lo >> 1) & m, b.hi & (b.hi >> 1) & m)};
+    }
+};
 
-// Plane bytes are 0..3: occupied <=> bit0|bit1, infectious <=> bit1, high rate <=> bit0&bit1.
-// Masks are 8 bits in NeighborIterator order.
-__device__ __forceinline__ uint32_t occupied_mask(const Rows3& r) {
-    const Nb8 b = neighbour_bytes(r.r0, r.r1, r.r2);
-    const uint32_t m = 0x01010101u;
-    return pack8((b.lo | (b.lo >> 1)) & m, (b.hi | (b.hi >> 1)) & m);
-}
-// Any infectious byte among the nine (the centre is vacant or the agent's own, never infectious).
-__device__ __forceinline__ bool any_infectious(const Rows3& r) { return ((r.r0 | r.r1 | r.r2) & 0x020202u) != 0u; }
-__device__ __forceinline__ uint32_t infectious_mask(const Rows3& r) {
-    const Nb8 b = neighbour_bytes(r.r0, r.r1, r.r2);
-    const uint32_t m = 0x01010101u;
-    return pack8((b.lo >> 1) & m, (b.hi >> 1) & m);
-}
-__device__ __forceinline__ uint32_t high_mask(const Rows3& r) {
-    const Nb8 b = neighbour_bytes(r.r0, r.r1, r.r2);
-    const uint32_t m = 0x01010101u;
-    return pack8(b.lo & (b.lo >> 1) & m, b.hi & (b.hi >> 1) & m);
-}
+// The engine's planes.  occ: one bit per cell, cell (x, y) bit (x + 1) & 31 of word
+// (y + 1) * PW + ((x + 1) >> 5) -- a 3x3 block is three words (six where it straddles one),
+// and the whole plane of a 2,500 grid is 0.8 MB where a byte plane took 6.3 MB, so the blocks
+// that sweep the agents find it in L1 far more often.  cls: class bytes, bit 0 of a byte an
+// infectious agent at the regular rate, bit 4 one at the high rate.  danger: infectious agents
+// among the 8 neighbours.
+struct BitView {
+    const uint32_t* __restrict__ occ;
+    const uint8_t* __restrict__ cls;
+    const uint8_t* __restrict__ danger;
+    int32_t G, WP;
+    uint32_t PW;
+    int* err;
+    __device__ __forceinline__ bool inside(int32_t x, int32_t y) const { return in_plane(G, err, x, y); }
+    __device__ __forceinline__ bool vacant(int32_t x, int32_t y) const {
+        if (!inside(x, y)) return false;
+        const uint32_t X = (uint32_t)x + 1u;
+        return ((__ldg(occ + ((uint32_t)y + 1u) * PW + (X >> 5)) >> (X & 31u)) & 1u) == 0u;
+    }
+    // bits of (x-1, y), (x, y), (x+1, y) in bits 0-2 (higher bits: later cells)
+    __device__ __forceinline__ uint32_t row(int32_t x, int32_t y) const {
+        const uint32_t* w = occ + ((uint32_t)y + 1u) * PW + ((uint32_t)x >> 5);
+        const uint32_t sh = (uint32_t)x & 31u;
+        const uint32_t lo = __ldg(w), hi = sh > 29u ? __ldg(w + 1) : 0u;
+        return __funnelshift_r(lo, hi, sh);
+    }
+    __device__ __forceinline__ Rows3 rows(int32_t x, int32_t y) const {
+        if (!inside(x, y)) return Rows3{7u, 7u, 7u};
+        return Rows3{row(x, y - 1), row(x, y), row(x, y + 1)};
+    }
+    static __device__ __forceinline__ bool centre_vacant(uint32_t r1) { return (r1 & 2u) == 0u; }
+    static __device__ __forceinline__ uint32_t occupied(const Rows3& r) {
+        return (r.r0 & 7u) | ((r.r1 & 7u) << 3) | ((r.r2 & 7u) << 6);
+    }
+    __device__ __forceinline__ bool safe(int32_t x, int32_t y) const {
+        return inside(x, y) && __ldg(danger + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1)) == 0u;
+    }
+    __device__ __forceinline__ InfMasks infectious(int32_t x, int32_t y) const {
+        if (!inside(x, y)) return InfMasks{0u, 0u};
+        const Nb8 b = neighbour_bytes(byte_row3(cls, WP, x, y - 1), byte_row3(cls, WP, x, y), byte_row3(cls, WP, x, y + 1));
+        const uint32_t m = 0x01010101u;
+        return InfMasks{pack8((b.lo | (b.lo >> 4)) & m, (b.hi | (b.hi >> 4)) & m), pack8((b.lo >> 4) & m, (b.hi >> 4) & m)};
+    }
+};
 
-// Neighbours of (x, y) inside area a and the grid (Area::get_neighbors_of filtered by
-// is_point_in_grid), as a mask in NeighborIterator order: three column and three row tests
-// (each one unsigned range compare) combined row by row.
-__device__ __forceinline__ uint32_t valid_neighbours(const Rect& a, int32_t G, int32_t x, int32_t y) {
+// Cells of the block around (x, y) inside area a and the grid, for (x, y) in the area or on the
+// plane's edge (Area::get_neighbors_of filtered by is_point_in_grid): three columns and three
+// rows, each a run of bits cut off on either side by as many cells as lie beyond the bounds
+// (shifts of 3 or more clear the run).
+__device__ __forceinline__ uint32_t valid_block(const Rect& a, int32_t G, int32_t x, int32_t y) {
     const int32_t lx = max(a.x0, 0), hx = min(a.x1, G - 1), ly = max(a.y0, 0), hy = min(a.y1, G - 1);
-    if (hx < lx || hy < ly) return 0u;
-    const uint32_t wx = (uint32_t)(hx - lx), wy = (uint32_t)(hy - ly);
-    const uint32_t dx = (uint32_t)(x - 1 - lx), dy = (uint32_t)(y - 1 - ly);
-    const uint32_t C = (uint32_t)(dx <= wx) | ((uint32_t)(dx + 1u <= wx) << 1) | ((uint32_t)(dx + 2u <= wx) << 2);
-    const uint32_t top = (dy <= wy) ? C : 0u, bot = (dy + 2u <= wy) ? C : 0u;
-    const uint32_t mid = (dy + 1u <= wy) ? ((C & 1u) | ((C >> 1) & 2u)) : 0u;
-    return top | (mid << 3) | (bot << 5);
+    const uint32_t cl = (uint32_t)max(lx - x + 1, 0), cr = (uint32_t)max(x + 1 - hx, 0);
+    const uint32_t rl = (uint32_t)max(ly - y + 1, 0), rr = (uint32_t)max(y + 1 - hy, 0);
+    const uint32_t cols = __funnelshift_lc(0u, 7u, cl) & __funnelshift_rc(7u, 0u, cr) & 7u;
+    const uint32_t rows = __funnelshift_lc(0u, 0x1FFu, 3u * rl) & __funnelshift_rc(0x1FFu, 0u, 3u * rr);
+    return (cols * 0x49u) & rows;
 }
 
-// Moore step of the j-th set bit of an 8-bit neighbour mask, as (dx + 1) | (dy + 1) << 2,
-// for every mask and j < popc(mask): one table read instead of the bit search.
-struct StepTable {
-    uint8_t v[256][8];
+// Moore step of the j-th set bit of a 9-cell mask, as (dx + 1) | (dy + 1) << 2, for every mask
+// and j < popc(mask): one table read instead of the bit search.  The kernels keep a copy in
+// shared memory, where lanes with different masks cost bank conflicts instead of cache lines.
+struct __align__(16) StepTable {
+    uint8_t v[512][8];
 };
 constexpr StepTable make_step_table() {
     StepTable t{};
-    for (int m = 0; m < 256; ++m) {
+    for (int m = 0; m < 512; ++m) {
         int j = 0;
-        for (int k = 0; k < 8; ++k)
-            if ((m >> k) & 1) {
-                const int dx = (int)((kMooreDx >> (2 * k)) & 3u), dy = (int)((kMooreDy >> (2 * k)) & 3u);
-                t.v[m][j++] = (uint8_t)(dx | (dy << 2));
-            }
+        for (int k = 0; k < 9; ++k)
+            if (k != 4 && ((m >> k) & 1)) t.v[m][j++] = (uint8_t)((k % 3) | ((k / 3) << 2));
     }
     return t;
 }
 __device__ const StepTable kStepTable = make_step_table();
+// The block's copy (the caller synchronises before it is read).
+__device__ __forceinline__ void stage_steps(StepTable& sh) {
+    const uint4* src = reinterpret_cast<const uint4*>(&kStepTable);
+    for (uint32_t k = threadIdx.x; k < sizeof(StepTable) / 16; k += blockDim.x) reinterpret_cast<uint4*>(&sh)[k] = __ldg(src + k);
+}
 
 // Lazily materialised Philox blocks of one agent-hour: m(0), m(1) the random-point words
 // and m(2) the choice word (Philox2x32 each), d(), d2() the disease blocks (Philox4x32).
@@ -215,96 +252,53 @@ __device__ __forceinline__ uint32_t cell_class(const DevParams& P, uint32_t s) {
     return 1u + rate_class(P.reg_start, P.high_start, P.last_day, d);
 }
 
-// Citizen::move_agent_from, citizen/mod.rs:415-432: uniform choice among the vacant
-// neighbours (of the cell, or of a random point of the area when outside it).
-__device__ __forceinline__ Cell move_agent_from(const PlaneView& pl, uint32_t s, const Rect& cur, Cell cell, Draws& dr) {
-    if (!can_move(s)) return cell;
+// A lane's move: act false keeps the cell.  jump is Citizen::goto_area of an agent that works
+// (citizen/mod.rs:367-395: a random point of the target area, kept when vacant), otherwise
+// Citizen::move_agent_from over the current area (citizen/mod.rs:415-432: uniform choice among
+// the vacant neighbours of the cell, or of a random point of the area when outside it); `area`
+// is the one or the other's.  Both are one code path: the centre is the lane's cell or its
+// random point, the row through it is read in the same pass (a jump tests the centre bit), and
+// walkers also read the rows above and below.  JUMPS false: no lane of the hour jumps but
+// hospital staff (rarely).
+template <bool JUMPS, class V>
+__device__ __forceinline__ Cell move_lane(const V& pl, const StepTable& steps, bool act, bool jump, const Rect& area, Cell cell,
+                                          Draws& dr) {
+    if (JUMPS) dr.prime(jump);
+    if (!act) return cell;
     Cell c = cell;
-    if (!rect_has(cur, cell.x, cell.y)) c = random_point(cur, dr.m(0), dr.m(1));
-    const Rows3 rows = rows_around(pl, c.x, c.y);
+    if (jump || !rect_has(area, cell.x, cell.y)) c = random_point(area, dr.m(0), dr.m(1));
+    if (!pl.inside(c.x, c.y)) return cell;  // reads as occupied (and is reported)
+    const uint32_t r1 = pl.row(c.x, c.y);
+    if (JUMPS && jump) return V::centre_vacant(r1) ? c : cell;
+    const Rows3 rows{pl.row(c.x, c.y - 1), r1, pl.row(c.x, c.y + 1)};
     // The choice word is drawn before the rows are used, so that its Philox rounds run while
     // the row loads are in flight (it is needed unless every neighbour is taken).
     const uint32_t u = dr.m(2);
-    const uint32_t cand = valid_neighbours(cur, pl.G, c.x, c.y) & ~occupied_mask(rows);
+    if (!JUMPS && jump) return V::centre_vacant(r1) ? c : cell;
+    const uint32_t cand = valid_block(area, pl.G, c.x, c.y) & ~V::occupied(rows) & kNeighbours9;
     if (!cand) return cell;
-    const uint32_t j = uniform_index(u, (uint32_t)__popc(cand));
-    const uint32_t e = __ldg(&kStepTable.v[cand][j]);
+    const uint32_t e = steps.v[cand][uniform_index(u, (uint32_t)__popc(cand))];
     return Cell{c.x + (int32_t)(e & 3u) - 1, c.y + (int32_t)(e >> 2) - 1};  // vacant by construction: move_agent keeps it
-}
-
-// Citizen::goto_area, citizen/mod.rs:367-395
-__device__ __forceinline__ Cell goto_area(const PlaneView& pl, uint32_t s, const Rect& cur, const Rect& target,
-                                          uint32_t home, uint32_t work, Cell cell, Draws& dr) {
-    const uint32_t ws = st_ws(s), v = s & kStateMask;
-    bool override_movement = false;
-    if (ws == EPI_WS_NORMAL || ws == EPI_WS_ESSENTIAL) {
-        if (rect_has(office_rect(work), cell.x, cell.y) && rect_eq(target, home_rect(home)) &&
-            (v == EPI_I_MILD || v == EPI_I_SEVERE))
-            override_movement = true;
-    }
-    if (!can_move(s) && !override_movement) return cell;
-    if (ws != EPI_WS_NA) {
-        Cell q = random_point(target, dr.m(0), dr.m(1));
-        return pl.vacant(q.x, q.y) ? q : cell;
-    }
-    return move_agent_from(pl, s, cur, cell, dr);
-}
-
-// One lane of an hour whose arms mix a jump and a walk, as one code path: jump lanes take
-// goto_area of a worker (Normal or Essential: a random point of the target area, kept when
-// vacant), walk lanes move_agent_from over the current area.  Both read the plane row through
-// their centre cell in the same pass (a jump tests its centre byte); walkers also read the
-// rows above and below.  Same words and outcomes as the two calls, without a warp running the
-// two arms' loads one after the other.  Used for hour 8 (workers to the office, the others a
-// walk): its k_decide went from 25.9 to 23.6 us at 1M agents.  In hours 7, 16 and 17 the two
-// plain calls were measured as fast.
-__device__ __forceinline__ Cell jump_or_walk(const PlaneView& pl, uint32_t s, bool jump, const Rect& cur,
-                                             const Rect& target, uint32_t home, uint32_t work, Cell cell, Draws& dr) {
-    bool act = can_move(s);
-    if (jump && !act) {  // goto_area's symptomatic override of a worker going home from the office
-        const uint32_t v = s & kStateMask;
-        act = rect_has(office_rect(work), cell.x, cell.y) && rect_eq(target, home_rect(home)) &&
-              (v == EPI_I_MILD || v == EPI_I_SEVERE);
-    }
-    if (!act) return cell;
-    Cell c = cell;
-    if (jump || !rect_has(cur, cell.x, cell.y)) c = random_point(jump ? target : cur, dr.m(0), dr.m(1));
-    if (!pl.inside(c.x, c.y)) {  // reads as occupied (and is reported), as rows_around and vacant do
-        atomicOr(pl.err, 1);
-        return cell;
-    }
-    const uint32_t r1 = pl.row3(c.x, c.y);
-    uint32_t r0 = 0u, r2 = 0u;
-    if (!jump) {
-        r0 = pl.row3(c.x, c.y - 1);
-        r2 = pl.row3(c.x, c.y + 1);
-    }
-    if (jump) return ((r1 >> 8) & 0xFFu) == 0u ? c : cell;
-    const uint32_t u = dr.m(2);
-    const uint32_t cand = valid_neighbours(cur, pl.G, c.x, c.y) & ~occupied_mask(Rows3{r0, r1, r2});
-    if (!cand) return cell;
-    const uint32_t j = uniform_index(u, (uint32_t)__popc(cand));
-    const uint32_t e = __ldg(&kStepTable.v[cand][j]);
-    return Cell{c.x + (int32_t)(e & 3u) - 1, c.y + (int32_t)(e >> 2) - 1};
 }
 
 // DiseaseStateMachine::next with the default DiseaseHandler (ddh:41-86) for the hour's
 // proposed cell; at is the Exposed/Pre at_hour word.
 // (The agent's current area, needed only when an infectious neighbour exists, is decoded from
 // its code and home / work corners here rather than by the caller.)
-__device__ __forceinline__ void infection_dynamics(const DevParams& P, const PlaneView& pl, uint32_t& s, uint32_t& at,
+template <class V>
+__device__ __forceinline__ void infection_dynamics(const DevParams& P, const V& pl, uint32_t& s, uint32_t& at,
                                                    uint32_t home, uint32_t work, Cell cell, uint32_t hour, Draws& dr) {
     const uint32_t v = s & kStateMask;
     if (v == EPI_S) {
         if (s & (kWq | kVacc)) return;
         // no infectious neighbour: no draw can succeed (the centre is vacant or the agent's own)
-        if (pl.danger && pl.danger_at(cell.x, cell.y) == 0u) return;
-        const Rows3 rows = rows_around(pl, cell.x, cell.y);
-        if (!any_infectious(rows)) return;
+        if (pl.safe(cell.x, cell.y)) return;
+        const InfMasks masks = pl.infectious(cell.x, cell.y);
+        if (!masks.inf) return;
         const Rect cur = area_rect(P, st_area(s), home, work);
-        const uint32_t cand = valid_neighbours(cur, pl.G, cell.x, cell.y) & infectious_mask(rows);
+        const uint32_t cand = neighbours8(valid_block(cur, pl.G, cell.x, cell.y)) & masks.inf;
         if (!cand) return;
-        const uint32_t high = high_mask(rows);
+        const uint32_t high = masks.high;
         const uint64_t thr_reg = P.thr_rate[1], thr_high = P.thr_rate[2];
         // neighbours in NeighborIterator order; the first successful Bernoulli exposes
 #pragma unroll
@@ -356,94 +350,74 @@ __host__ __device__ constexpr int hour_class(uint32_t hod) {
          : kHcMove;
 }
 
-// The HospitalStaff arm of Citizen::perform_movements (citizen/mod.rs:292-328).  Returns
-// false when the hour ends before the infection update (the two early returns).
-__device__ __forceinline__ bool staff_movements(const DevParams& P, const PlaneView& pl, uint32_t& s, uint32_t& wsa,
-                                                uint32_t home, uint32_t work, Cell cell, Cell& nc, uint32_t hod,
-                                                uint32_t hour, Draws& dr) {
-    const Rect cur = area_rect(P, st_area(s), home, work);
-    const uint32_t since = hour >= wsa ? hour - wsa : 0u;  // saturating_sub
-    if (since == 24u * 14u) {
-        s |= kWq;
-        return false;
-    }
-    if (since == 24u * 14u * 2u) {
-        nc = goto_area(pl, s, cur, home_rect(home), home, work, cell, dr);
-        s = with_area(s, kHome);
-        wsa = hour + 24u * 14u;
-        return false;
-    }
-    if (hod == 8u) {
-        const Rect hosp = P.area[P.hosp_code];
-        if (!rect_eq(cur, hosp) && wsa <= hour) {
-            nc = goto_area(pl, s, cur, hosp, home, work, cell, dr);
-            s = with_area(s, P.hosp_code);
-            wsa = hour;
-        }
-        s &= ~kWq;
-    } else if (hod == 16u) {
-        s |= kWq;
-    } else if (!(s & kWq) && can_move(s)) {
-        nc = move_agent_from(pl, s, cur, cell, dr);
-    }
-    return true;
-}
-
 // Citizen::perform_movements, citizen/mod.rs:257-349, for the movement classes (hours 7..22):
-// the work-status arms (Normal|Essential, HospitalStaff, NA) at hour class HC.  Returns the
-// proposed cell; infect is cleared when the hour ends before the infection update of
+// the work-status arms (Normal|Essential, HospitalStaff, NA) at hour class HC.  Each arm is a
+// jump, a walk or nothing (a non-worker's goto_area is move_agent_from over its current area),
+// so the arms only choose and one move_lane serves them all.  Returns the proposed cell;
+// infect is cleared when the hour ends before the infection update of
 // DiseaseStateMachine::next, which the caller runs on the proposed cell otherwise.
-template <int HC>
-__device__ __forceinline__ Cell perform_movements(const DevParams& P, const PlaneView& pl, uint32_t& s, uint32_t& wsa,
-                                                  uint32_t home, uint32_t work, Cell cell, uint32_t hod, uint32_t hour,
+template <int HC, class V>
+__device__ __forceinline__ Cell perform_movements(const DevParams& P, const V& pl, const StepTable& steps, uint32_t& s,
+                                                  uint32_t* wsa, uint32_t home, uint32_t work, Cell cell, uint32_t hour,
                                                   Draws& dr, bool& infect) {
     const uint32_t ws = st_ws(s);
-    Cell nc = cell;
+    Rect area = area_rect(P, st_area(s), home, work);
+    bool act = can_move(s), jump = false;
     infect = true;
-    if (ws == EPI_WS_HOSPITAL_STAFF) {
-        infect = staff_movements(P, pl, s, wsa, home, work, cell, nc, hod, hour, dr);
-    } else {
-        const Rect cur = area_rect(P, st_area(s), home, work);
-        const bool worker = ws != EPI_WS_NA;  // Normal or Essential here
-        // The arms of each class, as goto_area / move_agent_from calls of the reference.  A
-        // non-worker's goto_area is move_agent_from over its current area (work status NA), so
-        // a class's arms are a jump of some workers and a walk of everyone else (at noon, a
-        // walk of everyone: one call).  Where lanes differ, each computes its one Philox block
-        // before the branch, the point block for a jump and the choice block for a walk, so a
-        // warp runs the rounds once.
-        if (HC == kHcMove) {
-            nc = move_agent_from(pl, s, cur, cell, dr);
-        } else if (HC == kHcTransport) {
-            // worker with public transport: goto_area(transport); others: move_agent_from
-            const bool jump = worker && (s & kPt);
-            dr.prime(jump);
-            if (jump) {
-                nc = goto_area(pl, s, cur, P.area[kTransport], home, work, cell, dr);
-                s = with_area(s, kTransport);
-            } else {
-                nc = move_agent_from(pl, s, cur, cell, dr);
-            }
+    if (ws == EPI_WS_HOSPITAL_STAFF) {  // citizen/mod.rs:292-328; wsa: its work_start_at
+        const uint32_t w = *wsa, since = hour >= w ? hour - w : 0u;  // saturating_sub
+        if (since == 24u * 14u) {
+            s |= kWq;
+            act = infect = false;
+        } else if (since == 24u * 14u * 2u) {
+            jump = true;
+            area = home_rect(home);
+            s = with_area(s, kHome);
+            *wsa = hour + 24u * 14u;
+            infect = false;
         } else if (HC == kHcWork) {
-            // worker: goto_area(office); non-worker: goto_area(housing), a walk
-            dr.prime(worker);
-            nc = jump_or_walk(pl, s, worker, cur, office_rect(work), home, work, cell, dr);
+            jump = !rect_eq(area, P.area[P.hosp_code]) && w <= hour;
+            act = act && jump;
+            if (jump) {
+                area = P.area[P.hosp_code];
+                s = with_area(s, P.hosp_code);
+                *wsa = hour;
+            }
+            s &= ~kWq;
+        } else if (HC == kHcHome) {
+            s |= kWq;
+            act = false;
+        } else {
+            act = act && !(s & kWq);
+        }
+    } else {
+        const bool worker = ws != EPI_WS_NA;  // Normal or Essential here
+        if (HC == kHcTransport) {  // a worker with public transport: goto_area(transport)
+            jump = worker && (s & kPt);
+            if (jump) {
+                area = P.area[kTransport];
+                s = with_area(s, kTransport);
+            }
+        } else if (HC == kHcWork) {  // a worker: goto_area(office); the others: goto_area(housing), a walk
+            jump = worker;
+            if (jump) area = office_rect(work);
             s = with_area(s, worker ? kWork : kHousing);
-        } else if (HC == kHcNoon) {
-            // worker: move_agent_from; non-worker: goto_area(home), a walk
-            nc = move_agent_from(pl, s, cur, cell, dr);
+        } else if (HC == kHcNoon) {  // a worker walks; the others: goto_area(home), a walk
             if (!worker) s = with_area(s, kHome);
-        } else {  // kHcHome
-            // worker: goto_area(home); non-worker: move_agent_from
-            dr.prime(worker);
-            if (worker) {
-                nc = goto_area(pl, s, cur, home_rect(home), home, work, cell, dr);
+        } else if (HC == kHcHome) {  // a worker: goto_area(home)
+            jump = worker;
+            if (jump) {
+                area = home_rect(home);
                 s = with_area(s, kHome);
-            } else {
-                nc = move_agent_from(pl, s, cur, cell, dr);
             }
         }
+        if (jump && !act) {  // goto_area's symptomatic override of a worker going home from the office
+            const uint32_t v = s & kStateMask;
+            act = (v == EPI_I_MILD || v == EPI_I_SEVERE) && rect_has(office_rect(work), cell.x, cell.y) &&
+                  rect_eq(area, home_rect(home));
+        }
     }
-    return nc;
+    return move_lane<HC == kHcTransport || HC == kHcWork || HC == kHcHome>(pl, steps, act, jump, area, cell, dr);
 }
 
 // Hour 0 of the day: increment_infection_day, then Citizen::hospitalize
@@ -455,7 +429,8 @@ __device__ __forceinline__ bool wants_hospital(const DevParams& P, uint32_t s) {
     return (P.hosp_if_class >> rate_class(P.reg_start, P.high_start, P.last_day, d)) & 1u;
 }
 
-__device__ __forceinline__ Cell routine_start(const DevParams& P, const PlaneView& pl, uint32_t& s, uint32_t home,
+template <class V>
+__device__ __forceinline__ Cell routine_start(const DevParams& P, const V& pl, uint32_t& s, uint32_t home,
                                               Cell cell, uint32_t hosp_first, Draws& dr) {
     if (infected(s)) s = with_day(s, st_day(s) + 1u);
     if (!wants_hospital(P, s)) return cell;
@@ -468,7 +443,8 @@ __device__ __forceinline__ Cell routine_start(const DevParams& P, const PlaneVie
 }
 
 // Hour 23: Citizen::deceased with on_routine_end (citizen/mod.rs:397-413, ddh:88-102).
-__device__ __forceinline__ Cell routine_end(const DevParams& P, const PlaneView& pl, uint32_t& s, uint32_t home,
+template <class V>
+__device__ __forceinline__ Cell routine_end(const DevParams& P, const V& pl, uint32_t& s, uint32_t home,
                                             Cell cell, Draws& dr) {
     const uint32_t v = s & kStateMask, day = st_day(s);
     if (v == EPI_I_ASYM && day == 9u) s = with_state(s, EPI_R);          // ASYMPTOMATIC_LAST_DAY
@@ -504,18 +480,27 @@ __device__ __forceinline__ uint32_t target_xy(uint32_t t) { return t & 0x3FFF3FF
 __device__ __forceinline__ uint32_t target_class(uint32_t t) { return ((t >> 15) & 1u) | ((t >> 30) & 2u); }
 __device__ __forceinline__ uint32_t target_old_class(uint32_t t) { return ((t >> 14) & 1u) | ((t >> 29) & 2u); }
 
-// Add delta (+1 / -1) to the infectious-neighbour count of the 8 cells around the padded
-// plane index c (atomically, on the 32-bit words holding the bytes; counts stay in 0..8).
-__device__ __forceinline__ void danger_add(uint8_t* danger, size_t c, uint32_t WP, int delta) {
+// Class planes.  An infectious agent of plane class c (2 regular, 3 high rate) on a cell adds
+// one to its field of the cell's class byte and one to the infectious-neighbour count of the
+// 8 cells around; taking it away subtracts the same.  The updates of an hour only add up
+// (atomically, on the 32-bit words holding the bytes), so their order does not matter and a
+// proposal may be entered before its claim is settled and taken back after: at the end of the
+// hour class fields are 0 or 1 and counts 0..8.
+__device__ __forceinline__ void byte_add(uint8_t* plane, size_t c, uint32_t amount, bool minus) {
+    const uintptr_t a = (uintptr_t)(plane + c);
+    uint32_t* w = (uint32_t*)(a & ~(uintptr_t)3);
+    const uint32_t v = amount << ((a & 3u) * 8u);
+    atomicAdd(w, minus ? 0u - v : v);
+}
+__device__ __forceinline__ uint32_t class_amount(uint32_t cls) { return cls == 2u ? 0x01u : 0x10u; }
+// The agent of class cls >= 2 on cell (x, y) enters (minus false) or leaves the class planes.
+__device__ __forceinline__ void class_add(uint8_t* cls_plane, uint8_t* danger, uint32_t WP, uint32_t cell_xy, uint32_t cls,
+                                          bool minus) {
+    const size_t c = (size_t)(unpack_y(cell_xy) + 1) * WP + (size_t)(unpack_x(cell_xy) + 1);
+    byte_add(cls_plane, c, class_amount(cls), minus);
     const size_t nb[8] = {c - WP - 1, c - WP, c - WP + 1, c - 1, c + 1, c + WP - 1, c + WP, c + WP + 1};
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uintptr_t a = (uintptr_t)(danger + nb[k]);
-        uint32_t* w = (uint32_t*)(a & ~(uintptr_t)3);
-        const uint32_t one = 1u << ((a & 3u) * 8u);
-        if (delta > 0) atomicAdd(w, one);
-        else atomicSub(w, one);
-    }
+    for (int k = 0; k < 8; ++k) byte_add(danger, nb[k], 1u, minus);
 }
 
 }  // namespace epi

@@ -308,8 +308,9 @@ int epi_engine_restore_state(epi_engine* h);
 /* Number of engine kernels launched so far on this handle (graph nodes included). */
 int epi_engine_kernels_launched(const epi_engine* h, uint64_t* out);
 
-/* Launch shape of the tick kernels: the k_decide / k_sleep grid and the agents per k_commit
- * thread (its grid covers every agent once).  Results never depend on it. */
+/* Launch shape of the tick kernels: the grid of k_decide, k_commit and k_sleep.  commit_slots is
+ * checked, kept and reported as before, but k_commit takes its work from k_decide's lists and
+ * no longer has agents per thread.  Results never depend on the shape. */
 typedef struct {
     uint32_t decide_blocks;  /* 1 .. number of 256-agent chunks */
     uint32_t commit_slots;   /* 1 .. 8 */
@@ -329,7 +330,7 @@ int epi_engine_state_stream_close(epi_engine* h);
 
 /* Autotuner (no reference counterpart): time hours 1..hours (<= 168) of the current world
  * under each candidate shape -- k_decide grid = three quarters of the resident blocks, the
- * resident blocks, twice that, or one chunk per block; 1, 2 or 4 agents per k_commit thread --
+ * resident blocks, twice that, or one chunk per block --
  * from the same starting state, keep the fastest and restore the state.  Call it before simulating; it replaces the checkpoint of
  * epi_engine_save_state. */
 int epi_engine_autotune(epi_engine* h, uint32_t hours, epi_launch_shape* chosen);
