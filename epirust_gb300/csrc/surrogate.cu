@@ -6,14 +6,16 @@
 // are zero and stay zero: their inputs are zero, so are their gradients and Adam updates.
 // Per layer the device holds the FP32 master weights W (N x K) and b, Adam moments, and two
 // BF16 copies: W (the B operand of the forward product) and W^T (the B operand of the
-// input-gradient product).  Activations are kept in both orientations, written by the
+// input-gradient product).  Training activations are kept in both orientations, written by the
 // epilogues, so every product takes K-major operands:
 //   forward  H_{l+1} = gelu(H_l W_l^T + b_l)          A = H_l      B = W_l
 //   output   Y = H_{L-1} W^T + b, dY = 2 (Y - T) / (B * out_dim)   (fused, with the loss)
-//   weights  dW_l = dZ_l^T H_l                         A = dZ_l^T   B = H_l^T
 //   inputs   dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1})    A = dZ_l     B = W_l^T
-// A training step is one CUDA graph: gather, 2L + (L-1) products, L bias reductions, L Adam
-// updates and the step counter, replayed once per step.
+//   weights  dW_l = dZ_l^T H_l                         A = dZ_l^T   B = H_l^T   (fused with Adam)
+// A training step is 2 L launches (tc_train.cuh): L forward, then one launch per input
+// gradient, each carrying the weight gradients that have become ready.  The minibatches of a
+// chunk of steps are gathered by one launch; groups of kGroupSteps steps are one CUDA graph,
+// kept by the handle.  Inference runs the 128 x 128 products of tc_gemm.cuh.
 //
 // A handle holds E = cfg.members networks of the same shape (an ensemble).  Every buffer
 // carries a leading member axis and every kernel covers all members in one launch: the
@@ -33,6 +35,7 @@
 
 #include "../../include/epi_surrogate.h"
 #include "tc_gemm.cuh"
+#include "tc_train.cuh"
 
 using namespace epi::tc;
 
@@ -43,81 +46,96 @@ constexpr uint32_t kMaxMembers = 64;
 constexpr int kSmallThreads = 256;
 
 // ---------------------------------------------------------------- small kernels
-// Minibatch row r of member e (grid B x E) <- sample idx[e][step - step_base][r]: X rows (bf16,
-// already padded) in both orientations and the padded FP32 targets.
-__global__ void k_gather(const __nv_bfloat16* __restrict__ xs, const float* __restrict__ ys,
-                         const uint32_t* __restrict__ idx, uint32_t steps, const uint32_t* __restrict__ step,
-                         uint32_t step_base, uint32_t B, uint32_t out_pad, __nv_bfloat16* __restrict__ h0,
-                         __nv_bfloat16* __restrict__ h0t, float* __restrict__ t) {
-    const uint32_t r = blockIdx.x, e = blockIdx.y;
-    const uint32_t s = idx[((size_t)e * steps + (*step - step_base)) * B + r];
-    h0 += (size_t)e * B * kInPad;
-    h0t += (size_t)e * B * kInPad;
-    t += (size_t)e * B * out_pad;
-    for (uint32_t c = threadIdx.x; c < kInPad; c += blockDim.x) {
-        const __nv_bfloat16 v = xs[(size_t)s * kInPad + c];
-        h0[(size_t)r * kInPad + c] = v;
-        h0t[(size_t)c * B + r] = v;
-    }
-    for (uint32_t c = threadIdx.x; c < out_pad; c += blockDim.x) t[(size_t)r * out_pad + c] = ys[(size_t)s * out_pad + c];
-}
+// Host arrays travel as the caller lays them out; padding, conversion and (un)packing are
+// kernels (at 65,536 candidates the host loops they replace took a third of a score call).
 
-// db[n] = sum over the batch of dZ^T[n][:] (one warp per row; the members' rows follow one
-// another, so N counts the rows of all members).
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dzt, uint32_t N, uint32_t B, float* __restrict__ db) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (w >= N) return;
-    float s = 0.f;
-    for (uint32_t b = lane; b < B; b += 32) s += __bfloat162float(dzt[(size_t)w * B + b]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) db[w] = s;
-}
-
-struct AdamHyper {
-    float lr, beta1, beta2, eps;
-};
-
-// One Adam step (Kingma & Ba 2015, with bias correction) of member blockIdx.y; t = *step + 1.
-// Blocks below (N / 32) * (K / 32) take a 32 x 32 tile of W (N x K; both multiples of 32) and
-// write its BF16 copies W and W^T, the transpose through shared memory so that both stores
-// are coalesced; the blocks after them take 256 entries of b each.  256 threads.
-__device__ __forceinline__ float adam_update(float* p, float* m, float* v, float g, float c1, float c2, const AdamHyper& hp) {
-    const float mi = hp.beta1 * *m + (1.f - hp.beta1) * g;
-    const float vi = hp.beta2 * *v + (1.f - hp.beta2) * g * g;
-    *m = mi;
-    *v = vi;
-    const float np = *p - hp.lr * (mi / c1) / (sqrtf(vi / c2) + hp.eps);
-    *p = np;
-    return np;
-}
-
-__global__ void __launch_bounds__(256) k_adam(float* __restrict__ w, const float* __restrict__ gw, float* __restrict__ mw,
-                                              float* __restrict__ vw, float* __restrict__ b, const float* __restrict__ gb,
-                                              float* __restrict__ mb, float* __restrict__ vb, __nv_bfloat16* __restrict__ wb,
-                                              __nv_bfloat16* __restrict__ wtb, uint32_t N, uint32_t K,
-                                              const uint32_t* __restrict__ step, AdamHyper hp) {
-    __shared__ __nv_bfloat16 tile[32][34];
-    const float t = (float)(*step + 1u);
-    const float c1 = 1.f - powf(hp.beta1, t), c2 = 1.f - powf(hp.beta2, t);
-    const size_t nw = (size_t)N * K, ow = (size_t)blockIdx.y * nw, ob = (size_t)blockIdx.y * N;
-    const uint32_t tiles_k = K / 32u, n_tiles = N / 32u * tiles_k;
-    if (blockIdx.x < n_tiles) {
-        w += ow; gw += ow; mw += ow; vw += ow; wb += ow; wtb += ow;
-        const uint32_t n0 = blockIdx.x / tiles_k * 32u, k0 = blockIdx.x % tiles_k * 32u;
-        const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
-        for (uint32_t r = ty; r < 32u; r += 8u) {
-            const size_t i = (size_t)(n0 + r) * K + k0 + tx;
-            const __nv_bfloat16 q = __float2bfloat16_rn(adam_update(w + i, mw + i, vw + i, gw[i], c1, c2, hp));
-            wb[i] = q;
-            tile[r][tx] = q;
+// Rows of n x in_dim floats -> BF16 rows of kInPad, zero beyond in_dim and n (up to n_rows); xt,
+// when given, also receives the transpose (kInPad x n_rows).  One thread per two columns.
+__global__ void k_pad_inputs(const float* __restrict__ x, uint32_t n, uint32_t n_rows, uint32_t in_dim,
+                             __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ xt, uint32_t xt_pitch) {
+    const size_t total = (size_t)n_rows * (kInPad / 2);
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)(q / (kInPad / 2)), c = 2u * (uint32_t)(q % (kInPad / 2));
+        const float a = r < n && c < in_dim ? x[(size_t)r * in_dim + c] : 0.f;
+        const float b = r < n && c + 1 < in_dim ? x[(size_t)r * in_dim + c + 1] : 0.f;
+        const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+        reinterpret_cast<__nv_bfloat162*>(out)[q] = v;
+        if (xt) {
+            xt[(size_t)c * xt_pitch + r] = v.x;
+            xt[(size_t)(c + 1) * xt_pitch + r] = v.y;
         }
-        __syncthreads();
-        for (uint32_t r = ty; r < 32u; r += 8u) wtb[(size_t)(k0 + r) * N + n0 + tx] = tile[tx][r];
-    } else {
-        const uint32_t j = (blockIdx.x - n_tiles) * blockDim.x + threadIdx.x;
-        if (j < N) adam_update(b + ob + j, mb + ob + j, vb + ob + j, gb[ob + j], c1, c2, hp);
     }
+}
+
+// Rows of n x cols floats <-> rows of `pitch` (padding zero when written).
+__global__ void k_pad_rows(const float* __restrict__ in, uint32_t n, uint32_t cols, uint32_t pitch, float* __restrict__ out) {
+    const size_t total = (size_t)n * pitch;
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t c = (uint32_t)(q % pitch);
+        out[q] = c < cols ? in[q / pitch * cols + c] : 0.f;
+    }
+}
+__global__ void k_unpad_rows(const float* __restrict__ in, uint32_t n, uint32_t cols, uint32_t pitch, size_t member_in,
+                             float* __restrict__ out) {
+    const size_t total = (size_t)n * cols;
+    in += blockIdx.y * member_in;
+    out += blockIdx.y * total;
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x)
+        out[q] = in[q / cols * pitch + q % cols];
+}
+
+// One layer between the caller's flat layout (member blockIdx.y's block of `count` floats, W
+// row by row and then b from `first`) and its padded arrays; the padding stays zero.
+__global__ void k_params(float* __restrict__ flat, size_t count, size_t first, uint32_t n_real, uint32_t k_real,
+                         float* __restrict__ w, float* __restrict__ b, uint32_t N, uint32_t K, int to_flat) {
+    flat += blockIdx.y * count + first;
+    w += (size_t)blockIdx.y * N * K;
+    b += (size_t)blockIdx.y * N;
+    const size_t nw = (size_t)n_real * k_real, total = nw + n_real;
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x) {
+        float* p = q < nw ? w + q / k_real * K + q % k_real : b + (q - nw);
+        if (to_flat) flat[q] = *p;
+        else *p = flat[q];
+    }
+}
+
+// The minibatch inputs of a chunk of steps: row r of member e (grid rows / 32 x E) is sample
+// idx[r / B][e][r % B], in both orientations (out rows x kInPad, out_t kInPad x rows per member).
+__global__ void __launch_bounds__(256) k_gather(const __nv_bfloat16* __restrict__ xs, const uint32_t* __restrict__ idx,
+                                                uint32_t B, uint32_t rows_cap, __nv_bfloat16* __restrict__ out,
+                                                __nv_bfloat16* __restrict__ out_t) {
+    __shared__ __nv_bfloat16 tile[32][kInPad + 2];
+    const uint32_t e = blockIdx.y, r0 = blockIdx.x * 32u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    out += (size_t)e * rows_cap * kInPad;
+    out_t += (size_t)e * rows_cap * kInPad;
+    for (uint32_t k = warp; k < 32u; k += 8u) {
+        const uint32_t r = r0 + k, s = idx[((size_t)(r / B) * gridDim.y + e) * B + r % B];
+        const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162*>(xs + (size_t)s * kInPad)[lane];
+        reinterpret_cast<__nv_bfloat162*>(out + (size_t)r * kInPad)[lane] = v;
+        *reinterpret_cast<__nv_bfloat162*>(&tile[k][2u * lane]) = v;
+    }
+    __syncthreads();
+    for (uint32_t c = warp; c < kInPad; c += 8u) out_t[(size_t)c * rows_cap + r0 + lane] = tile[lane][c];
+}
+
+// A chunk of n steps begins (t0 steps taken before it): what they read on the device.  One block.
+__global__ void k_train_chunk(TrainDev* tr, const uint32_t* idx, const float* ys, float* loss, float4* corr, uint32_t n,
+                              uint32_t t0, AdamHyper hp) {
+    if (threadIdx.x == 0) {
+        tr->local = 0u;
+        tr->idx = idx;
+        tr->ys = ys;
+        tr->loss = loss;
+        tr->corr = corr;
+    }
+    for (uint32_t s = threadIdx.x; s < n; s += blockDim.x) {
+        const float t = (float)(t0 + s + 1u);
+        const float c1 = 1.f - powf(hp.beta1, t), c2 = 1.f - powf(hp.beta2, t);
+        corr[s] = make_float4(c1, c2, __frcp_rn(c1), __frcp_rn(c2));
+    }
+}
+__global__ void k_step_end(TrainDev* tr, uint32_t steps) {
+    tr->local += steps;
 }
 
 // BF16 copies of the master weights of member blockIdx.y (after initialisation or set_params).
@@ -131,8 +149,6 @@ __global__ void k_cast_weights(const float* __restrict__ w, __nv_bfloat16* __res
         wtb[(i % K) * N + i / K] = q;
     }
 }
-
-__global__ void k_step_end(uint32_t* step) { *step += 1u; }
 
 // ---------------------------------------------------------------- host helpers
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -174,11 +190,13 @@ struct MlpLayer {
     float *w = nullptr, *b = nullptr, *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
     float *gw = nullptr, *gb = nullptr;
     __nv_bfloat16 *wb = nullptr, *wtb = nullptr;
-    // training activations (batch rows, E members each)
+    // training activations (batch rows, E members each; layer 0's are a chunk's minibatches)
     __nv_bfloat16 *h = nullptr, *ht = nullptr;     // input of this layer, B x K and K x B
     float* z = nullptr;                             // pre-activation output, B x N (hidden layers)
     __nv_bfloat16 *dz = nullptr, *dzt = nullptr;    // gradient at the pre-activation, B x N and N x B
-    CUtensorMap t_h, t_w, t_dzt, t_ht, t_dz, t_wt;  // product operands
+    // training operands: A operands in boxes of 128 rows, B operands of 32 or 64
+    CUtensorMap t_h, t_w32, t_w64, t_dzt, t_ht32, t_ht64, t_dz, t_wt32, t_wt64;
+    CUtensorMap t_w;                                  // inference B operand (128 rows)
     // inference activations: the input layer's rows are shared by all members
     __nv_bfloat16* ph = nullptr;
     CUtensorMap t_ph;
@@ -187,19 +205,23 @@ struct MlpLayer {
 struct epi_mlp {
     epi_mlp_config cfg{};
     uint32_t E = 1;  // members
-    uint32_t L = 0, in_pad = kInPad, out_pad = 0, B = 0;
+    uint32_t L = 0, in_pad = kInPad, out_pad = 0, B = 0, sms = 0;
     std::vector<MlpLayer> layers;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     std::string err;
     int* d_err = nullptr;
-    uint32_t* d_step = nullptr;
-    float* d_t = nullptr;        // batch targets, E x B x out_pad
+    TrainDev* d_tr = nullptr;
+    uint32_t adam_steps = 0;     // Adam's t of the last step
+    float4* d_corr = nullptr;    // Adam's bias corrections of the chunk's steps
+    float* d_t = nullptr;        // targets of a gradients call, B x out_pad (all members)
     float* d_loss = nullptr;     // per-step losses, steps x E
-    float* d_step_loss = nullptr;  // losses of the step in flight, E
-    uint32_t loss_cap = 0;
-    uint32_t* d_idx = nullptr;   // minibatch indices of a train call, E x steps x B
+    size_t loss_cap = 0;
+    uint32_t chunk = 0;          // steps whose minibatches are gathered at once
+    uint32_t* d_idx = nullptr;   // minibatch indices of a train call, steps x E x B
     size_t idx_cap = 0;
+    float* d_raw = nullptr;      // caller arrays on their way in or out
+    size_t raw_cap = 0;
     __nv_bfloat16* d_xs = nullptr;  // dataset, n x 64 (bf16, padded)
     float* d_ys = nullptr;          // dataset, n x out_pad
     uint32_t n_data = 0;
@@ -208,7 +230,7 @@ struct epi_mlp {
     float* d_py = nullptr;        // E x n x out_pad
     float* d_pscore = nullptr;    // E x n
     float* d_ptarget = nullptr;   // out_pad
-    cudaGraphExec_t step_graph = nullptr;
+    cudaGraphExec_t step_graph = nullptr, group_graph = nullptr;  // one step, kGroupSteps steps
     uint64_t launches = 0;
 };
 
@@ -276,69 +298,160 @@ int cast_all(epi_mlp* h) {
     return EPI_OK;
 }
 
-// Forward + backward of one minibatch per member already in layers[0].h / .ht and d_t;
-// member e's loss added to loss[e].
-int enqueue_fwd_bwd(epi_mlp* h, float* loss) {
-    const uint32_t B = h->B, L = h->L;
+// A launch that may be scheduled while the kernel before it runs (its CTAs wait on the device).
+template <typename... KArgs, typename... Args>
+int launch_overlapped(epi_mlp* h, void (*kern)(KArgs...), dim3 grid, uint32_t smem, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTrainThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    MCK(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+    h->launches++;
+    return EPI_OK;
+}
+
+// The forward and backward launches of one step: of the gathered chunk's step tr->local + off
+// with its Adam updates, or (grads) of the one minibatch in row 0.. of the chunk buffers shared
+// by all members, with targets d_t, the gradients stored in gw / gb and the losses in d_loss.
+int enqueue_step(epi_mlp* h, uint32_t off, bool grads) {
+    const uint32_t B = h->B, L = h->L, E = h->E;
+    // Narrow tiles while a product's CTAs fit the SMs: one network's 256 x 512 product then
+    // runs on 32 SMs (6.0 us a launch on one GB300).  Five networks' would take 160 CTAs, two
+    // to an SM on some: 8.8 us, against 7.5 for 80 wide ones.
+    auto wide = [&](uint32_t N) { return B / kBM * (N / kTrainBN) * E > h->sms; };
+    // All K blocks in flight at once where a CTA has its SM to itself, else 4 (two CTAs an SM).
+    auto stages_for = [&](uint32_t nk, uint32_t ctas) { return std::min(nk, ctas <= h->sms ? kTrainStages : 4u); };
     for (uint32_t l = 0; l < L; ++l) {
         MlpLayer& ly = h->layers[l];
-        EpiArgs a;
+        const bool out = l + 1 == L, w = wide(ly.N);
+        const int bn = w ? kTrainWideBN : kTrainBN;
+        const dim3 grid(B / kBM, ly.N / bn, E);
+        ForwardArgs a{};
+        a.M = B;
+        a.N = ly.N;
+        a.nk = ly.K / kBK;
+        a.stages = stages_for(a.nk, grid.x * grid.y * grid.z);
+        a.first = l == 0;
+        a.shared_a = l == 0 && grads;
+        a.off = off;
         a.bias = ly.b;
-        a.ms_bias = ly.N;
-        if (l + 1 < L) {
-            MlpLayer& nx = h->layers[l + 1];
-            a.z = ly.z;
-            a.out = nx.h;
-            a.out_t = nx.ht;
-            a.ms_z = a.ms_out = (uint64_t)B * ly.N;
-            MRC((gemm<128, kEpHidden>(h, ly.t_h, ly.t_w, B, ly.N, ly.K, a)));
-        } else {
-            a.target = h->d_t;
-            a.out = ly.dz;
-            a.out_t = ly.dzt;
-            a.loss = loss;
+        a.z = ly.z;
+        a.out = out ? ly.dz : h->layers[l + 1].h;
+        a.out_t = out ? ly.dzt : h->layers[l + 1].ht;
+        if (out) {
+            a.target = grads ? h->d_t : nullptr;
+            a.loss = grads ? h->d_loss : nullptr;
             a.n_valid = h->cfg.out_dim;
-            a.m_valid = B;
             a.grad_scale = 2.0f / ((float)B * (float)h->cfg.out_dim);
-            a.ms_target = a.ms_out = (uint64_t)B * ly.N;
-            a.ms_loss = 1;
-            MRC((gemm<128, kEpOut>(h, ly.t_h, ly.t_w, B, ly.N, ly.K, a)));
         }
+        auto kern = out ? (w ? k_forward<true, kTrainWideBN> : k_forward<true, kTrainBN>)
+                        : (w ? k_forward<false, kTrainWideBN> : k_forward<false, kTrainBN>);
+        MRC(launch_overlapped(h, kern, grid, train_smem(bn, a.stages), ly.t_h, w ? ly.t_w64 : ly.t_w32, a,
+                              (const TrainDev*)h->d_tr, h->d_err));
     }
-    for (int l = (int)L - 1; l >= 0; --l) {
+    auto weight_job = [&](BackwardArgs& a, BackwardMaps& maps, int slot, uint32_t l, bool wide_w) {
         MlpLayer& ly = h->layers[l];
-        EpiArgs g;
-        g.outf = ly.gw;
-        g.ms_outf = (uint64_t)ly.N * ly.K;
-        if (ly.K == 64) MRC((gemm<64, kEpDw>(h, ly.t_dzt, ly.t_ht, ly.N, ly.K, B, g)));
-        else MRC((gemm<128, kEpDw>(h, ly.t_dzt, ly.t_ht, ly.N, ly.K, B, g)));
-        const uint32_t rows = ly.N * h->E;
-        k_bias_grad<<<(rows * 32 + kSmallThreads - 1) / kSmallThreads, kSmallThreads, 0, h->stream>>>(ly.dzt, rows, B,
-                                                                                                      ly.gb);
-        MCK(cudaGetLastError());
-        h->launches++;
+        WeightGrad& w = a.dw[slot];
+        w.tiles = ly.N / kBM * (ly.K / (wide_w ? kTrainWideBN : kTrainBN));
+        w.bias_blocks = (ly.N + kBiasRows - 1) / kBiasRows;
+        w.N = ly.N;
+        w.K = ly.K;
+        w.nk = B / kBK;
+        w.B = B;
+        w.first = l == 0;
+        w.shared_h = l == 0 && grads;
+        w.w = ly.w; w.mw = ly.mw; w.vw = ly.vw;
+        w.b = ly.b; w.mb = ly.mb; w.vb = ly.vb;
+        w.wb = ly.wb; w.wtb = ly.wtb;
+        w.dzt = ly.dzt;
+        w.gw = grads ? ly.gw : nullptr;
+        w.gb = grads ? ly.gb : nullptr;
+        maps.dw_a[slot] = ly.t_dzt;
+        maps.dw_b[slot] = wide_w ? ly.t_ht64 : ly.t_ht32;
+    };
+    // launch l computes dZ_{l-1} from dZ_l; W_{l+1}, whose last reader was the launch before,
+    // takes its update beside it; the last launch has those of layers 1 and 0
+    for (uint32_t l = L - 1; l + 1 > 0; --l) {
+        BackwardArgs a{};
+        BackwardMaps maps;
+        std::memset(&maps, 0, sizeof maps);
+        a.off = off;
+        a.grads = grads;
+        a.hp = AdamHyper{h->cfg.lr, h->cfg.beta1, h->cfg.beta2, h->cfg.eps};
+        const bool w = l > 0 && wide(h->layers[l].K);
+        // weight gradients: narrow while a hidden layer's fit two to an SM (200 steps on one
+        // GB300, narrow / wide: 3 networks 12.4 / 12.4 ms, 5 networks 19.6 / 18.8, 10 networks
+        // 32.1 / 30.7)
+        const bool ww = h->cfg.hidden / kBM * (h->cfg.hidden / kTrainBN) * E > 2 * h->sms;
+        const int bn = w ? kTrainWideBN : kTrainBN;
         if (l > 0) {
-            MlpLayer& pv = h->layers[l - 1];
-            EpiArgs d;
-            d.zin = pv.z;
-            d.out = pv.dz;
-            d.out_t = pv.dzt;
-            d.ms_zin = d.ms_out = (uint64_t)B * ly.K;
-            MRC((gemm<128, kEpDh>(h, ly.t_dz, ly.t_wt, B, ly.K, ly.N, d)));
+            MlpLayer &ly = h->layers[l], &pv = h->layers[l - 1];
+            a.dx.tiles = B / kBM * (ly.K / bn);
+            a.dx.M = B;
+            a.dx.N = ly.K;
+            a.dx.nk = ly.N / kBK;
+            a.dx.z = pv.z;
+            a.dx.out = pv.dz;
+            a.dx.out_t = pv.dzt;
+            maps.dx_a = ly.t_dz;
+            maps.dx_b = w ? ly.t_wt64 : ly.t_wt32;
+            if (l + 1 < L) weight_job(a, maps, 0, l + 1, ww);
+        } else {
+            weight_job(a, maps, 0, 1, ww);
+            weight_job(a, maps, 1, 0, ww);
         }
+        const uint32_t blocks = a.dx.tiles + a.dw[0].tiles + a.dw[1].tiles + a.dw[0].bias_blocks + a.dw[1].bias_blocks;
+        a.stages = stages_for(std::max(a.dx.nk, B / kBK), blocks * E);
+        auto kern = w ? (ww ? k_backward<kTrainWideBN, kTrainWideBN> : k_backward<kTrainWideBN, kTrainBN>)
+                      : (ww ? k_backward<kTrainBN, kTrainWideBN> : k_backward<kTrainBN, kTrainBN>);
+        MRC(launch_overlapped(h, kern, dim3(blocks, E), train_smem(w || ww ? kTrainWideBN : kTrainBN, a.stages), maps, a,
+                              (const TrainDev*)h->d_tr, h->d_err));
     }
     return EPI_OK;
 }
 
-int enqueue_adam(epi_mlp* h) {
-    const AdamHyper hp{h->cfg.lr, h->cfg.beta1, h->cfg.beta2, h->cfg.eps};
-    for (auto& ly : h->layers) {
-        const uint32_t blocks = ly.N / 32u * (ly.K / 32u) + (ly.N + kSmallThreads - 1) / kSmallThreads;
-        k_adam<<<dim3(blocks, h->E), kSmallThreads, 0, h->stream>>>(
-            ly.w, ly.gw, ly.mw, ly.vw, ly.b, ly.gb, ly.mb, ly.vb, ly.wb, ly.wtb, ly.N, ly.K, h->d_step, hp);
-        MCK(cudaGetLastError());
-        h->launches++;
+// Adam steps of a captured group, so that the gap between graph launches is paid once in four.
+constexpr uint32_t kGroupSteps = 4;
+
+int step_graph(epi_mlp* h, uint32_t steps, cudaGraphExec_t* out) {
+    if (*out) return EPI_OK;
+    cudaGraph_t g;
+    MCK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = EPI_OK;
+    for (uint32_t k = 0; k < steps && !rc; ++k) rc = enqueue_step(h, k, false);
+    if (!rc) k_step_end<<<1, 1, 0, h->stream>>>(h->d_tr, steps);
+    cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
+    if (rc) return rc;
+    if (ce == cudaSuccess) {
+        ce = cudaGraphInstantiate(out, g, 0);
+        cudaGraphDestroy(g);
     }
+    if (ce != cudaSuccess) { *out = nullptr; h->err = std::string("training graph: ") + cudaGetErrorString(ce); return EPI_ERR_CUDA; }
+    return EPI_OK;
+}
+
+void drop_graphs(epi_mlp* h) {
+    for (cudaGraphExec_t* g : {&h->step_graph, &h->group_graph}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+}
+
+// Device space for `floats` caller values.
+int ensure_raw(epi_mlp* h, size_t floats) {
+    if (floats <= h->raw_cap) return EPI_OK;
+    MCK(cudaStreamSynchronize(h->stream));
+    cudaFree(h->d_raw);
+    h->d_raw = nullptr;
+    h->raw_cap = 0;
+    MCK(cudaMalloc(&h->d_raw, floats * sizeof(float)));
+    h->raw_cap = floats;
     return EPI_OK;
 }
 
@@ -354,12 +467,29 @@ int check_err(epi_mlp* h) {
     return EPI_OK;
 }
 
-// Pad host inputs (n x in_dim, float) into BF16 rows of 64.
-std::vector<__nv_bfloat16> pad_inputs(const float* x, uint32_t n, uint32_t n_rows, uint32_t in_dim) {
-    std::vector<__nv_bfloat16> v((size_t)n_rows * kInPad, __float2bfloat16_rn(0.f));
-    for (uint32_t i = 0; i < n; ++i)
-        for (uint32_t c = 0; c < in_dim; ++c) v[(size_t)i * kInPad + c] = __float2bfloat16_rn(x[(size_t)i * in_dim + c]);
-    return v;
+// n caller rows of in_dim floats into BF16 rows of kInPad on the device (n_rows of them).
+int upload_inputs(epi_mlp* h, const float* x, uint32_t n, uint32_t n_rows, __nv_bfloat16* out, __nv_bfloat16* xt = nullptr,
+                  uint32_t xt_pitch = 0) {
+    const size_t floats = (size_t)n * h->cfg.in_dim;
+    MRC(ensure_raw(h, floats));
+    MCK(cudaMemcpyAsync(h->d_raw, x, floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    k_pad_inputs<<<blocks_for((size_t)n_rows * (kInPad / 2)), kSmallThreads, 0, h->stream>>>(h->d_raw, n, n_rows,
+                                                                                            h->cfg.in_dim, out, xt, xt_pitch);
+    MCK(cudaGetLastError());
+    h->launches++;
+    return EPI_OK;
+}
+
+// n caller rows of out_dim floats into rows of out_pad on the device.
+int upload_targets(epi_mlp* h, const float* y, uint32_t n, float* out) {
+    const size_t floats = (size_t)n * h->cfg.out_dim;
+    MRC(ensure_raw(h, floats));
+    MCK(cudaMemcpyAsync(h->d_raw, y, floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    k_pad_rows<<<blocks_for((size_t)n * h->out_pad), kSmallThreads, 0, h->stream>>>(h->d_raw, n, h->cfg.out_dim, h->out_pad,
+                                                                                   out);
+    MCK(cudaGetLastError());
+    h->launches++;
+    return EPI_OK;
 }
 
 int ensure_predict(epi_mlp* h, uint32_t n_pad) {
@@ -392,8 +522,7 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
     const uint32_t n_pad = std::max<uint32_t>(round_up(n, kBM), kBM);
     MRC(ensure_predict(h, n_pad));
     const uint64_t cap = h->p_cap;
-    std::vector<__nv_bfloat16> xs = pad_inputs(x, n, n_pad, h->cfg.in_dim);
-    MCK(cudaMemcpyAsync(h->layers[0].ph, xs.data(), xs.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice, h->stream));
+    MRC(upload_inputs(h, x, n, n_pad, h->layers[0].ph));
     if (target) {
         MCK(cudaMemcpyAsync(h->d_ptarget, target, h->cfg.out_dim * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         MCK(cudaMemsetAsync(h->d_pscore, 0, (size_t)h->E * cap * sizeof(float), h->stream));
@@ -423,14 +552,14 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
 }
 
 void free_all(epi_mlp* h) {
-    if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
+    drop_graphs(h);
     for (auto& ly : h->layers) {
         cudaFree(ly.w); cudaFree(ly.b); cudaFree(ly.mw); cudaFree(ly.vw); cudaFree(ly.mb); cudaFree(ly.vb);
         cudaFree(ly.gw); cudaFree(ly.gb); cudaFree(ly.wb); cudaFree(ly.wtb);
         cudaFree(ly.h); cudaFree(ly.ht); cudaFree(ly.z); cudaFree(ly.dz); cudaFree(ly.dzt); cudaFree(ly.ph);
     }
-    cudaFree(h->d_err); cudaFree(h->d_step); cudaFree(h->d_t); cudaFree(h->d_loss); cudaFree(h->d_step_loss);
-    cudaFree(h->d_idx);
+    cudaFree(h->d_err); cudaFree(h->d_tr); cudaFree(h->d_t); cudaFree(h->d_loss);
+    cudaFree(h->d_idx); cudaFree(h->d_raw); cudaFree(h->d_corr);
     cudaFree(h->d_xs); cudaFree(h->d_ys); cudaFree(h->d_py); cudaFree(h->d_pscore); cudaFree(h->d_ptarget);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
@@ -445,9 +574,15 @@ int init(epi_mlp* h) {
     const epi_mlp_config& c = h->cfg;
     MRC((allow_smem<128, kEpHidden>(h)));
     MRC((allow_smem<128, kEpOut>(h)));
-    MRC((allow_smem<128, kEpDh>(h)));
-    MRC((allow_smem<128, kEpDw>(h)));
-    MRC((allow_smem<64, kEpDw>(h)));
+    for (const void* k : {(const void*)k_forward<false, kTrainBN>, (const void*)k_forward<false, kTrainWideBN>,
+                          (const void*)k_forward<true, kTrainBN>, (const void*)k_forward<true, kTrainWideBN>,
+                          (const void*)k_backward<kTrainBN, kTrainBN>, (const void*)k_backward<kTrainBN, kTrainWideBN>,
+                          (const void*)k_backward<kTrainWideBN, kTrainBN>, (const void*)k_backward<kTrainWideBN, kTrainWideBN>})
+        MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem(kTrainWideBN, kTrainStages)));
+    int dev = 0, sms = 0;
+    MCK(cudaGetDevice(&dev));
+    MCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    h->sms = (uint32_t)sms;
     const uint32_t E = h->E;
     h->L = c.hidden_layers + 1;
     h->B = c.batch;
@@ -455,11 +590,14 @@ int init(epi_mlp* h) {
     MCK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     MCK(cudaMalloc(&h->d_err, sizeof(int)));
-    MCK(cudaMalloc(&h->d_step, sizeof(uint32_t)));
+    MCK(cudaMalloc(&h->d_tr, sizeof(TrainDev)));
     MCK(cudaMemset(h->d_err, 0, sizeof(int)));
-    MCK(cudaMemset(h->d_step, 0, sizeof(uint32_t)));
-    MCK(cudaMalloc(&h->d_t, (size_t)E * h->B * h->out_pad * sizeof(float)));
-    MCK(cudaMalloc(&h->d_step_loss, (size_t)E * sizeof(float)));
+    MCK(cudaMemset(h->d_tr, 0, sizeof(TrainDev)));
+    MCK(cudaMalloc(&h->d_t, (size_t)h->B * h->out_pad * sizeof(float)));
+    // steps gathered at once: up to 128, within 32 MB of inputs
+    h->chunk = (uint32_t)std::min<size_t>(128, std::max<size_t>(kGroupSteps, (32u << 20) / ((size_t)E * h->B * kInPad * 2)));
+    h->chunk -= h->chunk % kGroupSteps;
+    MCK(cudaMalloc(&h->d_corr, h->chunk * sizeof(float4)));
     MCK(cudaMalloc(&h->d_ptarget, (size_t)h->out_pad * sizeof(float)));
     h->layers.resize(h->L);
     for (uint32_t l = 0; l < h->L; ++l) {
@@ -468,7 +606,8 @@ int init(epi_mlp* h) {
         ly.n_real = l + 1 == h->L ? c.out_dim : c.hidden;
         ly.K = l == 0 ? kInPad : c.hidden;
         ly.N = l + 1 == h->L ? h->out_pad : c.hidden;
-        const size_t nw = (size_t)E * ly.N * ly.K, nb = (size_t)E * ly.N, act_in = (size_t)E * h->B * ly.K,
+        const uint32_t rows = l == 0 ? h->chunk * h->B : h->B;  // of the layer's input
+        const size_t nw = (size_t)E * ly.N * ly.K, nb = (size_t)E * ly.N, act_in = (size_t)E * rows * ly.K,
                      act_out = (size_t)E * h->B * ly.N;
         for (float** p : {&ly.w, &ly.mw, &ly.vw, &ly.gw}) MCK(cudaMalloc(p, nw * sizeof(float)));
         for (float** p : {&ly.b, &ly.mb, &ly.vb, &ly.gb}) MCK(cudaMalloc(p, nb * sizeof(float)));
@@ -483,12 +622,16 @@ int init(epi_mlp* h) {
         for (float* p : {ly.mb, ly.vb, ly.gb}) MCK(cudaMemset(p, 0, nb * sizeof(float)));
         // operands: forward A = h (B x K), B = W (N x K); weights A = dZ^T (N x B), B = H^T (K x B);
         // inputs A = dZ (B x N), B = W^T (K x N)
-        MRC(make_map(h, &ly.t_h, ly.h, h->B, ly.K, kBM, E));
+        MRC(make_map(h, &ly.t_h, ly.h, rows, ly.K, kBM, E));
         MRC(make_map(h, &ly.t_w, ly.wb, ly.N, ly.K, 128, E));
+        MRC(make_map(h, &ly.t_w32, ly.wb, ly.N, ly.K, kTrainBN, E));
+        MRC(make_map(h, &ly.t_w64, ly.wb, ly.N, ly.K, kTrainWideBN, E));
         MRC(make_map(h, &ly.t_dzt, ly.dzt, ly.N, h->B, kBM, E));
-        MRC(make_map(h, &ly.t_ht, ly.ht, ly.K, h->B, ly.K == 64 ? 64 : 128, E));
+        MRC(make_map(h, &ly.t_ht32, ly.ht, ly.K, rows, kTrainBN, E));
+        MRC(make_map(h, &ly.t_ht64, ly.ht, ly.K, rows, kTrainWideBN, E));
         MRC(make_map(h, &ly.t_dz, ly.dz, h->B, ly.N, kBM, E));
-        MRC(make_map(h, &ly.t_wt, ly.wtb, ly.K, ly.N, 128, E));
+        MRC(make_map(h, &ly.t_wt32, ly.wtb, ly.K, ly.N, kTrainBN, E));
+        MRC(make_map(h, &ly.t_wt64, ly.wtb, ly.K, ly.N, kTrainWideBN, E));
     }
     // torch.nn.Linear's default: W and b uniform in +-1/sqrt(fan_in); member m draws from
     // seed + m, layer by layer (W row by row, then b)
@@ -516,23 +659,26 @@ uint64_t member_params(const epi_mlp* h) {
     return n;
 }
 
-// Device W / b arrays of every layer (E padded members each) -> member-major unpadded host layout.
-int download_params(epi_mlp* h, float* const MlpLayer::*wp, float* const MlpLayer::*bp, float* out) {
+// Every layer's arrays (E padded members each) <-> the member-major unpadded layout in d_raw.
+int move_params(epi_mlp* h, float* const MlpLayer::*wp, float* const MlpLayer::*bp, bool to_flat) {
     const uint64_t count = member_params(h);
     size_t o = 0;
     for (auto& ly : h->layers) {
-        const size_t nw = (size_t)ly.N * ly.K;
-        std::vector<float> w(nw * h->E), b((size_t)ly.N * h->E);
-        MCK(cudaMemcpy(w.data(), ly.*wp, w.size() * sizeof(float), cudaMemcpyDeviceToHost));
-        MCK(cudaMemcpy(b.data(), ly.*bp, b.size() * sizeof(float), cudaMemcpyDeviceToHost));
-        for (uint32_t m = 0; m < h->E; ++m) {
-            size_t q = m * count + o;
-            for (uint32_t n = 0; n < ly.n_real; ++n)
-                for (uint32_t k = 0; k < ly.k_real; ++k) out[q++] = w[m * nw + (size_t)n * ly.K + k];
-            for (uint32_t n = 0; n < ly.n_real; ++n) out[q++] = b[(size_t)m * ly.N + n];
-        }
-        o += (size_t)ly.n_real * ly.k_real + ly.n_real;
+        const size_t total = (size_t)ly.n_real * ly.k_real + ly.n_real;
+        k_params<<<dim3(blocks_for(total), h->E), kSmallThreads, 0, h->stream>>>(h->d_raw, count, o, ly.n_real, ly.k_real,
+                                                                                ly.*wp, ly.*bp, ly.N, ly.K, to_flat);
+        MCK(cudaGetLastError());
+        h->launches++;
+        o += total;
     }
+    return EPI_OK;
+}
+int download_params(epi_mlp* h, float* const MlpLayer::*wp, float* const MlpLayer::*bp, float* out) {
+    const size_t floats = (size_t)member_params(h) * h->E;
+    MRC(ensure_raw(h, floats));
+    MRC(move_params(h, wp, bp, true));
+    MCK(cudaMemcpyAsync(out, h->d_raw, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    MCK(cudaStreamSynchronize(h->stream));
     return EPI_OK;
 }
 
@@ -573,10 +719,7 @@ int epi_mlp_set_stream(epi_mlp* h, void* cuda_stream) {
     if (h->own_stream) cudaStreamDestroy(h->stream);
     h->stream = static_cast<cudaStream_t>(cuda_stream);
     h->own_stream = false;
-    if (h->step_graph) {
-        cudaGraphExecDestroy(h->step_graph);
-        h->step_graph = nullptr;
-    }
+    drop_graphs(h);
     return EPI_OK;
 }
 
@@ -601,24 +744,16 @@ int epi_mlp_get_params(epi_mlp* h, float* out) {
 int epi_mlp_set_params(epi_mlp* h, const float* in) {
     if (!h || !in) return EPI_ERR_ARG;
     MCK(cudaStreamSynchronize(h->stream));
-    const uint64_t count = member_params(h);
-    size_t o = 0;
+    const size_t floats = (size_t)member_params(h) * h->E;
+    MRC(ensure_raw(h, floats));
+    MCK(cudaMemcpyAsync(h->d_raw, in, floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    MRC(move_params(h, &MlpLayer::w, &MlpLayer::b, false));
     for (auto& ly : h->layers) {
-        const size_t nw = (size_t)ly.N * ly.K;
-        std::vector<float> w(nw * h->E, 0.f), b((size_t)ly.N * h->E, 0.f);
-        for (uint32_t m = 0; m < h->E; ++m) {
-            size_t q = m * count + o;
-            for (uint32_t n = 0; n < ly.n_real; ++n)
-                for (uint32_t k = 0; k < ly.k_real; ++k) w[m * nw + (size_t)n * ly.K + k] = in[q++];
-            for (uint32_t n = 0; n < ly.n_real; ++n) b[(size_t)m * ly.N + n] = in[q++];
-        }
-        o += (size_t)ly.n_real * ly.k_real + ly.n_real;
-        MCK(cudaMemcpy(ly.w, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice));
-        MCK(cudaMemcpy(ly.b, b.data(), b.size() * sizeof(float), cudaMemcpyHostToDevice));
-        for (float* p : {ly.mw, ly.vw}) MCK(cudaMemset(p, 0, w.size() * sizeof(float)));
-        for (float* p : {ly.mb, ly.vb}) MCK(cudaMemset(p, 0, b.size() * sizeof(float)));
+        const size_t nw = (size_t)h->E * ly.N * ly.K * sizeof(float), nb = (size_t)h->E * ly.N * sizeof(float);
+        for (float* p : {ly.mw, ly.vw}) MCK(cudaMemsetAsync(p, 0, nw, h->stream));
+        for (float* p : {ly.mb, ly.vb}) MCK(cudaMemsetAsync(p, 0, nb, h->stream));
     }
-    MCK(cudaMemset(h->d_step, 0, sizeof(uint32_t)));
+    h->adam_steps = 0;
     MRC(cast_all(h));
     MCK(cudaStreamSynchronize(h->stream));
     return EPI_OK;
@@ -632,14 +767,11 @@ int epi_mlp_set_dataset(epi_mlp* h, const float* x, const float* y, uint32_t n) 
     h->d_xs = nullptr;
     h->d_ys = nullptr;
     h->n_data = 0;
-    std::vector<__nv_bfloat16> xs = pad_inputs(x, n, n, h->cfg.in_dim);
-    std::vector<float> ys((size_t)n * h->out_pad, 0.f);
-    for (uint32_t i = 0; i < n; ++i)
-        std::memcpy(&ys[(size_t)i * h->out_pad], y + (size_t)i * h->cfg.out_dim, h->cfg.out_dim * sizeof(float));
-    MCK(cudaMalloc(&h->d_xs, xs.size() * sizeof(__nv_bfloat16)));
-    MCK(cudaMalloc(&h->d_ys, ys.size() * sizeof(float)));
-    MCK(cudaMemcpy(h->d_xs, xs.data(), xs.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
-    MCK(cudaMemcpy(h->d_ys, ys.data(), ys.size() * sizeof(float), cudaMemcpyHostToDevice));
+    MCK(cudaMalloc(&h->d_xs, (size_t)n * kInPad * sizeof(__nv_bfloat16)));
+    MCK(cudaMalloc(&h->d_ys, (size_t)n * h->out_pad * sizeof(float)));
+    MRC(upload_inputs(h, x, n, n, h->d_xs));
+    MRC(upload_targets(h, y, n, h->d_ys));
+    MCK(cudaStreamSynchronize(h->stream));
     h->n_data = n;
     return EPI_OK;
 }
@@ -655,13 +787,12 @@ int epi_mlp_train(epi_mlp* h, uint32_t steps, uint64_t shuffle_seed, float* loss
     std::vector<uint32_t> idx((size_t)E * steps * B), perm(h->n_data);
     for (uint32_t m = 0; m < E; ++m) {
         SplitMix rng{shuffle_seed + m};
-        uint32_t* dst = &idx[(size_t)m * steps * B];
         for (uint32_t s = 0; s < steps; ++s) {
             if (s % per_epoch == 0) {
                 for (uint32_t i = 0; i < h->n_data; ++i) perm[i] = i;
                 for (uint32_t i = h->n_data - 1; i > 0; --i) std::swap(perm[i], perm[rng.next() % (i + 1)]);  // Fisher-Yates
             }
-            std::memcpy(dst + (size_t)s * B, &perm[(size_t)(s % per_epoch) * B], B * sizeof(uint32_t));
+            std::memcpy(&idx[((size_t)s * E + m) * B], &perm[(size_t)(s % per_epoch) * B], B * sizeof(uint32_t));
         }
     }
     MCK(cudaStreamSynchronize(h->stream));
@@ -677,45 +808,29 @@ int epi_mlp_train(epi_mlp* h, uint32_t steps, uint64_t shuffle_seed, float* loss
         h->d_loss = nullptr;
         h->loss_cap = 0;
         MCK(cudaMalloc(&h->d_loss, (size_t)steps * E * sizeof(float)));
-        h->loss_cap = steps * E;
+        h->loss_cap = (size_t)steps * E;
     }
     MCK(cudaMemcpyAsync(h->d_idx, idx.data(), idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
-    // Adam's step counter keeps counting across calls; this call's minibatch s is read at
-    // (*d_step - t0)
-    uint32_t t0 = 0;
-    MCK(cudaMemcpyAsync(&t0, h->d_step, sizeof t0, cudaMemcpyDeviceToHost, h->stream));
-    MCK(cudaStreamSynchronize(h->stream));
-    if (h->step_graph) {
-        cudaGraphExecDestroy(h->step_graph);
-        h->step_graph = nullptr;
-    }
-    cudaGraph_t g;
-    MCK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = EPI_OK;
-    {
-        MlpLayer& l0 = h->layers[0];
-        cudaError_t me = cudaMemsetAsync(h->d_step_loss, 0, (size_t)E * sizeof(float), h->stream);
-        if (me != cudaSuccess) rc = EPI_ERR_CUDA;
-        k_gather<<<dim3(B, E), 128, 0, h->stream>>>(h->d_xs, h->d_ys, h->d_idx, steps, h->d_step, t0, B, h->out_pad, l0.h,
-                                                    l0.ht, h->d_t);
-        if (!rc) rc = enqueue_fwd_bwd(h, h->d_step_loss);
-        if (!rc) rc = enqueue_adam(h);
-        if (!rc) k_step_end<<<1, 1, 0, h->stream>>>(h->d_step);
-    }
-    cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
-    if (rc) return rc;
-    if (ce != cudaSuccess) { h->err = std::string("capture: ") + cudaGetErrorString(ce); return EPI_ERR_CUDA; }
-    ce = cudaGraphInstantiate(&h->step_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (ce != cudaSuccess) { h->err = std::string("instantiate: ") + cudaGetErrorString(ce); return EPI_ERR_CUDA; }
-    // kernels per step (each covering all members): gather, L forward + L weight + (L - 1)
-    // input products, L bias reductions, L Adam updates, the step counter
-    const uint64_t per_step = 2 + 4 * (uint64_t)h->L + (h->L - 1);
-    for (uint32_t s = 0; s < steps; ++s) {
-        MCK(cudaGraphLaunch(h->step_graph, h->stream));
-        MCK(cudaMemcpyAsync(h->d_loss + (size_t)s * E, h->d_step_loss, E * sizeof(float), cudaMemcpyDeviceToDevice,
-                            h->stream));
-        h->launches += per_step;
+    MCK(cudaMemsetAsync(h->d_loss, 0, (size_t)steps * E * sizeof(float), h->stream));
+    if (steps >= kGroupSteps) MRC(step_graph(h, kGroupSteps, &h->group_graph));
+    if (steps % kGroupSteps) MRC(step_graph(h, 1, &h->step_graph));
+    const AdamHyper hp{h->cfg.lr, h->cfg.beta1, h->cfg.beta2, h->cfg.eps};
+    for (uint32_t s0 = 0; s0 < steps; s0 += h->chunk) {
+        const uint32_t n = std::min(h->chunk, steps - s0);
+        const uint32_t* idx0 = h->d_idx + (size_t)s0 * E * B;
+        k_train_chunk<<<1, 128, 0, h->stream>>>(h->d_tr, idx0, h->d_ys, h->d_loss + (size_t)s0 * E, h->d_corr, n,
+                                                h->adam_steps, hp);
+        h->adam_steps += n;  // Adam's t keeps counting across calls
+        k_gather<<<dim3(n * B / 32u, E), 256, 0, h->stream>>>(h->d_xs, idx0, B, h->chunk * B, h->layers[0].h,
+                                                              h->layers[0].ht);
+        MCK(cudaGetLastError());
+        for (uint32_t k = 0; k < n;) {
+            const uint32_t g = n - k >= kGroupSteps ? kGroupSteps : 1u;
+            MCK(cudaGraphLaunch(g == kGroupSteps ? h->group_graph : h->step_graph, h->stream));
+            h->launches += 2 * (uint64_t)h->L * g + 1;
+            k += g;
+        }
+        h->launches += 2;
     }
     MRC(check_err(h));
     if (losses) {
@@ -734,32 +849,22 @@ int epi_mlp_gradients(epi_mlp* h, const float* x, const float* y, uint32_t n, fl
     MCK(cudaStreamSynchronize(h->stream));
     const uint32_t E = h->E;
     MlpLayer& l0 = h->layers[0];
-    std::vector<__nv_bfloat16> xs = pad_inputs(x, n, n, h->cfg.in_dim), xt((size_t)kInPad * n);
-    for (uint32_t r = 0; r < n; ++r)
-        for (uint32_t c = 0; c < kInPad; ++c) xt[(size_t)c * n + r] = xs[(size_t)r * kInPad + c];
-    std::vector<float> ys((size_t)n * h->out_pad, 0.f);
-    for (uint32_t i = 0; i < n; ++i)
-        std::memcpy(&ys[(size_t)i * h->out_pad], y + (size_t)i * h->cfg.out_dim, h->cfg.out_dim * sizeof(float));
-    for (uint32_t m = 0; m < E; ++m) {  // every member sees the same minibatch
-        MCK(cudaMemcpyAsync(l0.h + (size_t)m * xs.size(), xs.data(), xs.size() * sizeof(__nv_bfloat16),
-                            cudaMemcpyHostToDevice, h->stream));
-        MCK(cudaMemcpyAsync(l0.ht + (size_t)m * xt.size(), xt.data(), xt.size() * sizeof(__nv_bfloat16),
-                            cudaMemcpyHostToDevice, h->stream));
-        MCK(cudaMemcpyAsync(h->d_t + (size_t)m * ys.size(), ys.data(), ys.size() * sizeof(float), cudaMemcpyHostToDevice,
-                            h->stream));
+    // every member sees the same minibatch: row 0.. of the chunk buffers, member 0's
+    MRC(upload_inputs(h, x, n, n, l0.h, l0.ht, h->chunk * h->B));
+    MRC(upload_targets(h, y, n, h->d_t));
+    if (E > h->loss_cap) {
+        cudaFree(h->d_loss);
+        h->d_loss = nullptr;
+        h->loss_cap = 0;
+        MCK(cudaMalloc(&h->d_loss, E * sizeof(float)));
+        h->loss_cap = E;
     }
-    float* d_l = nullptr;
-    MCK(cudaMalloc(&d_l, E * sizeof(float)));
-    MCK(cudaMemsetAsync(d_l, 0, E * sizeof(float), h->stream));
-    int rc = enqueue_fwd_bwd(h, d_l);
-    if (!rc) rc = check_err(h);
+    MCK(cudaMemsetAsync(h->d_loss, 0, E * sizeof(float), h->stream));
+    k_train_chunk<<<1, 1, 0, h->stream>>>(h->d_tr, nullptr, nullptr, nullptr, nullptr, 0u, 0u, AdamHyper{});
+    MRC(enqueue_step(h, 0, true));
     std::vector<float> lsum(E, 0.f);
-    if (!rc && cudaMemcpy(lsum.data(), d_l, E * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) rc = EPI_ERR_CUDA;
-    cudaFree(d_l);
-    if (rc) {
-        if (rc == EPI_ERR_CUDA && h->err.empty()) h->err = "gradients: device copy failed";
-        return rc;
-    }
+    MCK(cudaMemcpyAsync(lsum.data(), h->d_loss, E * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    MRC(check_err(h));
     if (loss)
         for (uint32_t m = 0; m < E; ++m) loss[m] = lsum[m] / ((float)n * (float)h->cfg.out_dim);
     return download_params(h, &MlpLayer::gw, &MlpLayer::gb, grads);
@@ -769,15 +874,14 @@ int epi_mlp_predict(epi_mlp* h, const float* x, uint32_t n, float* y) {
     if (!h || !x || !y) return EPI_ERR_ARG;
     if (n == 0) return EPI_OK;
     MRC(forward_n(h, x, n, nullptr));
+    const size_t floats = (size_t)h->E * n * h->cfg.out_dim;
+    MRC(ensure_raw(h, floats));
+    k_unpad_rows<<<dim3(blocks_for((size_t)n * h->cfg.out_dim), h->E), kSmallThreads, 0, h->stream>>>(
+        h->d_py, n, h->cfg.out_dim, h->out_pad, (size_t)h->p_cap * h->out_pad, h->d_raw);
+    MCK(cudaGetLastError());
+    h->launches++;
+    MCK(cudaMemcpyAsync(y, h->d_raw, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     MRC(check_err(h));
-    const size_t per = (size_t)h->p_cap * h->out_pad;
-    std::vector<float> tmp((size_t)n * h->out_pad);
-    for (uint32_t m = 0; m < h->E; ++m) {
-        MCK(cudaMemcpy(tmp.data(), h->d_py + m * per, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost));
-        float* ym = y + (size_t)m * n * h->cfg.out_dim;
-        for (uint32_t i = 0; i < n; ++i)
-            std::memcpy(ym + (size_t)i * h->cfg.out_dim, &tmp[(size_t)i * h->out_pad], h->cfg.out_dim * sizeof(float));
-    }
     return EPI_OK;
 }
 

@@ -1,5 +1,6 @@
-// tc_gemm.cuh -- BF16 matrix products on the sm_103a tensor cores (tcgen05 + TMA), with the
-// fused epilogues of the surrogate MLP.
+// tc_gemm.cuh -- BF16 matrix products on the sm_103a tensor cores (tcgen05 + TMA): the
+// building blocks of the surrogate MLP's kernels, and its inference products with their fused
+// epilogues (training's are in tc_train.cuh).
 //
 // D[m][n] = sum_k A[m][k] * B[n][k]: A is M x K and B is N x K, both row-major BF16 with K
 // contiguous ("K-major").  One CTA of 128 threads computes a 128 x BN tile of D:
@@ -27,44 +28,30 @@ constexpr uint32_t kSpinLimit = 1u << 22;  // polls (about 0.3 s with the back-o
 
 // Epilogues.
 enum Epilogue : int {
-    kEpHidden = 0,  // x = acc + bias; z = x (fp32, optional); out = gelu(x) (bf16) and out_t = its transpose
-    kEpOut = 1,     // x = acc + bias; outf = x (optional); with targets: loss += (x - t)^2 and
-                    // out/out_t = bf16(2 (x - t) / (rows * outputs)); with a score target: score[m] += (x - s)^2
-    kEpDh = 2,      // out/out_t = bf16(acc * gelu'(zin))
-    kEpDw = 3       // outf = acc (fp32)
+    kEpHidden = 0,  // x = acc + bias; out = gelu(x) (bf16)
+    kEpOut = 1      // x = acc + bias; outf = x (optional); with a score target: score[m] += (x - s)^2
 };
 
 // Pointers are those of member 0 of a stack of networks; member m (blockIdx.z) adds m times
-// the ms_* element stride of each (0: shared by all members).
+// the ms_* element stride of each.
 struct EpiArgs {
     const float* bias = nullptr;        // [N]
-    float* z = nullptr;                 // [M x N]
-    const float* zin = nullptr;         // [M x N]
     __nv_bfloat16* out = nullptr;       // [M x N]
-    __nv_bfloat16* out_t = nullptr;     // [N x M]
     float* outf = nullptr;              // [M x N]
-    const float* target = nullptr;      // [M x N] training targets (padding columns ignored)
     const float* score_target = nullptr;  // [n_valid]
-    float* loss = nullptr;              // one float, accumulated
     float* score = nullptr;             // [M], accumulated
     uint32_t n_valid = 0;               // real output columns
     uint32_t m_valid = 0;               // real sample rows
-    float grad_scale = 0.f;
-    uint64_t ms_bias = 0, ms_z = 0, ms_zin = 0, ms_out = 0, ms_outf = 0, ms_target = 0, ms_score = 0, ms_loss = 0;
+    uint64_t ms_bias = 0, ms_out = 0, ms_outf = 0, ms_score = 0;
 };
 
 // The member-m view of a.
 __device__ __forceinline__ EpiArgs member_args(const EpiArgs& a, uint32_t m) {
     EpiArgs b = a;
     if (b.bias) b.bias += m * a.ms_bias;
-    if (b.z) b.z += m * a.ms_z;
-    if (b.zin) b.zin += m * a.ms_zin;
     if (b.out) b.out += m * a.ms_out;
-    if (b.out_t) b.out_t += m * a.ms_out;  // both orientations hold M x N elements
     if (b.outf) b.outf += m * a.ms_outf;
-    if (b.target) b.target += m * a.ms_target;
     if (b.score) b.score += m * a.ms_score;
-    if (b.loss) b.loss += m * a.ms_loss;
     return b;
 }
 
@@ -93,6 +80,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (it >= 64) __nanosleep(32);
     }
     return false;
+}
+
+// The warp's number as a warp-uniform value, and one lane of a converged warp.  The roles below
+// are whole warps that branch uniformly and elect a lane only for the instruction itself: a
+// role that was a single thread of a diverged warp took 192 ns to issue the four MMAs of a K
+// block (their descriptors go through uniform registers) and 370 ns a block in all.
+__device__ __forceinline__ uint32_t uniform_warp() { return __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0u;
+}
+// Bounded wait of a whole warp: true on all lanes or on none.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity));
 }
 
 // Tile (x, y) of member z of a 3-D tensor map {K, rows, members}.
@@ -162,74 +164,32 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }
 
 template <int EP>
-__device__ __forceinline__ void epilogue16(const EpiArgs& a, uint32_t M, uint32_t N, uint32_t m, uint32_t n,
-                                           const float v[16], float& lsum, float& ssum) {
-    if (EP == kEpDw) {
-        float4* o = reinterpret_cast<float4*>(a.outf + (size_t)m * N + n);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        return;
-    }
+__device__ __forceinline__ void epilogue16(const EpiArgs& a, uint32_t N, uint32_t m, uint32_t n, const float v[16],
+                                           float& ssum) {
     float x[16];
-    __align__(16) __nv_bfloat16 hb[16];
-    bool write_bf16 = true;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = v[j] + __ldg(a.bias + n + j);
     if (EP == kEpHidden) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = v[j] + __ldg(a.bias + n + j);
-        if (a.z) {
-            float4* o = reinterpret_cast<float4*>(a.z + (size_t)m * N + n);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) o[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-        }
+        __align__(16) __nv_bfloat16 hb[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) hb[j] = __float2bfloat16_rn(gelu(x[j]));
-    } else if (EP == kEpOut) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = v[j] + __ldg(a.bias + n + j);
-        if (a.outf) {
-            float4* o = reinterpret_cast<float4*>(a.outf + (size_t)m * N + n);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) o[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-        }
-        const bool row_ok = m < a.m_valid;
-        if (a.score_target && row_ok) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (n + j < a.n_valid) {
-                    const float e = x[j] - __ldg(a.score_target + n + j);
-                    ssum += e * e;
-                }
-        }
-        write_bf16 = a.target != nullptr;
-        if (write_bf16) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                float d = 0.f;
-                if (row_ok && n + j < a.n_valid) d = x[j] - __ldg(a.target + (size_t)m * N + n + j);
-                lsum += d * d;
-                hb[j] = __float2bfloat16_rn(d * a.grad_scale);
-            }
-        }
-    } else {  // kEpDh
-        const float4* zi = reinterpret_cast<const float4*>(a.zin + (size_t)m * N + n);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float4 zz = zi[q];
-            hb[4 * q + 0] = __float2bfloat16_rn(v[4 * q + 0] * gelu_grad(zz.x));
-            hb[4 * q + 1] = __float2bfloat16_rn(v[4 * q + 1] * gelu_grad(zz.y));
-            hb[4 * q + 2] = __float2bfloat16_rn(v[4 * q + 2] * gelu_grad(zz.z));
-            hb[4 * q + 3] = __float2bfloat16_rn(v[4 * q + 3] * gelu_grad(zz.w));
-        }
-    }
-    if (!write_bf16) return;
-    if (a.out) {
         uint4* o = reinterpret_cast<uint4*>(a.out + (size_t)m * N + n);
         o[0] = *reinterpret_cast<const uint4*>(&hb[0]);
         o[1] = *reinterpret_cast<const uint4*>(&hb[8]);
+        return;
     }
-    if (a.out_t) {  // lanes hold consecutive rows m: each column's 32 values land side by side
+    if (a.outf) {
+        float4* o = reinterpret_cast<float4*>(a.outf + (size_t)m * N + n);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) a.out_t[(size_t)(n + j) * M + m] = hb[j];
+        for (int q = 0; q < 4; ++q) o[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    }
+    if (a.score_target && m < a.m_valid) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (n + j < a.n_valid) {
+                const float e = x[j] - __ldg(a.score_target + n + j);
+                ssum += e * e;
+            }
     }
 }
 
@@ -326,21 +286,14 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
         if (lane == 0) atomicOr(err, 2);
     } else {
         const uint32_t m = m0 + warp * 32u + lane;
-        float lsum = 0.f, ssum = 0.f;
+        float ssum = 0.f;
 #pragma unroll 1
         for (uint32_t c = 0; c < (uint32_t)BN; c += 16) {
             float v[16];
             tmem_ld16(tmem + ((warp * 32u) << 16) + c, v);
-            epilogue16<EP>(args, M, N, m, n0 + c, v, lsum, ssum);
+            epilogue16<EP>(args, N, m, n0 + c, v, ssum);
         }
-        if (EP == kEpOut) {
-            if (args.score && m < args.m_valid) atomicAdd(args.score + m, ssum);
-            if (args.loss && args.target) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xFFFFFFFFu, lsum, o);
-                if (lane == 0) atomicAdd(args.loss, lsum);
-            }
-        }
+        if (EP == kEpOut && args.score && m < args.m_valid) atomicAdd(args.score + m, ssum);
     }
     tc_fence_before();
     __syncthreads();
