@@ -70,6 +70,8 @@ struct epi_engine {
     int grid_blocks = 0;       // grid of the counting kernels (k_decide, k_sleep)
     int commit_slots = kCommitSlots;  // of the launch shape (k_commit takes its work from lists)
     int resident_blocks = 0;   // SMs x resident k_decide blocks per SM
+    bool small = false;        // a world that one cluster runs (k_small)
+    bool shape_set = false;    // a launch shape was asked for: hour kernels, whatever the size
     // device
     DevParams* d_params = nullptr;
     uint32_t* d_chunk_rep = nullptr;  // null for a single replicate
@@ -95,6 +97,7 @@ struct epi_engine {
     // host
     uint32_t* h_counts = nullptr;  // pinned mirror of d_counts
     SegDev* h_seg = nullptr;       // pinned staging of d_seg and d_ivn
+    int* h_err = nullptr;          // (in the same allocation, as is h_ivn)
     uint32_t* h_ivn = nullptr;
     int halt_row = -1;             // chain offset of the row the guard marked in the last chain
     cudaStream_t stream = nullptr;
@@ -348,11 +351,39 @@ static CommitKernel commit_kernel(bool patch, bool ensemble) {
 
 // The hours of day 7..22 write positions and occupancy to the other buffers, 16 a day, so the
 // buffer that holds the state after hour x is the parity of the number of such hours among
-// 1..x: a function of x mod 24.  The other hours patch the current buffers in place.
+// 1..x (hour_parity): a function of x mod 24.  The other hours patch the current buffers.
 static bool rebuild_hour(uint32_t hod) { return hod >= 7u && hod <= 22u; }
-static uint32_t hour_parity(uint32_t hod) { return (hod >= 7u ? std::min(hod, 22u) - 6u : 0u) & 1u; }
 static uint32_t* pos_buf(const epi_engine* h, uint32_t par) { return h->d_pos + (size_t)par * h->slots; }
 static uint32_t* occ_buf(const epi_engine* h, uint32_t par) { return h->d_occ + (size_t)par * h->occ_words; }
+
+static uint32_t small_threads(uint32_t n) {
+    return ((n + kSmallCluster - 1) / kSmallCluster + 31u) / 32u * 32u;
+}
+
+// Whether one cluster runs the world's hours: an agent per thread, a bit plane that the cluster
+// zeroes in a few stores per thread, and a device that schedules clusters of 16 CTAs.
+static bool fits_small(uint32_t n, size_t occ_words) {
+    if (n > kSmallAgents || occ_words > 16u * (size_t)kSmallCluster * small_threads(n)) return false;
+    if (cudaFuncSetAttribute(k_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSmallCluster);
+    cfg.blockDim = dim3(small_threads(n));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kSmallCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_small, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
+}
 
 // The arrays of a launch that starts from buffer par.
 static HourBuffers hour_buffers(const epi_engine* h, uint32_t par) {
@@ -482,6 +513,7 @@ static int piece_graph(epi_engine* h, uint32_t first_hour, uint32_t nh, cudaGrap
 }
 
 static int check_error_flag(epi_engine* h);
+static int report_error_flag(epi_engine* h, int e);
 
 // Replicate r's state in the buffers of parity par, and its other bit plane zero, as the hours
 // want it (a chain that starts out of step: a restore, hours run out of order).
@@ -504,31 +536,9 @@ static int move_to_buffer(epi_engine* h, uint32_t r, uint32_t par) {
 // fresh engine's 1M-agent 4,800-hour run 1.5 % faster than eight-day ones, at equal speed once warm.
 constexpr uint32_t kPieceHours = 24u * 2u;
 
-// Simulate hours first_hour .. first_hour + nh - 1 for every active replicate as one chain:
-// pieces of whole days, launched back to back with one host synchronisation at the end
-// (after each piece when profiling, whose events are read per launch).  The
-// counts of hour k of replicate r land in h_counts[(k * R + r) * 8 ..]; in the run loop,
-// h->halt_row is the chain offset of a row the guard marked, or -1.
-static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
-    h->halt_row = -1;
-    if (nh == 0) return EPI_OK;
-    if ((uint64_t)first_hour + nh > 0xFFFFFFFFull) { h->err = "hour out of range"; return EPI_ERR_ARG; }
-    int rc = ensure_counts(h, nh);
-    if (rc) return rc;
-    // claims left by an earlier hour of another window, or by a later hour, must go first
-    if (h->last_claim_hour >= 0 &&
-        ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
-        CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
-    h->last_claim_hour = (int64_t)first_hour + nh - 1;
-    // the chain reads the state after first_hour - 1 from its parity's buffers
-    const uint32_t need = hour_parity((first_hour + 23u) % 24u);
-    std::vector<uint8_t> ran(h->R(), 0);  // a world whose run has ended runs no hour kernel
-    for (uint32_t r = 0; r < h->R(); ++r) {
-        if (!h->reps[r].active) continue;
-        ran[r] = 1;
-        rc = move_to_buffer(h, r, need);
-        if (rc) return rc;
-    }
+// The chain's hours as captured pieces, launched back to back; the counts rows land in h_counts.
+static int run_pieces(epi_engine* h, uint32_t first_hour, uint32_t nh) {
+    int rc = EPI_OK;
     const size_t row_words = (size_t)h->R() * 8;
     CK(cudaMemsetAsync(h->d_counts, 0, (size_t)nh * row_words * sizeof(uint32_t), h->stream));
     if (h->stream_file) CK(cudaMemsetAsync(h->d_exc_n, 0, (size_t)nh * sizeof(uint32_t), h->stream));
@@ -561,12 +571,93 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     CK(cudaMemcpyAsync(h->h_counts, h->d_counts, (size_t)nh * row_words * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                        h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    return check_error_flag(h);
+}
+
+// The chain's hours of a small world in one launch (k_small), which writes the counts rows to
+// pinned memory itself: one launch and one wait per call, where a captured piece takes a copy
+// of the hour base, the graph, and two copies back with a wait each.
+static int run_small(epi_engine* h, uint32_t first_hour, uint32_t nh) {
+    const Replica& rep = h->reps[0];
+    SmallArgs a;
+    a.pos = pos_buf(h, rep.par);
+    for (uint32_t k = 0; k < 2; ++k) {
+        a.pos_buf[k] = pos_buf(h, k);
+        a.occ_buf[k] = occ_buf(h, k);
+    }
+    a.st = h->d_st;
+    a.home = h->d_home;
+    a.work = h->d_work;
+    a.wsa = h->d_wsa;
+    a.cls = h->d_cls;
+    a.danger = h->d_danger;
+    a.claim = h->d_claim;
+    a.occ_words = (uint32_t)h->occ_words;
+    a.first = first_hour;
+    a.hours = nh;
+    a.run_loop = h->stop_rule ? 1u : 0u;
+    a.ivn = h->d_ivn;
+    a.rows = h->h_counts;
+    a.err = h->d_err;
+    a.err_out = h->h_err;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSmallCluster);
+    cfg.blockDim = dim3(small_threads(rep.n));
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kSmallCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    *h->h_err = 0;
+    CK(cudaLaunchKernelEx(&cfg, k_small, (const DevParams*)h->d_params, a));
+    h->kernels_launched += 1;
+    CK(cudaStreamSynchronize(h->stream));
+    return report_error_flag(h, *h->h_err);
+}
+
+// Simulate hours first_hour .. first_hour + nh - 1 for every active replicate as one chain:
+// pieces of whole days, launched back to back with one host synchronisation at the end
+// (after each piece when profiling, whose events are read per launch).  The
+// counts of hour k of replicate r land in h_counts[(k * R + r) * 8 ..]; in the run loop,
+// h->halt_row is the chain offset of a row the guard marked, or -1.
+static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
+    h->halt_row = -1;
+    if (nh == 0) return EPI_OK;
+    if ((uint64_t)first_hour + nh > 0xFFFFFFFFull) { h->err = "hour out of range"; return EPI_ERR_ARG; }
+    int rc = ensure_counts(h, nh);
+    if (rc) return rc;
+    const bool small = h->small && !h->shape_set && !h->profiling && !h->stream_file;
+    // claims left by an earlier hour of another window, or by a later hour, must go first (all
+    // of them where the hours use the agents' bare indices)
+    if (h->last_claim_hour >= 0 && small)
+        CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
+    else if (h->last_claim_hour >= 0 &&
+        ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
+        CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
+    h->last_claim_hour = small ? -1 : (int64_t)first_hour + nh - 1;
+    // the chain reads the state after first_hour - 1 from its parity's buffers
+    const uint32_t need = hour_parity((first_hour + 23u) % 24u);
+    std::vector<uint8_t> ran(h->R(), 0);  // a world whose run has ended runs no hour kernel
+    for (uint32_t r = 0; r < h->R(); ++r) {
+        if (!h->reps[r].active) continue;
+        ran[r] = 1;
+        rc = move_to_buffer(h, r, need);
+        if (rc) return rc;
+    }
+    const size_t row_words = (size_t)h->R() * 8;
+    if (small) {
+        rc = run_small(h, first_hour, nh);
+        if (rc) return rc;
+    } else {
+        rc = run_pieces(h, first_hour, nh);
+        if (rc) return rc;
+    }
     for (uint32_t k = 1; k < nh; ++k)
         if (sleep_hour_skipped(first_hour, k))
             std::memcpy(h->h_counts + (size_t)k * row_words, h->h_counts + (size_t)(k - 1) * row_words,
                         row_words * sizeof(uint32_t));
-    rc = check_error_flag(h);
-    if (rc) return rc;
     std::vector<uint8_t> ended(h->R(), 0);  // stop rule met at an earlier hour of this chain
     std::vector<uint32_t> last(h->R(), nh - 1);  // the last row whose hour ran
     for (uint32_t k = 0; k < nh && h->halt_row < 0; ++k) {
@@ -598,6 +689,10 @@ static int check_error_flag(epi_engine* h) {
     int e = 0;
     CK(cudaMemcpyAsync(&e, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    return report_error_flag(h, e);
+}
+
+static int report_error_flag(epi_engine* h, int e) {
     if (e) {
         h->err = "device invariant violated (flag " + std::to_string(e) + "): a rule addressed a cell outside the plane";
         return EPI_ERR_INVARIANT;
@@ -868,7 +963,6 @@ static void free_device(epi_engine* h) {
     cudaFree(h->s_pos); cudaFree(h->s_wsa); cudaFree(h->s_st); cudaFree(h->s_occ); cudaFree(h->s_cls); cudaFree(h->s_danger);
     if (h->h_counts) cudaFreeHost(h->h_counts);
     if (h->h_seg) cudaFreeHost(h->h_seg);
-    if (h->h_ivn) cudaFreeHost(h->h_ivn);
     for (auto& pe : h->pending)
         if (pe.pooled) { cudaEventDestroy(pe.begin); cudaEventDestroy(pe.end); }
     for (auto e : h->event_pool) cudaEventDestroy(e);
@@ -1042,8 +1136,10 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     CK(cudaMemset(h->d_ivn, 0, R * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_err, sizeof(int)));
     CK(cudaMalloc(&h->d_scratch, 6 * sizeof(unsigned long long)));
-    CK(cudaMallocHost(&h->h_seg, sizeof(SegDev)));
-    CK(cudaMallocHost(&h->h_ivn, R * sizeof(uint32_t)));
+    CK(cudaMallocHost(&h->h_seg, sizeof(SegDev) + sizeof(int) + R * sizeof(uint32_t)));  // with h_err and h_ivn
+    h->h_err = reinterpret_cast<int*>(h->h_seg + 1);
+    h->h_ivn = reinterpret_cast<uint32_t*>(h->h_err + 1);
+    h->small = R == 1 && fits_small(h->reps[0].n, h->occ_words);
     int rc = ensure_counts(h, 48);
     if (rc) return rc;
     if (!recs) {
@@ -1185,6 +1281,7 @@ static int set_launch_shape(epi_engine* h, uint32_t decide_blocks, uint32_t comm
     CK(cudaStreamSynchronize(h->stream));
     h->grid_blocks = (int)decide_blocks;
     h->commit_slots = (int)commit_slots;
+    h->shape_set = true;
     destroy_graphs(h);  // they bake the launch shapes in
     return EPI_OK;
 }
@@ -1213,8 +1310,11 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
     if (rc) return rc;
     double best = 1e300;
     uint32_t best_g = (uint32_t)h->grid_blocks;
+    bool best_small = false;
+    if (h->small) grids.insert(grids.begin(), 0u);  // 0: no shape asked for, one cluster runs the hours
     for (uint32_t g : grids) {
-        rc = set_launch_shape(h, g, (uint32_t)h->commit_slots);
+        if (g) rc = set_launch_shape(h, g, (uint32_t)h->commit_slots);
+        else h->shape_set = false;
         double t_min = 1e300;
         for (int rep = 0; rep < 5 && !rc; ++rep) {  // the first pass captures the graphs
             rc = restore_state(h);
@@ -1225,10 +1325,15 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
             if (rep > 0) t_min = std::min(t_min, t);
         }
         if (rc) break;
-        if (t_min < best) { best = t_min; best_g = g; }
+        if (t_min < best) {
+            best = t_min;
+            best_small = g == 0u;
+            if (g) best_g = g;
+        }
     }
     h->profiling = prof;
     int rc2 = set_launch_shape(h, best_g, (uint32_t)h->commit_slots);
+    if (best_small) h->shape_set = false;
     if (!rc2) rc2 = restore_state(h);
     h->kernels_launched = launched;
     if (rc) return rc;

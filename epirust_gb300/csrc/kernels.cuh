@@ -269,7 +269,7 @@ struct AgentHour {
 // The rules of one agent for the hour: proposal, claim, infection update, state and position
 // words.  next is the replicate's zeroed bit plane, pos_next the other position buffer.
 template <int HC, bool PATCH>
-__device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitView& pl, const StepTable& steps,
+__device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitView<>& pl, const StepTable& steps,
                                                   uint32_t* __restrict__ next,
                                                   uint32_t* __restrict__ rclaim, uint32_t* __restrict__ wsa,
                                                   uint2* __restrict__ st, uint32_t* pos, uint32_t* pos_next, uint32_t slot,
@@ -382,7 +382,7 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
     if (!ENS) {
         if (blockIdx.x < n_chunks) switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
         if (blockIdx.x < n_chunks && P.active && !run_ended(prev_ptr(ha, hr.row), 0u)) {
-            const BitView pl{B.occ, B.cls, B.danger, P.G, P.WP, P.PW, B.err};
+            const BitView<> pl{B.occ, B.cls, B.danger, P.G, P.WP, P.PW, B.err};
             const uint32_t n = P.n;
             for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
                 const uint32_t slot = c * kChunk + threadIdx.x;  // = agent index (a lone world starts at slot 0)
@@ -432,7 +432,7 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                 ended = run_ended(prev_ptr(ha, hr.row), r);  // an earlier row: fixed during the launch
             }
             if (!P.active || ended) continue;
-            const BitView pl{B.occ + P.occ_off, B.cls + P.plane_off, B.danger + P.plane_off, P.G, P.WP, P.PW, B.err};
+            const BitView<> pl{B.occ + P.occ_off, B.cls + P.plane_off, B.danger + P.plane_off, P.G, P.WP, P.PW, B.err};
             const uint32_t i = slot - P.agent_off;  // index within the replicate
             const bool valid = i < P.n;
             const uint32_t s = valid ? sv.x : 0u, at = valid ? sv.y : 0u, p = valid ? pw : 0u;
@@ -550,6 +550,223 @@ __global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict
     if (next / kClaimWindow != hr.hour / kClaimWindow)
         for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < claim_cells; i += (size_t)gridDim.x * kThreads)
             B.claim[i] = kNoClaim;
+}
+
+// ---------------------------------------------------------------- small worlds
+// A world of a few thousand agents spends an hour on launches and latency: two launches of at
+// most 64 blocks, each a chain of dependent L2 round trips behind a launch.  One cluster runs
+// all hours of a chain instead: an agent per thread, its words in registers from hour to hour,
+// and two hardware cluster barriers per hour where the launches were.  One GB300, a waking
+// hour by launches / in one cluster: 2,000 agents 8.4 / 3.0 us, 10,000 8.0 / 5.2 us, 16,000
+// 8.6 / 6.1 us; of the 5.2 us the barriers with the atomics they wait for take 1.9, proposals
+// 1.6, the claims read back 0.5.  (A second agent per thread would reach 32,768 agents at an
+// extrapolated 9 us, no faster than the launches.)
+//   before the first   proposals, an atomicMin of the agent's index on the target's claim word,
+//                      infection update, counts
+//   between them       a mover reads its claim word back: it holds its index (it moves, and
+//                      frees the word) or not (a lower index has it, or the winner has already
+//                      freed it: it stays); occupancy bits and class planes are written, the
+//                      spent bit plane zeroed
+// Data that other SMs write is read at L2 (BitView<true>, __ldcg).  The counts of the hour are
+// summed in the first CTA's shared memory, where every CTA reads the stop rule and the run
+// loop's guard, and go to the caller's rows (pinned host memory) from there.
+constexpr uint32_t kSmallCluster = 16;
+constexpr uint32_t kSmallThreads = 1024;
+constexpr uint32_t kSmallAgents = kSmallCluster * kSmallThreads;  // most agents of a world run so
+
+struct SmallArgs {
+    uint32_t* pos;        // the buffer that holds the positions before the first hour
+    uint32_t* pos_buf[2];
+    uint32_t* occ_buf[2];
+    uint2* st;
+    const uint32_t *home, *work;
+    uint32_t* wsa;
+    uint8_t *cls, *danger;
+    uint32_t* claim;      // all kNoClaim, before and after
+    uint32_t occ_words;
+    uint32_t first, hours;
+    uint32_t run_loop;    // 1: the stop rule and the guard apply
+    uint32_t* ivn;        // the guard's new-infections figure
+    uint32_t* rows;       // hours x 8: bins, word 6 the halt mark; rows that did not run are zero
+    int* err;             // device error word
+    int* err_out;         // where the caller reads it
+};
+
+// The hours of day 7..22 write the other buffer, 16 a day (engine.cu: hour_parity).
+__host__ __device__ constexpr uint32_t hour_parity(uint32_t hod) {
+    return (hod >= 7u ? (hod < 22u ? hod : 22u) - 6u : 0u) & 1u;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The shared-memory address of p in the cluster's first CTA.
+__device__ __forceinline__ uint32_t in_first_cta(const void* p) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return a;
+}
+__device__ __forceinline__ void add_in_cluster(uint32_t addr, uint32_t v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t load_in_cluster(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// One movement hour of a lane's agent up to its claim and infection update (hours 7..22).
+template <int HC>
+__device__ __forceinline__ Cell small_move(const DevParams& P, const BitView<true>& pl, const StepTable& steps, uint32_t& s,
+                                           uint32_t* wsa, uint32_t hm, uint32_t wk, Cell cell, uint32_t hour, Draws& dr,
+                                           bool& infect) {
+    return perform_movements<HC>(P, pl, steps, s, wsa, hm, wk, cell, hour, dr, infect);
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __restrict__ Pall, const __grid_constant__ SmallArgs a) {
+    __shared__ uint32_t sh[8];
+    __shared__ uint32_t total[3][8];  // the first CTA's are the cluster's
+    __shared__ DevParams sP;
+    __shared__ StepTable steps;
+    const DevParams& P = sP;
+    const uint32_t rank = cluster_rank(), tid = threadIdx.x, i = rank * blockDim.x + tid;
+    stage_steps(steps);
+    for (uint32_t k = tid; k < sizeof(DevParams) / 4; k += blockDim.x)
+        reinterpret_cast<uint32_t*>(&sP)[k] = reinterpret_cast<const uint32_t*>(Pall)[k];
+    if (tid < 8) sh[tid] = total[0][tid] = total[1][tid] = total[2][tid] = 0u;
+    cluster_sync();  // every CTA of the cluster runs, and its counters are clear
+    const uint32_t sums = in_first_cta(&total[0][0]);
+    const bool valid = i < P.n;
+    uint32_t s = 0u, at = 0u, p = 0u, hm = 0u, wk = 0u;
+    if (valid) {
+        const uint2 sv = a.st[i];
+        s = sv.x;
+        at = sv.y;
+        p = a.pos[i];
+        hm = a.home[i];
+        wk = a.work[i];
+    }
+    uint32_t ivn = a.run_loop ? *a.ivn : 0u;
+    uint32_t slot = 0u;        // of total: the hour running
+    uint32_t last = a.first;   // the last hour that ran
+    uint32_t written = 0u;     // rows written by the first CTA
+    bool over = !P.active;
+    for (uint32_t k = 0; k < a.hours && !over; ++k) {
+        const uint32_t hour = a.first + k, hod = hour % 24u;
+        if (k > 0 && hod >= 2u && hod <= 6u) {  // hour 1 has sent everyone home: nothing changes
+            if (rank == 0 && tid < 8) a.rows[(size_t)k * 8u + tid] = 0u;
+            written = k + 1u;
+            last = hour;
+            continue;
+        }
+        Tally tally;
+        const uint32_t s0 = s;
+        if (hod >= 1u && hod <= 6u) {
+            if (valid && st_ws(s) != EPI_WS_HOSPITAL_STAFF) s = with_area(s, kHome);
+            tally.add(valid, count_bin(s));
+            tally.flush(sh);
+            cluster_sync();
+            if (tid < 6u) {
+                add_in_cluster(sums + (slot * 8u + tid) * 4u, sh[tid]);
+                sh[tid] = 0u;
+            }
+            cluster_sync();
+        } else {
+            const bool patch = hod == 0u || hod == 23u;
+            uint32_t* occ = a.occ_buf[hour_parity((hod + 23u) % 24u)];
+            uint32_t* next = a.occ_buf[hour_parity(hod)];
+            const BitView<true> pl{occ, a.cls, a.danger, P.G, P.WP, P.PW, a.err};
+            Cell cell{unpack_x(p), unpack_y(p)}, nc = cell;
+            Draws dr{i, hour, P.key0, P.key1, P.move_key};
+            bool infect = false;
+            if (hod == 0u) {
+                const bool need = valid && wants_hospital(P, infected(s) ? with_day(s, st_day(s) + 1u) : s);
+                const uint32_t hosp_first = __syncthreads_or(need) ? block_first_vacant(P, pl) : kNoAction;
+                if (valid) nc = routine_start(P, pl, s, hm, cell, hosp_first, dr);
+            } else if (valid) {
+                switch (hour_class(hod)) {
+                    case kHcEnd: nc = routine_end(P, pl, s, hm, cell, dr); break;
+                    case kHcTransport: nc = small_move<kHcTransport>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                    case kHcWork: nc = small_move<kHcWork>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                    case kHcNoon: nc = small_move<kHcNoon>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                    case kHcHome: nc = small_move<kHcHome>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                    default: nc = small_move<kHcMove>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                }
+            }
+            const bool moving = nc.x != cell.x || nc.y != cell.y;
+            uint32_t* claim = &a.claim[(size_t)nc.y * P.W + nc.x];
+            if (moving) atomicMin(claim, i);
+            if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
+            tally.add(valid, count_bin(s));
+            tally.flush(sh);
+            cluster_sync();  // every claim is in, and the bit plane of before has been read
+            if (tid < 6u) {
+                add_in_cluster(sums + (slot * 8u + tid) * 4u, sh[tid]);
+                sh[tid] = 0u;
+            }
+            bool win = false;
+            if (moving) {
+                win = __ldcg(claim) == i;
+                if (win) atomicMax(claim, kNoClaim);  // (not a plain store: see send_back)
+            }
+            const uint32_t q = win ? pack_xy(nc.x, nc.y) : p;
+            const uint32_t Xo = (uint32_t)cell.x + 1u, X = (uint32_t)unpack_x(q) + 1u;
+            uint32_t* word = &next[((uint32_t)unpack_y(q) + 1u) * P.PW + (X >> 5)];
+            if (patch ? win : valid) atomicOr(word, 1u << (X & 31u));
+            if (patch && win) atomicAnd(&next[((uint32_t)cell.y + 1u) * P.PW + (Xo >> 5)], ~(1u << (Xo & 31u)));
+            if (valid && (infected(s0) || infected(s))) {
+                const uint32_t cls0 = cell_class(P, s0), cls = cell_class(P, s);
+                if (win || cls != cls0) {
+                    if (cls0 >= 2u) class_add(a.cls, a.danger, (uint32_t)P.WP, p, cls0, true);
+                    if (cls >= 2u) class_add(a.cls, a.danger, (uint32_t)P.WP, q, cls, false);
+                }
+            }
+            p = q;
+            if (!patch)
+                for (uint32_t w = i; w < a.occ_words / 4u; w += kSmallCluster * blockDim.x)
+                    reinterpret_cast<uint4*>(occ)[w] = make_uint4(0u, 0u, 0u, 0u);
+            cluster_sync();
+        }
+        last = hour;
+        // the row, the stop rule and the guard, from the cluster's sums
+        const uint32_t at_sums = sums + slot * 32u;
+        const uint32_t e = load_in_cluster(at_sums + 4u), inf = load_in_cluster(at_sums + 8u), hos = load_in_cluster(at_sums + 12u);
+        bool fire = false;
+        if (a.run_loop) {
+            if (hod == 0u) {
+                const uint32_t fresh = inf > ivn ? inf - ivn : 0u;
+                ivn = fresh;
+                fire = ((P.guard_flags & kGuardLock) && inf > P.lock_threshold) ||
+                       ((P.guard_flags & kGuardSpread) && fresh >= P.spread_threshold) ||
+                       ((P.guard_flags & kGuardOccupancy) && hos >= P.occ_threshold);
+            }
+            over = fire || (e | inf | hos) == 0u;
+        }
+        if (rank == 0 && tid < 8u) {
+            a.rows[(size_t)k * 8u + tid] = tid < 6u ? total[slot][tid] : (tid == 6u && fire ? 1u : 0u);
+            // (cleared two hours before its next use: its readers have passed a barrier by then)
+            total[(slot + 2u) % 3u][tid] = 0u;
+        }
+        written = k + 1u;
+        slot = (slot + 1u) % 3u;
+    }
+    if (valid) {
+        a.st[i] = make_uint2(s, at);
+        (written ? a.pos_buf[hour_parity(last % 24u)] : a.pos)[i] = p;
+    }
+    if (rank == 0) {
+        for (uint32_t w = written * 8u + tid; w < a.hours * 8u; w += blockDim.x) a.rows[w] = 0u;
+        if (tid == 0) {
+            if (a.run_loop) *a.ivn = ivn;
+            *a.err_out = *(volatile int*)a.err;
+        }
+    }
+    cluster_sync();  // the first CTA's counters outlive their readers
 }
 
 // ---------------------------------------------------------------- the caller-owned planes

@@ -12,10 +12,15 @@ from helpers import COVID_FAST, make_config, rows_to_array
 pytestmark = pytest.mark.gpu
 
 
-def _engine(cfg):
+def _engine(cfg, hour_kernels=False):
+    """An engine of a small world runs its hours in one cluster; asked for a launch shape, with
+    the hour kernels of larger worlds."""
     from epirust_gb300 import Config, Epidemiology
 
-    return Epidemiology(Config(json.dumps(cfg)))
+    eng = Epidemiology(Config(json.dumps(cfg)))
+    if hour_kernels:
+        eng.set_launch_shape(max(1, (eng.population() + 255) // 256 - 1), 4)
+    return eng
 
 
 def _rows(r):
@@ -28,23 +33,25 @@ def _same_world(eng, sim):
 
 
 # G + 3 cells a row: one word short of a boundary, on it, one cell past it
+@pytest.mark.parametrize("hour_kernels", [False, True])
 @pytest.mark.parametrize("grid,n", [(60, 700), (61, 255), (62, 256), (92, 1700), (93, 257), (94, 2700), (125, 3000),
                                     (126, 4000)])
-def test_row_words_and_dense_claims(gpu, oracle_mod, grid, n):
+def test_row_words_and_dense_claims(gpu, oracle_mod, grid, n, hour_kernels):
     cfg = make_config(n=n, grid=grid, seed=grid * 7 + n, disease=COVID_FAST, starting=(4, 4, 4, 12), beds=0.01)
     sim = oracle_mod.O1(oracle_mod.params_from_config(cfg))
     want = rows_to_array(sim.run(1, 58, interventions=False, stop=False))
-    eng = _engine(cfg)
+    eng = _engine(cfg, hour_kernels)
     assert (_rows(eng.simulate_hours(1, 57)) == want).all()
     _same_world(eng, sim)
     eng.close()
 
 
+@pytest.mark.parametrize("hour_kernels", [False, True])
 @pytest.mark.parametrize("cuts", [(7, 8, 9, 22, 23, 24, 31), (1, 12, 13, 16, 17, 40, 47), tuple(range(1, 30))])
-def test_chains_from_either_buffer(gpu, oracle_mod, cuts):
+def test_chains_from_either_buffer(gpu, oracle_mod, cuts, hour_kernels):
     """Chains cut at hours of both parities, and hours run again after a restore."""
     cfg = make_config(n=1500, grid=93, seed=5, disease=COVID_FAST, starting=(2, 2, 4, 20))
-    eng = _engine(cfg)
+    eng = _engine(cfg, hour_kernels)
     eng.simulate_hours(1, 8)
     eng.save_state()
     for _ in range(2):
@@ -58,6 +65,37 @@ def test_chains_from_either_buffer(gpu, oracle_mod, cuts):
             first = cut
         eng.restore_state()
     eng.close()
+
+
+@pytest.mark.parametrize("n,grid", [(33, 60), (4096, 128), (16383, 260), (16384, 257), (16385, 261)])
+def test_one_cluster_equals_hour_kernels(gpu, n, grid):
+    """The run loop (lockdown, vaccination, hospital build, early stop) of the smallest and the
+    largest worlds that one cluster runs, and of one agent more, against the hour kernels; the
+    two also take over from each other in mid-run."""
+    cfg = make_config(n=n, grid=grid, hours=24 * 40, seed=n, disease=COVID_FAST, starting=(0, 0, 1, 3 + n // 500),
+                      beds=0.002, occupancy=0.5,
+                      interventions=[{"Lockdown": {"at_number_of_infections": 1 + n // 100, "essential_workers_population": 0.2}},
+                                     {"Vaccinate": {"at_hour": 300, "percent": 0.2}}])
+    one, other = _engine(cfg), _engine(cfg, hour_kernels=True)
+    one.save_state()
+    want = _rows(other.run())
+    assert (_rows(one.run()) == want).all()
+    assert (one.snapshot().view(np.uint8) == other.snapshot().view(np.uint8)).all()
+    one.check_invariants()
+    if n <= 16384:
+        assert one.kernels_launched() < other.kernels_launched() // 4
+    one.restore_state()
+    got, going = one.run_until(200)
+    one.set_launch_shape(1, 4)
+    if going:
+        got, going = one.run_until(333)
+    if going:
+        got = one.run()
+    assert (_rows(got) == want).all()
+    assert (one.snapshot().view(np.uint8) == other.snapshot().view(np.uint8)).all()
+    one.check_invariants()
+    one.close()
+    other.close()
 
 
 def test_replicates_that_end_early_keep_their_buffers(gpu):
