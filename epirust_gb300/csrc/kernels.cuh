@@ -47,6 +47,10 @@ struct Tally {
                        b2 = __ballot_sync(0xFFFFFFFFu, v & 4u);
         n += (uint32_t)__popc((b0 ^ n0) & (b1 ^ n1) & (b2 ^ n2));
     }
+    // all valid lanes in bin 0
+    __device__ __forceinline__ void add_susceptible(bool valid) {
+        n += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, valid)) & n0 & n1 & n2;
+    }
     __device__ __forceinline__ void flush(uint32_t* sh) {
         if ((threadIdx.x & 31u) < 6u && n) atomicAdd(&sh[threadIdx.x & 31u], n);
         n = 0;
@@ -112,7 +116,7 @@ __device__ __forceinline__ bool run_ended(const uint32_t* prev, uint32_t r) {
 // Switch the block to replicate r: flush the histogram of the previous one into its counts
 // row (counts[r * 8 + bin]), stage r's parameters, clear the histogram.  Block-uniform.
 __device__ __forceinline__ void switch_rep(BlockRep& br, uint32_t r, const DevParams* __restrict__ Pall, DevParams& sP,
-                                           Tally& tally, uint32_t* sh, uint32_t* counts) {
+                                           Tally& tally, uint32_t* sh, uint32_t* counts, Box* boxes = nullptr) {
     if (br.r != 0xFFFFFFFFu) tally.flush(sh);
     __syncthreads();
     if (br.r != 0xFFFFFFFFu && threadIdx.x < 6 && sh[threadIdx.x]) atomicAdd(&counts[br.r * 8 + threadIdx.x], sh[threadIdx.x]);
@@ -120,6 +124,7 @@ __device__ __forceinline__ void switch_rep(BlockRep& br, uint32_t r, const DevPa
     for (uint32_t k = threadIdx.x; k < sizeof(DevParams) / 4; k += blockDim.x)
         reinterpret_cast<uint32_t*>(&sP)[k] = reinterpret_cast<const uint32_t*>(Pall + r)[k];
     if (threadIdx.x < 8) sh[threadIdx.x] = 0;
+    if (boxes) stage_boxes(boxes, Pall[r]);
     __syncthreads();
     br.r = r;
 }
@@ -269,65 +274,56 @@ struct AgentHour {
 // The rules of one agent for the hour: proposal, claim, infection update, state and position
 // words.  next is the replicate's zeroed bit plane, pos_next the other position buffer.
 template <int HC, bool PATCH>
-__device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitView<>& pl, const StepTable& steps,
-                                                  uint32_t* __restrict__ next,
+__device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitView<>& pl, const MoveTables& tables,
+                                                  const Box* boxes, uint32_t* __restrict__ next,
                                                   uint32_t* __restrict__ rclaim, uint32_t* __restrict__ wsa,
                                                   uint2* __restrict__ st, uint32_t* pos, uint32_t* pos_next, uint32_t slot,
                                                   uint32_t i, uint32_t s, uint32_t at, uint32_t p, uint32_t hm, uint32_t wk,
                                                   uint32_t hour, uint32_t hosp_first) {
     const uint32_t s0 = s, at0 = at;
-    const Cell cell{unpack_x(p), unpack_y(p)};
     Draws dr{i, hour, P.key0, P.key1, P.move_key};
-    Cell nc;
+    uint32_t q;  // the proposal: the agent's cell, a vacant cell or a valid neighbour, so inside the plane
     bool infect = false;
-    if (HC == kHcStart) {
-        nc = routine_start(P, pl, s, hm, cell, hosp_first, dr);
-    } else if (HC == kHcEnd) {
-        nc = routine_end(P, pl, s, hm, cell, dr);
-    } else {
-        nc = perform_movements<HC>(P, pl, steps, s, wsa + slot, hm, wk, cell, hour, dr, infect);
-    }
-    // (a proposal is the agent's cell, a vacant cell or a valid neighbour: inside the plane)
-    bool moving = nc.x != cell.x || nc.y != cell.y;
+    if (HC == kHcStart) q = routine_start(P, pl, s, hm, p, hosp_first, dr);
+    else if (HC == kHcEnd) q = routine_end(P, pl, s, hm, p, dr);
+    else q = perform_movements<HC>(P, pl, tables, boxes, s, wsa + slot, hm, wk, p, hour, dr, infect);
     // The claim goes out before the infection update so that its round trip overlaps it.
     AgentHour out;
-    const uint32_t key = claim_key(hour, i);
-    const uint32_t found = moving ? atomicMin(&rclaim[(size_t)nc.y * P.W + nc.x], key) : kNoClaim;
-    if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
+    const uint32_t key = claim_key(hour, i), wanted = q;
+    const uint32_t found = q != p ? atomicMin(&rclaim[(q >> 16) * (uint32_t)P.W + (q & 0xFFFFu)], key) : kNoClaim;
+    if (infect) infection_dynamics(P, pl, tables, boxes, s, at, hm, wk, wanted, hour, dr);
     // (an untouched word looks like a key of the window's first hour, but for its index)
     if (found != kNoClaim && (found >> kClaimAgentBits) == (key >> kClaimAgentBits)) {
         const uint32_t j = found & kMaxAgentsPerWorld;
-        if (j < i) {
-            moving = false;
-            nc = cell;
-        } else {
-            out.displaces = true;
-            out.loser = P.agent_off + j;
-        }
+        out.displaces = j > i;
+        out.loser = P.agent_off + j;
+        if (j < i) q = p;
     }
-    const uint32_t q = pack_xy(nc.x, nc.y);
+    const bool moving = q != p;
     if (!PATCH) {
         if (!out.displaces) {
-            const uint32_t X = (uint32_t)nc.x + 1u;
-            atomicOr(&next[((uint32_t)nc.y + 1u) * P.PW + (X >> 5)], 1u << (X & 31u));
+            const uint32_t X = (q & 0xFFFFu) + 1u;
+            atomicOr(&next[((q >> 16) + 1u) * P.PW + (X >> 5)], 1u << (X & 31u));
         }
         pos_next[slot] = q;
     }
-    if (infected(s0) || infected(s)) {  // the planes follow its class (a healthy agent's is 1 throughout)
-        const uint32_t cls0 = cell_class(P, s0), cls = cell_class(P, s);
-        out.act = (cls0 >= 2u || cls >= 2u) && (moving || cls != cls0);
-        out.target = encode_target(nc, cls, cls0);
+    out.bin = count_bin(s);
+    if (out.bin != 0u) {  // not susceptible: infectious, perhaps, before or after
+        if (infected(s0) || infected(s)) {  // the planes follow its class (a healthy agent's is 1 throughout)
+            const uint32_t cls0 = cell_class(P, s0), cls = cell_class(P, s);
+            out.act = (cls0 >= 2u || cls >= 2u) && (moving || cls != cls0);
+            out.target = encode_target(q, cls, cls0);
+        }
     }
     if (PATCH && moving && !out.act) {
         out.act = true;
-        out.target = encode_target(nc, 1u, 1u);
+        out.target = encode_target(q, 1u, 1u);
     }
     if (PATCH && out.act) {
         pos_next[slot] = p;
         if (moving) pos[slot] = q;
     }
     if (s != s0 || at != at0) st[slot] = make_uint2(s, at);
-    out.bin = count_bin(s);
     return out;
 }
 
@@ -369,9 +365,10 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
     constexpr bool PATCH = HC == kHcStart || HC == kHcEnd;
     __shared__ uint32_t sh[8];
     __shared__ DevParams sP;
-    __shared__ StepTable steps;
+    __shared__ MoveTables tables;
+    __shared__ Box boxes[kNumAreas];
     const DevParams& P = sP;
-    if (!PATCH) stage_steps(steps);  // read after switch_rep's barriers
+    if (!PATCH) stage_tables(tables);  // read after switch_rep's barriers
     dep_wait();
     const HourRow hr = hour_row(ha);
     const uint32_t hour = hr.hour;
@@ -380,7 +377,7 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
     uint32_t hosp_first = kNoAction, n_displaced = 0u, n_acts = 0u;
     bool hosp_known = false;
     if (!ENS) {
-        if (blockIdx.x < n_chunks) switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+        if (blockIdx.x < n_chunks) switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row), boxes);
         if (blockIdx.x < n_chunks && P.active && !run_ended(prev_ptr(ha, hr.row), 0u)) {
             const BitView<> pl{B.occ, B.cls, B.danger, P.G, P.WP, P.PW, B.err};
             const uint32_t n = P.n;
@@ -403,10 +400,13 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                 }
                 AgentHour a;
                 if (valid)
-                    a = decide_agent<HC, PATCH>(P, pl, steps, B.occ_next, B.claim, B.wsa, B.st, B.pos, B.pos_next, slot, slot, s, at, p,
+                    a = decide_agent<HC, PATCH>(P, pl, tables, boxes, B.occ_next, B.claim, B.wsa, B.st, B.pos, B.pos_next, slot, slot, s, at, p,
                                                 B.home[slot], B.work[slot], hour, hosp_first);
-                tally.add(valid, a.bin);
-                if (__any_sync(0xFFFFFFFFu, a.displaces || a.act)) {
+                // most warps of a young epidemic: all susceptible, no one displaced
+                if (!__any_sync(0xFFFFFFFFu, a.bin != 0u || a.displaces || a.act)) {
+                    tally.add_susceptible(valid);
+                } else {
+                    tally.add(valid, a.bin);
                     list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
                     list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
                 }
@@ -427,7 +427,7 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
             const uint2 sv = B.st[slot];
             const uint32_t pw = B.pos[slot], hw = B.home[slot], ww = B.work[slot];
             if (r != br.r) {
-                switch_rep(br, r, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+                switch_rep(br, r, Pall, sP, tally, sh, row_ptr(ha, hr.row), boxes);
                 hosp_known = false;
                 ended = run_ended(prev_ptr(ha, hr.row), r);  // an earlier row: fixed during the launch
             }
@@ -445,10 +445,12 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
             }
             AgentHour a;
             if (valid)
-                a = decide_agent<HC, PATCH>(P, pl, steps, B.occ_next + P.occ_off, B.claim + P.claim_off, B.wsa, B.st, B.pos,
+                a = decide_agent<HC, PATCH>(P, pl, tables, boxes, B.occ_next + P.occ_off, B.claim + P.claim_off, B.wsa, B.st, B.pos,
                                             B.pos_next, slot, i, s, at, p, hw, ww, hour, hosp_first);
-            tally.add(valid, a.bin);
-            if (__any_sync(0xFFFFFFFFu, a.displaces || a.act)) {
+            if (!__any_sync(0xFFFFFFFFu, a.bin != 0u || a.displaces || a.act)) {
+                tally.add_susceptible(valid);
+            } else {
+                tally.add(valid, a.bin);
                 list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
                 list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
             }
@@ -622,20 +624,22 @@ __device__ __forceinline__ uint32_t load_in_cluster(uint32_t addr) {
 
 // One movement hour of a lane's agent up to its claim and infection update (hours 7..22).
 template <int HC>
-__device__ __forceinline__ Cell small_move(const DevParams& P, const BitView<true>& pl, const StepTable& steps, uint32_t& s,
-                                           uint32_t* wsa, uint32_t hm, uint32_t wk, Cell cell, uint32_t hour, Draws& dr,
-                                           bool& infect) {
-    return perform_movements<HC>(P, pl, steps, s, wsa, hm, wk, cell, hour, dr, infect);
+__device__ __forceinline__ uint32_t small_move(const DevParams& P, const BitView<true>& pl, const MoveTables& tables,
+                                               const Box* boxes, uint32_t& s, uint32_t* wsa, uint32_t hm, uint32_t wk,
+                                               uint32_t p, uint32_t hour, Draws& dr, bool& infect) {
+    return perform_movements<HC>(P, pl, tables, boxes, s, wsa, hm, wk, p, hour, dr, infect);
 }
 
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __restrict__ Pall, const __grid_constant__ SmallArgs a) {
     __shared__ uint32_t sh[8];
     __shared__ uint32_t total[3][8];  // the first CTA's are the cluster's
     __shared__ DevParams sP;
-    __shared__ StepTable steps;
+    __shared__ MoveTables tables;
+    __shared__ Box boxes[kNumAreas];
     const DevParams& P = sP;
     const uint32_t rank = cluster_rank(), tid = threadIdx.x, i = rank * blockDim.x + tid;
-    stage_steps(steps);
+    stage_tables(tables);
+    stage_boxes(boxes, Pall[0]);
     for (uint32_t k = tid; k < sizeof(DevParams) / 4; k += blockDim.x)
         reinterpret_cast<uint32_t*>(&sP)[k] = reinterpret_cast<const uint32_t*>(Pall)[k];
     if (tid < 8) sh[tid] = total[0][tid] = total[1][tid] = total[2][tid] = 0u;
@@ -681,27 +685,27 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
             uint32_t* occ = a.occ_buf[hour_parity((hod + 23u) % 24u)];
             uint32_t* next = a.occ_buf[hour_parity(hod)];
             const BitView<true> pl{occ, a.cls, a.danger, P.G, P.WP, P.PW, a.err};
-            Cell cell{unpack_x(p), unpack_y(p)}, nc = cell;
+            uint32_t nc = p;
             Draws dr{i, hour, P.key0, P.key1, P.move_key};
             bool infect = false;
             if (hod == 0u) {
                 const bool need = valid && wants_hospital(P, infected(s) ? with_day(s, st_day(s) + 1u) : s);
                 const uint32_t hosp_first = __syncthreads_or(need) ? block_first_vacant(P, pl) : kNoAction;
-                if (valid) nc = routine_start(P, pl, s, hm, cell, hosp_first, dr);
+                if (valid) nc = routine_start(P, pl, s, hm, p, hosp_first, dr);
             } else if (valid) {
                 switch (hour_class(hod)) {
-                    case kHcEnd: nc = routine_end(P, pl, s, hm, cell, dr); break;
-                    case kHcTransport: nc = small_move<kHcTransport>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
-                    case kHcWork: nc = small_move<kHcWork>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
-                    case kHcNoon: nc = small_move<kHcNoon>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
-                    case kHcHome: nc = small_move<kHcHome>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
-                    default: nc = small_move<kHcMove>(P, pl, steps, s, a.wsa + i, hm, wk, cell, hour, dr, infect); break;
+                    case kHcEnd: nc = routine_end(P, pl, s, hm, p, dr); break;
+                    case kHcTransport: nc = small_move<kHcTransport>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcWork: nc = small_move<kHcWork>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcNoon: nc = small_move<kHcNoon>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcHome: nc = small_move<kHcHome>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    default: nc = small_move<kHcMove>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
                 }
             }
-            const bool moving = nc.x != cell.x || nc.y != cell.y;
-            uint32_t* claim = &a.claim[(size_t)nc.y * P.W + nc.x];
+            const bool moving = nc != p;
+            uint32_t* claim = &a.claim[(nc >> 16) * (uint32_t)P.W + (nc & 0xFFFFu)];
             if (moving) atomicMin(claim, i);
-            if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
+            if (infect) infection_dynamics(P, pl, tables, boxes, s, at, hm, wk, nc, hour, dr);
             tally.add(valid, count_bin(s));
             tally.flush(sh);
             cluster_sync();  // every claim is in, and the bit plane of before has been read
@@ -714,11 +718,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
                 win = __ldcg(claim) == i;
                 if (win) atomicMax(claim, kNoClaim);  // (not a plain store: see send_back)
             }
-            const uint32_t q = win ? pack_xy(nc.x, nc.y) : p;
-            const uint32_t Xo = (uint32_t)cell.x + 1u, X = (uint32_t)unpack_x(q) + 1u;
-            uint32_t* word = &next[((uint32_t)unpack_y(q) + 1u) * P.PW + (X >> 5)];
+            const uint32_t q = win ? nc : p;
+            const uint32_t Xo = (p & 0xFFFFu) + 1u, X = (q & 0xFFFFu) + 1u;
+            uint32_t* word = &next[((q >> 16) + 1u) * P.PW + (X >> 5)];
             if (patch ? win : valid) atomicOr(word, 1u << (X & 31u));
-            if (patch && win) atomicAnd(&next[((uint32_t)cell.y + 1u) * P.PW + (Xo >> 5)], ~(1u << (Xo & 31u)));
+            if (patch && win) atomicAnd(&next[((p >> 16) + 1u) * P.PW + (Xo >> 5)], ~(1u << (Xo & 31u)));
             if (valid && (infected(s0) || infected(s))) {
                 const uint32_t cls0 = cell_class(P, s0), cls = cell_class(P, s);
                 if (win || cls != cls0) {
@@ -782,9 +786,10 @@ __global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __re
                                                            HourArgs ha, int* err) {
     __shared__ uint32_t sh[8];
     __shared__ DevParams sP;
-    __shared__ StepTable steps;
+    __shared__ MoveTables tables;
+    __shared__ Box boxes[kNumAreas];
     const DevParams& P = sP;
-    stage_steps(steps);  // read after switch_rep's barriers
+    stage_tables(tables);  // read after switch_rep's barriers
     const HourRow hr = hour_row(ha);
     const uint32_t hour = hr.hour;
     BlockRep br;
@@ -792,7 +797,7 @@ __global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __re
     uint32_t hosp_first = kNoAction;
     bool hosp_known = false;
     if (blockIdx.x >= n_chunks) return;  // block-uniform
-    switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row));
+    switch_rep(br, 0u, Pall, sP, tally, sh, row_ptr(ha, hr.row), boxes);
     const ByteView pl{plane, P.G, P.WP, err};
     for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         const uint32_t i = c * kChunk + threadIdx.x;
@@ -809,22 +814,16 @@ __global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __re
         }
         if (valid) {
             const uint32_t hm = home[i], wk = work[i];
-            const Cell cell{unpack_x(p), unpack_y(p)};
             Draws dr{i, hour, P.key0, P.key1, P.move_key};
-            Cell nc;
+            uint32_t q;
             bool infect = false;
-            if (HC == kHcStart) {
-                nc = routine_start(P, pl, s, hm, cell, hosp_first, dr);
-            } else if (HC == kHcEnd) {
-                nc = routine_end(P, pl, s, hm, cell, dr);
-            } else {
-                nc = perform_movements<HC>(P, pl, steps, s, wsa + i, hm, wk, cell, hour, dr, infect);
-            }
-            const bool moving = nc.x != cell.x || nc.y != cell.y;
-            if (moving) atomicMin(&claim[(size_t)nc.y * P.W + nc.x], i);
-            if (infect) infection_dynamics(P, pl, s, at, hm, wk, nc, hour, dr);
+            if (HC == kHcStart) q = routine_start(P, pl, s, hm, p, hosp_first, dr);
+            else if (HC == kHcEnd) q = routine_end(P, pl, s, hm, p, dr);
+            else q = perform_movements<HC>(P, pl, tables, boxes, s, wsa + i, hm, wk, p, hour, dr, infect);
+            if (q != p) atomicMin(&claim[(size_t)(q >> 16) * P.W + (q & 0xFFFFu)], i);
+            if (infect) infection_dynamics(P, pl, tables, boxes, s, at, hm, wk, q, hour, dr);
             const uint32_t cls0 = cell_class(P, sv.x), cls = cell_class(P, s);
-            tgt[i] = moving || cls != cls0 ? encode_target(nc, cls, cls0) : kNoAction;
+            tgt[i] = q != p || cls != cls0 ? encode_target(q, cls, cls0) : kNoAction;
             if (s != sv.x || at != sv.y) st[i] = make_uint2(s, at);
         }
         tally.add(valid, valid ? count_bin(s) : 0u);

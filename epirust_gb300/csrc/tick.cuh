@@ -146,8 +146,9 @@ struct BitView {
     static __device__ __forceinline__ uint32_t occupied(const Rows3& r) {
         return (r.r0 & 7u) | ((r.r1 & 7u) << 3) | ((r.r2 & 7u) << 6);
     }
+    // (x, y) is a proposal: inside the plane
     __device__ __forceinline__ bool safe(int32_t x, int32_t y) const {
-        return inside(x, y) && plane_load<CG>(danger + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1)) == 0u;
+        return plane_load<CG>(danger + (size_t)(y + 1) * (size_t)WP + (size_t)(x + 1)) == 0u;
     }
     __device__ __forceinline__ InfMasks infectious(int32_t x, int32_t y) const {
         if (!inside(x, y)) return InfMasks{0u, 0u};
@@ -157,39 +158,71 @@ struct BitView {
     }
 };
 
-// Cells of the block around (x, y) inside area a and the grid, for (x, y) in the area or on the
-// plane's edge (Area::get_neighbors_of filtered by is_point_in_grid): three columns and three
-// rows, each a run of bits cut off on either side by as many cells as lie beyond the bounds
-// (shifts of 3 or more clear the run).
-__device__ __forceinline__ uint32_t valid_block(const Rect& a, int32_t G, int32_t x, int32_t y) {
-    const int32_t lx = max(a.x0, 0), hx = min(a.x1, G - 1), ly = max(a.y0, 0), hy = min(a.y1, G - 1);
-    const uint32_t cl = (uint32_t)max(lx - x + 1, 0), cr = (uint32_t)max(x + 1 - hx, 0);
-    const uint32_t rl = (uint32_t)max(ly - y + 1, 0), rr = (uint32_t)max(y + 1 - hy, 0);
-    const uint32_t cols = __funnelshift_lc(0u, 7u, cl) & __funnelshift_rc(7u, 0u, cr) & 7u;
-    const uint32_t rows = __funnelshift_lc(0u, 0x1FFu, 3u * rl) & __funnelshift_rc(0x1FFu, 0u, 3u * rr);
-    return (cols * 0x49u) & rows;
+// Cells and areas as packed words, x | y << 16: bounds are tested and clamped for both
+// coordinates at once (values stay below 2^14, so sums with kHalf = 2^14 per half never carry).
+// An area is its low and high corner, both inside it.
+struct Box {
+    uint32_t lo, hi;
+};
+constexpr uint32_t kHalf = 0x40004000u;
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ bool box_has(const Box& b, uint32_t c) {
+    return (max2(b.lo + kHalf - c, kHalf) | max2(c + kHalf - b.hi, kHalf)) == kHalf;
 }
 
-// Moore step of the j-th set bit of a 9-cell mask, as (dx + 1) | (dy + 1) << 2, for every mask
-// and j < popc(mask): one table read instead of the bit search.  The kernels keep a copy in
-// shared memory, where lanes with different masks cost bank conflicts instead of cache lines.
-struct __align__(16) StepTable {
-    uint8_t v[512][8];
+// Tables of the kernels' shared memory.
+//   valid[i]   cells of a 3x3 block inside bounds, i = columns cut off on the left | rows cut
+//              off above << 2 | columns on the right << 4 | rows below << 6 (3 cuts all)
+//   step[m][j] Moore step of the j-th set bit of a 9-cell mask m, (dx + 1) | (dy + 1) << 4
+// Lanes with different entries cost bank conflicts there instead of cache lines.
+struct __align__(16) MoveTables {
+    uint16_t valid[256];
+    uint8_t step[512][8];
 };
-constexpr StepTable make_step_table() {
-    StepTable t{};
+constexpr MoveTables make_move_tables() {
+    MoveTables t{};
+    for (int i = 0; i < 256; ++i) {
+        const int cl = i & 3, rl = (i >> 2) & 3, cr = (i >> 4) & 3, rr = (i >> 6) & 3;
+        int m = 0;
+        for (int k = 0; k < 9; ++k) {
+            const int c = k % 3, r = k / 3;
+            if (c >= cl && c < 3 - cr && r >= rl && r < 3 - rr) m |= 1 << k;
+        }
+        t.valid[i] = (uint16_t)m;
+    }
     for (int m = 0; m < 512; ++m) {
         int j = 0;
         for (int k = 0; k < 9; ++k)
-            if (k != 4 && ((m >> k) & 1)) t.v[m][j++] = (uint8_t)((k % 3) | ((k / 3) << 2));
+            if (k != 4 && ((m >> k) & 1)) t.step[m][j++] = (uint8_t)((k % 3) | ((k / 3) << 4));
     }
     return t;
 }
-__device__ const StepTable kStepTable = make_step_table();
+__device__ const MoveTables kMoveTables = make_move_tables();
 // The block's copy (the caller synchronises before it is read).
-__device__ __forceinline__ void stage_steps(StepTable& sh) {
-    const uint4* src = reinterpret_cast<const uint4*>(&kStepTable);
-    for (uint32_t k = threadIdx.x; k < sizeof(StepTable) / 16; k += blockDim.x) reinterpret_cast<uint4*>(&sh)[k] = __ldg(src + k);
+__device__ __forceinline__ void stage_tables(MoveTables& sh) {
+    const uint4* src = reinterpret_cast<const uint4*>(&kMoveTables);
+    for (uint32_t k = threadIdx.x; k < sizeof(MoveTables) / 16; k += blockDim.x)
+        reinterpret_cast<uint4*>(&sh)[k] = __ldg(src + k);
+}
+
+// Cells of the block around c inside area b and the grid (last = the grid's last cell
+// G - 1 | G - 1 << 16; Area::get_neighbors_of filtered by is_point_in_grid): how many columns
+// and rows lie beyond the bounds on either side, clamped to 0..3, index the table.
+__device__ __forceinline__ uint32_t valid_block(const MoveTables& t, const Box& b, uint32_t last, uint32_t c) {
+    const uint32_t beyond = kHalf + 0x00010001u;
+    const uint32_t l = min2(max2(b.lo + beyond - c, kHalf), kHalf | 0x00030003u);
+    const uint32_t h = min2(max2(c + beyond - min2(b.hi, last), kHalf), kHalf | 0x00030003u);
+    const uint32_t i = (l | (h << 4)) & 0x00330033u;  // columns in bits 0-1, 4-5; rows in 16-17, 20-21
+    return t.valid[(i | (i >> 14)) & 0xFFu];
 }
 
 // Lazily materialised Philox blocks of one agent-hour: m(0), m(1) the random-point words
@@ -227,25 +260,27 @@ struct Draws {
 
 struct Cell { int32_t x, y; };
 
-__device__ __forceinline__ Cell random_point(const Rect& a, uint32_t ux, uint32_t uy) {
-    Cell c;
-    c.x = a.x0 + (int32_t)uniform_index(ux, (uint32_t)(a.x1 - a.x0 + 1));
-    c.y = a.y0 + (int32_t)uniform_index(uy, (uint32_t)(a.y1 - a.y0 + 1));
-    return c;
+// (house and office corners are packed words already)
+__device__ __forceinline__ Box home_box(uint32_t home) { return Box{home, home + 0x00010001u}; }
+__device__ __forceinline__ Box office_box(uint32_t work) { return Box{work, work + 0x00090009u}; }
+// The area of a code; boxes holds the packed global areas.
+__device__ __forceinline__ Box area_box(const Box* boxes, uint32_t code, uint32_t home, uint32_t work) {
+    Box b;
+    b.lo = code == kWork ? work : home;
+    b.hi = b.lo + (code == kWork ? 0x00090009u : 0x00010001u);
+    if (code >= kTransport) b = boxes[code];
+    return b;
 }
-
-__device__ __forceinline__ Rect home_rect(uint32_t home) {
-    int32_t x = unpack_x(home), y = unpack_y(home);
-    return Rect{x, y, x + 1, y + 1};
+// The packed global areas of P into shared memory (the caller synchronises).
+__device__ __forceinline__ void stage_boxes(Box* boxes, const DevParams& P) {
+    if (threadIdx.x < kNumAreas) {
+        const Rect& r = P.area[threadIdx.x];
+        boxes[threadIdx.x] = Box{pack_xy(r.x0, r.y0), pack_xy(r.x1, r.y1)};
+    }
 }
-__device__ __forceinline__ Rect office_rect(uint32_t work) {
-    int32_t x = unpack_x(work), y = unpack_y(work);
-    return Rect{x, y, x + 9, y + 9};
-}
-__device__ __forceinline__ Rect area_rect(const DevParams& P, uint32_t code, uint32_t home, uint32_t work) {
-    if (code == kHome) return home_rect(home);
-    if (code == kWork) return office_rect(work);
-    return P.area[code];
+__device__ __forceinline__ uint32_t random_cell(const Box& b, uint32_t ux, uint32_t uy) {
+    const uint32_t w = b.hi - b.lo + 0x00010001u;
+    return b.lo + (uniform_index(ux, w & 0xFFFFu) | (uniform_index(uy, w >> 16) << 16));
 }
 
 // Citizen::can_move, citizen/mod.rs:452-454
@@ -261,7 +296,7 @@ __device__ __forceinline__ uint32_t cell_class(const DevParams& P, uint32_t s) {
     return 1u + rate_class(P.reg_start, P.high_start, P.last_day, d);
 }
 
-// A lane's move: act false keeps the cell.  jump is Citizen::goto_area of an agent that works
+// A lane's move: act false keeps the cell p.  jump is Citizen::goto_area of an agent that works
 // (citizen/mod.rs:367-395: a random point of the target area, kept when vacant), otherwise
 // Citizen::move_agent_from over the current area (citizen/mod.rs:415-432: uniform choice among
 // the vacant neighbours of the cell, or of a random point of the area when outside it); `area`
@@ -270,24 +305,29 @@ __device__ __forceinline__ uint32_t cell_class(const DevParams& P, uint32_t s) {
 // walkers also read the rows above and below.  JUMPS false: no lane of the hour jumps but
 // hospital staff (rarely).
 template <bool JUMPS, class V>
-__device__ __forceinline__ Cell move_lane(const V& pl, const StepTable& steps, bool act, bool jump, const Rect& area, Cell cell,
-                                          Draws& dr) {
+__device__ __forceinline__ uint32_t move_lane(const V& pl, const MoveTables& tables, bool act, bool jump, const Box& area,
+                                              uint32_t p, Draws& dr) {
     if (JUMPS) dr.prime(jump);
-    if (!act) return cell;
-    Cell c = cell;
-    if (jump || !rect_has(area, cell.x, cell.y)) c = random_point(area, dr.m(0), dr.m(1));
-    if (!pl.inside(c.x, c.y)) return cell;  // reads as occupied (and is reported)
-    const uint32_t r1 = pl.row(c.x, c.y);
-    if (JUMPS && jump) return V::centre_vacant(r1) ? c : cell;
-    const Rows3 rows{pl.row(c.x, c.y - 1), r1, pl.row(c.x, c.y + 1)};
+    if (!act) return p;
+    uint32_t c = p;
+    if (jump || !box_has(area, p)) c = random_cell(area, dr.m(0), dr.m(1));
+    const uint32_t edge = (uint32_t)pl.G * 0x00010001u;
+    if (max2(c, edge) != edge) {  // reads as occupied (and is reported)
+        atomicOr(pl.err, 1);
+        return p;
+    }
+    const int32_t x = (int32_t)(c & 0xFFFFu), y = (int32_t)(c >> 16);
+    const uint32_t r1 = pl.row(x, y);
+    if (JUMPS && jump) return V::centre_vacant(r1) ? c : p;
+    const Rows3 rows{pl.row(x, y - 1), r1, pl.row(x, y + 1)};
     // The choice word is drawn before the rows are used, so that its Philox rounds run while
     // the row loads are in flight (it is needed unless every neighbour is taken).
     const uint32_t u = dr.m(2);
-    if (!JUMPS && jump) return V::centre_vacant(r1) ? c : cell;
-    const uint32_t cand = valid_block(area, pl.G, c.x, c.y) & ~V::occupied(rows) & kNeighbours9;
-    if (!cand) return cell;
-    const uint32_t e = steps.v[cand][uniform_index(u, (uint32_t)__popc(cand))];
-    return Cell{c.x + (int32_t)(e & 3u) - 1, c.y + (int32_t)(e >> 2) - 1};  // vacant by construction: move_agent keeps it
+    if (!JUMPS && jump) return V::centre_vacant(r1) ? c : p;
+    const uint32_t cand = valid_block(tables, area, edge - 0x00010001u, c) & ~V::occupied(rows) & kNeighbours9;
+    if (!cand) return p;
+    const uint32_t e = tables.step[cand][uniform_index(u, (uint32_t)__popc(cand))];
+    return c + ((e | (e << 12)) & 0x00030003u) - 0x00010001u;  // vacant by construction: move_agent keeps it
 }
 
 // DiseaseStateMachine::next with the default DiseaseHandler (ddh:41-86) for the hour's
@@ -295,8 +335,10 @@ __device__ __forceinline__ Cell move_lane(const V& pl, const StepTable& steps, b
 // (The agent's current area, needed only when an infectious neighbour exists, is decoded from
 // its code and home / work corners here rather than by the caller.)
 template <class V>
-__device__ __forceinline__ void infection_dynamics(const DevParams& P, const V& pl, uint32_t& s, uint32_t& at,
-                                                   uint32_t home, uint32_t work, Cell cell, uint32_t hour, Draws& dr) {
+__device__ __forceinline__ void infection_dynamics(const DevParams& P, const V& pl, const MoveTables& tables,
+                                                   const Box* boxes, uint32_t& s, uint32_t& at, uint32_t home,
+                                                   uint32_t work, uint32_t p, uint32_t hour, Draws& dr) {
+    const Cell cell{(int32_t)(p & 0xFFFFu), (int32_t)(p >> 16)};
     const uint32_t v = s & kStateMask;
     if (v == EPI_S) {
         if (s & (kWq | kVacc)) return;
@@ -304,8 +346,8 @@ __device__ __forceinline__ void infection_dynamics(const DevParams& P, const V& 
         if (pl.safe(cell.x, cell.y)) return;
         const InfMasks masks = pl.infectious(cell.x, cell.y);
         if (!masks.inf) return;
-        const Rect cur = area_rect(P, st_area(s), home, work);
-        const uint32_t cand = neighbours8(valid_block(cur, pl.G, cell.x, cell.y)) & masks.inf;
+        const Box cur = area_box(boxes, st_area(s), home, work);
+        const uint32_t cand = neighbours8(valid_block(tables, cur, (uint32_t)(pl.G - 1) * 0x00010001u, p)) & masks.inf;
         if (!cand) return;
         const uint32_t high = masks.high;
         const uint64_t thr_reg = P.thr_rate[1], thr_high = P.thr_rate[2];
@@ -366,11 +408,11 @@ __host__ __device__ constexpr int hour_class(uint32_t hod) {
 // infect is cleared when the hour ends before the infection update of
 // DiseaseStateMachine::next, which the caller runs on the proposed cell otherwise.
 template <int HC, class V>
-__device__ __forceinline__ Cell perform_movements(const DevParams& P, const V& pl, const StepTable& steps, uint32_t& s,
-                                                  uint32_t* wsa, uint32_t home, uint32_t work, Cell cell, uint32_t hour,
-                                                  Draws& dr, bool& infect) {
+__device__ __forceinline__ uint32_t perform_movements(const DevParams& P, const V& pl, const MoveTables& tables,
+                                                      const Box* boxes, uint32_t& s, uint32_t* wsa, uint32_t home,
+                                                      uint32_t work, uint32_t p, uint32_t hour, Draws& dr, bool& infect) {
     const uint32_t ws = st_ws(s);
-    Rect area = area_rect(P, st_area(s), home, work);
+    Box area = area_box(boxes, st_area(s), home, work);
     bool act = can_move(s), jump = false;
     infect = true;
     if (ws == EPI_WS_HOSPITAL_STAFF) {  // citizen/mod.rs:292-328; wsa: its work_start_at
@@ -380,15 +422,16 @@ __device__ __forceinline__ Cell perform_movements(const DevParams& P, const V& p
             act = infect = false;
         } else if (since == 24u * 14u * 2u) {
             jump = true;
-            area = home_rect(home);
+            area = home_box(home);
             s = with_area(s, kHome);
             *wsa = hour + 24u * 14u;
             infect = false;
         } else if (HC == kHcWork) {
-            jump = !rect_eq(area, P.area[P.hosp_code]) && w <= hour;
+            const Box hosp = boxes[P.hosp_code];
+            jump = (area.lo != hosp.lo || area.hi != hosp.hi) && w <= hour;
             act = act && jump;
             if (jump) {
-                area = P.area[P.hosp_code];
+                area = hosp;
                 s = with_area(s, P.hosp_code);
                 *wsa = hour;
             }
@@ -404,29 +447,30 @@ __device__ __forceinline__ Cell perform_movements(const DevParams& P, const V& p
         if (HC == kHcTransport) {  // a worker with public transport: goto_area(transport)
             jump = worker && (s & kPt);
             if (jump) {
-                area = P.area[kTransport];
+                area = boxes[kTransport];
                 s = with_area(s, kTransport);
             }
         } else if (HC == kHcWork) {  // a worker: goto_area(office); the others: goto_area(housing), a walk
             jump = worker;
-            if (jump) area = office_rect(work);
+            if (jump) area = office_box(work);
             s = with_area(s, worker ? kWork : kHousing);
         } else if (HC == kHcNoon) {  // a worker walks; the others: goto_area(home), a walk
             if (!worker) s = with_area(s, kHome);
         } else if (HC == kHcHome) {  // a worker: goto_area(home)
             jump = worker;
             if (jump) {
-                area = home_rect(home);
+                area = home_box(home);
                 s = with_area(s, kHome);
             }
         }
         if (jump && !act) {  // goto_area's symptomatic override of a worker going home from the office
             const uint32_t v = s & kStateMask;
-            act = (v == EPI_I_MILD || v == EPI_I_SEVERE) && rect_has(office_rect(work), cell.x, cell.y) &&
-                  rect_eq(area, home_rect(home));
+            const Box house = home_box(home);
+            act = (v == EPI_I_MILD || v == EPI_I_SEVERE) && box_has(office_box(work), p) && area.lo == house.lo &&
+                  area.hi == house.hi;
         }
     }
-    return move_lane<HC == kHcTransport || HC == kHcWork || HC == kHcHome>(pl, steps, act, jump, area, cell, dr);
+    return move_lane<HC == kHcTransport || HC == kHcWork || HC == kHcHome>(pl, tables, act, jump, area, p, dr);
 }
 
 // Hour 0 of the day: increment_infection_day, then Citizen::hospitalize
@@ -439,32 +483,32 @@ __device__ __forceinline__ bool wants_hospital(const DevParams& P, uint32_t s) {
 }
 
 template <class V>
-__device__ __forceinline__ Cell routine_start(const DevParams& P, const V& pl, uint32_t& s, uint32_t home,
-                                              Cell cell, uint32_t hosp_first, Draws& dr) {
+__device__ __forceinline__ uint32_t routine_start(const DevParams& P, const V& pl, uint32_t& s, uint32_t home, uint32_t p,
+                                                  uint32_t hosp_first, Draws& dr) {
     if (infected(s)) s = with_day(s, st_day(s) + 1u);
-    if (!wants_hospital(P, s)) return cell;
+    if (!wants_hospital(P, s)) return p;
     if (hosp_first != kNoAction) {
         s |= kHosp;
-        return Cell{unpack_x(hosp_first), unpack_y(hosp_first)};
+        return hosp_first;
     }
-    Cell q = random_point(home_rect(home), dr.m(0), dr.m(1));
-    return pl.vacant(q.x, q.y) ? q : cell;
+    const uint32_t q = random_cell(home_box(home), dr.m(0), dr.m(1));
+    return pl.vacant(unpack_x(q), unpack_y(q)) ? q : p;
 }
 
 // Hour 23: Citizen::deceased with on_routine_end (citizen/mod.rs:397-413, ddh:88-102).
 template <class V>
-__device__ __forceinline__ Cell routine_end(const DevParams& P, const V& pl, uint32_t& s, uint32_t home,
-                                            Cell cell, Draws& dr) {
+__device__ __forceinline__ uint32_t routine_end(const DevParams& P, const V& pl, uint32_t& s, uint32_t home, uint32_t p,
+                                                Draws& dr) {
     const uint32_t v = s & kStateMask, day = st_day(s);
     if (v == EPI_I_ASYM && day == 9u) s = with_state(s, EPI_R);          // ASYMPTOMATIC_LAST_DAY
     else if (v == EPI_I_MILD && day == 12u) s = with_state(s, EPI_R);    // MILD_INFECTED_LAST_DAY
     else if (v == EPI_I_SEVERE && day == P.last_day)
         s = with_state(s, (uint64_t)dr.m(2) < P.thr_death ? EPI_D : EPI_R);
-    Cell nc = cell;
+    uint32_t nc = p;
     const uint32_t nv = s & kStateMask;
     if (nv == EPI_R) {
-        Cell q = random_point(home_rect(home), dr.m(0), dr.m(1));
-        if (pl.vacant(q.x, q.y)) nc = q;
+        const uint32_t q = random_cell(home_box(home), dr.m(0), dr.m(1));
+        if (pl.vacant(unpack_x(q), unpack_y(q))) nc = q;
     }
     if (nv == EPI_R || nv == EPI_D) s &= ~kHosp;
     return nc;
@@ -472,18 +516,15 @@ __device__ __forceinline__ Cell routine_end(const DevParams& P, const V& pl, uin
 
 // Counts::update_counts bin (counts.rs:126-140): 0 S, 1 E, 2 I, 3 H, 4 R, 5 D.
 __device__ __forceinline__ uint32_t count_bin(uint32_t s) {
-    uint32_t v = s & kStateMask;
-    if (v == EPI_S) return 0u;
-    if (v == EPI_E) return 1u;
-    if (v == EPI_R) return 4u;
-    if (v == EPI_D) return 5u;
-    return (s & kHosp) ? 3u : 2u;
+    // bins of the eight states, four bits each (2..5 are the infected ones)
+    const uint32_t bin = (0x54222210u >> ((s & kStateMask) * 4u)) & 7u;
+    return bin == 2u && (s & kHosp) ? 3u : bin;
 }
 
 // tgt word: target x | y << 16 (14 bits each, grids up to 16,383) with the new plane class
 // in bits 15 (low) and 31 (high) and the class before the hour in bits 14 and 30.
-__device__ __forceinline__ uint32_t encode_target(Cell c, uint32_t cls, uint32_t old_cls) {
-    return pack_xy(c.x, c.y) | ((cls & 1u) << 15) | ((cls >> 1) << 31) | ((old_cls & 1u) << 14) | ((old_cls >> 1) << 30);
+__device__ __forceinline__ uint32_t encode_target(uint32_t xy, uint32_t cls, uint32_t old_cls) {
+    return xy | ((cls & 1u) << 15) | ((cls >> 1) << 31) | ((old_cls & 1u) << 14) | ((old_cls >> 1) << 30);
 }
 __device__ __forceinline__ uint32_t target_xy(uint32_t t) { return t & 0x3FFF3FFFu; }
 __device__ __forceinline__ uint32_t target_class(uint32_t t) { return ((t >> 15) & 1u) | ((t >> 30) & 2u); }
