@@ -1198,43 +1198,24 @@ static int finish_upload(epi_engine* h) {
     return check_error_flag(h);
 }
 
+// Replicate r's records.  They are laid out on the device in the claim plane (free between
+// chains: the next chain resets it), as many at a time as it holds.
 static int snapshot_replica(epi_engine* h, uint32_t r, epi_agent_record* out, size_t n) {
     const Replica& rep = h->reps[r];
     if (!out || n != rep.n) return EPI_ERR_ARG;
-    const size_t off = rep.hp.agent_off;
-    std::vector<uint32_t> pos(n), home(n), work(n), wsa(n);
-    std::vector<uint2> st(n);
-    CK(cudaMemcpyAsync(pos.data(), pos_buf(h, rep.par) + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(home.data(), h->d_home + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(work.data(), h->d_work + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(wsa.data(), h->d_wsa + off, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(st.data(), h->d_st + off, n * sizeof(uint2), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    for (size_t i = 0; i < n; ++i) {
-        epi_agent_record& a = out[i];
-        std::memset(&a, 0, sizeof a);
-        const uint32_t s = st[i].x, v = s & kStateMask;
-        a.x = unpack_x(pos[i]);
-        a.y = unpack_y(pos[i]);
-        a.state = (uint8_t)v;
-        a.flags = (uint8_t)(((s & kHosp) ? EPI_F_HOSPITALIZED : 0) | ((s & kIso) ? EPI_F_ISOLATED : 0) |
-                            ((s & kVacc) ? EPI_F_VACCINATED : 0) | ((s & kWq) ? EPI_F_WORK_QUARANTINED : 0) |
-                            ((s & kPt) ? EPI_F_PUBLIC_TRANSPORT : 0));
-        a.work_status = (uint8_t)st_ws(s);
-        a.immunity = (int8_t)st_imm(s);
-        a.at_hour = (v == EPI_E || v == EPI_I_PRE) ? st[i].y : 0u;
-        a.infection_day = infected(s) ? st_day(s) : 0u;
-        a.work_start_at = st_ws(s) == EPI_WS_HOSPITAL_STAFF ? wsa[i] : 0u;
-        a.home_x = unpack_x(home[i]);
-        a.home_y = unpack_y(home[i]);
-        a.work_x = unpack_x(work[i]);
-        a.work_y = unpack_y(work[i]);
-        const uint32_t code = st_area(s);
-        Rect ar = code == kHome ? Rect{a.home_x, a.home_y, a.home_x + 1, a.home_y + 1}
-                  : code == kWork ? Rect{a.work_x, a.work_y, a.work_x + 9, a.work_y + 9}
-                                  : rep.hp.area[code < kNumAreas ? code : kHome];
-        a.area_x0 = ar.x0; a.area_y0 = ar.y0; a.area_x1 = ar.x1; a.area_y1 = ar.y1;
+    const size_t room = h->claim_cells * sizeof(uint32_t) / sizeof(epi_agent_record);
+    if (room == 0) { h->err = "snapshot: world without cells"; return EPI_ERR_INVARIANT; }
+    h->last_claim_hour = INT64_MAX;
+    touch_pages(out, n * sizeof(epi_agent_record));
+    for (size_t first = 0; first < n; first += room) {
+        const uint32_t count = (uint32_t)std::min(room, n - first);
+        k_unpack_records<<<(count + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(
+            h->d_params, r, rep.hp.agent_off, (uint32_t)first, count, pos_buf(h, rep.par), h->d_st, h->d_home, h->d_work,
+            h->d_wsa, h->d_claim);
+        CK(cudaGetLastError());  // (not counted: the counter is of the simulation's launches)
+        CK(cudaMemcpyAsync(out + first, h->d_claim, count * sizeof(epi_agent_record), cudaMemcpyDeviceToHost, h->stream));
     }
+    CK(cudaStreamSynchronize(h->stream));
     return EPI_OK;
 }
 

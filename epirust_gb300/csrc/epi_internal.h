@@ -18,6 +18,7 @@
 //   claim      a u32 per cell of (G+1) x (G+1), without border: the smallest claim key
 #pragma once
 
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/epi_engine.h"
@@ -163,6 +164,15 @@ EPI_HD int record_words(const DevParams& hp, const epi_agent_record& a, AgentWor
     w = AgentWords{pack_xy(a.x, a.y), s, a.at_hour, pack_xy(a.home_x, a.home_y), pack_xy(a.work_x, a.work_y),
                    a.work_start_at};
     return 0;
+}
+
+// One write to every page of a caller's buffer that a device copy is about to fill: a copy into
+// pages that the process has never touched waits for them one by one on the device's side (a
+// GB300's records of 300,000 agents: 2.2 to 9.2 ms into fresh pages, 0.7 ms after this).
+inline void touch_pages(void* p, size_t bytes) {
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t b = 0; b < bytes; b += 4096) c[b] = 0;
+    if (bytes) c[bytes - 1] = 0;
 }
 
 constexpr uint32_t kChunk = 256;  // agent slots per chunk; replicates start on chunk boundaries

@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "../../include/epi_surrogate.h"
+#include "epi_internal.h"
 #include "tc_gemm.cuh"
 #include "tc_train.cuh"
 
@@ -677,6 +678,7 @@ int download_params(epi_mlp* h, float* const MlpLayer::*wp, float* const MlpLaye
     const size_t floats = (size_t)member_params(h) * h->E;
     MRC(ensure_raw(h, floats));
     MRC(move_params(h, wp, bp, true));
+    epi::touch_pages(out, floats * sizeof(float));
     MCK(cudaMemcpyAsync(out, h->d_raw, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     MCK(cudaStreamSynchronize(h->stream));
     return EPI_OK;
@@ -880,6 +882,7 @@ int epi_mlp_predict(epi_mlp* h, const float* x, uint32_t n, float* y) {
         h->d_py, n, h->cfg.out_dim, h->out_pad, (size_t)h->p_cap * h->out_pad, h->d_raw);
     MCK(cudaGetLastError());
     h->launches++;
+    epi::touch_pages(y, floats * sizeof(float));
     MCK(cudaMemcpyAsync(y, h->d_raw, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     MRC(check_err(h));
     return EPI_OK;
@@ -889,6 +892,7 @@ int epi_mlp_score(epi_mlp* h, const float* x, uint32_t n, const float* target, f
     if (!h || !x || !target || !score) return EPI_ERR_ARG;
     if (n == 0) return EPI_OK;
     MRC(forward_n(h, x, n, target));
+    epi::touch_pages(score, (size_t)h->E * n * sizeof(float));
     MRC(check_err(h));
     for (uint32_t m = 0; m < h->E; ++m)
         MCK(cudaMemcpy(score + (size_t)m * n, h->d_pscore + (size_t)m * h->p_cap, (size_t)n * sizeof(float),

@@ -184,5 +184,51 @@ __global__ void __launch_bounds__(kThreads) k_pack_records(const DevParams* __re
     }
 }
 
+// The way back: the SoA words of agents first .. first + count - 1 of one replicate (its agents
+// start at slot off) as records, 256 to a block.  A record is 14 words that a thread lays out in
+// shared memory, from where the block writes them as one run; the host then takes the records
+// with one copy.  (Five copies of words and a host loop over the agents took 4.7 ms for 1M
+// agents on one GB300 and 22.7 ms for 4M; now 2.2 and 8.4 ms, most of it the first touch of
+// the caller's pages: the copy alone takes 0.3 and 1.2.)
+__global__ void __launch_bounds__(kThreads) k_unpack_records(const DevParams* __restrict__ Pall, uint32_t r, uint32_t off,
+                                                             uint32_t first, uint32_t count, const uint32_t* __restrict__ pos,
+                                                             const uint2* __restrict__ st, const uint32_t* __restrict__ home,
+                                                             const uint32_t* __restrict__ work,
+                                                             const uint32_t* __restrict__ wsa, uint32_t* __restrict__ out) {
+    static_assert(sizeof(epi_agent_record) == 56, "14 words a record");
+    __shared__ uint32_t words[kThreads * 14];
+    const uint32_t k0 = blockIdx.x * kThreads, k = k0 + threadIdx.x;
+    if (k < count) {
+        const size_t slot = (size_t)off + first + k;
+        const uint2 sv = st[slot];
+        const uint32_t s = sv.x, v = s & kStateMask, p = pos[slot], h = home[slot], w = work[slot], code = st_area(s);
+        const uint32_t flags = ((s & kHosp) ? EPI_F_HOSPITALIZED : 0u) | ((s & kIso) ? EPI_F_ISOLATED : 0u) |
+                               ((s & kVacc) ? EPI_F_VACCINATED : 0u) | ((s & kWq) ? EPI_F_WORK_QUARANTINED : 0u) |
+                               ((s & kPt) ? EPI_F_PUBLIC_TRANSPORT : 0u);
+        const int32_t hx = unpack_x(h), hy = unpack_y(h), wx = unpack_x(w), wy = unpack_y(w);
+        const Rect a = code == kHome ? Rect{hx, hy, hx + 1, hy + 1}
+                     : code == kWork ? Rect{wx, wy, wx + 9, wy + 9}
+                                     : Pall[r].area[code < kNumAreas ? code : kHome];
+        uint32_t* o = words + threadIdx.x * 14u;
+        o[0] = (uint32_t)unpack_x(p);
+        o[1] = (uint32_t)unpack_y(p);
+        o[2] = v | (flags << 8) | (st_ws(s) << 16) | ((uint32_t)(st_imm(s) & 0xFF) << 24);
+        o[3] = (v == EPI_E || v == EPI_I_PRE) ? sv.y : 0u;
+        o[4] = infected(s) ? st_day(s) : 0u;
+        o[5] = st_ws(s) == EPI_WS_HOSPITAL_STAFF ? wsa[slot] : 0u;
+        o[6] = (uint32_t)hx;
+        o[7] = (uint32_t)hy;
+        o[8] = (uint32_t)wx;
+        o[9] = (uint32_t)wy;
+        o[10] = (uint32_t)a.x0;
+        o[11] = (uint32_t)a.y0;
+        o[12] = (uint32_t)a.x1;
+        o[13] = (uint32_t)a.y1;
+    }
+    __syncthreads();
+    const uint32_t n_words = min(count - k0, (uint32_t)kThreads) * 14u;
+    for (uint32_t q = threadIdx.x; q < n_words; q += kThreads) out[(size_t)k0 * 14u + q] = words[q];
+}
+
 }  // namespace kern
 }  // namespace epi
