@@ -36,6 +36,7 @@
 #include "../../include/epi_surrogate.h"
 #include "epi_internal.h"
 #include "tc_gemm.cuh"
+#include "tc_infer.cuh"
 #include "tc_train.cuh"
 
 using namespace epi::tc;
@@ -266,6 +267,24 @@ int make_map(epi_mlp* h, CUtensorMap* map, const void* base, uint32_t rows, uint
     return EPI_OK;
 }
 
+// A launch that may be scheduled while the kernel before it runs (its CTAs wait on the device).
+template <typename... KArgs, typename... Args>
+int launch_overlapped(epi_mlp* h, void (*kern)(KArgs...), dim3 grid, int threads, uint32_t smem, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    MCK(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+    h->launches++;
+    return EPI_OK;
+}
+
 // One product per member (grid z = E); za = 0 when every member reads member 0's A.
 template <int BN, int EP>
 int gemm(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, uint32_t N, uint32_t K, const EpiArgs& a,
@@ -275,10 +294,23 @@ int gemm(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, u
         return EPI_ERR_ARG;
     }
     constexpr uint32_t smem = gemm_smem_bytes<BN>();
-    k_gemm<BN, EP><<<dim3(M / kBM, N / BN, h->E), kGemmThreads, smem, h->stream>>>(ta, tb, M, N, K, a, za, 1u, h->d_err);
-    MCK(cudaGetLastError());
-    h->launches++;
-    return EPI_OK;
+    return launch_overlapped(h, k_gemm<BN, EP>, dim3(M / kBM, N / BN, h->E), kGemmThreads, smem, ta, tb, M, N, K, a, za, 1u,
+                             h->d_err);
+}
+
+// The same by k_infer, for K up to its resident panel (512); wider layers take k_gemm.  Whole
+// rows per item, two blocks at a time, where the 128-row panels fill the SMs (65,536 rows x 5:
+// 206 us a hidden layer, 235 a block at a time); below that one block per item (1,024 rows x 5:
+// 14 us on 152 SMs; whole rows would leave 112 of them idle).
+template <int EP>
+int infer_product(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, uint32_t N, uint32_t K,
+                  const EpiArgs& a, uint32_t za) {
+    if (K / kBK > kInferMaxK) return gemm<128, EP>(h, ta, tb, M, N, K, a, za);
+    const uint32_t panels = M / kBM * h->E, blocks = N / kInferBN;
+    const uint32_t wide = panels < h->sms ? 1u : 2u, run = panels < h->sms ? 1u : blocks;
+    const uint32_t items = panels * (blocks / run);
+    return launch_overlapped(h, k_infer<EP>, dim3(std::min(items, h->sms)), kInferThreads, infer_smem(K / kBK), ta, tb, M, N,
+                             K / kBK, wide, run, items, a, za, h->d_err);
 }
 
 #define MRC(x)                 \
@@ -296,24 +328,6 @@ int cast_all(epi_mlp* h) {
         MCK(cudaGetLastError());
         h->launches++;
     }
-    return EPI_OK;
-}
-
-// A launch that may be scheduled while the kernel before it runs (its CTAs wait on the device).
-template <typename... KArgs, typename... Args>
-int launch_overlapped(epi_mlp* h, void (*kern)(KArgs...), dim3 grid, uint32_t smem, Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kTrainThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = h->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    MCK(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
-    h->launches++;
     return EPI_OK;
 }
 
@@ -353,7 +367,7 @@ int enqueue_step(epi_mlp* h, uint32_t off, bool grads) {
         }
         auto kern = out ? (w ? k_forward<true, kTrainWideBN> : k_forward<true, kTrainBN>)
                         : (w ? k_forward<false, kTrainWideBN> : k_forward<false, kTrainBN>);
-        MRC(launch_overlapped(h, kern, grid, train_smem(bn, a.stages), ly.t_h, w ? ly.t_w64 : ly.t_w32, a,
+        MRC(launch_overlapped(h, kern, grid, kTrainThreads, train_smem(bn, a.stages), ly.t_h, w ? ly.t_w64 : ly.t_w32, a,
                               (const TrainDev*)h->d_tr, h->d_err));
     }
     auto weight_job = [&](BackwardArgs& a, BackwardMaps& maps, int slot, uint32_t l, bool wide_w) {
@@ -411,7 +425,7 @@ int enqueue_step(epi_mlp* h, uint32_t off, bool grads) {
         a.stages = stages_for(std::max(a.dx.nk, B / kBK), blocks * E);
         auto kern = w ? (ww ? k_backward<kTrainWideBN, kTrainWideBN> : k_backward<kTrainWideBN, kTrainBN>)
                       : (ww ? k_backward<kTrainBN, kTrainWideBN> : k_backward<kTrainBN, kTrainBN>);
-        MRC(launch_overlapped(h, kern, dim3(blocks, E), train_smem(w || ww ? kTrainWideBN : kTrainBN, a.stages), maps, a,
+        MRC(launch_overlapped(h, kern, dim3(blocks, E), kTrainThreads, train_smem(w || ww ? kTrainWideBN : kTrainBN, a.stages), maps, a,
                               (const TrainDev*)h->d_tr, h->d_err));
     }
     return EPI_OK;
@@ -537,7 +551,7 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
         if (l + 1 < h->L) {
             a.out = h->layers[l + 1].ph;
             a.ms_out = cap * ly.N;
-            MRC((gemm<128, kEpHidden>(h, ly.t_ph, ly.t_w, n_pad, ly.N, ly.K, a, za)));
+            MRC(infer_product<kEpHidden>(h, ly.t_ph, ly.t_w, n_pad, ly.N, ly.K, a, za));
         } else {
             a.outf = target ? nullptr : h->d_py;
             a.score_target = target ? h->d_ptarget : nullptr;
@@ -546,7 +560,7 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
             a.m_valid = n;
             a.ms_outf = cap * ly.N;
             a.ms_score = cap;
-            MRC((gemm<128, kEpOut>(h, ly.t_ph, ly.t_w, n_pad, ly.N, ly.K, a, za)));
+            MRC(infer_product<kEpOut>(h, ly.t_ph, ly.t_w, n_pad, ly.N, ly.K, a, za));
         }
     }
     return EPI_OK;
@@ -575,6 +589,8 @@ int init(epi_mlp* h) {
     const epi_mlp_config& c = h->cfg;
     MRC((allow_smem<128, kEpHidden>(h)));
     MRC((allow_smem<128, kEpOut>(h)));
+    for (const void* k : {(const void*)k_infer<kEpHidden>, (const void*)k_infer<kEpOut>})
+        MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)infer_smem(kInferMaxK)));
     for (const void* k : {(const void*)k_forward<false, kTrainBN>, (const void*)k_forward<false, kTrainWideBN>,
                           (const void*)k_forward<true, kTrainBN>, (const void*)k_forward<true, kTrainWideBN>,
                           (const void*)k_backward<kTrainBN, kTrainBN>, (const void*)k_backward<kTrainBN, kTrainWideBN>,

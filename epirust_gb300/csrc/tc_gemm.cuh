@@ -1,14 +1,16 @@
 // tc_gemm.cuh -- BF16 matrix products on the sm_103a tensor cores (tcgen05 + TMA): the
-// building blocks of the surrogate MLP's kernels, and its inference products with their fused
-// epilogues (training's are in tc_train.cuh).
+// building blocks of the surrogate MLP's kernels, and k_gemm, a tile per CTA, for the inference
+// products of networks wider than k_infer's resident panel (K > 512; the others are in
+// tc_infer.cuh, training's in tc_train.cuh).
 //
 // D[m][n] = sum_k A[m][k] * B[n][k]: A is M x K and B is N x K, both row-major BF16 with K
-// contiguous ("K-major").  One CTA of 128 threads computes a 128 x BN tile of D:
-//   thread 0      issues TMA loads of 128 x 64 (A) and BN x 64 (B) tiles into a 2-stage ring
-//                 of shared memory (128-byte swizzle), and tcgen05.mma (M = 128, N = BN,
-//                 K = 16) on each stage, accumulating in FP32 in tensor memory;
-//   all 4 warps   wait for the last MMA, read their 32 lanes (rows) of the accumulator with
-//                 tcgen05.ld, apply the epilogue and store.
+// contiguous ("K-major").  One CTA of 256 threads computes a 128 x BN tile of D:
+//   warp 0        issues TMA loads of 128 x 64 (A) and BN x 64 (B) tiles into a 2-stage ring
+//                 of shared memory (128-byte swizzle);
+//   warp 1        issues tcgen05.mma (M = 128, N = BN, K = 16) on each stage, accumulating in
+//                 FP32 in tensor memory;
+//   all 8 warps   wait for the last MMA, read 32 rows x half the columns of the accumulator
+//                 each with tcgen05.ld, apply the epilogue and store.
 // Every wait on an mbarrier is bounded: on expiry the kernel raises a flag in *err, waits
 // (again bounded) for its own copies and MMAs still in flight, frees tensor memory and exits.
 #pragma once
@@ -23,7 +25,7 @@ namespace tc {
 constexpr int kBM = 128;         // rows of a tile (MMA M)
 constexpr int kBK = 64;          // K per stage: one 128-byte row of BF16
 constexpr int kStages = 2;
-constexpr int kGemmThreads = 128;
+constexpr int kGemmThreads = 256;
 constexpr uint32_t kSpinLimit = 1u << 22;  // polls (about 0.3 s with the back-off) before a wait fails
 
 // Epilogues.
@@ -196,8 +198,8 @@ __device__ __forceinline__ void epilogue16(const EpiArgs& a, uint32_t N, uint32_
 // Stage ring + 1 KB for the 1024-byte alignment of the swizzled tiles: 65 KB with BN = 128,
 // so three CTAs share an SM and one's epilogue overlaps the others' copies and products.
 // (Measured on the screen of 65,536 candidates by 5 members: a hidden 512 x 512 product took
-// 650 us with 3 stages and one CTA per SM, 418 us with two CTAs, 347 us with 2 stages and
-// three CTAs.)
+// 650 us with 3 stages and one CTA per SM, 418 us with two CTAs, 331 us with 2 stages and
+// three CTAs of four warps, 322 us with eight.)
 template <int BN>
 constexpr uint32_t gemm_smem_bytes() {
     return (uint32_t)kStages * (uint32_t)(kBM + BN) * kBK * 2u + 1024u;
@@ -219,7 +221,8 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     __shared__ __align__(8) uint64_t done_bar;
     __shared__ uint32_t tmem_base;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    __shared__ uint32_t issued, bad;
+    const uint32_t warp = uniform_warp(), lane = threadIdx.x & 31u;
     const uint32_t m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
     const uint32_t nk = K / kBK;
 
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
             mbar_init(&empty_bar[s], 1);
         }
         mbar_init(&done_bar, 1);
+        issued = bad = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -243,60 +247,78 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
     tc_fence_after();
     const uint32_t tmem = tmem_base;
 
-    if (threadIdx.x == 0) {
-        const uint32_t idesc = instr_desc(kBM, BN);
-        uint32_t issued = 0, consumed = 0;
-        bool ok = true;
-        auto load_stage = [&](uint32_t kb) {
-            const uint32_t s = kb % kStages;
-            uint8_t* sa = smem + s * kStageBytes;
-            mbar_expect_tx(&full_bar[s], kStageBytes);
-            tma_load_3d(sa, &ta, (int32_t)(kb * kBK), (int32_t)m0, (int32_t)(blockIdx.z * za), &full_bar[s]);
-            tma_load_3d(sa + kABytes, &tb, (int32_t)(kb * kBK), (int32_t)n0, (int32_t)(blockIdx.z * zb), &full_bar[s]);
-            ++issued;
-        };
-        for (uint32_t kb = 0; kb < nk && kb < (uint32_t)kStages; ++kb) load_stage(kb);
-        for (uint32_t kb = 0; kb < nk; ++kb) {
-            const uint32_t s = kb % kStages, ph = (kb / kStages) & 1u;
-            if (!mbar_wait(&full_bar[s], ph)) { ok = false; break; }
-            ++consumed;
-            tc_fence_after();
-            const uint32_t sa = smem_u32(smem + s * kStageBytes), sb = sa + kABytes;
-#pragma unroll
-            for (int j = 0; j < kBK / 16; ++j)  // K = 16 per MMA: advance 32 bytes within the swizzled row
-                mma_bf16(tmem, smem_desc(sa + 32u * j), smem_desc(sb + 32u * j), idesc, (kb | (uint32_t)j) != 0u);
-            mma_commit(&empty_bar[s]);
-            if (kb + kStages < nk) {
-                if (!mbar_wait(&empty_bar[s], ph)) { ok = false; break; }  // stage s read by its MMAs
-                load_stage(kb + kStages);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the inputs are the kernel before's outputs
+    if (warp == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");
+        const bool lead = elect_one();
+        uint32_t kb = 0;
+        for (; kb < nk; ++kb) {
+            const uint32_t s = kb % kStages, round = kb / kStages;
+            if (round > 0 && !warp_wait(&empty_bar[s], (round - 1u) & 1u)) {
+                if (lead) {
+                    atomicOr(err, 1);
+                    bad = 1;
+                }
+                break;
+            }
+            if (lead) {
+                uint8_t* sa = smem + s * kStageBytes;
+                mbar_expect_tx(&full_bar[s], kStageBytes);
+                tma_load_3d(sa, &ta, (int32_t)(kb * kBK), (int32_t)m0, (int32_t)(blockIdx.z * za), &full_bar[s]);
+                tma_load_3d(sa + kABytes, &tb, (int32_t)(kb * kBK), (int32_t)n0, (int32_t)(blockIdx.z * zb), &full_bar[s]);
             }
         }
-        if (!ok) {
-            atomicOr(err, 1);
-            // drain: copies issued but not consumed
-            for (uint32_t kb = consumed; kb < issued; ++kb) mbar_wait(&full_bar[kb % kStages], (kb / kStages) & 1u);
+        if (lead) issued = kb;
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = instr_desc(kBM, BN);
+        const uint64_t da = smem_desc(smem_u32(smem)), db = smem_desc(smem_u32(smem) + kABytes);
+        const bool lead = elect_one();
+        for (uint32_t kb = 0; kb < nk; ++kb) {
+            const uint32_t s = kb % kStages;
+            if (!warp_wait(&full_bar[s], (kb / kStages) & 1u)) {
+                if (lead) {
+                    atomicOr(err, 1);
+                    bad = 1;
+                }
+                break;
+            }
+            tc_fence_after();
+            if (lead) {
+                const uint64_t off = (uint64_t)(s * (kStageBytes >> 4));
+#pragma unroll
+                for (int j = 0; j < kBK / 16; ++j)  // K = 16 per MMA: advance 32 bytes within the swizzled row
+                    mma_bf16(tmem, da + off + 2u * j, db + off + 2u * j, idesc, (kb | (uint32_t)j) != 0u);
+                mma_commit(&empty_bar[s]);
+            }
+            __syncwarp();
         }
-        mma_commit(&done_bar);  // arrives when every MMA issued above has completed
+        if (lead) mma_commit(&done_bar);  // arrives when every MMA issued above has completed
     }
     __syncwarp();
     // warp-uniform, so that tcgen05.ld below runs on all 32 lanes or none
-    const bool done = __all_sync(0xFFFFFFFFu, mbar_wait(&done_bar, 0));
+    const bool done = warp_wait(&done_bar, 0);
     tc_fence_after();
     if (!done) {
         if (lane == 0) atomicOr(err, 2);
-    } else {
-        const uint32_t m = m0 + warp * 32u + lane;
+    } else {  // a warp takes its quarter of the rows and its share of the columns
+        constexpr uint32_t kCols = BN / (kGemmThreads / 128);
+        const uint32_t row = (warp & 3u) * 32u, c0 = (warp >> 2) * kCols, m = m0 + row + lane;
         float ssum = 0.f;
 #pragma unroll 1
-        for (uint32_t c = 0; c < (uint32_t)BN; c += 16) {
+        for (uint32_t c = c0; c < c0 + kCols; c += 16) {
             float v[16];
-            tmem_ld16(tmem + ((warp * 32u) << 16) + c, v);
+            tmem_ld16(tmem + (row << 16) + c, v);
             epilogue16<EP>(args, N, m, n0 + c, v, ssum);
         }
         if (EP == kEpOut && args.score && m < args.m_valid) atomicAdd(args.score + m, ssum);
     }
     tc_fence_before();
     __syncthreads();
+    if (bad && threadIdx.x == 0)  // a copy may still be in flight: wait (bounded) for the last one of every stage
+        for (uint32_t kb = issued > (uint32_t)kStages ? issued - kStages : 0u; kb < issued; ++kb)
+            mbar_wait(&full_bar[kb % kStages], (kb / kStages) & 1u);
+    __syncwarp();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN) : "memory");
 }
