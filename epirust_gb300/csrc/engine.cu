@@ -61,6 +61,9 @@ struct Replica {
     std::vector<epi_counts> s_rows;
 };
 
+// How one launch runs a world's hours (k_small): not, in one cluster, or on a grid of all SMs.
+enum class Together { kNo, kCluster, kGrid };
+
 struct epi_engine {
     std::vector<Replica> reps;
     uint32_t slots = 0;        // agent slots (chunk-padded replicates)
@@ -70,7 +73,8 @@ struct epi_engine {
     int grid_blocks = 0;       // grid of the counting kernels (k_decide, k_sleep)
     int commit_slots = kCommitSlots;  // of the launch shape (k_commit takes its work from lists)
     int resident_blocks = 0;   // SMs x resident k_decide blocks per SM
-    bool small = false;        // a world that one cluster runs (k_small)
+    uint32_t sms = 0;
+    Together together = Together::kNo;  // a world whose hours one launch runs (k_small)
     bool shape_set = false;    // a launch shape was asked for: hour kernels, whatever the size
     // device
     DevParams* d_params = nullptr;
@@ -86,6 +90,7 @@ struct epi_engine {
     uint32_t* d_claim = nullptr;
     uint32_t* d_displaced = nullptr;  // the hour's lists (HourLists)
     uint2 *d_acts = nullptr, *d_list_n = nullptr;
+    uint32_t* d_sums = nullptr;     // SmallArgs::sums
     uint32_t* d_piece_rep = nullptr;  // replicate of every kPieceWords of the bit planes (ensembles)
     uint32_t* d_par = nullptr;        // Replica::par, uploaded for the checks
     uint32_t* d_counts = nullptr;  // [hour of segment][replicate][8]
@@ -356,33 +361,39 @@ static bool rebuild_hour(uint32_t hod) { return hod >= 7u && hod <= 22u; }
 static uint32_t* pos_buf(const epi_engine* h, uint32_t par) { return h->d_pos + (size_t)par * h->slots; }
 static uint32_t* occ_buf(const epi_engine* h, uint32_t par) { return h->d_occ + (size_t)par * h->occ_words; }
 
-static uint32_t small_threads(uint32_t n) {
-    return ((n + kSmallCluster - 1) / kSmallCluster + 31u) / 32u * 32u;
-}
+static uint32_t threads_of(uint32_t n, uint32_t blocks) { return ((n + blocks - 1) / blocks + 31u) / 32u * 32u; }
 
-// Whether one cluster runs the world's hours: an agent per thread, a bit plane that the cluster
-// zeroes in a few stores per thread, and a device that schedules clusters of 16 CTAs.
-static bool fits_small(uint32_t n, size_t occ_words) {
-    if (n > kSmallAgents || occ_words > 16u * (size_t)kSmallCluster * small_threads(n)) return false;
-    if (cudaFuncSetAttribute(k_small, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+// How one launch can run the world's hours: an agent per thread, a bit plane that the threads
+// zero in a few stores each, and a device that schedules clusters of 16 CTAs, or an SM for
+// each block.
+constexpr uint32_t kShortCall = 12, kSharedThreads = 256;  // (see run_hours_chunk)
+static Together runs_together(uint32_t n, size_t occ_words, uint32_t sms) {
+    if (n <= kSmallAgents && occ_words <= 16u * (size_t)kSmallCluster * threads_of(n, kSmallCluster)) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kSmallCluster);
+        cfg.blockDim = dim3(threads_of(n, kSmallCluster));
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kSmallCluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(k_small<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, k_small<false>, &cfg) == cudaSuccess && clusters > 0)
+            return Together::kCluster;
         cudaGetLastError();
-        return false;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kSmallCluster);
-    cfg.blockDim = dim3(small_threads(n));
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kSmallCluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, k_small, &cfg) != cudaSuccess) {
+    const uint32_t threads = threads_of(n, sms);
+    if (threads <= kSmallThreads && occ_words <= 16u * (size_t)sms * threads) {
+        int dev = 0, cooperative = 0, per_sm = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && cooperative &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_small<true>, (int)threads, 0) == cudaSuccess && per_sm > 0)
+            return Together::kGrid;
         cudaGetLastError();
-        return false;
     }
-    return clusters > 0;
+    return Together::kNo;
 }
 
 // The arrays of a launch that starts from buffer par.
@@ -577,7 +588,7 @@ static int run_pieces(epi_engine* h, uint32_t first_hour, uint32_t nh) {
 // The chain's hours of a small world in one launch (k_small), which writes the counts rows to
 // pinned memory itself: one launch and one wait per call, where a captured piece takes a copy
 // of the hour base, the graph, and two copies back with a wait each.
-static int run_small(epi_engine* h, uint32_t first_hour, uint32_t nh) {
+static int run_together(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     const Replica& rep = h->reps[0];
     SmallArgs a;
     a.pos = pos_buf(h, rep.par);
@@ -592,26 +603,35 @@ static int run_small(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     a.cls = h->d_cls;
     a.danger = h->d_danger;
     a.claim = h->d_claim;
+    a.claim_cells = (uint32_t)h->claim_cells;
     a.occ_words = (uint32_t)h->occ_words;
     a.first = first_hour;
     a.hours = nh;
     a.run_loop = h->stop_rule ? 1u : 0u;
     a.ivn = h->d_ivn;
+    a.sums = h->d_sums;
     a.rows = h->h_counts;
     a.err = h->d_err;
     a.err_out = h->h_err;
+    const bool grid = h->together == Together::kGrid;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kSmallCluster);
-    cfg.blockDim = dim3(small_threads(rep.n));
+    cfg.blockDim = dim3(threads_of(rep.n, grid ? h->sms : kSmallCluster));
+    cfg.gridDim = dim3(grid ? (rep.n + cfg.blockDim.x - 1) / cfg.blockDim.x : kSmallCluster);
     cfg.stream = h->stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kSmallCluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    if (grid) {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        CK(cudaMemsetAsync(h->d_sums, 0, kGridWords * sizeof(uint32_t), h->stream));
+    } else {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kSmallCluster;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    }
     cfg.attrs = at;
     cfg.numAttrs = 1;
     *h->h_err = 0;
-    CK(cudaLaunchKernelEx(&cfg, k_small, (const DevParams*)h->d_params, a));
+    CK(cudaLaunchKernelEx(&cfg, grid ? k_small<true> : k_small<false>, (const DevParams*)h->d_params, a));
     h->kernels_launched += 1;
     CK(cudaStreamSynchronize(h->stream));
     return report_error_flag(h, *h->h_err);
@@ -628,15 +648,18 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     if ((uint64_t)first_hour + nh > 0xFFFFFFFFull) { h->err = "hour out of range"; return EPI_ERR_ARG; }
     int rc = ensure_counts(h, nh);
     if (rc) return rc;
-    const bool small = h->small && !h->shape_set && !h->profiling && !h->stream_file;
-    // claims left by an earlier hour of another window, or by a later hour, must go first (all
-    // of them where the hours use the agents' bare indices)
-    if (h->last_claim_hour >= 0 && small)
-        CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
-    else if (h->last_claim_hour >= 0 &&
+    // k_small: any call of a cluster's world.  A grid's world takes it where four such grids fit
+    // the SMs (256 threads each: engines of several threads then still run side by side; 30,000
+    // agents, two weeks in ms, one / four engines: 1.65 / 2.32, captured launches 1.79 / 2.22),
+    // and larger ones for calls of a few hours, where the launch itself is the time (98,000
+    // agents: two weeks 2.02 / 7.68, launches 1.91 / 2.89, but six hours 48 us for 66).
+    const bool small = h->together != Together::kNo && !h->shape_set && !h->profiling && !h->stream_file &&
+                       (h->together == Together::kCluster || nh <= kShortCall || threads_of(h->reps[0].n, h->sms) <= kSharedThreads);
+    // claims left by an earlier hour of another window, or by a later hour, must go first
+    if (h->last_claim_hour >= 0 &&
         ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
         CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
-    h->last_claim_hour = small ? -1 : (int64_t)first_hour + nh - 1;
+    h->last_claim_hour = (int64_t)first_hour + nh - 1;
     // the chain reads the state after first_hour - 1 from its parity's buffers
     const uint32_t need = hour_parity((first_hour + 23u) % 24u);
     std::vector<uint8_t> ran(h->R(), 0);  // a world whose run has ended runs no hour kernel
@@ -648,7 +671,7 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     }
     const size_t row_words = (size_t)h->R() * 8;
     if (small) {
-        rc = run_small(h, first_hour, nh);
+        rc = run_together(h, first_hour, nh);
         if (rc) return rc;
     } else {
         rc = run_pieces(h, first_hour, nh);
@@ -959,6 +982,7 @@ static void free_device(epi_engine* h) {
     cudaFree(h->d_params); cudaFree(h->d_chunk_rep); cudaFree(h->d_pos); cudaFree(h->d_home); cudaFree(h->d_work);
     cudaFree(h->d_wsa); cudaFree(h->d_st); cudaFree(h->d_occ); cudaFree(h->d_cls); cudaFree(h->d_danger); cudaFree(h->d_claim);
     cudaFree(h->d_displaced); cudaFree(h->d_acts); cudaFree(h->d_list_n); cudaFree(h->d_piece_rep); cudaFree(h->d_par);
+    cudaFree(h->d_sums);
     cudaFree(h->d_counts); cudaFree(h->d_seg); cudaFree(h->d_ivn); cudaFree(h->d_err); cudaFree(h->d_scratch);
     cudaFree(h->s_pos); cudaFree(h->s_wsa); cudaFree(h->s_st); cudaFree(h->s_occ); cudaFree(h->s_cls); cudaFree(h->s_danger);
     if (h->h_counts) cudaFreeHost(h->h_counts);
@@ -1096,6 +1120,7 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     per_sm = std::max(per_sm, 1);
     const uint64_t n_chunks = slots / kChunk;
     h->resident_blocks = sms * per_sm;
+    h->sms = (uint32_t)sms;
     h->grid_blocks = (int)std::min<uint64_t>(n_chunks, (uint64_t)h->resident_blocks);
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
@@ -1139,7 +1164,8 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     CK(cudaMallocHost(&h->h_seg, sizeof(SegDev) + sizeof(int) + R * sizeof(uint32_t)));  // with h_err and h_ivn
     h->h_err = reinterpret_cast<int*>(h->h_seg + 1);
     h->h_ivn = reinterpret_cast<uint32_t*>(h->h_err + 1);
-    h->small = R == 1 && fits_small(h->reps[0].n, h->occ_words);
+    if (R == 1) h->together = runs_together(h->reps[0].n, h->occ_words, h->sms);
+    if (h->together == Together::kGrid) CK(cudaMalloc(&h->d_sums, kGridWords * sizeof(uint32_t)));
     int rc = ensure_counts(h, 48);
     if (rc) return rc;
     if (!recs) {
@@ -1292,7 +1318,7 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
     double best = 1e300;
     uint32_t best_g = (uint32_t)h->grid_blocks;
     bool best_small = false;
-    if (h->small) grids.insert(grids.begin(), 0u);  // 0: no shape asked for, one cluster runs the hours
+    if (h->together != Together::kNo) grids.insert(grids.begin(), 0u);  // 0: no shape asked for, one launch runs the hours
     for (uint32_t g : grids) {
         if (g) rc = set_launch_shape(h, g, (uint32_t)h->commit_slots);
         else h->shape_set = false;

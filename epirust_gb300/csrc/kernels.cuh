@@ -555,23 +555,27 @@ __global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict
 }
 
 // ---------------------------------------------------------------- small worlds
-// A world of a few thousand agents spends an hour on launches and latency: two launches of at
-// most 64 blocks, each a chain of dependent L2 round trips behind a launch.  One cluster runs
-// all hours of a chain instead: an agent per thread, its words in registers from hour to hour,
-// and two hardware cluster barriers per hour where the launches were.  One GB300, a waking
-// hour by launches / in one cluster: 2,000 agents 8.4 / 3.0 us, 10,000 8.0 / 5.2 us, 16,000
-// 8.6 / 6.1 us; of the 5.2 us the barriers with the atomics they wait for take 1.9, proposals
-// 1.6, the claims read back 0.5.  (A second agent per thread would reach 32,768 agents at an
-// extrapolated 9 us, no faster than the launches.)
-//   before the first   proposals, an atomicMin of the agent's index on the target's claim word,
-//                      infection update, counts
-//   between them       a mover reads its claim word back: it holds its index (it moves, and
-//                      frees the word) or not (a lower index has it, or the winner has already
-//                      freed it: it stays); occupancy bits and class planes are written, the
+// An hour of a world of a few thousand agents is launches and latency: two launches of at most
+// 64 blocks, each a chain of dependent L2 round trips.  k_small runs all hours of a call in one
+// launch: an agent per thread, its words in registers from hour to hour, and two barriers per
+// hour where the launches were.
+//   before the first   proposals, an atomicMin of the agent's claim key on the target's claim
+//                      word, infection update, the block's counts added to the world's
+//   between them       a mover reads its claim word back: it holds its key (it moves) or a lower
+//                      index's (it stays); occupancy bits and class planes are written, the
 //                      spent bit plane zeroed
-// Data that other SMs write is read at L2 (BitView<true>, __ldcg).  The counts of the hour are
-// summed in the first CTA's shared memory, where every CTA reads the stop rule and the run
-// loop's guard, and go to the caller's rows (pinned host memory) from there.
+// The stop rule and the run loop's guard are read from the world's counts by every thread, and
+// the rows go to the caller (pinned host memory) from the first block.  Two forms:
+//   GRID false  one cluster of 16 CTAs, hardware barriers, counts in the first CTA's shared
+//               memory: up to 16,384 agents.  An hour of day 7..22 on one GB300, launches /
+//               cluster: 2,000 agents LA2 / CL2 us, 10,000 LA10 / CL10, 16,000 LA16 / CL16; of the
+//               10,000's the barriers with the atomics they wait for take 1.7, proposals 1.6.
+//   GRID true   a cooperative grid of one CTA per SM, barriers at L2: up to 155,648 agents.
+//               96 hours of 30,000 / 98,000 agents, ms: hour by hour 3.8 / 3.8 by captured
+//               launches, 1.9 / 2.0 here; six hours a call 1.01 / 1.05 and 0.66 / 0.77; in one
+//               call 0.49 / 0.53 and 0.44 / 0.55 (the rule of use: run_hours_chunk).  Its counts
+//               lie a cache line per bin apart: side by side, 152 blocks' atomics on one sector
+//               held every barrier up (98,000 agents, a day's mean hour 7.4 us, 6.0 apart).
 constexpr uint32_t kSmallCluster = 16;
 constexpr uint32_t kSmallThreads = 1024;
 constexpr uint32_t kSmallAgents = kSmallCluster * kSmallThreads;  // most agents of a world run so
@@ -584,11 +588,14 @@ struct SmallArgs {
     const uint32_t *home, *work;
     uint32_t* wsa;
     uint8_t *cls, *danger;
-    uint32_t* claim;      // all kNoClaim, before and after
+    uint32_t* claim;      // no keys but earlier hours' of the first hour's window
+    uint32_t claim_cells;
     uint32_t occ_words;
     uint32_t first, hours;
     uint32_t run_loop;    // 1: the stop rule and the guard apply
     uint32_t* ivn;        // the guard's new-infections figure
+    uint32_t* sums;       // k_small<true>: zero, kGridWords: 3 x 8 sums of an hour's counts and the barrier's
+                          // arrivals, a cache line each
     uint32_t* rows;       // hours x 8: bins, word 6 the halt mark; rows that did not run are zero
     int* err;             // device error word
     int* err_out;         // where the caller reads it
@@ -601,11 +608,6 @@ __host__ __device__ constexpr uint32_t hour_parity(uint32_t hod) {
 
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
 }
 // The shared-memory address of p in the cluster's first CTA.
 __device__ __forceinline__ uint32_t in_first_cta(const void* p) {
@@ -622,14 +624,28 @@ __device__ __forceinline__ uint32_t load_in_cluster(uint32_t addr) {
     return v;
 }
 
-// One movement hour of a lane's agent up to its claim and infection update (hours 7..22).
-template <int HC>
-__device__ __forceinline__ uint32_t small_move(const DevParams& P, const BitView<true>& pl, const MoveTables& tables,
-                                               const Box* boxes, uint32_t& s, uint32_t* wsa, uint32_t hm, uint32_t wk,
-                                               uint32_t p, uint32_t hour, Draws& dr, bool& infect) {
-    return perform_movements<HC>(P, pl, tables, boxes, s, wsa, hm, wk, p, hour, dr, infect);
+// The barrier of a grid whose blocks all run (a cooperative launch): false, on every thread of
+// the block, when the others did not arrive within some seconds.
+constexpr uint32_t kLineWords = 32, kGridWords = 25 * kLineWords;
+constexpr uint32_t kGridSpinLimit = 1u << 22;
+__device__ __forceinline__ bool grid_sync(uint32_t* arrived, uint32_t& target) {
+    target += gridDim.x;
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("fence.acq_rel.gpu;\n\tred.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+        ok = false;
+        for (uint32_t it = 0; it < kGridSpinLimit && !ok; ++it) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+            ok = (int32_t)(v - target) >= 0;
+        }
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    return !__syncthreads_or(!ok);
 }
 
+template <bool GRID>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __restrict__ Pall, const __grid_constant__ SmallArgs a) {
     __shared__ uint32_t sh[8];
     __shared__ uint32_t total[3][8];  // the first CTA's are the cluster's
@@ -637,14 +653,33 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
     __shared__ MoveTables tables;
     __shared__ Box boxes[kNumAreas];
     const DevParams& P = sP;
-    const uint32_t rank = cluster_rank(), tid = threadIdx.x, i = rank * blockDim.x + tid;
+    const uint32_t rank = blockIdx.x, tid = threadIdx.x, i = rank * blockDim.x + tid;
     stage_tables(tables);
     stage_boxes(boxes, Pall[0]);
     for (uint32_t k = tid; k < sizeof(DevParams) / 4; k += blockDim.x)
         reinterpret_cast<uint32_t*>(&sP)[k] = reinterpret_cast<const uint32_t*>(Pall)[k];
     if (tid < 8) sh[tid] = total[0][tid] = total[1][tid] = total[2][tid] = 0u;
-    cluster_sync();  // every CTA of the cluster runs, and its counters are clear
-    const uint32_t sums = in_first_cta(&total[0][0]);
+    if (GRID) __syncthreads();
+    else cluster_sync();  // every CTA of the cluster runs, and its counters are clear
+    const uint32_t sums = GRID ? 0u : in_first_cta(&total[0][0]);
+    uint32_t arrivals = 0u;  // GRID: of all blocks at all barriers so far
+    bool ok = true;
+    // the counts of the hour, from a block's sums to the world's
+    auto add_counts = [&](uint32_t slot) {
+        if (tid < 6u) {
+            if (!sh[tid]) return;
+            if (GRID) atomicAdd(&a.sums[(slot * 8u + tid) * kLineWords], sh[tid]);
+            else add_in_cluster(sums + (slot * 8u + tid) * 4u, sh[tid]);
+            sh[tid] = 0u;
+        }
+    };
+    auto count_of = [&](uint32_t slot, uint32_t bin) {
+        return GRID ? __ldcg(&a.sums[(slot * 8u + bin) * kLineWords]) : load_in_cluster(sums + (slot * 8u + bin) * 4u);
+    };
+    auto sync = [&] {
+        if (GRID) ok = grid_sync(a.sums + 24u * kLineWords, arrivals) && ok;
+        else cluster_sync();
+    };
     const bool valid = i < P.n;
     uint32_t s = 0u, at = 0u, p = 0u, hm = 0u, wk = 0u;
     if (valid) {
@@ -659,8 +694,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
     uint32_t slot = 0u;        // of total: the hour running
     uint32_t last = a.first;   // the last hour that ran
     uint32_t written = 0u;     // rows written by the first CTA
+    uint32_t window = a.first / kClaimWindow;  // of the claim plane's keys
     bool over = !P.active;
-    for (uint32_t k = 0; k < a.hours && !over; ++k) {
+    for (uint32_t k = 0; k < a.hours && !over && ok; ++k) {
         const uint32_t hour = a.first + k, hod = hour % 24u;
         if (k > 0 && hod >= 2u && hod <= 6u) {  // hour 1 has sent everyone home: nothing changes
             if (rank == 0 && tid < 8) a.rows[(size_t)k * 8u + tid] = 0u;
@@ -670,18 +706,22 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
         }
         Tally tally;
         const uint32_t s0 = s;
+        uint32_t e, inf, hos;
         if (hod >= 1u && hod <= 6u) {
             if (valid && st_ws(s) != EPI_WS_HOSPITAL_STAFF) s = with_area(s, kHome);
             tally.add(valid, count_bin(s));
             tally.flush(sh);
-            cluster_sync();
-            if (tid < 6u) {
-                add_in_cluster(sums + (slot * 8u + tid) * 4u, sh[tid]);
-                sh[tid] = 0u;
-            }
-            cluster_sync();
+            __syncthreads();
+            add_counts(slot);
+            sync();
+            e = count_of(slot, 1u), inf = count_of(slot, 2u), hos = count_of(slot, 3u);
         } else {
             const bool patch = hod == 0u || hod == 23u;
+            if (hour / kClaimWindow != window) {
+                for (uint32_t c = i; c < a.claim_cells; c += gridDim.x * blockDim.x) a.claim[c] = kNoClaim;
+                window = hour / kClaimWindow;
+                sync();
+            }
             uint32_t* occ = a.occ_buf[hour_parity((hod + 23u) % 24u)];
             uint32_t* next = a.occ_buf[hour_parity(hod)];
             const BitView<true> pl{occ, a.cls, a.danger, P.G, P.WP, P.PW, a.err};
@@ -695,29 +735,25 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
             } else if (valid) {
                 switch (hour_class(hod)) {
                     case kHcEnd: nc = routine_end(P, pl, s, hm, p, dr); break;
-                    case kHcTransport: nc = small_move<kHcTransport>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
-                    case kHcWork: nc = small_move<kHcWork>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
-                    case kHcNoon: nc = small_move<kHcNoon>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
-                    case kHcHome: nc = small_move<kHcHome>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
-                    default: nc = small_move<kHcMove>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcTransport: nc = perform_movements<kHcTransport>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcWork: nc = perform_movements<kHcWork>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcNoon: nc = perform_movements<kHcNoon>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    case kHcHome: nc = perform_movements<kHcHome>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
+                    default: nc = perform_movements<kHcMove>(P, pl, tables, boxes, s, a.wsa + i, hm, wk, p, hour, dr, infect); break;
                 }
             }
             const bool moving = nc != p;
             uint32_t* claim = &a.claim[(nc >> 16) * (uint32_t)P.W + (nc & 0xFFFFu)];
-            if (moving) atomicMin(claim, i);
+            const uint32_t key = claim_key(hour, i);
+            if (moving) atomicMin(claim, key);
             if (infect) infection_dynamics(P, pl, tables, boxes, s, at, hm, wk, nc, hour, dr);
             tally.add(valid, count_bin(s));
             tally.flush(sh);
-            cluster_sync();  // every claim is in, and the bit plane of before has been read
-            if (tid < 6u) {
-                add_in_cluster(sums + (slot * 8u + tid) * 4u, sh[tid]);
-                sh[tid] = 0u;
-            }
-            bool win = false;
-            if (moving) {
-                win = __ldcg(claim) == i;
-                if (win) atomicMax(claim, kNoClaim);  // (not a plain store: see send_back)
-            }
+            __syncthreads();
+            add_counts(slot);
+            sync();  // every claim is in, and the bit plane of before has been read
+            e = count_of(slot, 1u), inf = count_of(slot, 2u), hos = count_of(slot, 3u);
+            const bool win = moving && *(volatile const uint32_t*)claim == key;
             const uint32_t q = win ? nc : p;
             const uint32_t Xo = (p & 0xFFFFu) + 1u, X = (q & 0xFFFFu) + 1u;
             uint32_t* word = &next[((q >> 16) + 1u) * P.PW + (X >> 5)];
@@ -732,14 +768,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
             }
             p = q;
             if (!patch)
-                for (uint32_t w = i; w < a.occ_words / 4u; w += kSmallCluster * blockDim.x)
+                for (uint32_t w = i; w < a.occ_words / 4u; w += gridDim.x * blockDim.x)
                     reinterpret_cast<uint4*>(occ)[w] = make_uint4(0u, 0u, 0u, 0u);
-            cluster_sync();
+            sync();
         }
         last = hour;
-        // the row, the stop rule and the guard, from the cluster's sums
-        const uint32_t at_sums = sums + slot * 32u;
-        const uint32_t e = load_in_cluster(at_sums + 4u), inf = load_in_cluster(at_sums + 8u), hos = load_in_cluster(at_sums + 12u);
+        // the row, the stop rule and the guard
         bool fire = false;
         if (a.run_loop) {
             if (hod == 0u) {
@@ -752,9 +786,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
             over = fire || (e | inf | hos) == 0u;
         }
         if (rank == 0 && tid < 8u) {
-            a.rows[(size_t)k * 8u + tid] = tid < 6u ? total[slot][tid] : (tid == 6u && fire ? 1u : 0u);
+            a.rows[(size_t)k * 8u + tid] = tid < 6u ? count_of(slot, tid) : (tid == 6u && fire ? 1u : 0u);
             // (cleared two hours before its next use: its readers have passed a barrier by then)
-            total[(slot + 2u) % 3u][tid] = 0u;
+            if (GRID) a.sums[((slot + 2u) % 3u * 8u + tid) * kLineWords] = 0u;
+            else total[(slot + 2u) % 3u][tid] = 0u;
         }
         written = k + 1u;
         slot = (slot + 1u) % 3u;
@@ -770,7 +805,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
             *a.err_out = *(volatile int*)a.err;
         }
     }
-    cluster_sync();  // the first CTA's counters outlive their readers
+    if (!GRID) cluster_sync();  // the first CTA's counters outlive their readers
+    if (!ok && tid == 0) *(volatile int*)a.err_out = 4;
 }
 
 // ---------------------------------------------------------------- the caller-owned planes

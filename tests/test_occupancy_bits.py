@@ -124,3 +124,40 @@ def test_replicates_that_end_early_keep_their_buffers(gpu):
     for eng in lone:
         eng.close()
     ens.close()
+
+
+@pytest.mark.parametrize("n,grid", [(16385, 280), (38912, 420), (38913, 421), (155648, 800), (155649, 800)])
+def test_one_grid_equals_hour_kernels(gpu, n, grid):
+    """The smallest and the largest worlds whose hours one grid runs (for calls of a few hours, and
+    up to 38,912 agents for all), and one agent more, against the hour kernels, in calls of one to
+    thirty hours over a boundary of the claim keys' window (128 hours), taking over from each
+    other in between."""
+    cfg = make_config(n=n, grid=grid, hours=24 * 9, seed=n, disease=COVID_FAST, starting=(0, 0, 1, 3 + n // 300), beds=0.002)
+    one, other = _engine(cfg), _engine(cfg, hour_kernels=True)
+    hour = 1
+    for k in (1, 1, 5, 1, 1, 12, 30, 13, 11, 30, 1, 24, 2, 12):
+        if hour in (53, 77):
+            one.set_launch_shape(2, 4)  # from here on the hour kernels
+        assert (_rows(one.simulate_hours(hour, k)) == _rows(other.simulate_hours(hour, k))).all(), hour
+        hour += k
+    assert hour > 130
+    assert (one.snapshot().view(np.uint8) == other.snapshot().view(np.uint8)).all()
+    one.check_invariants()
+    one.close()
+    other.close()
+
+
+@pytest.mark.parametrize("n,grid", [(16385, 261), (30000, 430)])
+def test_one_grid_runs_the_run_loop(gpu, n, grid):
+    """Lockdown, vaccination, hospital build and the early stop, as the hour kernels have them."""
+    cfg = make_config(n=n, grid=grid, hours=24 * 40, seed=n, disease=COVID_FAST, starting=(0, 0, 1, 3 + n // 500),
+                      beds=0.002, occupancy=0.5,
+                      interventions=[{"Lockdown": {"at_number_of_infections": 1 + n // 100, "essential_workers_population": 0.2}},
+                                     {"Vaccinate": {"at_hour": 300, "percent": 0.2}}])
+    one, other = _engine(cfg), _engine(cfg, hour_kernels=True)
+    assert (_rows(one.run()) == _rows(other.run())).all()
+    assert (one.snapshot().view(np.uint8) == other.snapshot().view(np.uint8)).all()
+    one.check_invariants()
+    assert one.kernels_launched() < other.kernels_launched() // 4
+    one.close()
+    other.close()
