@@ -169,11 +169,7 @@ EPI_HD int record_words(const DevParams& hp, const epi_agent_record& a, AgentWor
 // One write to every page of a caller's buffer that a device copy is about to fill: a copy into
 // pages that the process has never touched waits for them one by one on the device's side (a
 // GB300's records of 300,000 agents: 2.2 to 9.2 ms into fresh pages, 0.7 ms after this).
-inline void touch_pages(void* p, size_t bytes) {
-    volatile char* c = static_cast<volatile char*>(p);
-    for (size_t b = 0; b < bytes; b += 4096) c[b] = 0;
-    if (bytes) c[bytes - 1] = 0;
-}
+void touch_pages(void* p, size_t bytes);
 
 constexpr uint32_t kChunk = 256;  // agent slots per chunk; replicates start on chunk boundaries
 

@@ -10,6 +10,8 @@
 #include <cstring>
 #include <ctime>
 #include <stdexcept>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 
 #include "json.hpp"
@@ -550,6 +552,30 @@ int write_outputs(const std::string& dir, const std::string& engine_id, const st
     std::fprintf(f, "]");
     std::fclose(f);
     return EPI_OK;
+}
+
+// Fresh pages cost the kernel's zeroing, 30 GB/s a core, so large buffers take up to four
+// threads (fresh 12 / 40 / 160 MB on the Grace host: one 0.39 / 1.34 / 5.4 ms, two 0.29 / 0.79 /
+// 3.0, four 0.22 / 0.48 / 1.65, eight no better; 4 MB 0.13 ms with one, 0.16 with two).
+void touch_pages(void* p, size_t bytes) {
+    constexpr size_t kPerThread = (size_t)3 << 20, kMost = 4;
+    const size_t parts = std::min(std::max(bytes / kPerThread, (size_t)1), kMost), per = bytes / parts;
+    const auto touch = [p](size_t from, size_t to) {
+        volatile char* c = static_cast<volatile char*>(p);
+        for (size_t b = from; b < to; b += 4096) c[b] = 0;
+        if (to > from) c[to - 1] = 0;
+    };
+    std::thread others[kMost - 1];
+    size_t started = 1;  // parts with a thread, the caller's own included
+    try {
+        for (; started < parts; ++started)
+            others[started - 1] = std::thread(touch, started * per, started + 1 == parts ? bytes : (started + 1) * per);
+    } catch (const std::system_error&) {  // no more threads: the caller takes the rest
+        touch(started * per, bytes);
+    }
+    touch(0, parts > 1 ? per : bytes);
+    for (std::thread& t : others)
+        if (t.joinable()) t.join();
 }
 
 }  // namespace epi

@@ -567,9 +567,10 @@ __global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict
 // The stop rule and the run loop's guard are read from the world's counts by every thread, and
 // the rows go to the caller (pinned host memory) from the first block.  Two forms:
 //   GRID false  one cluster of 16 CTAs, hardware barriers, counts in the first CTA's shared
-//               memory: up to 16,384 agents.  An hour of day 7..22 on one GB300, launches /
-//               cluster: 2,000 agents LA2 / CL2 us, 10,000 LA10 / CL10, 16,000 LA16 / CL16; of the
-//               10,000's the barriers with the atomics they wait for take 1.7, proposals 1.6.
+//               memory: up to 16,384 agents.  Two weeks of hours on one GB300, captured
+//               launches / cluster: 2,000 agents 1.53 / 0.84 ms, 10,000 1.62 / 1.16, 16,000
+//               1.63 / 1.48.  An hour of the 10,000's spends 1.7 of its 4.6 us in the barriers
+//               and the atomics they wait for, 1.6 in proposals.
 //   GRID true   a cooperative grid of one CTA per SM, barriers at L2: up to 155,648 agents.
 //               96 hours of 30,000 / 98,000 agents, ms: hour by hour 3.8 / 3.8 by captured
 //               launches, 1.9 / 2.0 here; six hours a call 1.01 / 1.05 and 0.66 / 0.77; in one

@@ -259,7 +259,7 @@ class Epidemiology:
 
     def snapshot(self) -> np.ndarray:
         n = self.population()
-        out = np.zeros(n, dtype=AGENT_DTYPE)
+        out = np.empty(n, dtype=AGENT_DTYPE)  # the call writes every byte
         check(lib().epi_engine_snapshot(self._h, out.ctypes.data, n), self._h)
         return out
 
@@ -362,7 +362,7 @@ class Ensemble:
         return [rows[r, : n[r]] for r in range(self.replicates)]
 
     def snapshot(self, r: int) -> np.ndarray:
-        out = np.zeros(self.params[r].number_of_agents, dtype=AGENT_DTYPE)
+        out = np.empty(self.params[r].number_of_agents, dtype=AGENT_DTYPE)
         self._check(lib().epi_ensemble_snapshot(self._h, r, out.ctypes.data, len(out)))
         return out
 

@@ -192,7 +192,7 @@ class Surrogate:
 
     def get_params(self) -> np.ndarray:
         """(n_params,) for one member, else (members, n_params)."""
-        out = np.zeros((self.members, self.n_params), dtype=np.float32)
+        out = np.empty((self.members, self.n_params), dtype=np.float32)
         self._check(lib().epi_mlp_get_params(self._h, self._ptr(out)))
         return self._shape(out)
 
@@ -234,7 +234,7 @@ class Surrogate:
         """Loss and gradients of one minibatch: (float, (n_params,)) for one member, else
         ((members,), (members, n_params))."""
         x, y = self._f32(x), self._f32(y)
-        g = np.zeros((self.members, self.n_params), dtype=np.float32)
+        g = np.empty((self.members, self.n_params), dtype=np.float32)
         loss = np.zeros(self.members, dtype=np.float32)
         self._check(lib().epi_mlp_gradients(self._h, self._ptr(x), self._ptr(y), x.shape[0], self._ptr(g),
                                             self._ptr(loss)))
@@ -243,7 +243,7 @@ class Surrogate:
     def predict_members(self, x) -> np.ndarray:
         """Every member's curves: (members, n, out_dim)."""
         x = self._f32(x)
-        y = np.zeros((self.members, x.shape[0], self.cfg.out_dim), dtype=np.float32)
+        y = np.empty((self.members, x.shape[0], self.cfg.out_dim), dtype=np.float32)  # the call writes all of it
         self._check(lib().epi_mlp_predict(self._h, self._ptr(x), x.shape[0], self._ptr(y)))
         return self._from_z(y)
 
@@ -257,7 +257,7 @@ class Surrogate:
         training scale (the standardised outputs when set_output_scaling was called):
         (members, n)."""
         x, t = self._f32(x), self._to_z(np.asarray(target)[None])[0]
-        s = np.zeros((self.members, x.shape[0]), dtype=np.float32)
+        s = np.empty((self.members, x.shape[0]), dtype=np.float32)
         self._check(lib().epi_mlp_score(self._h, self._ptr(x), x.shape[0], self._ptr(t), self._ptr(s)))
         return s
 
