@@ -401,9 +401,11 @@ int enqueue_step(epi_mlp* h, uint32_t off, bool grads) {
         a.hp = AdamHyper{h->cfg.lr, h->cfg.beta1, h->cfg.beta2, h->cfg.eps};
         const bool w = l > 0 && wide(h->layers[l].K);
         // weight gradients: narrow while a hidden layer's fit two to an SM (200 steps on one
-        // GB300, narrow / wide: 3 networks 12.4 / 12.4 ms, 5 networks 19.6 / 18.8, 10 networks
-        // 32.1 / 30.7)
-        const bool ww = h->cfg.hidden / kBM * (h->cfg.hidden / kTrainBN) * E > 2 * h->sms;
+        // GB300, narrow / wide: 3 networks 12.4 / 12.4 ms, 8 networks 27.4 / 28.2, 16 networks
+        // 46.8 / 44.9); in the last launch, which has nothing beside them, while they fit three
+        // times (5 networks 19.3 / 20.5, 10 networks 32.3 / 33.1, 16 networks 45.2 / 44.9)
+        const uint32_t narrow = h->cfg.hidden / kBM * (h->cfg.hidden / kTrainBN) * E;
+        const bool ww = narrow > (l > 0 ? 2u : 6u) * h->sms;
         const int bn = w ? kTrainWideBN : kTrainBN;
         if (l > 0) {
             MlpLayer &ly = h->layers[l], &pv = h->layers[l - 1];
