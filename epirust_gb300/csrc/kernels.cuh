@@ -57,14 +57,14 @@ struct Tally {
     }
 };
 
-// Consecutive chunks a block takes per grid-stride step.  An ensemble block that strides one
-// chunk at a time switches replicate at nearly every step (a parameter reload and a
-// histogram flush); groups of 8 made the 256-replicate ensemble 10 % faster.  A single world
-// keeps 1: the plain stride, where the resident blocks sweep one contiguous band of agents,
-// was measured fastest (groups of 2, 4, 8 were 2, 8, 15 % slower, a scattered chunk order
-// 6 % slower).
-constexpr uint32_t kEnsembleChunkGroup = 8;
-constexpr uint32_t kWorldChunkGroup = 1;
+// Consecutive chunks a block takes per grid-stride step.  A single world takes 1: the plain
+// stride, where the resident blocks sweep one contiguous band of agents, was measured fastest
+// (groups of 2, 4, 8 were 2, 8, 15 % slower, a scattered chunk order 6 % slower).  An ensemble
+// block that strides one chunk at a time switches replicate at nearly every step (a parameter
+// reload and a histogram flush), so it takes groups of `size`; inverse = ceil(2^32 / size).
+struct ChunkGroup {
+    uint32_t size, inverse;
+};
 
 // Block-uniform bookkeeping of the replicate a block is working on.
 struct BlockRep {
@@ -168,7 +168,7 @@ __device__ __forceinline__ void sleep_agent(uint2* __restrict__ st, uint32_t slo
 }
 
 __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict__ Pall, const uint32_t* __restrict__ chunk_rep,
-                                                    uint32_t n_chunks, uint2* __restrict__ st, HourArgs ha) {
+                                                    uint32_t n_chunks, uint32_t grp, uint2* __restrict__ st, HourArgs ha) {
     __shared__ uint32_t sh[8];
     __shared__ DevParams sP;
     dep_wait();
@@ -200,7 +200,6 @@ __global__ void __launch_bounds__(kThreads) k_sleep(const DevParams* __restrict_
         flush_rep(br, tally, sh, row_ptr(ha, hr.row));
         return;
     }
-    const uint32_t grp = kEnsembleChunkGroup;  // chunks per stride step
     for (uint32_t c = blockIdx.x * grp, k = 0; c < n_chunks;
          c = (++k < grp) ? c + 1u : c + (gridDim.x - 1u) * grp + 1u, k = (k < grp) ? k : 0u) {
         const uint32_t r = chunk_rep ? chunk_rep[c] : 0u;
@@ -244,22 +243,22 @@ struct HourLists {
     uint2* n;             // per warp: entries of the two lists
 };
 
-// The k-th chunk of block b (a grid of blocks): plain stride for a single world, groups of
-// kEnsembleChunkGroup for an ensemble.
+// The k-th chunk of this block: plain stride for a single world, groups for an ensemble.
 template <bool ENS>
-__device__ __forceinline__ uint32_t chunk_at(uint32_t b, uint32_t grid, uint32_t k) {
-    if (!ENS) return b + k * grid;
-    return ((k / kEnsembleChunkGroup) * grid + b) * kEnsembleChunkGroup + k % kEnsembleChunkGroup;
+__device__ __forceinline__ uint32_t chunk_at(ChunkGroup g, uint32_t k) {
+    if (!ENS) return blockIdx.x + k * gridDim.x;
+    const uint32_t q = g.size > 1u ? __umulhi(k, g.inverse) : k;  // k / size (k < 2^28)
+    return (q * gridDim.x + blockIdx.x) * g.size + (k - q * g.size);
 }
 template <bool ENS>
-__device__ __forceinline__ uint32_t list_slot(uint32_t e) {
-    return chunk_at<ENS>(blockIdx.x, gridDim.x, e >> 5) * kChunk + (threadIdx.x & ~31u) + (e & 31u);
+__device__ __forceinline__ uint32_t list_slot(ChunkGroup g, uint32_t e) {
+    return chunk_at<ENS>(g, e >> 5) * kChunk + (threadIdx.x & ~31u) + (e & 31u);
 }
 // Append the entries of the lanes with f set to the warp's list (whole warps; n is uniform).
 template <bool ENS, class T>
-__device__ __forceinline__ void list_append(T* list, uint32_t& n, bool f, const T& v) {
+__device__ __forceinline__ void list_append(ChunkGroup g, T* list, uint32_t& n, bool f, const T& v) {
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, f);
-    if (f) list[list_slot<ENS>(n + (uint32_t)__popc(m & ((1u << (threadIdx.x & 31u)) - 1u)))] = v;
+    if (f) list[list_slot<ENS>(g, n + (uint32_t)__popc(m & ((1u << (threadIdx.x & 31u)) - 1u)))] = v;
     n += (uint32_t)__popc(m);
 }
 
@@ -356,6 +355,7 @@ struct HourBuffers {
     uint8_t *cls, *danger;
     uint32_t* claim;
     HourLists lists;
+    ChunkGroup group;
     int* err;
 };
 
@@ -407,8 +407,8 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                     tally.add_susceptible(valid);
                 } else {
                     tally.add(valid, a.bin);
-                    list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
-                    list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
+                    list_append<ENS>(B.group, B.lists.displaced, n_displaced, a.displaces, a.loser);
+                    list_append<ENS>(B.group, B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
                 }
             }
         }
@@ -417,12 +417,16 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
         // The replicate of the next chunk is read one chunk ahead, and a chunk's agent words are
         // read before its replicate is known (every chunk of an ensemble is whole in the slot
         // arrays), so neither waits on the other.
-        uint32_t c = chunk_at<true>(blockIdx.x, gridDim.x, 0u);
+        uint32_t c = blockIdx.x * B.group.size, left = B.group.size;
         uint32_t r_next = c < n_chunks ? chunk_rep[c] : 0u;
-        for (uint32_t k = 0; c < n_chunks; ++k) {
+        while (c < n_chunks) {
             const uint32_t r = r_next;
             const uint32_t slot = c * kChunk + threadIdx.x;
-            c = chunk_at<true>(blockIdx.x, gridDim.x, k + 1u);
+            ++c;
+            if (--left == 0u) {  // the block's next group
+                c += (gridDim.x - 1u) * B.group.size;
+                left = B.group.size;
+            }
             r_next = c < n_chunks ? chunk_rep[c] : 0u;
             const uint2 sv = B.st[slot];
             const uint32_t pw = B.pos[slot], hw = B.home[slot], ww = B.work[slot];
@@ -451,8 +455,8 @@ __device__ __forceinline__ void decide_body(const DevParams* __restrict__ Pall, 
                 tally.add_susceptible(valid);
             } else {
                 tally.add(valid, a.bin);
-                list_append<ENS>(B.lists.displaced, n_displaced, a.displaces, a.loser);
-                list_append<ENS>(B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
+                list_append<ENS>(B.group, B.lists.displaced, n_displaced, a.displaces, a.loser);
+                list_append<ENS>(B.group, B.lists.acts, n_acts, a.act, make_uint2(slot, a.target));
             }
         }
     }
@@ -514,12 +518,12 @@ __global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict
     const uint32_t* old = PATCH ? B.pos_next : B.pos;
     uint32_t* occ = PATCH ? B.occ : B.occ_next;
     for (uint32_t e = lane; e < n.x; e += 32u) {
-        const uint32_t slot = B.lists.displaced[list_slot<ENS>(e)];
+        const uint32_t slot = B.lists.displaced[list_slot<ENS>(B.group, e)];
         const DevParams& P = Pall[ENS ? chunk_rep[slot / kChunk] : 0u];
         send_back<PATCH>(P, slot, B.st, dest, old, occ + P.occ_off, B.cls + P.plane_off, B.danger + P.plane_off);
     }
     for (uint32_t e = lane; e < n.y; e += 32u) {
-        const uint2 a = B.lists.acts[list_slot<ENS>(e)];
+        const uint2 a = B.lists.acts[list_slot<ENS>(B.group, e)];
         const DevParams& P = Pall[ENS ? chunk_rep[a.x / kChunk] : 0u];
         const uint32_t o = old[a.x], t = target_xy(a.y), cls = target_class(a.y), cls0 = target_old_class(a.y);
         uint8_t *cp = B.cls + P.plane_off, *dg = B.danger + P.plane_off;

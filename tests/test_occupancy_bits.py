@@ -161,3 +161,21 @@ def test_one_grid_runs_the_run_loop(gpu, n, grid):
     assert one.kernels_launched() < other.kernels_launched() // 4
     one.close()
     other.close()
+
+
+# chunks a block takes at a time on 152 SMs: 1, 3, 5, 9 (the last a group of 9 with one block's cut short)
+@pytest.mark.parametrize("replicates,n", [(3, 700), (40, 13000), (70, 16500), (80, 24100)])
+def test_replicates_in_groups_of_chunks_equal_lone_engines(gpu, replicates, n):
+    from epirust_gb300 import Config, Ensemble
+
+    cfgs = [make_config(n=n - 97 * (i % 5), grid=int((n / 0.2) ** 0.5) + i % 3, hours=40, seed=7 + i, disease=COVID_FAST,
+                        starting=(0, 0, n // 100, n // 50)) for i in range(replicates)]
+    ens = Ensemble([Config(json.dumps(c)).params for c in cfgs])
+    rows = ens.run()
+    ens.check_invariants()
+    for r in (0, replicates // 2, replicates - 1):
+        eng = _engine(cfgs[r], hour_kernels=True)
+        assert (_rows(rows[r]) == _rows(eng.run())).all(), r
+        assert (ens.snapshot(r).view(np.uint8) == eng.snapshot().view(np.uint8)).all(), r
+        eng.close()
+    ens.close()
