@@ -229,7 +229,8 @@ struct epi_mlp {
     uint32_t n_data = 0;
     // inference
     uint32_t p_cap = 0;
-    float* d_py = nullptr;        // E x n x out_pad
+    uint8_t* d_predict = nullptr; // the layers' ph, then
+    float* d_py = nullptr;        // E x n x out_pad (the caller's rows before that)
     float* d_pscore = nullptr;    // E x n
     float* d_ptarget = nullptr;   // out_pad
     cudaGraphExec_t step_graph = nullptr, group_graph = nullptr;  // one step, kGroupSteps steps
@@ -485,12 +486,15 @@ int check_err(epi_mlp* h) {
 }
 
 // n caller rows of in_dim floats into BF16 rows of kInPad on the device (n_rows of them).
-int upload_inputs(epi_mlp* h, const float* x, uint32_t n, uint32_t n_rows, __nv_bfloat16* out, __nv_bfloat16* xt = nullptr,
-                  uint32_t xt_pitch = 0) {
+int upload_inputs(epi_mlp* h, const float* x, uint32_t n, uint32_t n_rows, float* stage, __nv_bfloat16* out,
+                  __nv_bfloat16* xt = nullptr, uint32_t xt_pitch = 0) {
     const size_t floats = (size_t)n * h->cfg.in_dim;
-    MRC(ensure_raw(h, floats));
-    MCK(cudaMemcpyAsync(h->d_raw, x, floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-    k_pad_inputs<<<blocks_for((size_t)n_rows * (kInPad / 2)), kSmallThreads, 0, h->stream>>>(h->d_raw, n, n_rows,
+    if (!stage) {
+        MRC(ensure_raw(h, floats));
+        stage = h->d_raw;
+    }
+    MCK(cudaMemcpyAsync(stage, x, floats * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    k_pad_inputs<<<blocks_for((size_t)n_rows * (kInPad / 2)), kSmallThreads, 0, h->stream>>>(stage, n, n_rows,
                                                                                             h->cfg.in_dim, out, xt, xt_pitch);
     MCK(cudaGetLastError());
     h->launches++;
@@ -511,23 +515,27 @@ int upload_targets(epi_mlp* h, const float* y, uint32_t n, float* out) {
 
 int ensure_predict(epi_mlp* h, uint32_t n_pad) {
     if (n_pad <= h->p_cap) return EPI_OK;
-    for (auto& ly : h->layers) {
-        if (ly.ph) cudaFree(ly.ph);
-        ly.ph = nullptr;
-    }
-    cudaFree(h->d_py);
-    cudaFree(h->d_pscore);
-    h->d_py = nullptr;
-    h->d_pscore = nullptr;
+    cudaFree(h->d_predict);
+    h->d_predict = nullptr;
     h->p_cap = 0;
+    // one allocation for all of them (a first call of a few rows is mostly allocations)
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255u) / 256u * 256u;
+        return at;
+    };
+    std::vector<size_t> ph(h->L);
+    for (uint32_t l = 0; l < h->L; ++l) ph[l] = take((size_t)(l == 0 ? 1u : h->E) * n_pad * h->layers[l].K * sizeof(__nv_bfloat16));
+    const size_t py = take((size_t)h->E * n_pad * h->out_pad * sizeof(float)), ps = take((size_t)h->E * n_pad * sizeof(float));
+    MCK(cudaMalloc(&h->d_predict, bytes));
     for (uint32_t l = 0; l < h->L; ++l) {
         MlpLayer& ly = h->layers[l];
-        const uint32_t depth = l == 0 ? 1u : h->E;
-        MCK(cudaMalloc(&ly.ph, (size_t)depth * n_pad * ly.K * sizeof(__nv_bfloat16)));
-        MRC(make_map(h, &ly.t_ph, ly.ph, n_pad, ly.K, kBM, depth));
+        ly.ph = reinterpret_cast<__nv_bfloat16*>(h->d_predict + ph[l]);
+        MRC(make_map(h, &ly.t_ph, ly.ph, n_pad, ly.K, kBM, l == 0 ? 1u : h->E));
     }
-    MCK(cudaMalloc(&h->d_py, (size_t)h->E * n_pad * h->out_pad * sizeof(float)));
-    MCK(cudaMalloc(&h->d_pscore, (size_t)h->E * n_pad * sizeof(float)));
+    h->d_py = reinterpret_cast<float*>(h->d_predict + py);
+    h->d_pscore = reinterpret_cast<float*>(h->d_predict + ps);
     h->p_cap = n_pad;
     return EPI_OK;
 }
@@ -539,7 +547,8 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
     const uint32_t n_pad = std::max<uint32_t>(round_up(n, kBM), kBM);
     MRC(ensure_predict(h, n_pad));
     const uint64_t cap = h->p_cap;
-    MRC(upload_inputs(h, x, n, n_pad, h->layers[0].ph));
+    // (the outputs' buffer, unused until the last layer, holds the caller's rows: in_dim <= 64 < out_pad)
+    MRC(upload_inputs(h, x, n, n_pad, h->d_py, h->layers[0].ph));
     if (target) {
         MCK(cudaMemcpyAsync(h->d_ptarget, target, h->cfg.out_dim * sizeof(float), cudaMemcpyHostToDevice, h->stream));
         MCK(cudaMemsetAsync(h->d_pscore, 0, (size_t)h->E * cap * sizeof(float), h->stream));
@@ -573,11 +582,11 @@ void free_all(epi_mlp* h) {
     for (auto& ly : h->layers) {
         cudaFree(ly.w); cudaFree(ly.b); cudaFree(ly.mw); cudaFree(ly.vw); cudaFree(ly.mb); cudaFree(ly.vb);
         cudaFree(ly.gw); cudaFree(ly.gb); cudaFree(ly.wb); cudaFree(ly.wtb);
-        cudaFree(ly.h); cudaFree(ly.ht); cudaFree(ly.z); cudaFree(ly.dz); cudaFree(ly.dzt); cudaFree(ly.ph);
+        cudaFree(ly.h); cudaFree(ly.ht); cudaFree(ly.z); cudaFree(ly.dz); cudaFree(ly.dzt);
     }
     cudaFree(h->d_err); cudaFree(h->d_tr); cudaFree(h->d_t); cudaFree(h->d_loss);
     cudaFree(h->d_idx); cudaFree(h->d_raw); cudaFree(h->d_corr);
-    cudaFree(h->d_xs); cudaFree(h->d_ys); cudaFree(h->d_py); cudaFree(h->d_pscore); cudaFree(h->d_ptarget);
+    cudaFree(h->d_xs); cudaFree(h->d_ys); cudaFree(h->d_predict); cudaFree(h->d_ptarget);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -789,7 +798,7 @@ int epi_mlp_set_dataset(epi_mlp* h, const float* x, const float* y, uint32_t n) 
     h->n_data = 0;
     MCK(cudaMalloc(&h->d_xs, (size_t)n * kInPad * sizeof(__nv_bfloat16)));
     MCK(cudaMalloc(&h->d_ys, (size_t)n * h->out_pad * sizeof(float)));
-    MRC(upload_inputs(h, x, n, n, h->d_xs));
+    MRC(upload_inputs(h, x, n, n, nullptr, h->d_xs));
     MRC(upload_targets(h, y, n, h->d_ys));
     MCK(cudaStreamSynchronize(h->stream));
     h->n_data = n;
@@ -870,7 +879,7 @@ int epi_mlp_gradients(epi_mlp* h, const float* x, const float* y, uint32_t n, fl
     const uint32_t E = h->E;
     MlpLayer& l0 = h->layers[0];
     // every member sees the same minibatch: row 0.. of the chunk buffers, member 0's
-    MRC(upload_inputs(h, x, n, n, l0.h, l0.ht, h->chunk * h->B));
+    MRC(upload_inputs(h, x, n, n, nullptr, l0.h, l0.ht, h->chunk * h->B));
     MRC(upload_targets(h, y, n, h->d_t));
     if (E > h->loss_cap) {
         cudaFree(h->d_loss);
