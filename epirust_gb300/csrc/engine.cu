@@ -396,12 +396,14 @@ static Together runs_together(uint32_t n, size_t occ_words, uint32_t sms) {
     return Together::kNo;
 }
 
+constexpr uint32_t kEnsembleBlockChunks = 18;  // (see the default grid)
+
 // The group of an ensemble's launch: 1 to 16 chunks, by the time of the busiest block, whose
 // chunks are whole groups and each group a switch of replicate, 0.2 chunks of time; 8 from 32
 // chunks a block, where the last group is a small part.  (One GB300,
 // groups of 1 / 2 / 4 / 7 / 8 / 14 / 28: 64 replicates of 50,000 agents, 13.8 chunks a block,
-// 51.7 / 47.8 / 45.8 / 45.1 / 48.0 / 45.2 / 56 ms; 256 replicates, 142 chunks a block, 145 / 134 /
-// 125.5 / 121.7 / 122.0 / 122.9 / 143 ms.  Chosen here / always 8: 4 replicates of 3,000 to
+// 51.7 / 47.8 / 45.8 / 45.1 / 48.0 / 45.2 / 56 ms; 256 replicates on the resident grid, 142 chunks
+// a block, 145 / 134 / 125.5 / 121.7 / 122.0 / 122.9 / 143 ms.  Chosen here / always 8: 4 replicates of 3,000 to
 // 10,000 agents 0.61 / 1.48 ms for 100 hours, 32 of 10,000 to 100,000 2.5 / 2.7.)
 static ChunkGroup chunk_group(uint32_t n_chunks, uint32_t grid) {
     uint32_t best = 8u;
@@ -1144,7 +1146,12 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     const uint64_t n_chunks = slots / kChunk;
     h->resident_blocks = sms * per_sm;
     h->sms = (uint32_t)sms;
-    h->grid_blocks = (int)std::min<uint64_t>(n_chunks, (uint64_t)h->resident_blocks);
+    // A world takes the resident grid (4M agents, 15,625 chunks: 68.8 ms a run; a block per 4 chunks
+    // 88, per chunk 111).  A large ensemble takes more blocks, whose uneven chunks then spread
+    // over the SMs as they come (256 replicates, 130,000 chunks: resident 122 ms, a block per 24 /
+    // 18 / 14 / 10 chunks 113.7 / 112.2 / 114 / 113; 43,000 chunks 10.4 ms, 10.5 per 18).
+    h->grid_blocks = (int)std::min<uint64_t>(
+        n_chunks, std::max<uint64_t>(h->resident_blocks, R > 1 ? n_chunks / kEnsembleBlockChunks : 0u));
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     CK(cudaMalloc(&h->d_params, R * sizeof(DevParams)));
@@ -1327,7 +1334,7 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
     std::vector<uint32_t> grids;
     // three quarters of the resident grid too: fewer warps per SM share the L1 that holds the
     // plane rows their agents read
-    const uint64_t cand[4] = {(uint64_t)h->resident_blocks * 3u / 4u, (uint64_t)h->resident_blocks,
+    const uint64_t cand[5] = {(uint64_t)h->grid_blocks, (uint64_t)h->resident_blocks * 3u / 4u, (uint64_t)h->resident_blocks,
                               2ull * (uint64_t)h->resident_blocks, (uint64_t)n_chunks};
     for (uint64_t g : cand) {
         const uint32_t v = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(g, n_chunks));

@@ -337,9 +337,9 @@ __device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitV
 // hours: 1M agents 5.39 ms at 5 blocks, 5.43 at 6, 6.08 at 7; 4M agents 5.83, 5.69, 6.15; the
 // 256-replicate ensemble 49.9 at 4 blocks, 48.0 at 5, 47.1 at 6, 60.1 at 8.)
 //
-// What bounds it: issue and dependent latency together.  A walking agent costs about 390 warp
-// instructions per 32 agents and three dependent L2 round trips (its words, the rows around
-// its cell, the claim); 60 % of the issue slots are busy while warps are resident.
+// What bounds it: dependent latency with issue behind it.  Walking agents cost about 350 warp
+// instructions per 32 and three dependent L2 round trips (words, the rows around the cell, the
+// claim); 42 % of the issue slots are busy (1M agents cold, 4 blocks per SM).
 constexpr int kWorldMinBlocks = 5;
 constexpr int kEnsembleMinBlocks = 6;
 
