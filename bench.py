@@ -36,10 +36,10 @@ sys.path.insert(0, ROOT)
 DEFAULT_CONFIG = os.path.join(ROOT, "tests", "golden", "small_pox_1m_2500.json")
 METRIC = "agent-hours/s"
 # Algorithmic bytes of one k_decide launch per agent: pos 4 + st 8 + home 4 + work 4 read,
-# st 8 + tgt 4 written; plus one read of the (G+1)^2 byte occupancy plane and of the
-# (G+1)^2 infectious-neighbour counts.
-DECIDE_BYTES_PER_AGENT = 32
-DECIDE_PLANES = 2
+# pos 4 written; and per cell the two occupancy bit planes (one read, one written) and a byte of
+# infectious-neighbour counts.
+DECIDE_BYTES_PER_AGENT = 24
+DECIDE_PLANES = 1.25
 # Whole-tick algorithmic bytes per agent-hour of the reference-layout accounting (agent record
 # read 25 B + written 11 B, claim write and clear, plane write, and the occupancy and
 # infectiousness planes amortised over the agents -- 76 B at 1M agents / 2500 grid in a
