@@ -540,6 +540,11 @@ int ensure_predict(epi_mlp* h, uint32_t n_pad) {
     return EPI_OK;
 }
 
+// Whether the last product leaves the rows in d_py as the caller has them ([member][n][out_dim]):
+// k_infer stores 32 bytes at a time, so out_dim is a multiple of 8.  Else they have out_pad columns
+// and p_cap rows a member, and k_unpad_rows makes a copy for the caller.
+bool outputs_as_asked(const epi_mlp* h) { return h->cfg.out_dim % 8u == 0u && h->layers[h->L - 1].K / kBK <= kInferMaxK; }
+
 // Forward pass of n host samples through every member; outputs stay in d_py (and scores in
 // d_pscore when target).  The buffers hold p_cap rows per member (the largest call so far):
 // member m's rows start at m * p_cap in every buffer and tensor map, whatever n is.
@@ -569,7 +574,8 @@ int forward_n(epi_mlp* h, const float* x, uint32_t n, const float* target) {
             a.score = target ? h->d_pscore : nullptr;
             a.n_valid = h->cfg.out_dim;
             a.m_valid = n;
-            a.ms_outf = cap * ly.N;
+            a.ld_outf = outputs_as_asked(h) ? h->cfg.out_dim : ly.N;
+            a.ms_outf = outputs_as_asked(h) ? (uint64_t)n * h->cfg.out_dim : cap * ly.N;
             a.ms_score = cap;
             MRC(infer_product<kEpOut>(h, ly.t_ph, ly.t_w, n_pad, ly.N, ly.K, a, za));
         }
@@ -904,13 +910,17 @@ int epi_mlp_predict(epi_mlp* h, const float* x, uint32_t n, float* y) {
     if (n == 0) return EPI_OK;
     MRC(forward_n(h, x, n, nullptr));
     const size_t floats = (size_t)h->E * n * h->cfg.out_dim;
-    MRC(ensure_raw(h, floats));
-    k_unpad_rows<<<dim3(blocks_for((size_t)n * h->cfg.out_dim), h->E), kSmallThreads, 0, h->stream>>>(
-        h->d_py, n, h->cfg.out_dim, h->out_pad, (size_t)h->p_cap * h->out_pad, h->d_raw);
-    MCK(cudaGetLastError());
-    h->launches++;
+    const float* rows = h->d_py;
+    if (!outputs_as_asked(h)) {
+        MRC(ensure_raw(h, floats));
+        k_unpad_rows<<<dim3(blocks_for((size_t)n * h->cfg.out_dim), h->E), kSmallThreads, 0, h->stream>>>(
+            h->d_py, n, h->cfg.out_dim, h->out_pad, (size_t)h->p_cap * h->out_pad, h->d_raw);
+        MCK(cudaGetLastError());
+        h->launches++;
+        rows = h->d_raw;
+    }
     epi::touch_pages(y, floats * sizeof(float));
-    MCK(cudaMemcpyAsync(y, h->d_raw, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    MCK(cudaMemcpyAsync(y, rows, floats * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     MRC(check_err(h));
     return EPI_OK;
 }

@@ -39,11 +39,12 @@ enum Epilogue : int {
 struct EpiArgs {
     const float* bias = nullptr;        // [N]
     __nv_bfloat16* out = nullptr;       // [M x N]
-    float* outf = nullptr;              // [M x N]
+    float* outf = nullptr;              // [M x N] (k_infer: [m_valid x ld_outf])
     const float* score_target = nullptr;  // [n_valid]
     float* score = nullptr;             // [M], accumulated
     uint32_t n_valid = 0;               // real output columns
     uint32_t m_valid = 0;               // real sample rows
+    uint32_t ld_outf = 0;
     uint64_t ms_bias = 0, ms_out = 0, ms_outf = 0, ms_score = 0;
 };
 

@@ -100,10 +100,11 @@ __device__ __forceinline__ void infer_epilogue(const EpiArgs& a, uint32_t N, uin
         }
         return;
     }
-    if (a.outf) {
-        float* o = a.outf + (size_t)m * N + n;
+    if (a.outf && m < a.m_valid) {
+        float* o = a.outf + (size_t)m * a.ld_outf + n;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) store_32b(o + 8 * q, reinterpret_cast<const uint32_t*>(x + 8 * q));
+        for (int q = 0; q < 4; ++q)
+            if (n + 8 * q < a.n_valid) store_32b(o + 8 * q, reinterpret_cast<const uint32_t*>(x + 8 * q));
     }
     if (a.score_target) {  // (padded to N: the bound only keeps the padding out of the sum)
         const float4* target = reinterpret_cast<const float4*>(a.score_target + n);

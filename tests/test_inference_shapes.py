@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 # (in_dim, hidden, hidden_layers, out_dim, members, rows)
 SHAPES = [(1, 128, 1, 1, 1, 1), (8, 512, 3, 600, 2, 12801), (64, 384, 2, 129, 3, 7000), (5, 640, 2, 300, 2, 700),
-          (8, 256, 1, 100, 40, 500), (3, 896, 2, 128, 1, 20000)]
+          (8, 256, 1, 100, 40, 500), (3, 896, 2, 128, 1, 20000), (8, 128, 1, 200, 3, 129)]
 
 
 @pytest.mark.parametrize("shape", SHAPES)
