@@ -15,7 +15,7 @@
 // A training step is 2 L launches (tc_train.cuh): L forward, then one launch per input
 // gradient, each carrying the weight gradients that have become ready.  The minibatches of a
 // chunk of steps are gathered by one launch; groups of kGroupSteps steps are one CUDA graph,
-// kept by the handle.  Inference runs the 128 x 128 products of tc_gemm.cuh.
+// kept by the handle.  Inference runs the products of tc_infer.cuh (tc_gemm.cuh where K > 512).
 //
 // A handle holds E = cfg.members networks of the same shape (an ensemble).  Every buffer
 // carries a leading member axis and every kernel covers all members in one launch: the
