@@ -684,7 +684,7 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     if (h->last_claim_hour >= 0 &&
         ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
         CK(cudaMemsetAsync(h->d_claim, 0xFF, h->claim_cells * sizeof(uint32_t), h->stream));
-    h->last_claim_hour = (int64_t)first_hour + nh - 1;
+    h->last_claim_hour = INT64_MAX;  // until the hours have run
     // the chain reads the state after first_hour - 1 from its parity's buffers
     const uint32_t need = hour_parity((first_hour + 23u) % 24u);
     std::vector<uint8_t> ran(h->R(), 0);  // a world whose run has ended runs no hour kernel
@@ -730,6 +730,10 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
         if (h->halt_row >= 0) last[r] = std::min(last[r], (uint32_t)h->halt_row);
         h->reps[r].par = hour_parity((first_hour + last[r]) % 24u);
     }
+    // The hour kernels open every claim window of the chain, whether or not a world still runs;
+    // k_small none that its world did not get to.
+    if (!small) h->last_claim_hour = (int64_t)first_hour + nh - 1;
+    else if (ran[0]) h->last_claim_hour = (int64_t)first_hour + last[0];
     return EPI_OK;
 }
 

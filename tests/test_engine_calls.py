@@ -1,0 +1,45 @@
+"""Calls that follow one another on one engine: hours after a run that ended early."""
+import json
+
+import numpy as np
+import pytest
+
+from helpers import COVID_FAST, make_config, rows_to_array
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(cfg, **kw):
+    from epirust_gb300 import Config, Epidemiology
+
+    return Epidemiology(Config(json.dumps(cfg)), **kw)
+
+
+def _rows(r):
+    return np.stack([r[k] for k in r.dtype.names], axis=1).astype(np.int64)
+
+
+def _same_world(eng, sim):
+    eng.check_invariants()
+    assert (eng.snapshot().view(np.uint8) == sim.export().view(np.uint8)).all()
+
+
+@pytest.mark.parametrize("hour_kernels", [False, True])
+@pytest.mark.parametrize("n,grid", [(1500, 93), (17000, 290)])
+def test_hours_after_a_run_that_ended_early(gpu, oracle_mod, n, grid, hour_kernels):
+    """The run's last chain reaches into a claim window (128 hours) that its world never gets to;
+    hours of that window then find no claim of the window before."""
+    disease = dict(COVID_FAST, last_day=4, high_transmission_start_day=3, regular_transmission_rate=0.0,
+                   high_transmission_rate=0.0)
+    cfg = make_config(n=n, grid=grid, hours=193, seed=n, disease=disease, starting=(0, 0, 3, 0))
+    sim = oracle_mod.O1(oracle_mod.params_from_config(cfg))
+    want = rows_to_array(sim.run(1, 193, interventions=True, stop=True))
+    assert 24 < len(want) < 128
+    eng = _engine(cfg)
+    assert (_rows(eng.run()) == want).all()
+    if hour_kernels:
+        eng.set_launch_shape((n + 255) // 256, 4)
+    want = rows_to_array(sim.run(200, 220, interventions=False, stop=False))
+    assert (_rows(eng.simulate_hours(200, 20)) == want).all()
+    _same_world(eng, sim)
+    eng.close()
