@@ -75,6 +75,7 @@ struct epi_engine {
     int resident_blocks = 0;   // SMs x resident k_decide blocks per SM
     uint32_t sms = 0;
     Together together = Together::kNo;  // a world whose hours one launch runs (k_small)
+    uint32_t wait_polls = kGridSpinLimit;  // SmallArgs::polls
     bool shape_set = false;    // a launch shape was asked for: hour kernels, whatever the size
     // device
     DevParams* d_params = nullptr;
@@ -102,7 +103,7 @@ struct epi_engine {
     // host
     uint32_t* h_counts = nullptr;  // pinned mirror of d_counts
     SegDev* h_seg = nullptr;       // pinned staging of d_seg and d_ivn
-    int* h_err = nullptr;          // (in the same allocation, as is h_ivn)
+    int* h_err = nullptr;          // SmallArgs::err_out (in the same allocation, as is h_ivn)
     uint32_t* h_ivn = nullptr;
     int halt_row = -1;             // chain offset of the row the guard marked in the last chain
     cudaStream_t stream = nullptr;
@@ -637,6 +638,7 @@ static int run_together(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     a.sums = h->d_sums;
     a.rows = h->h_counts;
     a.err = h->d_err;
+    a.polls = h->wait_polls;
     a.err_out = h->h_err;
     const bool grid = h->together == Together::kGrid;
     cudaLaunchConfig_t cfg = {};
@@ -655,11 +657,11 @@ static int run_together(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     }
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    *h->h_err = 0;
+    h->h_err[0] = h->h_err[1] = 0;
     CK(cudaLaunchKernelEx(&cfg, grid ? k_small<true> : k_small<false>, (const DevParams*)h->d_params, a));
     h->kernels_launched += 1;
     CK(cudaStreamSynchronize(h->stream));
-    return report_error_flag(h, *h->h_err);
+    return report_error_flag(h, h->h_err[0] | h->h_err[1]);
 }
 
 // Simulate hours first_hour .. first_hour + nh - 1 for every active replicate as one chain:
@@ -745,6 +747,10 @@ static int check_error_flag(epi_engine* h) {
 }
 
 static int report_error_flag(epi_engine* h, int e) {
+    if (e & kErrWait) {
+        h->err = "a block gave up waiting for the others of its launch; the world is somewhere within an hour";
+        return EPI_ERR_TIMEOUT;
+    }
     if (e) {
         h->err = "device invariant violated (flag " + std::to_string(e) + "): a rule addressed a cell outside the plane";
         return EPI_ERR_INVARIANT;
@@ -1195,9 +1201,9 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     CK(cudaMemset(h->d_ivn, 0, R * sizeof(uint32_t)));
     CK(cudaMalloc(&h->d_err, sizeof(int)));
     CK(cudaMalloc(&h->d_scratch, 6 * sizeof(unsigned long long)));
-    CK(cudaMallocHost(&h->h_seg, sizeof(SegDev) + sizeof(int) + R * sizeof(uint32_t)));  // with h_err and h_ivn
+    CK(cudaMallocHost(&h->h_seg, sizeof(SegDev) + 2 * sizeof(int) + R * sizeof(uint32_t)));  // with h_err and h_ivn
     h->h_err = reinterpret_cast<int*>(h->h_seg + 1);
-    h->h_ivn = reinterpret_cast<uint32_t*>(h->h_err + 1);
+    h->h_ivn = reinterpret_cast<uint32_t*>(h->h_err + 2);
     if (R == 1) h->together = runs_together(h->reps[0].n, h->occ_words, h->sms);
     if (h->together == Together::kGrid) CK(cudaMalloc(&h->d_sums, kGridWords * sizeof(uint32_t)));
     int rc = ensure_counts(h, 48);
@@ -1993,6 +1999,12 @@ int epi_engine_state_stream_close(epi_engine* h) {
 int epi_engine_set_launch_shape(epi_engine* h, const epi_launch_shape* shape) {
     if (!h || !shape) return EPI_ERR_ARG;
     return set_launch_shape(h, shape->decide_blocks, shape->commit_slots);
+}
+
+int epi_engine_set_wait_limit(epi_engine* h, uint32_t polls) {
+    if (!h) return EPI_ERR_ARG;
+    h->wait_polls = polls;
+    return EPI_OK;
 }
 
 int epi_engine_launch_shape(const epi_engine* h, epi_launch_shape* out) {

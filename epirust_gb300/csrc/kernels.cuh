@@ -602,9 +602,12 @@ struct SmallArgs {
     uint32_t* sums;       // k_small<true>: zero, kGridWords: 3 x 8 sums of an hour's counts and the barrier's
                           // arrivals, a cache line each
     uint32_t* rows;       // hours x 8: bins, word 6 the halt mark; rows that did not run are zero
+    uint32_t polls;       // k_small<true>: of a barrier before its block gives up
     int* err;             // device error word
-    int* err_out;         // where the caller reads it
+    int* err_out;         // where the caller reads it: [0] what the first block finds there at its end, [1] kErrWait
+                          // from a block that gave up (a word of its own, so that neither undoes the other)
 };
+constexpr int kErrWait = 4;  // the error word: a wait for the other blocks ran out
 
 // The hours of day 7..22 write the other buffer, 16 a day (engine.cu: hour_parity).
 __host__ __device__ constexpr uint32_t hour_parity(uint32_t hod) {
@@ -630,17 +633,17 @@ __device__ __forceinline__ uint32_t load_in_cluster(uint32_t addr) {
 }
 
 // The barrier of a grid whose blocks all run (a cooperative launch): false, on every thread of
-// the block, when the others did not arrive within some seconds.
+// the block, when the others did not arrive within `polls` (kGridSpinLimit: some seconds).
 constexpr uint32_t kLineWords = 32, kGridWords = 25 * kLineWords;
 constexpr uint32_t kGridSpinLimit = 1u << 22;
-__device__ __forceinline__ bool grid_sync(uint32_t* arrived, uint32_t& target) {
+__device__ __forceinline__ bool grid_sync(uint32_t* arrived, uint32_t& target, uint32_t polls) {
     target += gridDim.x;
     bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("fence.acq_rel.gpu;\n\tred.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
         ok = false;
-        for (uint32_t it = 0; it < kGridSpinLimit && !ok; ++it) {
+        for (uint32_t it = 0; it < polls && !ok; ++it) {
             uint32_t v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
             ok = (int32_t)(v - target) >= 0;
@@ -682,7 +685,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
         return GRID ? __ldcg(&a.sums[(slot * 8u + bin) * kLineWords]) : load_in_cluster(sums + (slot * 8u + bin) * 4u);
     };
     auto sync = [&] {
-        if (GRID) ok = grid_sync(a.sums + 24u * kLineWords, arrivals) && ok;
+        if (GRID) ok = grid_sync(a.sums + 24u * kLineWords, arrivals, a.polls) && ok;
         else cluster_sync();
     };
     const bool valid = i < P.n;
@@ -811,7 +814,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const DevParams* __r
         }
     }
     if (!GRID) cluster_sync();  // the first CTA's counters outlive their readers
-    if (!ok && tid == 0) *(volatile int*)a.err_out = 4;
+    if (!ok && tid == 0) {
+        atomicOr(a.err, kErrWait);  // stays: the world is somewhere within an hour
+        *(volatile int*)(a.err_out + 1) = kErrWait;
+    }
 }
 
 // ---------------------------------------------------------------- the caller-owned planes

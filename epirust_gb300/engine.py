@@ -319,6 +319,11 @@ class Epidemiology:
         check(lib().epi_engine_launch_shape(self._h, C.byref(s)), self._h)
         return {"decide_blocks": s.decide_blocks, "commit_slots": s.commit_slots}
 
+    def set_wait_limit(self, polls: int) -> None:
+        """How often a block of a world that runs as one grid looks for the others before the call
+        ends with EPI_ERR_TIMEOUT."""
+        check(lib().epi_engine_set_wait_limit(self._h, polls), self._h)
+
     def hour_bytes(self, hour: int) -> float:
         b = C.c_double(0.0)
         check(lib().epi_engine_hour_bytes(self._h, hour, C.byref(b)), self._h)

@@ -337,6 +337,11 @@ int epi_engine_autotune(epi_engine* h, uint32_t hours, epi_launch_shape* chosen)
 int epi_engine_set_launch_shape(epi_engine* h, const epi_launch_shape* shape);
 int epi_engine_launch_shape(const epi_engine* h, epi_launch_shape* out);
 
+/* Polls (default 2^22, some seconds) after which a block of a world that runs as one grid gives up
+ * waiting for the other blocks of its launch.  The call then ends with EPI_ERR_TIMEOUT, and so
+ * does every later hour of this engine: its world is somewhere within an hour. */
+int epi_engine_set_wait_limit(epi_engine* h, uint32_t polls);
+
 /* Kernel timing: when enabled, every kernel launch of the engine is bracketed by CUDA
  * events on the launching stream and CUDA graphs are not used.  kernel_stats returns, per
  * kernel kind k < n, its launch count and total milliseconds; names via kernel_name. */

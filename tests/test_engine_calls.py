@@ -1,4 +1,5 @@
-"""Calls that follow one another on one engine: hours after a run that ended early."""
+"""Calls that follow one another on one engine: hours after a run that ended early, and after a
+launch whose blocks did not find one another."""
 import json
 
 import numpy as np
@@ -43,3 +44,27 @@ def test_hours_after_a_run_that_ended_early(gpu, oracle_mod, n, grid, hour_kerne
     assert (_rows(eng.simulate_hours(200, 20)) == want).all()
     _same_world(eng, sim)
     eng.close()
+
+
+@pytest.mark.parametrize("hour", [1, 9])
+def test_a_wait_that_runs_out_ends_the_call_and_the_engine(gpu, hour):
+    """A world that runs as one grid, its blocks given no time to wait for one another: the call
+    reports it, the engine takes no more hours in either form, and others are not touched by it."""
+    from epirust_gb300 import EpiError
+
+    cfg = make_config(n=17000, grid=290, seed=2, disease=COVID_FAST, starting=(0, 0, 5, 50))
+    want = _engine(cfg).simulate_hours(1, 24)
+    eng = _engine(cfg)
+    if hour > 1:
+        eng.simulate_hours(1, hour - 1)
+    eng.set_wait_limit(0)
+    with pytest.raises(EpiError, match="TIMEOUT.*gave up waiting"):
+        eng.simulate(hour)
+    eng.set_wait_limit(1 << 22)
+    with pytest.raises(EpiError, match="TIMEOUT"):
+        eng.simulate(hour + 1)
+    eng.set_launch_shape(16, 4)
+    with pytest.raises(EpiError, match="TIMEOUT"):
+        eng.simulate(hour + 1)
+    eng.close()
+    assert (_engine(cfg).simulate_hours(1, 24) == want).all()
