@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __re
     __shared__ uint32_t sh[8];
     __shared__ DevParams sP;
     __shared__ MoveTables tables;
-    __shared__ Box boxes[kNumAreas];
+    __shared__ Box boxes[8];  // (the caller's state words hold any 3-bit code)
     const DevParams& P = sP;
     stage_tables(tables);  // read after switch_rep's barriers
     const HourRow hr = hour_row(ha);
@@ -867,6 +867,12 @@ __global__ void __launch_bounds__(kThreads) k_decide_bytes(const DevParams* __re
             if (HC == kHcStart) q = routine_start(P, pl, s, hm, p, hosp_first, dr);
             else if (HC == kHcEnd) q = routine_end(P, pl, s, hm, p, dr);
             else q = perform_movements<HC>(P, pl, tables, boxes, s, wsa + i, hm, wk, p, hour, dr, infect);
+            // house and office words are as the caller has them: no proposal outside the plane from them
+            const uint32_t edge = (uint32_t)P.G * 0x00010001u;
+            if (q != p && max2(q, edge) != edge) {
+                atomicOr(err, 1);
+                q = p;
+            }
             if (q != p) atomicMin(&claim[(size_t)(q >> 16) * P.W + (q & 0xFFFFu)], i);
             if (infect) infection_dynamics(P, pl, tables, boxes, s, at, hm, wk, q, hour, dr);
             const uint32_t cls0 = cell_class(P, sv.x), cls = cell_class(P, s);
