@@ -70,6 +70,7 @@ struct epi_engine {
     size_t plane_bytes = 0;    // all bordered byte planes
     size_t occ_words = 0;      // all bit planes (one buffer)
     size_t claim_cells = 0;    // all claim planes
+    size_t claim_bytes = 0;    // of d_claim
     int grid_blocks = 0;       // grid of the counting kernels (k_decide, k_sleep)
     int commit_slots = kCommitSlots;  // of the launch shape (k_commit takes its work from lists)
     int resident_blocks = 0;   // SMs x resident k_decide blocks per SM
@@ -1195,7 +1196,9 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     CK(cudaMalloc(&h->d_acts, slots * sizeof(uint2)));
     CK(cudaMalloc(&h->d_list_n, n_chunks * (kThreads / 32) * sizeof(uint2)));  // grids have at most n_chunks blocks
     CK(cudaMalloc(&h->d_par, R * sizeof(uint32_t)));
-    CK(cudaMalloc(&h->d_claim, h->claim_cells * sizeof(uint32_t)));
+    // (room for one record, which snapshots lay out here: a grid of 2 has 9 cells)
+    h->claim_bytes = std::max(h->claim_cells * sizeof(uint32_t), sizeof(epi_agent_record));
+    CK(cudaMalloc(&h->d_claim, h->claim_bytes));
     CK(cudaMalloc(&h->d_seg, sizeof(SegDev)));
     CK(cudaMalloc(&h->d_ivn, R * sizeof(uint32_t)));
     CK(cudaMemset(h->d_ivn, 0, R * sizeof(uint32_t)));
@@ -1269,8 +1272,7 @@ static int finish_upload(epi_engine* h) {
 static int snapshot_replica(epi_engine* h, uint32_t r, epi_agent_record* out, size_t n) {
     const Replica& rep = h->reps[r];
     if (!out || n != rep.n) return EPI_ERR_ARG;
-    const size_t room = h->claim_cells * sizeof(uint32_t) / sizeof(epi_agent_record);
-    if (room == 0) { h->err = "snapshot: world without cells"; return EPI_ERR_INVARIANT; }
+    const size_t room = h->claim_bytes / sizeof(epi_agent_record);
     h->last_claim_hour = INT64_MAX;
     touch_pages(out, n * sizeof(epi_agent_record));
     for (size_t first = 0; first < n; first += room) {

@@ -1,5 +1,5 @@
-"""Calls that follow one another on one engine: hours after a run that ended early, and after a
-launch whose blocks did not find one another."""
+"""Calls that follow one another on one engine -- hours after a run that ended early, and after a
+launch whose blocks did not find one another -- and worlds at the small end of what is accepted."""
 import json
 
 import numpy as np
@@ -68,3 +68,22 @@ def test_a_wait_that_runs_out_ends_the_call_and_the_engine(gpu, hour):
         eng.simulate(hour + 1)
     eng.close()
     assert (_engine(cfg).simulate_hours(1, 24) == want).all()
+
+
+@pytest.mark.parametrize("grid", [1, 2, 3, 5])
+def test_records_of_the_smallest_grids(gpu, oracle_mod, grid):
+    """Two agents at home in worlds of 4 to 36 cells: their records come back, hour after hour."""
+    cfg = make_config(n=2, grid=grid, seed=9, starting=(0, 0, 0, 0))
+    p = oracle_mod.params_from_config(cfg)
+    recs = oracle_mod.O1(oracle_mod.params_from_config(make_config(n=2, grid=60, seed=9, starting=(0, 0, 0, 0)))).export()
+    for k in (0, 1):
+        for name, v in [("x", k), ("y", k), ("flags", 0), ("work_status", 3), ("work_start_at", 0), ("home_x", 0), ("home_y", 0),
+                        ("work_x", 0), ("work_y", 0), ("area_x0", 0), ("area_y0", 0), ("area_x1", 1), ("area_y1", 1)]:
+            recs[name][k] = v
+    sim = oracle_mod.O1(p, records=recs)
+    eng = _engine(cfg, records=recs)
+    _same_world(eng, sim)
+    want = rows_to_array(sim.run(1, 49, interventions=False, stop=False))
+    assert (_rows(eng.simulate_hours(1, 48)) == want).all()
+    _same_world(eng, sim)
+    eng.close()
