@@ -368,7 +368,6 @@ static uint32_t threads_of(uint32_t n, uint32_t blocks) { return ((n + blocks - 
 // How one launch can run the world's hours: an agent per thread, a bit plane that the threads
 // zero in a few stores each, and a device that schedules clusters of 16 CTAs, or an SM for
 // each block.
-constexpr uint32_t kShortCall = 12, kSharedThreads = 256;  // (see run_hours_chunk)
 static Together runs_together(uint32_t n, size_t occ_words, uint32_t sms) {
     if (n <= kSmallAgents && occ_words <= 16u * (size_t)kSmallCluster * threads_of(n, kSmallCluster)) {
         cudaLaunchConfig_t cfg = {};
@@ -612,6 +611,23 @@ static int run_pieces(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     return check_error_flag(h);
 }
 
+// The longest call that one launch runs.  A cluster's world: any.  A grid has a block on every SM,
+// and the grids of engines in other threads run beside it only while all their threads fit
+// (64 registers each: 1,024 threads an SM).  Two weeks of hours in one call, ms, one / four
+// engines, one GB300: 30,000 agents (224 threads) 1.63 / 2.30, captured launches 1.76 / 2.20;
+// 98,000 (672) 2.02 / 7.68, launches 1.91 / 2.89; so any call while four grids fit.  Above that a
+// short call is still mostly launch and wait, which the grid has one of: 96 hours in calls of 1 /
+// 3 / 6 hours, ms, grid : launches, 77,000 agents, one engine 2.12 : 3.89, 1.11 : 1.65, 0.86 : 1.10,
+// four 3.97 : 5.16, 1.90 : 2.29, 1.60 : 1.55, eight 8.56 : 9.07, 3.59 : 3.61, 3.15 : 2.54; 98,000 agents, one
+// 2.22 : 3.89, 1.17 : 1.69, 0.92 : 1.15, four 3.75 : 5.17, 2.80 : 2.34, 2.47 : 1.61.  So 3 hours while two grids
+// fit and 1 hour beyond: no number of engines up to eight is slower than by launches.
+constexpr uint32_t kSharedThreads = 256;
+static uint32_t longest_together(const epi_engine* h) {
+    if (h->together != Together::kGrid) return h->together == Together::kCluster ? 0xFFFFFFFFu : 0u;
+    const uint32_t threads = threads_of(h->reps[0].n, h->sms);
+    return threads <= kSharedThreads ? 0xFFFFFFFFu : threads <= 2u * kSharedThreads ? 3u : 1u;
+}
+
 // The chain's hours of a small world in one launch (k_small), which writes the counts rows to
 // pinned memory itself: one launch and one wait per call, where a captured piece takes a copy
 // of the hour base, the graph, and two copies back with a wait each.
@@ -676,13 +692,7 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     if ((uint64_t)first_hour + nh > 0xFFFFFFFFull) { h->err = "hour out of range"; return EPI_ERR_ARG; }
     int rc = ensure_counts(h, nh);
     if (rc) return rc;
-    // k_small: any call of a cluster's world.  A grid's world takes it where four such grids fit
-    // the SMs (256 threads each: engines of several threads then still run side by side; 30,000
-    // agents, two weeks in ms, one / four engines: 1.65 / 2.32, captured launches 1.79 / 2.22),
-    // and larger ones for calls of a few hours, where the launch itself is the time (98,000
-    // agents: two weeks 2.02 / 7.68, launches 1.91 / 2.89, but six hours 48 us for 66).
-    const bool small = h->together != Together::kNo && !h->shape_set && !h->profiling && !h->stream_file &&
-                       (h->together == Together::kCluster || nh <= kShortCall || threads_of(h->reps[0].n, h->sms) <= kSharedThreads);
+    const bool small = nh <= longest_together(h) && !h->shape_set && !h->profiling && !h->stream_file;
     // claims left by an earlier hour of another window, or by a later hour, must go first
     if (h->last_claim_hour >= 0 &&
         ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))

@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kThreads) k_commit(const DevParams* __restrict
 //   GRID true   a cooperative grid of one CTA per SM, barriers at L2: up to 155,648 agents.
 //               96 hours of 30,000 / 98,000 agents, ms: hour by hour 3.8 / 3.8 by captured
 //               launches, 1.9 / 2.0 here; six hours a call 1.01 / 1.05 and 0.66 / 0.77; in one
-//               call 0.49 / 0.53 and 0.44 / 0.55 (the rule of use: run_hours_chunk).  Its counts
+//               call 0.49 / 0.53 and 0.44 / 0.55 (the rule of use: longest_together).  Its counts
 //               lie a cache line per bin apart: side by side, 152 blocks' atomics on one sector
 //               held every barrier up (98,000 agents, a day's mean hour 7.4 us, 6.0 apart).
 constexpr uint32_t kSmallCluster = 16;

@@ -1,6 +1,8 @@
 """Calls that follow one another on one engine -- hours after a run that ended early, and after a
-launch whose blocks did not find one another -- and worlds at the small end of what is accepted."""
+launch whose blocks did not find one another --, worlds at the small end of what is accepted, and
+engines that share the GPU from several threads."""
 import json
+import threading
 
 import numpy as np
 import pytest
@@ -87,3 +89,50 @@ def test_records_of_the_smallest_grids(gpu, oracle_mod, grid):
     assert (_rows(eng.simulate_hours(1, 48)) == want).all()
     _same_world(eng, sim)
     eng.close()
+
+
+# sizes of 128, 256, 288, 512 and 544 threads a block on 152 SMs, and the longest call of one launch
+@pytest.mark.parametrize("n,grid,longest", [(16_385, 330, 100), (38_912, 494, 100), (38_913, 495, 3), (77_824, 700, 3),
+                                            (77_825, 700, 1), (155_648, 990, 1)])
+def test_longest_call_of_one_launch(gpu, n, grid, longest):
+    """Beyond it an engine would hold every SM against engines of other threads for too long."""
+    eng = _engine(make_config(n=n, grid=grid, seed=3, starting=(0, 0, 0, 50)))
+    hour = 1
+    for k in (1, longest, min(longest + 1, 100)):
+        launched = eng.kernels_launched()
+        eng.simulate_hours(hour, k)
+        assert (eng.kernels_launched() - launched == 1) == (k <= longest), k
+        hour += k
+    eng.close()
+
+
+@pytest.mark.parametrize("n,grid", [(9_000, 240), (30_000, 433), (60_000, 612), (98_000, 783)])
+def test_engines_of_several_threads(gpu, n, grid):
+    """Four engines stepped from four threads at once, in calls of one launch and of many, have the
+    hours that each has alone by hour kernels."""
+    cfgs = [make_config(n=n, grid=grid, seed=70 + i, disease=COVID_FAST, starting=(0, 0, 5, 60)) for i in range(4)]
+    cuts = [1, 2, 3, 6, 7, 8, 11, 14, 26, 27, 50, 73]
+    got, errors = [None] * 4, []
+
+    def work(i):
+        try:
+            eng = _engine(cfgs[i])
+            rows = [_rows(eng.simulate_hours(a, b - a)) for a, b in zip(cuts, cuts[1:])]
+            got[i] = (np.concatenate(rows), eng.snapshot())
+            eng.check_invariants()
+            eng.close()
+        except Exception as e:  # reported below, in the test's own thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for i in range(4):
+        eng = _engine(cfgs[i])
+        eng.set_launch_shape((n + 255) // 256, 4)
+        assert (got[i][0] == _rows(eng.simulate_hours(1, 72))).all(), i
+        assert (got[i][1].view(np.uint8) == eng.snapshot().view(np.uint8)).all(), i
+        eng.close()
