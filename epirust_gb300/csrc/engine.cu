@@ -77,7 +77,8 @@ struct epi_engine {
     uint32_t sms = 0;
     Together together = Together::kNo;  // a world whose hours one launch runs (k_small)
     uint32_t wait_polls = kGridSpinLimit;  // SmallArgs::polls
-    bool shape_set = false;    // a launch shape was asked for: hour kernels, whatever the size
+    uint32_t together_most = 0;  // hours of the longest call that one launch runs: longest_together, 0 once a launch
+                                 // shape was asked for, fewer where the autotuner found a grid faster
     // device
     DevParams* d_params = nullptr;
     uint32_t* d_chunk_rep = nullptr;  // null for a single replicate
@@ -621,11 +622,11 @@ static int run_pieces(epi_engine* h, uint32_t first_hour, uint32_t nh) {
 // four 3.97 : 5.16, 1.90 : 2.29, 1.60 : 1.55, eight 8.56 : 9.07, 3.59 : 3.61, 3.15 : 2.54; 98,000 agents, one
 // 2.22 : 3.89, 1.17 : 1.69, 0.92 : 1.15, four 3.75 : 5.17, 2.80 : 2.34, 2.47 : 1.61.  So 3 hours while two grids
 // fit and 1 hour beyond: no number of engines up to eight is slower than by launches.
-constexpr uint32_t kSharedThreads = 256;
+constexpr uint32_t kSharedThreads = 256, kShortHours = 3;
 static uint32_t longest_together(const epi_engine* h) {
     if (h->together != Together::kGrid) return h->together == Together::kCluster ? 0xFFFFFFFFu : 0u;
     const uint32_t threads = threads_of(h->reps[0].n, h->sms);
-    return threads <= kSharedThreads ? 0xFFFFFFFFu : threads <= 2u * kSharedThreads ? 3u : 1u;
+    return threads <= kSharedThreads ? 0xFFFFFFFFu : threads <= 2u * kSharedThreads ? kShortHours : 1u;
 }
 
 // The chain's hours of a small world in one launch (k_small), which writes the counts rows to
@@ -692,7 +693,7 @@ static int run_hours_chunk(epi_engine* h, uint32_t first_hour, uint32_t nh) {
     if ((uint64_t)first_hour + nh > 0xFFFFFFFFull) { h->err = "hour out of range"; return EPI_ERR_ARG; }
     int rc = ensure_counts(h, nh);
     if (rc) return rc;
-    const bool small = nh <= longest_together(h) && !h->shape_set && !h->profiling && !h->stream_file;
+    const bool small = nh <= h->together_most && !h->profiling && !h->stream_file;
     // claims left by an earlier hour of another window, or by a later hour, must go first
     if (h->last_claim_hour >= 0 &&
         ((int64_t)first_hour <= h->last_claim_hour || first_hour / kClaimWindow != (uint64_t)h->last_claim_hour / kClaimWindow))
@@ -1219,6 +1220,7 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     h->h_ivn = reinterpret_cast<uint32_t*>(h->h_err + 2);
     if (R == 1) h->together = runs_together(h->reps[0].n, h->occ_words, h->sms);
     if (h->together == Together::kGrid) CK(cudaMalloc(&h->d_sums, kGridWords * sizeof(uint32_t)));
+    h->together_most = longest_together(h);
     int rc = ensure_counts(h, 48);
     if (rc) return rc;
     if (!recs) {
@@ -1340,14 +1342,13 @@ static int set_launch_shape(epi_engine* h, uint32_t decide_blocks, uint32_t comm
     CK(cudaStreamSynchronize(h->stream));
     h->grid_blocks = (int)decide_blocks;
     h->commit_slots = (int)commit_slots;
-    h->shape_set = true;
     destroy_graphs(h);  // they bake the launch shapes in
     return EPI_OK;
 }
 
 // Launch-shape autotuner: times hours 1..hours of the engine's current world under each
-// candidate k_decide grid (three quarters of the resident grid, the resident grid, twice it,
-// one chunk per block), restarting every candidate from the same state, and keeps the fastest.
+// candidate k_decide grid (the present one, three quarters of the resident grid, the resident
+// grid, twice it, one chunk per block) and, where it applies, in one launch, restarting every candidate from the same state, and keeps the fastest.
 // Results do not depend on the shape; the state, the run's rows and the launch counter are
 // restored afterwards (the saved checkpoint is replaced).
 static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
@@ -1369,11 +1370,13 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
     if (rc) return rc;
     double best = 1e300;
     uint32_t best_g = (uint32_t)h->grid_blocks;
-    bool best_small = false;
-    if (h->together != Together::kNo) grids.insert(grids.begin(), 0u);  // 0: no shape asked for, one launch runs the hours
+    // one launch for the hours (0) is a candidate where it would run a call of so many
+    const uint32_t most = longest_together(h), before = h->together_most;
+    bool keep_together = hours > most;
+    if (hours <= most) grids.insert(grids.begin(), 0u);
     for (uint32_t g : grids) {
+        h->together_most = g ? 0u : most;
         if (g) rc = set_launch_shape(h, g, (uint32_t)h->commit_slots);
-        else h->shape_set = false;
         double t_min = 1e300;
         for (int rep = 0; rep < 5 && !rc; ++rep) {  // the first pass captures the graphs
             rc = restore_state(h);
@@ -1386,13 +1389,14 @@ static int autotune(epi_engine* h, uint32_t hours, epi_launch_shape* out) {
         if (rc) break;
         if (t_min < best) {
             best = t_min;
-            best_small = g == 0u;
+            keep_together = g == 0u || hours > most;
             if (g) best_g = g;
         }
     }
     h->profiling = prof;
     int rc2 = set_launch_shape(h, best_g, (uint32_t)h->commit_slots);
-    if (best_small) h->shape_set = false;
+    // a grid that beat one launch over these hours has shorter calls, mostly launch and wait, left to it
+    h->together_most = rc ? before : keep_together ? most : std::min({most, hours - 1u, kShortHours});
     if (!rc2) rc2 = restore_state(h);
     h->kernels_launched = launched;
     if (rc) return rc;
@@ -2010,7 +2014,9 @@ int epi_engine_state_stream_close(epi_engine* h) {
 
 int epi_engine_set_launch_shape(epi_engine* h, const epi_launch_shape* shape) {
     if (!h || !shape) return EPI_ERR_ARG;
-    return set_launch_shape(h, shape->decide_blocks, shape->commit_slots);
+    const int rc = set_launch_shape(h, shape->decide_blocks, shape->commit_slots);
+    if (!rc) h->together_most = 0;  // a shape that was asked for runs the hour kernels
+    return rc;
 }
 
 int epi_engine_set_wait_limit(epi_engine* h, uint32_t polls) {

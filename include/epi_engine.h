@@ -310,7 +310,8 @@ int epi_engine_kernels_launched(const epi_engine* h, uint64_t* out);
 
 /* Launch shape of the tick kernels: the grid of k_decide, k_commit and k_sleep.  commit_slots is
  * checked, kept and reported as before, but k_commit takes its work from k_decide's lists and
- * no longer has agents per thread.  Results never depend on the shape. */
+ * no longer has agents per thread.  Once a shape is set, these kernels run every hour, whatever
+ * the world's size.  Results never depend on the shape. */
 typedef struct {
     uint32_t decide_blocks;  /* 1 .. number of 256-agent chunks */
     uint32_t commit_slots;   /* 1 .. 8 */
@@ -329,10 +330,11 @@ int epi_engine_state_stream_open(epi_engine* h, const char* path);
 int epi_engine_state_stream_close(epi_engine* h);
 
 /* Autotuner (no reference counterpart): time hours 1..hours (<= 168) of the current world
- * under each candidate shape -- k_decide grid = three quarters of the resident blocks, the
- * resident blocks, twice that, or one chunk per block --
- * from the same starting state, keep the fastest and restore the state.  Call it before simulating; it replaces the checkpoint of
- * epi_engine_save_state. */
+ * under each candidate shape (k_decide grid = three quarters of the resident blocks, the resident
+ * blocks, twice that, or one chunk per block; also one launch for all hours where a call of so
+ * many would have it) from the same starting state, keep the fastest and restore the state.  A grid that wins is for the calls the hour kernels run;
+ * calls of up to 3 hours that one launch runs faster stay with it.  Call it before simulating; it
+ * replaces the checkpoint of epi_engine_save_state. */
 int epi_engine_autotune(epi_engine* h, uint32_t hours, epi_launch_shape* chosen);
 int epi_engine_set_launch_shape(epi_engine* h, const epi_launch_shape* shape);
 int epi_engine_launch_shape(const epi_engine* h, epi_launch_shape* out);

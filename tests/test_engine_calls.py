@@ -136,3 +136,20 @@ def test_engines_of_several_threads(gpu, n, grid):
         assert (got[i][0] == _rows(eng.simulate_hours(1, 72))).all(), i
         assert (got[i][1].view(np.uint8) == eng.snapshot().view(np.uint8)).all(), i
         eng.close()
+
+
+def test_short_calls_after_the_autotuner(gpu):
+    """A grid tuned on a day of hours leaves calls of an hour to the one launch that runs them, and a
+    shape that is asked for does not."""
+    for n, grid in [(3_000, 150), (30_000, 433), (60_000, 612), (98_000, 783), (150_000, 975)]:
+        eng = _engine(make_config(n=n, grid=grid, seed=4, starting=(0, 0, 0, 50)))
+        eng.autotune(24)
+        launched = eng.kernels_launched()
+        eng.simulate(1)
+        eng.simulate(7)
+        assert eng.kernels_launched() == launched + 2, n
+        shape = eng.launch_shape()
+        eng.set_launch_shape(**shape)
+        eng.simulate(8)
+        assert eng.kernels_launched() > launched + 3, n
+        eng.close()
