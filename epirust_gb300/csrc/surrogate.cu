@@ -219,7 +219,9 @@ struct epi_mlp {
     float* d_t = nullptr;        // targets of a gradients call, B x out_pad (all members)
     float* d_loss = nullptr;     // per-step losses, steps x E
     size_t loss_cap = 0;
-    uint32_t chunk = 0;          // steps whose minibatches are gathered at once
+    __nv_bfloat16* d_chunk = nullptr;  // layer 0's input in both orientations
+    uint32_t chunk = 0;          // steps whose minibatches layer 0's input has room for
+    uint32_t chunk_most = 0;     // most steps whose minibatches are gathered at once
     uint32_t* d_idx = nullptr;   // minibatch indices of a train call, steps x E x B
     size_t idx_cap = 0;
     float* d_raw = nullptr;      // caller arrays on their way in or out
@@ -588,12 +590,44 @@ void free_all(epi_mlp* h) {
     for (auto& ly : h->layers) {
         cudaFree(ly.w); cudaFree(ly.b); cudaFree(ly.mw); cudaFree(ly.vw); cudaFree(ly.mb); cudaFree(ly.vb);
         cudaFree(ly.gw); cudaFree(ly.gb); cudaFree(ly.wb); cudaFree(ly.wtb);
-        cudaFree(ly.h); cudaFree(ly.ht); cudaFree(ly.z); cudaFree(ly.dz); cudaFree(ly.dzt);
+        if (&ly != &h->layers[0]) {  // (layer 0's lie in d_chunk)
+            cudaFree(ly.h);
+            cudaFree(ly.ht);
+        }
+        cudaFree(ly.z); cudaFree(ly.dz); cudaFree(ly.dzt);
     }
+    cudaFree(h->d_chunk);
     cudaFree(h->d_err); cudaFree(h->d_tr); cudaFree(h->d_t); cudaFree(h->d_loss);
     cudaFree(h->d_idx); cudaFree(h->d_raw); cudaFree(h->d_corr);
     cudaFree(h->d_xs); cudaFree(h->d_ys); cudaFree(h->d_predict); cudaFree(h->d_ptarget);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
+}
+
+// The operands that lie in a layer's input (rows of it a member).
+int input_maps(epi_mlp* h, MlpLayer& ly, uint32_t rows) {
+    MRC(make_map(h, &ly.t_h, ly.h, rows, ly.K, kBM, h->E));
+    MRC(make_map(h, &ly.t_ht32, ly.ht, ly.K, rows, kTrainBN, h->E));
+    MRC(make_map(h, &ly.t_ht64, ly.ht, ly.K, rows, kTrainWideBN, h->E));
+    return EPI_OK;
+}
+
+// Room for the minibatches of so many steps in layer 0's input (nothing of the handle runs): one at
+// first, for gradients, and as many as a training call gathers at once from that call on, so that
+// handles that only predict do without (five members, batch 256: 42 MB).
+int ensure_chunk(epi_mlp* h, uint32_t steps) {
+    if (steps <= h->chunk) return EPI_OK;
+    MlpLayer& ly = h->layers[0];
+    drop_graphs(h);  // they bake the maps in
+    cudaFree(h->d_chunk);
+    h->d_chunk = nullptr;
+    h->chunk = 0;
+    const size_t elements = (size_t)h->E * steps * h->B * ly.K;  // (a multiple of 128 x 64)
+    MCK(cudaMalloc(&h->d_chunk, 2 * elements * sizeof(__nv_bfloat16)));
+    ly.h = h->d_chunk;
+    ly.ht = h->d_chunk + elements;
+    MRC(input_maps(h, ly, steps * h->B));
+    h->chunk = steps;
+    return EPI_OK;
 }
 
 template <int BN, int EP>
@@ -628,10 +662,10 @@ int init(epi_mlp* h) {
     MCK(cudaMemset(h->d_err, 0, sizeof(int)));
     MCK(cudaMemset(h->d_tr, 0, sizeof(TrainDev)));
     MCK(cudaMalloc(&h->d_t, (size_t)h->B * h->out_pad * sizeof(float)));
-    // steps gathered at once: up to 128, within 32 MB of inputs
-    h->chunk = (uint32_t)std::min<size_t>(128, std::max<size_t>(kGroupSteps, (32u << 20) / ((size_t)E * h->B * kInPad * 2)));
-    h->chunk -= h->chunk % kGroupSteps;
-    MCK(cudaMalloc(&h->d_corr, h->chunk * sizeof(float4)));
+    // steps gathered at once: up to 128, within 32 MB of inputs in each orientation
+    h->chunk_most = (uint32_t)std::min<size_t>(128, std::max<size_t>(kGroupSteps, (32u << 20) / ((size_t)E * h->B * kInPad * 2)));
+    h->chunk_most -= h->chunk_most % kGroupSteps;
+    MCK(cudaMalloc(&h->d_corr, h->chunk_most * sizeof(float4)));
     MCK(cudaMalloc(&h->d_ptarget, (size_t)h->out_pad * sizeof(float)));
     h->layers.resize(h->L);
     for (uint32_t l = 0; l < h->L; ++l) {
@@ -640,29 +674,30 @@ int init(epi_mlp* h) {
         ly.n_real = l + 1 == h->L ? c.out_dim : c.hidden;
         ly.K = l == 0 ? kInPad : c.hidden;
         ly.N = l + 1 == h->L ? h->out_pad : c.hidden;
-        const uint32_t rows = l == 0 ? h->chunk * h->B : h->B;  // of the layer's input
-        const size_t nw = (size_t)E * ly.N * ly.K, nb = (size_t)E * ly.N, act_in = (size_t)E * rows * ly.K,
+        const size_t nw = (size_t)E * ly.N * ly.K, nb = (size_t)E * ly.N, act_in = (size_t)E * h->B * ly.K,
                      act_out = (size_t)E * h->B * ly.N;
         for (float** p : {&ly.w, &ly.mw, &ly.vw, &ly.gw}) MCK(cudaMalloc(p, nw * sizeof(float)));
         for (float** p : {&ly.b, &ly.mb, &ly.vb, &ly.gb}) MCK(cudaMalloc(p, nb * sizeof(float)));
         MCK(cudaMalloc(&ly.wb, nw * sizeof(__nv_bfloat16)));
         MCK(cudaMalloc(&ly.wtb, nw * sizeof(__nv_bfloat16)));
-        MCK(cudaMalloc(&ly.h, act_in * sizeof(__nv_bfloat16)));
-        MCK(cudaMalloc(&ly.ht, act_in * sizeof(__nv_bfloat16)));
+        if (l == 0) {
+            MRC(ensure_chunk(h, 1));
+        } else {
+            MCK(cudaMalloc(&ly.h, act_in * sizeof(__nv_bfloat16)));
+            MCK(cudaMalloc(&ly.ht, act_in * sizeof(__nv_bfloat16)));
+            MRC(input_maps(h, ly, h->B));
+        }
         if (l + 1 < h->L) MCK(cudaMalloc(&ly.z, act_out * sizeof(float)));
         MCK(cudaMalloc(&ly.dz, act_out * sizeof(__nv_bfloat16)));
         MCK(cudaMalloc(&ly.dzt, act_out * sizeof(__nv_bfloat16)));
         for (float* p : {ly.mw, ly.vw, ly.gw}) MCK(cudaMemset(p, 0, nw * sizeof(float)));
         for (float* p : {ly.mb, ly.vb, ly.gb}) MCK(cudaMemset(p, 0, nb * sizeof(float)));
-        // operands: forward A = h (B x K), B = W (N x K); weights A = dZ^T (N x B), B = H^T (K x B);
-        // inputs A = dZ (B x N), B = W^T (K x N)
-        MRC(make_map(h, &ly.t_h, ly.h, rows, ly.K, kBM, E));
+        // operands (and input_maps): forward A = h (B x K), B = W (N x K); weights A = dZ^T (N x B),
+        // B = H^T (K x B); inputs A = dZ (B x N), B = W^T (K x N)
         MRC(make_map(h, &ly.t_w, ly.wb, ly.N, ly.K, 128, E));
         MRC(make_map(h, &ly.t_w32, ly.wb, ly.N, ly.K, kTrainBN, E));
         MRC(make_map(h, &ly.t_w64, ly.wb, ly.N, ly.K, kTrainWideBN, E));
         MRC(make_map(h, &ly.t_dzt, ly.dzt, ly.N, h->B, kBM, E));
-        MRC(make_map(h, &ly.t_ht32, ly.ht, ly.K, rows, kTrainBN, E));
-        MRC(make_map(h, &ly.t_ht64, ly.ht, ly.K, rows, kTrainWideBN, E));
         MRC(make_map(h, &ly.t_dz, ly.dz, h->B, ly.N, kBM, E));
         MRC(make_map(h, &ly.t_wt32, ly.wtb, ly.K, ly.N, kTrainBN, E));
         MRC(make_map(h, &ly.t_wt64, ly.wtb, ly.K, ly.N, kTrainWideBN, E));
@@ -845,6 +880,7 @@ int epi_mlp_train(epi_mlp* h, uint32_t steps, uint64_t shuffle_seed, float* loss
         MCK(cudaMalloc(&h->d_loss, (size_t)steps * E * sizeof(float)));
         h->loss_cap = (size_t)steps * E;
     }
+    MRC(ensure_chunk(h, round_up(std::min(steps, h->chunk_most), kGroupSteps)));
     MCK(cudaMemcpyAsync(h->d_idx, idx.data(), idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
     MCK(cudaMemsetAsync(h->d_loss, 0, (size_t)steps * E * sizeof(float), h->stream));
     if (steps >= kGroupSteps) MRC(step_graph(h, kGroupSteps, &h->group_graph));
@@ -883,6 +919,7 @@ int epi_mlp_gradients(epi_mlp* h, const float* x, const float* y, uint32_t n, fl
     if (n != h->B) { h->err = "gradients take exactly one minibatch"; return EPI_ERR_ARG; }
     MCK(cudaStreamSynchronize(h->stream));
     const uint32_t E = h->E;
+    MRC(ensure_chunk(h, 1));
     MlpLayer& l0 = h->layers[0];
     // every member sees the same minibatch: row 0.. of the chunk buffers, member 0's
     MRC(upload_inputs(h, x, n, n, nullptr, l0.h, l0.ht, h->chunk * h->B));

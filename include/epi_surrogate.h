@@ -64,7 +64,9 @@ int epi_mlp_set_params(epi_mlp* h, const float* in);
 int epi_mlp_set_dataset(epi_mlp* h, const float* x, const float* y, uint32_t n);
 /* Run `steps` Adam steps on minibatches of the uploaded set, reshuffled every epoch from
  * shuffle_seed (+ m for member m); losses (may be NULL, else members x steps) receives the
- * mean squared error of every member's every step. */
+ * mean squared error of every member's every step.  A handle that has trained keeps its buffer of
+ * minibatches gathered ahead: 256 B a row, up to 128 steps and 64 MB (five members at batch 256: 42 MB;
+ * 4 steps of larger ones). */
 int epi_mlp_train(epi_mlp* h, uint32_t steps, uint64_t shuffle_seed, float* losses);
 /* Losses (members values) and gradients (same layout as epi_mlp_get_params) of every member
  * on one minibatch of exactly `batch` samples, without updating the weights. */
