@@ -10,7 +10,6 @@
 #include <cstring>
 #include <ctime>
 #include <stdexcept>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 
@@ -570,7 +569,7 @@ void touch_pages(void* p, size_t bytes) {
     try {
         for (; started < parts; ++started)
             others[started - 1] = std::thread(touch, started * per, started + 1 == parts ? bytes : (started + 1) * per);
-    } catch (const std::system_error&) {  // no more threads: the caller takes the rest
+    } catch (...) {  // no more threads, or no memory for one: the caller takes the rest
         touch(started * per, bytes);
     }
     touch(0, parts > 1 ? per : bytes);
