@@ -4,7 +4,7 @@
 // boundary, so a chunk belongs to one replicate (chunk_rep[c]; absent when there is one).
 // The counting kernels walk chunks with a grid-stride loop, stage the chunk's replicate
 // parameters in shared memory and flush their per-block histogram whenever the replicate
-// changes; the commit kernel runs one thread per slot.  Philox counters and claim values use
+// changes; the commit kernel takes the lists they leave.  Philox counters and claim values use
 // the agent's index within its replicate, so a replicate evolves exactly as a lone engine
 // with the same parameters would.
 //

@@ -932,7 +932,6 @@ int epi_mlp_gradients(epi_mlp* h, const float* x, const float* y, uint32_t n, fl
         h->loss_cap = E;
     }
     MCK(cudaMemsetAsync(h->d_loss, 0, E * sizeof(float), h->stream));
-    k_train_chunk<<<1, 1, 0, h->stream>>>(h->d_tr, nullptr, nullptr, nullptr, nullptr, 0u, 0u, AdamHyper{});
     MRC(enqueue_step(h, 0, true));
     std::vector<float> lsum(E, 0.f);
     MCK(cudaMemcpyAsync(lsum.data(), h->d_loss, E * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
