@@ -82,7 +82,6 @@ EPI_HD int32_t unpack_y(uint32_t p) { return (int32_t)((p >> 16) & 0x7FFFu); }
 
 struct Rect { int32_t x0, y0, x1, y1; };
 
-EPI_HD bool rect_has(const Rect& r, int32_t x, int32_t y) { return r.x0 <= x && x <= r.x1 && r.y0 <= y && y <= r.y1; }
 EPI_HD bool rect_eq(const Rect& a, const Rect& b) { return a.x0 == b.x0 && a.y0 == b.y0 && a.x1 == b.x1 && a.y1 == b.y1; }
 
 // Per-engine constants, in device global memory (read through a const __restrict__ pointer).

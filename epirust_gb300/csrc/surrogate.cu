@@ -289,15 +289,14 @@ int launch_overlapped(epi_mlp* h, void (*kern)(KArgs...), dim3 grid, int threads
 }
 
 // One product per member (grid z = E); za = 0 when every member reads member 0's A.
-template <int BN, int EP>
+template <int EP>
 int gemm(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, uint32_t N, uint32_t K, const EpiArgs& a,
          uint32_t za = 1) {
-    if (M % kBM || N % BN || K % kBK || K == 0) {
+    if (M % kBM || N % kGemmBN || K % kBK || K == 0) {
         h->err = "gemm shape " + std::to_string(M) + "x" + std::to_string(N) + "x" + std::to_string(K);
         return EPI_ERR_ARG;
     }
-    constexpr uint32_t smem = gemm_smem_bytes<BN>();
-    return launch_overlapped(h, k_gemm<BN, EP>, dim3(M / kBM, N / BN, h->E), kGemmThreads, smem, ta, tb, M, N, K, a, za, 1u,
+    return launch_overlapped(h, k_gemm<EP>, dim3(M / kBM, N / kGemmBN, h->E), kGemmThreads, kGemmSmem, ta, tb, M, N, K, a, za,
                              h->d_err);
 }
 
@@ -308,7 +307,7 @@ int gemm(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, u
 template <int EP>
 int infer_product(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, uint32_t N, uint32_t K,
                   const EpiArgs& a, uint32_t za) {
-    if (K / kBK > kInferMaxK) return gemm<128, EP>(h, ta, tb, M, N, K, a, za);
+    if (K / kBK > kInferMaxK) return gemm<EP>(h, ta, tb, M, N, K, a, za);
     const uint32_t panels = M / kBM * h->E, blocks = N / kInferBN;
     const uint32_t wide = panels < h->sms ? 1u : 2u, run = panels < h->sms ? 1u : blocks;
     const uint32_t items = panels * (blocks / run);
@@ -630,16 +629,10 @@ int ensure_chunk(epi_mlp* h, uint32_t steps) {
     return EPI_OK;
 }
 
-template <int BN, int EP>
-int allow_smem(epi_mlp* h) {
-    MCK(cudaFuncSetAttribute(k_gemm<BN, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes<BN>()));
-    return EPI_OK;
-}
-
 int init(epi_mlp* h) {
     const epi_mlp_config& c = h->cfg;
-    MRC((allow_smem<128, kEpHidden>(h)));
-    MRC((allow_smem<128, kEpOut>(h)));
+    for (const void* k : {(const void*)k_gemm<kEpHidden>, (const void*)k_gemm<kEpOut>})
+        MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
     for (const void* k : {(const void*)k_infer<kEpHidden>, (const void*)k_infer<kEpOut>})
         MCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)infer_smem(kInferMaxK)));
     for (const void* k : {(const void*)k_forward<false, kTrainBN>, (const void*)k_forward<false, kTrainWideBN>,

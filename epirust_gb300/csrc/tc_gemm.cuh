@@ -4,10 +4,10 @@
 // tc_infer.cuh, training's in tc_train.cuh).
 //
 // D[m][n] = sum_k A[m][k] * B[n][k]: A is M x K and B is N x K, both row-major BF16 with K
-// contiguous ("K-major").  One CTA of 256 threads computes a 128 x BN tile of D:
-//   warp 0        issues TMA loads of 128 x 64 (A) and BN x 64 (B) tiles into a 2-stage ring
+// contiguous ("K-major").  One CTA of 256 threads computes a 128 x 128 tile of D:
+//   warp 0        issues TMA loads of 128 x 64 tiles of A and B into a 2-stage ring
 //                 of shared memory (128-byte swizzle);
-//   warp 1        issues tcgen05.mma (M = 128, N = BN, K = 16) on each stage, accumulating in
+//   warp 1        issues tcgen05.mma (M = 128, N = 128, K = 16) on each stage, accumulating in
 //                 FP32 in tensor memory;
 //   all 8 warps   wait for the last MMA, read 32 rows x half the columns of the accumulator
 //                 each with tcgen05.ld, apply the epilogue and store.
@@ -196,24 +196,22 @@ __device__ __forceinline__ void epilogue16(const EpiArgs& a, uint32_t N, uint32_
     }
 }
 
-// Stage ring + 1 KB for the 1024-byte alignment of the swizzled tiles: 65 KB with BN = 128,
-// so three CTAs share an SM and one's epilogue overlaps the others' copies and products.
+// Stage ring + 1 KB for the 1024-byte alignment of the swizzled tiles: 65 KB, so three CTAs share
+// an SM and one's epilogue overlaps the others' copies and products.
 // (Measured on the screen of 65,536 candidates by 5 members: a hidden 512 x 512 product took
 // 650 us with 3 stages and one CTA per SM, 418 us with two CTAs, 331 us with 2 stages and
 // three CTAs of four warps, 322 us with eight.)
-template <int BN>
-constexpr uint32_t gemm_smem_bytes() {
-    return (uint32_t)kStages * (uint32_t)(kBM + BN) * kBK * 2u + 1024u;
-}
+constexpr int kGemmBN = 128;
+constexpr uint32_t kGemmSmem = (uint32_t)kStages * (uint32_t)(kBM + kGemmBN) * kBK * 2u + 1024u;
 
-// Grid (M / 128, N / BN, members); M % 128 == 0, N % BN == 0, K % 64 == 0 (checked by the
-// host).  za / zb: 1 when A / B differ per member, 0 when the member stack shares member 0's.
-template <int BN, int EP>
+// Grid (M / 128, N / 128, members); M % 128 == 0, N % 128 == 0, K % 64 == 0 (checked by the
+// host).  za: 1 when A differs per member, 0 when the member stack shares member 0's.
+template <int EP>
 __global__ void __launch_bounds__(kGemmThreads, 3)
     k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, uint32_t M, uint32_t N,
-           uint32_t K, EpiArgs margs, uint32_t za, uint32_t zb, int* err) {
+           uint32_t K, EpiArgs margs, uint32_t za, int* err) {
     const EpiArgs args = member_args(margs, blockIdx.z);
-    static_assert(BN == 64 || BN == 128 || BN == 256, "UMMA N");
+    constexpr int BN = kGemmBN;
     constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = BN * kBK * 2, kStageBytes = kABytes + kBBytes;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -267,7 +265,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3)
                 uint8_t* sa = smem + s * kStageBytes;
                 mbar_expect_tx(&full_bar[s], kStageBytes);
                 tma_load_3d(sa, &ta, (int32_t)(kb * kBK), (int32_t)m0, (int32_t)(blockIdx.z * za), &full_bar[s]);
-                tma_load_3d(sa + kABytes, &tb, (int32_t)(kb * kBK), (int32_t)n0, (int32_t)(blockIdx.z * zb), &full_bar[s]);
+                tma_load_3d(sa + kABytes, &tb, (int32_t)(kb * kBK), (int32_t)n0, (int32_t)blockIdx.z, &full_bar[s]);
             }
         }
         if (lead) issued = kb;

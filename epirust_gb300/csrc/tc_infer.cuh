@@ -19,8 +19,7 @@
 // 512 -> 640 with the score): a tile per CTA with three CTAs per SM (k_gemm) 218, 322, 250;
 // persistent with N = 128, 4 ring blocks and 16-byte stores 188, 235, 210; N = 256, 6 blocks and
 // 32-byte stores 172, 206, 161.  1,024 rows x 5 members, one block per item: 12 to 14 us a
-// launch.  What bounds it now: the epilogue's issue slots, 70 % busy.  Not better:
-// pairs of CTAs that multicast the weight blocks (a hidden layer 250 us, fours 400).
+// launch.  What bounds it now: the epilogue's issue slots, 70 % busy.
 #pragma once
 
 #include "tc_gemm.cuh"

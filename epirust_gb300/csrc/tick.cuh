@@ -139,10 +139,6 @@ struct BitView {
         const uint32_t lo = plane_load<SHARED>(w), hi = sh > 29u ? plane_load<SHARED>(w + 1) : 0u;
         return __funnelshift_r(lo, hi, sh);
     }
-    __device__ __forceinline__ Rows3 rows(int32_t x, int32_t y) const {
-        if (!inside(x, y)) return Rows3{7u, 7u, 7u};
-        return Rows3{row(x, y - 1), row(x, y), row(x, y + 1)};
-    }
     static __device__ __forceinline__ bool centre_vacant(uint32_t r1) { return (r1 & 2u) == 0u; }
     static __device__ __forceinline__ uint32_t occupied(const Rows3& r) {
         return (r.r0 & 7u) | ((r.r1 & 7u) << 3) | ((r.r2 & 7u) << 6);
