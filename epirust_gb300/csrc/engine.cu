@@ -2066,10 +2066,10 @@ size_t epi_abi_struct_size(const char* name) {
 }
 
 // Algorithmic bytes of one hour over all replicates (the roofline numerator): the agent
-// words the hour's kernels must read and write plus one pass over each plane.
-//   movement hours and hours 0/23: decide reads pos 4 + st 8 + home 4 + work 4, writes st 8 +
-//   tgt 4; commit reads tgt 4 + pos 4 + lost 4, writes pos 4; the occupancy plane and the
-//   infectious-neighbour counts, (G+1)^2 bytes each, read once.
+// words the hour's kernels must read and write plus one pass over each plane they touch throughout.
+//   hours 7..22: pos 4 + st 8 + home 4 + work 4 read, pos 4 written; per cell of (G+1)^2 a bit read,
+//   a bit written and an infectious-neighbour count of a byte read.
+//   hours 0 and 23: the same words read; the few agents that act patch theirs and the planes.
 //   hour 1: st.x read 4 + write 4; hours 2-6 of a segment move no data.
 int epi_engine_hour_bytes(const epi_engine* h, uint32_t hour, double* bytes) {
     if (!h || !bytes) return EPI_ERR_ARG;
@@ -2078,7 +2078,7 @@ int epi_engine_hour_bytes(const epi_engine* h, uint32_t hour, double* bytes) {
     for (const auto& rep : h->reps) {
         const double n = (double)rep.n, side = (double)rep.p.grid_size + 1.0;
         if (hod >= 1u && hod <= 6u) b += hod == 1u ? n * 8.0 : 0.0;
-        else b += n * 48.0 + 2.0 * side * side;
+        else b += rebuild_hour(hod) ? n * 24.0 + 1.25 * side * side : n * 20.0;
     }
     *bytes = b;
     return EPI_OK;

@@ -153,3 +153,19 @@ def test_short_calls_after_the_autotuner(gpu):
         eng.simulate(8)
         assert eng.kernels_launched() > launched + 3, n
         eng.close()
+
+
+def test_algorithmic_bytes_of_an_hour(gpu):
+    """The agent words and planes that the hour kernels move: 24 B an agent and 1.25 B a cell while
+    people are about, and the figure that bench.py takes for one launch."""
+    import bench
+
+    n, grid = 5000, 120
+    eng = _engine(make_config(n=n, grid=grid, seed=1))
+    cells = (grid + 1) ** 2
+    for hour in range(24, 48):
+        hod = hour % 24
+        want = n * 8.0 if hod == 1 else 0.0 if hod < 7 and hod else n * 20.0 if hod in (0, 23) else n * 24.0 + 1.25 * cells
+        assert eng.hour_bytes(hour) == want, hod
+    assert eng.hour_bytes(9) == bench.DECIDE_BYTES_PER_AGENT * n + bench.DECIDE_PLANES * cells
+    eng.close()
