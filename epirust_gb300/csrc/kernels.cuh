@@ -339,7 +339,7 @@ __device__ __forceinline__ AgentHour decide_agent(const DevParams& P, const BitV
 //
 // What bounds it: dependent latency with issue behind it.  Walking agents cost about 350 warp
 // instructions per 32 and three dependent L2 round trips (words, the rows around the cell, the
-// claim); 42 % of the issue slots are busy (1M agents cold, 4 blocks per SM).
+// claim); 48 % of the issue slots are busy (1M agents cold, 5 blocks per SM).
 constexpr int kWorldMinBlocks = 5;
 constexpr int kEnsembleMinBlocks = 6;
 

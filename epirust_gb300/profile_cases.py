@@ -4,9 +4,9 @@ package and exits.
     python -m epirust_gb300.profile_cases tick --agents 1000000 --grid 2500 --hours 48
         the 1M-agent / 2,500-grid small-pox world (tests/golden/small_pox_1m_2500.json) resized, hours 1..hours-1
         through simulate_hours (one CUDA graph per call, or one launch for a small world);
-        --events adds CUDA events per kernel, --shape 608,2 sets the launch shape (grid of the
+        --events adds CUDA events per kernel, --shape 760,2 sets the launch shape (grid of the
         hour kernels; the second number is accepted and has no effect)
-    python -m epirust_gb300.profile_cases run [--shape 608,2]
+    python -m epirust_gb300.profile_cases run [--shape 760,2]
         the 1M-agent / 2,500-grid run loop once (bench.py's step: 4,799 hours with the interventions)
     python -m epirust_gb300.profile_cases ensemble --replicates 256 --hours 49
         the 256-replicate ensemble (30.6M agents) through the run loop, hours
@@ -130,7 +130,7 @@ def main() -> None:
     t.add_argument("--events", action="store_true")
     t.add_argument("--shape", default="", help="launch shape 'blocks,slots' (grid of the hour kernels, 1-8)")
     r = sub.add_parser("run")
-    r.add_argument("--shape", default="608,2", help="launch shape 'blocks,slots' (grid of the hour kernels, 1-8)")
+    r.add_argument("--shape", default="760,2", help="launch shape 'blocks,slots' (grid of the hour kernels, 1-8)")
     e = sub.add_parser("ensemble")
     e.add_argument("--replicates", type=int, default=256)
     e.add_argument("--hours", type=int, default=49)
