@@ -24,9 +24,8 @@ __global__ void both(const float* m, const float* v, const float* c1, const floa
         float p = 0.f, mi = m[i], vi = v[i];
         const float4 c = make_float4(c1[i], c2[i], __frcp_rn(c1[i]), __frcp_rn(c2[i]));
         const AdamHyper hp{lr, 1.f, 1.f, eps};
-        float top = epi::tc::adam_ranged(c, hp) ? 0.f : 2.f * epi::tc::kAdamTop;
-        epi::tc::adam_update(p, mi, vi, 0.f, c, hp, top);
-        if (!(top <= epi::tc::kAdamTop)) p = epi::tc::adam_exact(0.f, mi, vi, c, lr, eps);
+        epi::tc::adam_update(p, mi, vi, 0.f, epi::tc::adam_corrections(c, hp), hp);
+        if (epi::tc::either_nan(p, p)) p = epi::tc::adam_exact(0.f, mi, vi, c, lr, eps);
         mine[i] = p;
         const float step = __fdiv_rn(__fmul_rn(lr, __fdiv_rn(m[i], c1[i])),
                                      __fadd_rn(__fsqrt_rn(__fdiv_rn(v[i], c2[i])), eps));
