@@ -55,6 +55,18 @@ def tick_bytes_per_agent_hour(hod: int, agents: int, grid: int) -> float:
     return 36.0 + 8.0 + 1.0 + 5.0 * (grid + 1) ** 2 / agents
 
 
+def moved_bytes(hod: int, agents: int, grid: int) -> float:
+    """Bytes that one hour's kernels have to move as the engine lays a world out
+    (epi_engine_hour_bytes): the second numerator of the run roofline."""
+    if hod == 1:
+        return 8.0 * agents
+    if 2 <= hod <= 6:
+        return 0.0
+    if hod in (0, 23):
+        return 20.0 * agents
+    return DECIDE_BYTES_PER_AGENT * agents + DECIDE_PLANES * (grid + 1) ** 2
+
+
 def _peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -495,6 +507,8 @@ def run_gpu(args, cfg):
     # run roofline: every simulated hour's algorithmic bytes over the timed step
     run_bytes = sum(n * tick_bytes_per_agent_hour(h % 24, n, G) for h in range(1, hours_per_step + 1))
     run_achieved = run_bytes / (ms_total / args.steps / 1000.0) / 1e9
+    run_moved = sum(moved_bytes(h % 24, n, G) for h in range(1, hours_per_step + 1))
+    moved_achieved = run_moved / (ms_total / args.steps / 1000.0) / 1e9
 
     batched = run_batched(args, stream, flush) if not args.no_batched else None
 
@@ -517,7 +531,10 @@ def run_gpu(args, cfg):
                          "run": {"achieved": run_achieved, "peak": peak, "unit": "GB/s", "frac": run_achieved / peak,
                                  "bytes_per_step": run_bytes,
                                  "basis": "whole run: per agent-hour 76 B (movement hours at 1M/2500), 16 B (hour 0), "
-                                          "3 B (hours 1-6), 12 B (hour 23), reference-layout accounting"},
+                                          "3 B (hours 1-6), 12 B (hour 23), reference-layout accounting",
+                                 "moved": {"achieved": moved_achieved, "frac": moved_achieved / peak,
+                                           "bytes_per_step": run_moved,
+                                           "basis": "the words and planes this layout's kernels have to move"}},
                          "kernels": {k: {"launches": v[0], "ms": v[1]} for k, v in stats.items() if v[0]}},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": METRIC, "h2d_bytes_per_step": int(host_records.nbytes),

@@ -1171,7 +1171,8 @@ static int engine_init(epi_engine* h, const epi_params* params, const epi_agent_
     // A world takes the resident grid (4M agents, 15,625 chunks: 68.8 ms a run; a block per 4 chunks
     // 88, per chunk 111).  A large ensemble takes more blocks, whose uneven chunks then spread
     // over the SMs as they come (256 replicates, 130,000 chunks: resident 122 ms, a block per 24 /
-    // 18 / 14 / 10 chunks 113.7 / 112.2 / 114 / 113; 43,000 chunks 10.4 ms, 10.5 per 18).
+    // 18 / 14 / 10 chunks 113.7 / 112.2 / 114 / 113; resident / per 18, ms: 25,700 chunks 10.6 / 11.1, 38,600
+    // 14.8 / 14.8, 52,500 11.55 / 11.33, 78,600 17.3 / 16.6, 120,000 22.2 / 21.1, 183,000 35.3 / 31.4).
     h->grid_blocks = (int)std::min<uint64_t>(
         n_chunks, std::max<uint64_t>(h->resident_blocks, R > 1 ? n_chunks / kEnsembleBlockChunks : 0u));
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));

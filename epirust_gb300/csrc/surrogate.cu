@@ -303,7 +303,9 @@ int gemm(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, u
 // The same by k_infer, for K up to its resident panel (512); wider layers take k_gemm.  Whole
 // rows per item, two blocks at a time, where the 128-row panels fill the SMs (65,536 rows x 5:
 // 206 us a hidden layer, 235 a block at a time); below that one block per item (1,024 rows x 5:
-// 14 us on 152 SMs; whole rows would leave 112 of them idle).
+// 14 us on 152 SMs; whole rows would leave 112 of them idle).  Just above the line some CTAs have
+// two items and the others one: screens of 40 / 140 / 150 / 155 / 200 / 310 / 600 panels take 117 / 152 /
+// 151 / 187 / 187 / 227 / 282 us, by k_gemm 146 / 206 / 214 / 223 / 243 / 313 / 504.
 template <int EP>
 int infer_product(epi_mlp* h, const CUtensorMap& ta, const CUtensorMap& tb, uint32_t M, uint32_t N, uint32_t K,
                   const EpiArgs& a, uint32_t za) {

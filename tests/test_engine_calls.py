@@ -166,6 +166,6 @@ def test_algorithmic_bytes_of_an_hour(gpu):
     for hour in range(24, 48):
         hod = hour % 24
         want = n * 8.0 if hod == 1 else 0.0 if hod < 7 and hod else n * 20.0 if hod in (0, 23) else n * 24.0 + 1.25 * cells
-        assert eng.hour_bytes(hour) == want, hod
+        assert eng.hour_bytes(hour) == want == bench.moved_bytes(hod, n, grid), hod
     assert eng.hour_bytes(9) == bench.DECIDE_BYTES_PER_AGENT * n + bench.DECIDE_PLANES * cells
     eng.close()
