@@ -29,7 +29,8 @@
 using namespace epi;
 using namespace epi::kern;
 
-// k_commit takes no slots per thread any more; the launch shape keeps the field.
+// A field of the launch shape that k_commit, which takes its work from lists, has no use for: the
+// value reported by default and the largest accepted, as callers know them.
 constexpr int kCommitSlots = 4, kMaxCommitSlots = 8;
 
 enum KernelKind { kKDecide = 0, kKCommit, kKSleep, kKLock, kKVaccinate, kKBuildPlane, kKCheck, kKindCount };

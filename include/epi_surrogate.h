@@ -78,7 +78,7 @@ int epi_mlp_predict(epi_mlp* h, const float* x, uint32_t n, float* y);
  * (members x n), computed on the device (the outputs themselves stay there). */
 int epi_mlp_score(epi_mlp* h, const float* x, uint32_t n, const float* target, float* score);
 
-/* Kernel launches so far (the GEMM, gather, bias-gradient, Adam and step kernels). */
+/* Kernel launches so far (products, gathers, padding and packing, step counters). */
 int epi_mlp_kernels_launched(const epi_mlp* h, uint64_t* out);
 
 #ifdef __cplusplus
